@@ -19,11 +19,13 @@ constexpr int WARPS = 4;
 constexpr int MAX_DK = 640;  // most lanes of a query and a key
 constexpr int MAX_DV = 512;  // most lanes of a value
 
-template <typename T>
+// ACC: 32 value lanes each.  WIDE: the runs of a query and a key are read four lanes at a time (their lengths, strides and bases
+// allow it).  The order of every addition is that of the plain form.
+template <typename T, int ACC, bool WIDE>
 __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsArgs<T> a) {
-    __shared__ float q_s[WARPS][MAX_DK];
+    __shared__ __align__(16) float q_s[WARPS][MAX_DK];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * WARPS + warp;
+    const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
     if (item >= (long long)a.n_tokens * a.H) return;
     const int t = (int)(item / a.H), h = (int)(item - (long long)t * a.H);
     const int r = a.token_request[t];
@@ -37,7 +39,6 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
     const float slope = a.slopes ? a.slopes[h] : 0.f;
 
     const int* table = a.page_table + (size_t)r * a.table_width;
-    constexpr int ACC = MAX_DV / 32;
     float first[ACC];  // with two maps a head: what the first map's softmax gave
 #pragma unroll
     for (int i = 0; i < ACC; ++i) first[i] = 0.f;
@@ -63,11 +64,25 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
             const int j = c + lane;
             const bool visible = (j >= lo && j <= pos) || j < kept;
             float s = -INFINITY;
+            long long value_at = 0;  // where the lane's key has its value
             if (visible) {
                 const int page = table[j / a.page_size], off = j % a.page_size;
                 const T* kp = a.keys + (long long)page * a.k_page + (long long)kvh * a.k_head + (long long)off * a.k_token + map * a.k_map;
+                value_at = (long long)page * a.v_page + (long long)kvh * a.v_head + (long long)off * a.v_token;
                 float dot = 0.f;
-                for (int d = 0; d < dk; ++d) dot = fmaf(q_s[warp][d], to_float(kp[d]), dot);
+                if constexpr (WIDE) {
+                    // a key row is the lane's alone: sixteen wide loads on their way hide what one scalar after the other shows
+#pragma unroll 16
+                    for (int d = 0; d < dk; d += 4) {
+                        float kv[4], qv[4];
+                        load4(kp + d, kv);
+                        load4(q_s[warp] + d, qv);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) dot = fmaf(qv[e], kv[e], dot);
+                    }
+                } else {
+                    for (int d = 0; d < dk; ++d) dot = fmaf(q_s[warp][d], to_float(kp[d]), dot);
+                }
                 s = dot * a.scale;
                 if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
                 s -= slope * (float)(pos - j);
@@ -79,18 +94,21 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
 #pragma unroll
             for (int i = 0; i < ACC; ++i) acc[i] *= rescale;
             m = m_new;
-            const int count = min(32, pos - c + 1);
-            for (int jj = 0; jj < count; ++jj) {
-                const float pj = __shfl_sync(0xffffffffu, p, jj);
-                if (pj == 0.f) continue;  // uniform across the warp
-                const int key = c + jj;
-                const int page = table[key / a.page_size], off = key % a.page_size;
-                const T* vp = a.values + (long long)page * a.v_page + (long long)kvh * a.v_head + (long long)off * a.v_token;
+            // eight keys' values on their way at a time; a key of weight 0 is passed by
+#pragma unroll 1
+            for (int j0 = 0; j0 < min(32, pos - c + 1); j0 += 8) {
+                float v[8][ACC], pj[8];
 #pragma unroll
-                for (int i = 0; i < ACC; ++i) {
-                    const int d = lane + 32 * i;
-                    if (d < dv) acc[i] = fmaf(pj, to_float(vp[d]), acc[i]);
+                for (int u = 0; u < 8; ++u) {
+                    pj[u] = __shfl_sync(0xffffffffu, p, j0 + u);
+                    const T* vp = a.values + __shfl_sync(0xffffffffu, value_at, j0 + u);
+#pragma unroll
+                    for (int i = 0; i < ACC; ++i) v[u][i] = pj[u] != 0.f && lane + 32 * i < dv ? to_float(vp[lane + 32 * i]) : 0.f;
                 }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+#pragma unroll
+                    for (int i = 0; i < ACC; ++i) acc[i] = pj[u] != 0.f ? fmaf(pj[u], v[u][i], acc[i]) : acc[i];
             }
         }
         const float inv = 1.f / l;
@@ -116,13 +134,26 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
                   a.out + (long long)t * a.out_token + (long long)h * a.out_head);
 }
 
+template <typename T, int ACC>
+int launch_rows_of(const RowsArgs<T>& a, cudaStream_t stream) {
+    const long long items = (long long)a.n_tokens * a.H;
+    // few rows (decode steps): a warp a CTA, so that each has an SM of its own
+    const int warps = items <= 512 ? 1 : WARPS;
+    const long long blocks = (items + warps - 1) / warps;
+    if (blocks > 0x7fffffffLL) return LLM_ERR_UNSUPPORTED;
+    const bool wide = !(a.d0 & 3) && !(a.d1 & 3) && !((a.k_page | a.k_head | a.k_token | (a.maps == 2 ? a.k_map : 0)) & 3) &&
+                      !((uintptr_t)a.keys & (4 * sizeof(T) - 1));
+    if (wide) attention_rows_kernel<T, ACC, true><<<(unsigned)blocks, warps * 32, 0, stream>>>(a);
+    else attention_rows_kernel<T, ACC, false><<<(unsigned)blocks, warps * 32, 0, stream>>>(a);
+    return launch_status();
+}
+
 template <typename T>
 int launch_rows(const RowsArgs<T>& a, cudaStream_t stream) {
-    const long long items = (long long)a.n_tokens * a.H;
-    const long long blocks = (items + WARPS - 1) / WARPS;
-    if (blocks > 0x7fffffffLL) return LLM_ERR_UNSUPPORTED;
-    attention_rows_kernel<T><<<(unsigned)blocks, WARPS * 32, 0, stream>>>(a);
-    return launch_status();
+    if (a.dv <= 64) return launch_rows_of<T, 2>(a, stream);
+    if (a.dv <= 128) return launch_rows_of<T, 4>(a, stream);
+    if (a.dv <= 256) return launch_rows_of<T, 8>(a, stream);
+    return launch_rows_of<T, MAX_DV / 32>(a, stream);
 }
 
 }  // namespace
