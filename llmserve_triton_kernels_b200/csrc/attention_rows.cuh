@@ -57,7 +57,13 @@ struct RowsArgs {
     // head's output, lanes m and m + dv/2 (turn_neighbours: 2m and 2m + 1), is turned back by the query token's row
     const float2* turn;
     int turn_neighbours;
+    // the keys and values cached before this step were written behind a full dependency (not by a kernel that may still be running
+    // when a kernel launched early starts): they may be read before pdl_wait
+    int cached_early;
 };
+
+// attention_rows_few.cu: steps that bring few rows per request and key/value head
+int launch_rows_few(const RowsArgs<__nv_bfloat16>& a, int requests, int max_query_len, int splits, float* part_o, float* part_ml, cudaStream_t stream);
 
 // The end of one head's output: y [dv] in shared memory, complete and visible to this warp; turned back where the values were
 // turned (`turn`: the token's row or null), gated (`gate`: the head's first gate or null, `gate_step` apart) and written.

@@ -469,50 +469,95 @@ merge_two_parts_kernel(const bf16* __restrict__ o1, long long o1_token, long lon
 
 // For steps of few rows whose keys were cut over `splits` CTAs: the merge of the partial results, the product with a
 // per-head matrix w [H, n_out, dv] (the value up-projection of latent attention) and an optional sigmoid gate, in one
-// kernel; one CTA per (token, head).  out[t, h * n_out + e] = gate(g[t, h * n_out + e]) * sum_r w[h, e, r] merged[r].
+// kernel.  out[t, h * n_out + e] = gate(g[t, h * n_out + e]) * sum_r w[h, e, r] merged[r].
+//
+// Bound by latency: a CTA per (token, head, PROJECT_ROWS of the n_out rows), each merging for itself.  A warp's four rows of w
+// are on their way before the kernel in front has ended, and so, behind the wait, are eight shares at a time (a share of weight 0 was
+// perhaps never written: it is read and not used).  In a decode step of a model with 16 or 32 heads it took 16 to 18 us as one CTA a
+// head with a row after the other, and takes 6.
+constexpr int PROJECT_ROWS = 16;
+
+// eight elements from r on (WIDE: 16-byte aligned), zeros behind the row's end
+template <bool WIDE>
+__device__ __forceinline__ void load8(const bf16* row, int r, int dv, float (&v)[8]) {
+    if (WIDE && r + 8 <= dv) {
+        const uint4 u = *reinterpret_cast<const uint4*>(row + r);
+        const unsigned words[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[2 * i] = __uint_as_float(words[i] << 16);
+            v[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000u);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = r + i < dv ? __bfloat162float(row[r + i]) : 0.f;
+    }
+}
+
+template <bool WIDE>
 __global__ void __launch_bounds__(128)
 merge_project_gate_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,
                           const bf16* __restrict__ w, const bf16* __restrict__ gate, int ldg, bf16* __restrict__ out, int H,
                           int dv, int n_out, int gate_per_head) {
-    extern __shared__ float merged[];  // dv floats, then the splits' weights
-    float* weights = merged + dv;
+    extern __shared__ __align__(16) float merged[];  // dv floats, rounded up to 8
+    constexpr int MINE = PROJECT_ROWS / 4;
     const int item = blockIdx.x, t = item / H, h = item - t * H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e0 = blockIdx.y * PROJECT_ROWS + warp * MINE;
+    const bf16* wh = w + (size_t)h * n_out * dv;
+    float wv[MINE][8];
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) load8<WIDE>(wh + (size_t)min(e0 + i, n_out - 1) * dv, lane * 8, dv, wv[i]);
     pdl_trigger();
     pdl_wait();
     const float* ml = part_ml + (size_t)item * splits * 2;
-    if (warp == 0) {
-        const float ms = lane < splits ? ml[2 * lane] : -INFINITY, ls = lane < splits ? ml[2 * lane + 1] : 0.f;
-        const float M = warp_max(ms);
-        const float ws = ms == -INFINITY ? 0.f : exp2f(ms - M);
-        const float inv = 1.f / warp_sum(ws * ls);
-        if (lane < splits) weights[lane] = ws * inv;
-    }
-    __syncthreads();
+    const float ms = lane < splits ? ml[2 * lane] : -INFINITY, ls = lane < splits ? ml[2 * lane + 1] : 0.f;
+    float gates[MINE];
+#pragma unroll
+    for (int i = 0; i < MINE; ++i)
+        gates[i] = gate ? __bfloat162float(gate[(size_t)t * ldg + (gate_per_head ? (size_t)h : (size_t)h * n_out + min(e0 + i, n_out - 1))]) : 0.f;
+    const float M = warp_max(ms);
+    const float ws = ms == -INFINITY ? 0.f : exp2f(ms - M);
+    const float weight = ws / warp_sum(ws * ls);
     const float* po = part_o + (size_t)item * splits * dv;
-    for (int r = threadIdx.x; r < dv; r += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < splits; ++s) {
-            const float ws = weights[s];
-            if (ws != 0.f) acc = fmaf(ws, po[(size_t)s * dv + r], acc);
+    for (int r0 = 0; r0 < dv; r0 += 256) {
+        const int r = r0 + threadIdx.x * 2;  // (dv is even)
+        float2 acc = make_float2(0.f, 0.f);
+        for (int s0 = 0; s0 < splits; s0 += 8) {
+            float2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                v[u] = s0 + u < splits && r < dv ? *reinterpret_cast<const float2*>(po + (size_t)(s0 + u) * dv + r) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float here = __shfl_sync(0xffffffffu, weight, (s0 + u) & 31);
+                if (s0 + u < splits && here != 0.f) {
+                    acc.x = fmaf(here, v[u].x, acc.x);
+                    acc.y = fmaf(here, v[u].y, acc.y);
+                }
+            }
         }
-        merged[r] = acc;
+        if (r < ((dv + 7) & ~7)) *reinterpret_cast<float2*>(merged + r) = acc;
     }
     __syncthreads();
-    const bf16* wh = w + (size_t)h * n_out * dv;
-    for (int e = warp; e < n_out; e += 4) {
-        const bf16* row = wh + (size_t)e * dv;
-        float acc = 0.f;
-        for (int r = lane * 2; r < dv; r += 64) {
-            const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(row + r);
-            acc = fmaf(__low2float(v), merged[r], acc);
-            acc = fmaf(__high2float(v), merged[r + 1], acc);
+    float sums[MINE];
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) sums[i] = 0.f;
+    for (int r = lane * 8; r < dv; r += 256) {
+        float m8[8];
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(m8 + i) = *reinterpret_cast<const float4*>(merged + r + i);
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+            if (r >= 256) load8<WIDE>(wh + (size_t)min(e0 + i, n_out - 1) * dv, r, dv, wv[i]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sums[i] = fmaf(wv[i][j], m8[j], sums[i]);
         }
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            const size_t col = (size_t)h * n_out + e;
-            if (gate) acc *= 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)t * ldg + (gate_per_head ? (size_t)h : col)])));
-            out[(size_t)t * H * n_out + col] = __float2bfloat16_rn(acc);
-        }
+    }
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+        const float total = warp_sum(sums[i]);
+        if (lane == i && e0 + i < n_out)
+            out[(size_t)t * H * n_out + (size_t)h * n_out + e0 + i] = __float2bfloat16_rn(gate ? total / (1.f + expf(-gates[i])) : total);
     }
 }
 
@@ -536,7 +581,9 @@ int launch(const RowsArgs<bf16>& a, int requests, int max_query_len, int splits,
 // As llm_attention_rows, for bfloat16 with every run of lanes a multiple of 16 and 16-byte aligned rows; dv <= 256.
 // `max_query_len`: the most tokens a request brings (it sizes the grid); skip_from > 0: requests of that many tokens and more are
 // left out.  `splits` > 1 cuts every row tile's keys over that many CTAs; part_o [n_tokens * H * maps * splits * dv] and part_ml [n_tokens * H * maps * splits * 2] (float32) then hold the
-// partial results until the merge that follows.  Returns LLM_ERR_UNSUPPORTED for shapes it does not take.
+// partial results until the merge that follows.  `few` (requests that bring few rows): the kernel that cuts the keys over warps and
+// merges in the cluster; 2: keys cached before this step were written behind a full dependency and may be read before the kernel in
+// front has ended.  Returns LLM_ERR_UNSUPPORTED for shapes it does not take.
 LLM_EXPORT int llm_attention_rows_mma(const void* q0, long long q0_token, long long q0_head, int d0, const void* q1,
                                       long long q1_token, long long q1_head, int d1, void* out, long long out_token,
                                       long long out_head, const void* keys, long long k_page, long long k_head,
@@ -548,13 +595,13 @@ LLM_EXPORT int llm_attention_rows_mma(const void* q0, long long q0_token, long l
                                       long long k1_token, int fresh_d0, float* stats, const float* sinks, const float* gate,
                                       long long gate_token, int keep_first, int chunk, float softcap, int gate_per_head, int maps,
                                       long long q_map, long long k_map, float diff_weight, float diff_eps, float diff_scale,
-                                      const void* turn, int turn_neighbours, int skip_from, cudaStream_t stream) {
+                                      const void* turn, int turn_neighbours, int skip_from, int few, cudaStream_t stream) {
     if (n_tokens <= 0 || requests <= 0) return 0;
     if (maps < 1 || maps > 2 || (maps == 2 && (d1 != 0 || sinks || key_part != 0 || stats)) || (turn && (key_part != 0 || stats)))
         return LLM_ERR_BAD_ARGUMENT;
     if (maps == 2 && (k_map != d0 || (q_map & 7))) return LLM_ERR_UNSUPPORTED;
     if (d0 <= 0 || d1 < 0 || dv <= 0 || H <= 0 || KV <= 0 || H % KV || page_size <= 0 || table_width <= 0 || splits < 1 ||
-        max_query_len < 1 || (d1 > 0 && q1 == nullptr) || (splits > 1 && (part_o == nullptr || part_ml == nullptr)))
+        max_query_len < 1 || (d1 > 0 && q1 == nullptr) || (splits > 1 && !few && (part_o == nullptr || part_ml == nullptr)))
         return LLM_ERR_BAD_ARGUMENT;
     const int dk = maps * d0 + d1;
     auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
@@ -587,6 +634,8 @@ LLM_EXPORT int llm_attention_rows_mma(const void* q0, long long q0_token, long l
     a.maps = maps; a.q_map = q_map; a.k_map = k_map; a.skip_from = skip_from;
     a.diff_weight = diff_weight; a.diff_eps = diff_eps; a.diff_scale = diff_scale;
     a.turn = (const float2*)turn; a.turn_neighbours = turn_neighbours;
+    a.cached_early = few == 2;
+    if (few) return launch_rows_few(a, requests, max_query_len, splits, part_o, part_ml, stream);
     const bool alias = key_part != 2 && values == keys && v_page == k_page && v_head == k_head && v_token == k_token;
     // a tile's queries, two stages of keys and of values; at the end, where values turn back, the tile's rows in 32-bit instead
     auto smem_for = [&](int bn, int bm = 64) {
@@ -629,9 +678,12 @@ LLM_EXPORT int llm_merge_project_gate(const float* part_o, const float* part_ml,
                                       int ldg, void* out, int n_tokens, int H, int dv, int n_out, int gate_per_head, cudaStream_t stream) {
     if (n_tokens <= 0 || H <= 0) return 0;
     if (splits < 1 || splits > 32 || dv <= 0 || (dv & 1) || n_out <= 0 || ((uintptr_t)w & 3)) return LLM_ERR_BAD_ARGUMENT;
-    const size_t smem = (size_t)(dv + 32) * sizeof(float);
-    return launch_pdl(merge_project_gate_kernel, dim3((unsigned)(n_tokens * H)), dim3(128), smem, stream, part_o, part_ml, splits,
-                      (const bf16*)w, (const bf16*)gate, ldg, (bf16*)out, H, dv, n_out, gate_per_head);
+    const size_t smem = (size_t)((dv + 7) & ~7) * sizeof(float);
+    const dim3 grid((unsigned)(n_tokens * H), (unsigned)((n_out + PROJECT_ROWS - 1) / PROJECT_ROWS));
+    if (grid.y > 65535) return LLM_ERR_UNSUPPORTED;
+    auto kernel = (dv & 7) || ((uintptr_t)w & 15) ? merge_project_gate_kernel<false> : merge_project_gate_kernel<true>;
+    return launch_pdl(kernel, grid, dim3(128), smem, stream, part_o, part_ml, splits, (const bf16*)w, (const bf16*)gate, ldg, (bf16*)out,
+                      H, dv, n_out, gate_per_head);
 }
 
 // Two parts of one softmax, each normalised by itself (o [n, H, dv] bfloat16 with token and head strides, stats [n, H, 2] =

@@ -50,6 +50,9 @@ class StepContext:
     # them before the step, which a mixer may use to leave out the work over cached rows.  A graph is captured for one
     # value of this and replayed only for steps of the same kind.
     fresh_requests: bool = False
+    # True if a full dependency (a copy, the start of a graph) lies between the kernels of this step and those of the steps before:
+    # what was cached before the step may be read by a kernel that is launched before the one in front of it has ended
+    steps_apart: bool = False
     # what the parts of one pass hand to one another across layers (a tensor of this step's tokens that a later layer
     # reads, by a key the two agree on); emptied when a pass starts
     shared: dict = field(default_factory=dict)
@@ -92,7 +95,7 @@ def pack_step(entries: list[StepEntry], lengths: list[int], state_slots: np.ndar
         return dev[offsets[i] : offsets[i] + pieces[i].size]
 
     ctx = StepContext(
-        num_tokens=n,
+        num_tokens=n, steps_apart=True,
         num_requests=r,
         num_logits=len(rows),
         token_ids=piece(0),

@@ -72,7 +72,7 @@ class StepGraph:
         self.decode_only = all(c == 1 for c in self.counts) and all(w == (0,) for w in self.wants)
         d = self._piece
         self.ctx = StepContext(
-            num_tokens=N, num_requests=R, num_logits=P,
+            num_tokens=N, num_requests=R, num_logits=P, steps_apart=True,
             token_ids=d(0), positions=d(1), token_request=d(2), cu_tokens=d(3), context_lens=d(4), logit_rows=d(5),
             state_slots=d(6), host_cu_tokens=cu.tolist(), host_context_lens=None, host_state_slots=None,
             max_query_len=max(self.counts), max_context_len=self.max_positions, static_decode=self.decode_only,

@@ -48,7 +48,7 @@ _SIGNATURES = {
     "llm_unary": [_vp, _i, _vp, _i, _i, _i, _i, _i, _f, _vp],
     "llm_gate_mul": [_vp, _ll, _ll, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
     "llm_mingru_scan": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
-    "llm_latent_prepare": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _vp],
+    "llm_latent_prepare": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp],
     "llm_merge_project_gate": [_vp, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
     "llm_merge_two_parts": [_vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _i, _i, _i, _vp],
     "llm_unit_norm_kv_write": [_vp, _i, _i, _vp, _vp, _f, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -57,7 +57,7 @@ _SIGNATURES = {
                            _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _vp],
     "llm_attention_rows_mma": [_vp, _ll, _ll, _i, _vp, _ll, _ll, _i, _vp, _ll, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _i,
                                _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp, _ll, _i, _vp, _vp, _vp, _ll, _i, _i, _f,
-                               _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _i, _vp],
+                               _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _i, _i, _vp],
     "llm_attention_tcgen05_general": [_vp, _i, _vp, _i, _vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,
                                       _vp, _ll, _vp, _f, _f, _f, _vp, _vp],
     "llm_gemm_simt_batched": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _vp],
@@ -1081,7 +1081,7 @@ def mingru_scan(proj: torch.Tensor, bias_z, bias_u, states: torch.Tensor, state_
 
 def latent_prepare(proj: torch.Tensor, positions: torch.Tensor, slot_map: torch.Tensor, plane: torch.Tensor, weight: torch.Tensor,
                    freq: torch.Tensor, eps: float, heads: int, dim: int, rot: int, rank: int, fresh: bool = False,
-                   queries: torch.Tensor | None = None, kv_col: int = 0, halves: bool = False):
+                   queries: torch.Tensor | None = None, kv_col: int = 0, halves: bool = False, w_up: torch.Tensor | None = None):
     """For latent attention, from a token's stacked projections ``proj`` = ``[heads x (dim | rot) | rank | rot | ...]``:
     the queries' rotated parts (interleaved pairs, angles ``position * freq[i]`` in 32-bit) are returned as
     ``[N, heads, rot]``; the latent, RMS-normed with ``weight``, and the rotated shared key part are written to the
@@ -1089,7 +1089,9 @@ def latent_prepare(proj: torch.Tensor, positions: torch.Tensor, slot_map: torch.
     token, ``[N, rank + rot]``: the result is then the pair ``(rotated query parts, rows)``.  ``queries``
     (``[N, heads x (dim | rot)]``, rows may have a pitch): the queries lie there and ``proj`` holds ``[rank | rot]`` from
     column ``kv_col`` on (queries that come through a latent of their own are a later product than the keys' latent).
-    ``halves``: the rotated lanes pair as ``(i, i + rot_dims / 2)`` instead of ``(2i, 2i + 1)``."""
+    ``halves``: the rotated lanes pair as ``(i, i + rot_dims / 2)`` instead of ``(2i, 2i + 1)``.  ``w_up [heads, rank, dim]``
+    (see :func:`latent_prepare_takes_up`): the result is ``(rotated query parts, head_linear(the queries' plain lanes, w_up))``, in one
+    launch."""
     if queries is None:
         _need(proj.dim() == 2 and proj.stride(1) == 1 and proj.shape[1] >= heads * (dim + rot) + rank + rot, "latent_prepare: proj rows are too short")
     else:
@@ -1103,11 +1105,24 @@ def latent_prepare(proj: torch.Tensor, positions: torch.Tensor, slot_map: torch.
     rot_dims = 2 * freq.numel()
     q_rot = torch.empty((proj.shape[0], heads, rot), dtype=proj.dtype, device=proj.device)
     rows = torch.empty((proj.shape[0], rank + rot), dtype=proj.dtype, device=proj.device) if fresh else None
+    q_up = None
+    if w_up is not None:
+        _need(not fresh and latent_prepare_takes_up(proj, dim), "latent_prepare: the up product is for few bfloat16 tokens")
+        _need(w_up.dtype == proj.dtype and w_up.is_contiguous() and tuple(w_up.shape) == (heads, rank, dim), "latent_prepare: w_up [heads, rank, dim]")
+        q_up = torch.empty((proj.shape[0], heads, rank), dtype=proj.dtype, device=proj.device)
     code = _launch("llm_latent_prepare", _ptr(proj), _code(proj.dtype), proj.stride(0), _ptr(q_rot), _ptr(rows), _ptr(positions),
                    _ptr(slot_map), _ptr(plane), _ptr(weight), _ptr(freq), float(eps), proj.shape[0], heads, dim, rot, rank, rot_dims,
-                   _ptr(queries), 0 if queries is None else queries.stride(0), int(kv_col), int(halves), _stream())
+                   _ptr(queries), 0 if queries is None else queries.stride(0), int(kv_col), int(halves), _ptr(w_up), _ptr(q_up), _stream())
     _check(code, "latent_prepare")
+    if w_up is not None:
+        return q_rot, q_up
     return (q_rot, rows) if fresh else q_rot
+
+
+def latent_prepare_takes_up(proj: torch.Tensor, dim: int) -> bool:
+    """Whether :func:`latent_prepare` does the key up-projection of the queries too: steps of few tokens, whose product is bound by its
+    launch (the library's batched product took 2.5 us a layer and let nothing start before its end)."""
+    return proj.is_cuda and proj.dtype == torch.bfloat16 and proj.shape[0] <= 16 and dim % 16 == 0 and 16 <= dim <= 128
 
 
 def unit_norm_kv_write(qkv: torch.Tensor, slot_map: torch.Tensor, pool: torch.Tensor, eps: float | None, heads: int, kv_heads: int,
@@ -1147,6 +1162,27 @@ def head_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 # lanes: no second one fits).  Measured with the merge behind it, against 256 keys and one CTA an SM: 32 heads on 8 of 64 lanes, window
 # 512: 18.4 -> 12.4 us for one request, 22.1 -> 14.1 us for 8; all of 2,048 keys, 8 requests: 73.0 -> 38.9 us.
 _ROWS_SPLIT_KEYS = 128
+
+# Requests that bring at most so many rows (tokens times the query heads that share a key head), and at most 16 tokens, take the kernel
+# that cuts the keys over warps and merges in the cluster.  Measured against the kernel for many rows and its merge, back to back in a
+# graph: 32 heads on 8 of 64 lanes, window 512 of 2,000 keys: 13.4 -> 5.6 us for one token, 18.2 -> 7.5 for 8 requests, 14.4 -> 8.0
+# for 16 tokens of one (64 rows); all of 2,000 keys, 8 requests: 38.3 -> 14.4; two maps of 64 on values of 128, 128 rows: 20.3 ->
+# 11.3.  Latents of 256 + 32 with 32 heads (with the product behind them): 20.8 -> 12.1 at 32 rows, 25.1 -> 16.0 at 128, but 31.6 ->
+# 34.9 at 512, where sixteen rows a CTA read the keys too often.
+_ROWS_FEW = 128
+
+
+def _few_splits(longest: int, base: int, dk: int, dv: int, leave: bool, bytes_a_split: int) -> int:
+    """How many CTAs share the keys of a tile of 16 rows, of which there are ``base``: a pass of a CTA takes 128 keys (64 where two warps
+    share the value lanes); an SM holds two such CTAs of short keys, else one.  CTAs of one cluster: a power of two up to 8."""
+    small = dk <= 64 and dv <= 64
+    want = -(-longest // (128 if dk <= 128 and dv <= 128 else 64))
+    room = max(1, (2 if small else 1) * _sm_count() // base)
+    if leave:
+        return max(1, min(want, room, 32, _SPLIT_SCRATCH_BYTES // bytes_a_split))
+    most = min(want, room, 8)
+    return 8 if most >= 8 else 4 if most >= 4 else 2 if most >= 2 else 1
+
 
 
 def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, page_table, page_size: int, ctx, *, num_heads: int,
@@ -1215,25 +1251,34 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
         splits = max(1, min(-(-longest // _ROWS_SPLIT_KEYS), (2 if value_dim <= 128 else 1) * _sm_count() // ctas, 16, _SPLIT_SCRATCH_BYTES // (n * num_heads * maps * value_dim * 4)))
         if key_part or want_stats:
             splits = 1
+        dk = maps * d0 + d1
+        few = (most <= 16 and most * group * maps <= _ROWS_FEW and not key_part and not want_stats and dk % 32 == 0 and value_dim % 64 == 0
+               and ((dk <= 128 and value_dim <= 128) or (maps == 1 and dk <= 320)))
+        leave = leave_parts and splits > 1
+        if few:
+            splits = _few_splits(longest, -(-most * group * maps // 16) * num_kv_heads * ctx.num_requests, dk, value_dim,
+                                 leave_parts, n * num_heads * value_dim * 4)
+            leave = leave_parts and splits > 1
+            few = 2 if getattr(ctx, "steps_apart", False) else 1
         stats = torch.empty((n, num_heads, 2), dtype=torch.float32, device=q0.device) if want_stats else None
         part_o = part_ml = None
-        if splits > 1:
+        if splits > 1 and (leave or not few):
             part_o = torch.empty((n * num_heads * maps * splits * value_dim,), dtype=torch.float32, device=q0.device)
             part_ml = torch.empty((n * num_heads * maps * splits * 2,), dtype=torch.float32, device=q0.device)
         code = _launch(
             "llm_attention_rows_mma", _ptr(q0), q0.stride(0), q0.stride(1), d0, _ptr(q1), 0 if q1 is None else q1.stride(0),
-            0 if q1 is None else q1.stride(1), d1, None if (leave_parts and splits > 1) else _ptr(out), out.stride(0), out.stride(1),
+            0 if q1 is None else q1.stride(1), d1, None if leave else _ptr(out), out.stride(0), out.stride(1),
             keys, *k_strides, values, *v_strides,
             value_dim, _ptr(page_table), page_table.shape[1], _ptr(ctx.token_request), _ptr(ctx.cu_tokens), _ptr(ctx.context_lens),
             _ptr(slopes), n, ctx.num_requests, most, num_heads, num_kv_heads, page_size, int(window or 0), float(scale),
             splits, _ptr(part_o), _ptr(part_ml), int(key_part), keys1, int(k1_token), int(fresh_d0), _ptr(stats), _ptr(sinks), _ptr(gate),
-            gate_token, keep_first, chunk, softcap, *more, int(skip_from), _stream(),
+            gate_token, keep_first, chunk, softcap, *more, int(skip_from), int(few), _stream(),
         )
         if code != 10002:
             _check(code, "attention_rows (tensor cores)")
-            if leave_parts and splits > 1:
+            if leave:
                 return AttentionParts(part_o, part_ml, splits, n, num_heads, value_dim)
-            add_launches(int(splits > 1))
+            add_launches(int(splits > 1 and not few))
             return (out, stats) if want_stats else out
         add_launches(-1)  # a layout the kernel does not take: the general one below
     _need(not key_part and not want_stats, "attention over a part of the keys runs on the tensor cores only (bfloat16, lanes in multiples of 16)")

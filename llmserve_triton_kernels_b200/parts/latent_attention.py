@@ -123,20 +123,24 @@ class LatentAttention(Mixer):
         proj = ops.linear(x, self.w_in)  # [N, H (dim | rot) | rank | rot | gate], or [N, query rank | rank | rot | gate]
         two_parts = ops.latent_two_parts(ctx, proj.dtype, dim, rot, rank, self.value_dim)
         halves = self.rotary_layout == "half"
+        up = {"w_up": self.w_uk_t} if not two_parts and ops.latent_prepare_takes_up(proj, dim) else {}
         if self.query_rank:
             # the queries' latent is normed (32-bit statistics) and expanded: a product of its own behind the stacked one
             q_all = ops.linear(ops.row_rmsnorm(proj[:, : self.query_rank], self.q_weight, self.norm_eps), self.w_uq)
             gate_col = self.query_rank + rank + rot
             prepared = ops.latent_prepare(
                 proj, ctx.positions, cache.slot_map, cache.pool, self.latent_weight, self.freq, self.norm_eps, H, dim, rot, rank,
-                fresh=two_parts, queries=q_all, kv_col=self.query_rank, halves=halves,
+                fresh=two_parts, queries=q_all, kv_col=self.query_rank, halves=halves, **up,
             )
         else:
             q_all, gate_col = proj, H * (dim + rot) + rank + rot
             prepared = ops.latent_prepare(
                 proj, ctx.positions, cache.slot_map, cache.pool, self.latent_weight, self.freq, self.norm_eps, H, dim, rot, rank,
-                fresh=two_parts, halves=halves,
+                fresh=two_parts, halves=halves, **up,
             )
+        q_lat = None
+        if up:
+            prepared, q_lat = prepared
         q_rot, fresh = prepared if two_parts else (prepared, None)
         q_plain = q_all.as_strided((q_all.shape[0], H, dim), (q_all.stride(0), dim + rot, 1), q_all.storage_offset())
         if two_parts:
@@ -156,7 +160,8 @@ class LatentAttention(Mixer):
                 )
                 heads = ops.merge_two_parts(own, own_stats, ops.head_linear(cached, self.w_uv), cached_stats)
         else:
-            q_lat = ops.head_linear(q_plain, self.w_uk_t)  # [N, H, rank]
+            if q_lat is None:
+                q_lat = ops.head_linear(q_plain, self.w_uk_t)  # [N, H, rank]
             mixed = ops.latent_paged_attention(
                 q_lat, q_rot, cache.pool, cache.page_table, ctx, rank=rank, scale=self.scale, window=self.window,
                 leave_parts=ctx.num_tokens <= 16,
