@@ -60,6 +60,7 @@ _SIGNATURES = {
                                _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _i, _i, _vp],
     "llm_attention_tcgen05_general": [_vp, _i, _vp, _i, _vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,
                                       _vp, _ll, _vp, _f, _f, _f, _vp, _vp],
+    "llm_experts_few": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp],
     "llm_gemm_simt_batched": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _vp],
     "llm_sample": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "llm_sigmoid_attention": [_vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i,
@@ -1646,6 +1647,57 @@ def expert_gated_act(x: torch.Tensor, experts: int, ff: int, shared_ff: int, lim
                    _ptr(table), top, vocab, x.shape[0], experts, ff, shared_ff, float(limit), float(shared_limit), float(slope), float(up_shift), _stream())
     _check(code, "expert_gated_act")
     return out
+
+
+_EXPERTS_FEW = 8  # tokens, see experts_few
+
+
+def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, ff: int, shared_ff: int, *, activation: str | None = None,
+                limit: float = 0.0, shared_limit: float = 0.0, slope: float = 1.0, up_shift: float = 0.0, weights: torch.Tensor | None = None,
+                ids: torch.Tensor | None = None, table: torch.Tensor | None = None, sink: "ResidualSink | None" = None):
+    """A mixture of experts for few bfloat16 tokens, of which only the experts that one of them uses are read: the product with ``w_up``,
+    the activation (``activation``: one of :func:`expert_act_scale`'s; None: the bounded gated one of :func:`expert_gated_act`) times the
+    tokens' weights, and the product with ``w_down``.  Returns ``[N, hidden]`` float32, or what ``sink.linear`` returns; None for
+    a step that it does not take.  Up to 8 tokens: with 4 of 32 experts each (2,048 wide, 704 inside, a shared one of 1,408), cold and
+    with the start of a graph, the two kernels took 27 us for one token, 49 for 4 and 70 for 8, whose experts are then two thirds of all,
+    against 70 for the products over all experts and the activation between them."""
+    m, k = x.shape
+    n, c = w_down.shape
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and m <= _EXPERTS_FEW and x.stride(1) == 1 and w_up.is_contiguous() and w_down.is_contiguous()):
+        return None
+    gated = activation is None
+    _need(w_up.dtype == w_down.dtype == x.dtype and tuple(w_up.shape) == ((2 if gated else 1) * (experts * ff + shared_ff), k) and c == experts * ff + shared_ff,
+          "experts_few: the stacked matrices do not match the experts")
+    ldw = top = vocab = 0
+    if weights is not None:
+        _need(weights.dtype == torch.float32 and weights.stride(1) == 1 and weights.shape[0] == m and weights.shape[1] >= experts + int(shared_ff > 0), "experts_few: weights are float32 [N, experts (+ 1)]")
+        ldw = weights.stride(0)
+    else:
+        _i32(ids, "ids")
+        _need(table is not None and table.dtype == torch.int32 and table.is_contiguous() and table.dim() == 2 and ids.numel() == m, "experts_few: table is int32 [vocab, top]")
+        vocab, top = table.shape
+    resid = norm_w = out = xw = ss = None
+    alpha = 1.0
+    if sink is not None and sink.resid.is_contiguous() and tuple(sink.resid.shape) == (m, n):
+        resid, alpha = sink.resid, sink.alpha
+        if sink.weight is not None and alpha == 1.0:
+            norm_w = sink.weight
+            xw = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+            ss = torch.empty((-(-n // 16), m), dtype=torch.float32, device=x.device)
+    else:
+        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    act = torch.empty((m, c), dtype=x.dtype, device=x.device)
+    code = _launch("llm_experts_few", _ptr(x), x.stride(0), _ptr(w_up), _ptr(w_down), _ptr(act), m, k, n, experts, ff, shared_ff,
+                   -1 if gated else _UNARY_KINDS[activation], float(limit), float(shared_limit), float(slope), float(up_shift), _ptr(weights), ldw,
+                   _ptr(ids), _ptr(table), top, vocab, _ptr(out), _ptr(resid), _ptr(norm_w), _ptr(xw), _ptr(ss), float(alpha), _error_flag_ptr(), _stream())
+    if code == 10002:
+        add_launches(-1)
+        return None
+    _check(code, "experts_few")
+    add_launches(1)
+    if resid is None:
+        return out
+    return NormedInput(xw, ss, sink.eps, sink.norm) if norm_w is not None else ADDED
 
 
 # ------------------------------------------------------------------------------------------------

@@ -1,0 +1,88 @@
+"""A mixture of experts for few tokens, of which only the used experts are read, beside the double statement of the same: token counts at
+the edges of its tiles, widths that leave warps without work, every form of weights and of ends; experts that nobody uses hold NaN."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, dtype=torch.bfloat16, seed=0, scale=1.0):
+    g = torch.Generator().manual_seed(seed + sum(shape))
+    return (torch.randn(*shape, generator=g) * scale).to(dtype).to(DEV)
+
+
+def stated(x, w_up, w_down, E, ff, fs, wts, act, limits, slope, shift):
+    out, per = 0, 1 if act else 2
+    for e in range(E + (fs > 0)):
+        f = fs if e == E else ff
+        use = wts[:, e] != 0
+        up = x.double() @ w_up[e * per * ff : e * per * ff + per * f].double().T
+        if act is None:
+            g, u = up[:, :f].clamp(max=limits[e == E]), up[:, f:].clamp(-limits[e == E], limits[e == E])
+            y = g * torch.sigmoid(slope * g) * (u + shift)
+        else:
+            y = {"relu2": lambda v: torch.relu(v) ** 2, "silu": torch.nn.functional.silu,
+                 "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](up)
+        y = y * wts[:, e : e + 1].double()
+        part = y @ w_down[:, e * ff : e * ff + f].double().T
+        out = out + torch.where(use[:, None], part, torch.zeros_like(part))
+    return out
+
+
+@pytest.mark.parametrize("m", [1, 3, 8])
+@pytest.mark.parametrize("K, N, E, ff, fs", [(2048, 2048, 32, 704, 1408), (1024, 1024, 16, 512, 1024), (32, 16, 1, 32, 0), (992, 48, 37, 64, 32),
+                                             (2048, 160, 256, 32, 0), (96, 32, 9, 1568, 800)])
+@pytest.mark.parametrize("form", ["gated", "table", "relu2", "silu", "gelu_tanh"])
+def test_used_experts_alone(m, K, N, E, ff, fs, form):
+    from llmserve_triton_kernels_b200 import ops
+
+    act = form if form in ("relu2", "silu", "gelu_tanh") else None
+    per, top = 1 if act else 2, min(4, E)
+    x = rnd(m, K + 8, seed=1)[:, :K]
+    w_up, w_down = rnd(per * (E * ff + fs), K, seed=2, scale=K**-0.5), rnd(N, E * ff + fs, seed=3, scale=ff**-0.5)
+    g = torch.Generator().manual_seed(m)
+    chosen = torch.rand(m, E, generator=g).argsort(1)[:, :top].to(DEV)
+    kw = dict(activation=act) if act else dict(limit=1.5, shared_limit=1.0, slope=1.702, up_shift=1.0)
+    if form == "table":
+        table = torch.zeros(50, top, dtype=torch.int32, device=DEV)
+        ids = torch.arange(m, dtype=torch.int32, device=DEV) * 2 + 1
+        table[ids.long()] = chosen.int()
+        kw.update(ids=ids, table=table)
+        wts = torch.zeros(m, E + 1, device=DEV).scatter(1, chosen, 1.0 / top)
+        wts[:, E] = 1.0
+    else:
+        wts = torch.zeros(m, E + 1, device=DEV).scatter(1, chosen, rnd(m, top, dtype=torch.float32, seed=5).abs() + 0.1)
+        wts[:, E] = rnd(m, dtype=torch.float32, seed=6).abs() + 0.1
+        kw.update(weights=wts[:, : E + (fs > 0)].contiguous())
+    for e in range(E):
+        if not bool((wts[:, e] != 0).any()):
+            w_up[e * per * ff : (e + 1) * per * ff] = torch.nan
+            w_down[:, e * ff : (e + 1) * ff] = torch.nan
+    want = stated(x, w_up, w_down, E, ff, fs, wts, act, (1.5, 1.0), 1.702, 1.0)
+    got = ops.experts_few(x, w_up, w_down, E, ff, fs, **kw)
+    # the activations are rounded to bfloat16 (2^-9 each, signs at random), the sums are 32-bit
+    assert float((got.double() - want).norm()) <= 3e-3 * float(want.norm())
+    resid, weight = rnd(m, N, dtype=torch.float32, seed=7), rnd(N, dtype=torch.float32, seed=8)
+    stream = resid.clone()
+    handed = ops.experts_few(x, w_up, w_down, E, ff, fs, **kw, sink=ops.ResidualSink(stream, weight, 1e-5))
+    new = resid.double() + got.double()
+    torch.testing.assert_close(stream.double(), new, rtol=1e-6, atol=1e-5)
+    torch.testing.assert_close(handed.xw.double(), new * weight.double(), rtol=2.0**-8, atol=1e-5)
+    torch.testing.assert_close(handed.ss.sum(0).double(), (new * new).sum(1), rtol=1e-5, atol=1e-5)
+    stream = resid.clone()
+    assert ops.experts_few(x, w_up, w_down, E, ff, fs, **kw, sink=ops.ResidualSink(stream, None, 1e-5, alpha=0.5)) is ops.ADDED
+    torch.testing.assert_close(stream.double(), resid.double() + 0.5 * got.double(), rtol=1e-6, atol=1e-5)
+
+
+def test_what_it_does_not_take_goes_the_other_way():
+    from llmserve_triton_kernels_b200 import ops
+
+    def call(m, K, N, ff, dtype=torch.bfloat16):
+        return ops.experts_few(rnd(m, K, dtype=dtype), rnd(4 * ff, K, dtype=dtype), rnd(N, 4 * ff, dtype=dtype), 4, ff, 0, activation="silu",
+                               weights=torch.ones(m, 4, device=DEV))
+
+    assert call(2, 64, 32, 32) is not None
+    for args in ((9, 64, 32, 32), (2, 48, 32, 32), (2, 2080, 32, 32), (2, 64, 24, 32), (2, 64, 32, 48), (2, 64, 32, 32, torch.float32)):
+        assert call(*args) is None, args
