@@ -79,6 +79,21 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return scratch[32];
 }
 
+// K sums over a block at once, the same values to every thread, one meeting more than none: every warp adds up all warps' parts.
+// `scratch` holds K * 32 floats of shared memory that nobody else uses before the block's next meeting.
+template <int K>
+__device__ __forceinline__ void block_sums(float (&v)[K], float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        v[k] = warp_sum(v[k]);
+        if (lane == 0) scratch[k * 32 + warp] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < nwarps ? scratch[k * 32 + lane] : 0.f);
+}
+
 static inline int launch_status() { return (int)cudaGetLastError(); }
 
 // Programmatic dependent launch: a kernel launched through launch_pdl may start while the kernel

@@ -16,7 +16,8 @@
 //   warm:      queries times 1 + coef * ln(floor((position + 1) / every) + 1)
 // Queries go to q_out [N, Hq * D]; keys and values into the token's slot of pool [pages, 2, Hk, page_size, Dp].  With maps = 2
 // every two key heads in a row share a value head and a row of the pool [pages, 2, Hk / 2, page_size, Dp], side by side.
-// Everything is computed in 32-bit.  One CTA per token, one warp per head at a time; where no head is normed by itself and
+// Everything is computed in 32-bit.  One CTA per token (several that share its heads in steps of few tokens: a warp that takes five heads
+// one after the other shows five loads' latency, 10.7 us a layer of a decode step), one warp per head at a time; where no head is normed by itself and
 // everything lies on boundaries of four lanes, a second kernel takes four neighbouring pairs of lanes a thread instead.
 #include <type_traits>
 
@@ -58,7 +59,7 @@ head_prepare_kernel(const TI* __restrict__ proj, int ldp, const float* __restric
     const int page = slot / page_size, off = slot % page_size;
     __syncthreads();
     pdl_wait();
-    if (turn_out)
+    if (turn_out && blockIdx.y == 0)
         for (int i = threadIdx.x; i < v_half; i += blockDim.x) turn_out[(size_t)t * v_half + i] = v_turn[i];
     const TI* row = proj + (size_t)t * ldp;
     float whole[2] = {1.f, 1.f};  // the scales of all query heads and of all key heads together
@@ -77,7 +78,8 @@ head_prepare_kernel(const TI* __restrict__ proj, int ldp, const float* __restric
     }
     float* buf = smem + warp * D;
     const int per_head = D - half;  // work items a head: `half` pairs, then the lanes that pass
-    for (int head = warp; head < Hq + Hk; head += WARPS) {
+    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    for (int head = blockIdx.y * WARPS + warp; head < Hq + Hk; head += gridDim.y * WARPS) {
         const bool is_q = head < Hq;
         const int base = head * D;  // keys follow the queries in the row and in the bias
         TK* vdst = (!is_q && values_are_keys) ? pool + ((((size_t)page * 2 + 1) * Hk + (head - Hq)) * page_size + off) * Dp : nullptr;  // (one map)
@@ -127,7 +129,7 @@ head_prepare_kernel(const TI* __restrict__ proj, int ldp, const float* __restric
     if (Hk > 0 && !values_are_keys) {
         const int vbase = (Hq + Hk) * D;
         if (v_freq) {
-            for (int i = threadIdx.x; i < Gv * v_half; i += blockDim.x) {
+            for (int i = first; i < Gv * v_half; i += step) {
                 const int kh = i / v_half, m = i - kh * v_half;
                 const int da = interleaved ? 2 * m : m, db = interleaved ? 2 * m + 1 : m + v_half;
                 float u = to_float(row[vbase + kh * V + da]), v = to_float(row[vbase + kh * V + db]);
@@ -139,7 +141,7 @@ head_prepare_kernel(const TI* __restrict__ proj, int ldp, const float* __restric
             }
             return;
         }
-        for (int i = threadIdx.x; i < Gv * V; i += blockDim.x) {
+        for (int i = first; i < Gv * V; i += step) {
             const int kh = i / V, d = i % V;
             float v = to_float(row[vbase + i]);
             if (bias) v += bias[vbase + i];
@@ -283,7 +285,8 @@ LLM_EXPORT int llm_head_prepare(const void* proj, int in_dtype, int ldp, const f
     const size_t smem = ((size_t)WARPS * D + 1) * sizeof(float) + (size_t)(rot / 2 + 1 + (v_freq ? V / 2 : 0)) * sizeof(float2);
     auto go = [&](auto kernel, auto* in, auto* qo) {
         using TK = std::remove_pointer_t<decltype(qo)>;
-        return launch_pdl(kernel, dim3(N), dim3(WARPS * 32), smem, stream, in, ldp, bias, qo, ldq, (TK*)pool, slot_map, page_size, Dp, qw, kw,
+        const int rounds = (Hq + Hk + WARPS - 1) / WARPS, room = 2 * 148 / N;
+        return launch_pdl(kernel, dim3(N, rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room)), dim3(WARPS * 32), smem, stream, in, ldp, bias, qo, ldq, (TK*)pool, slot_map, page_size, Dp, qw, kw,
                           eps, normed, freq, rot, positions, warm_coef, warm_every, Hq, Hk, D, V, values_are_keys, interleaved, v_keep, v_first, v_lambda, maps, v_freq,
                           (float2*)turn_out);
     };

@@ -150,7 +150,8 @@ sum_parts_kernel(const float* __restrict__ part, TO* __restrict__ out, const int
 //   rotate:  in every head, lanes i and i + rot/2 (i < rot/2) turn by position * freq[i]; lanes >= rot pass
 //   keys:    times k_scale
 //   queries go to q_out [N, Hq * D]; keys to k_out [N, Hk * D], or with the values into the token's slot of
-//   pool [pages, 2, Hk, page_size, Dp].  One CTA per token.
+//   pool [pages, 2, Hk, page_size, Dp].  One CTA per token, or in steps of few tokens several that share its lanes, each of
+//   which works out the token's angles and sums for itself.
 template <typename TI, typename TQ, typename TK>
 __global__ void __launch_bounds__(256)
 qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, int ldq, TK* __restrict__ k_out, int ldk,
@@ -158,7 +159,7 @@ qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, 
                   const float* __restrict__ kw, float eps, const float* __restrict__ freq, int rot,
                   const int* __restrict__ positions, float k_scale, int Hq, int Hk, int D, int V) {
     extern __shared__ float2 turn[];  // (cos, sin) of the token's angles
-    __shared__ float scratch[33];
+    __shared__ float scratch[2 * 32];
     pdl_trigger();
     const int t = blockIdx.x;
     const int half = rot >> 1;
@@ -173,18 +174,20 @@ qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, 
     const TI* row = proj + (size_t)t * ldp;
     float q_scale = 1.f, kn_scale = 1.f;
     if (qw) {
-        float sq = 0.f, sk = 0.f;
-        for (int i = threadIdx.x; i < Hq * D; i += blockDim.x) { const float v = to_float(row[i]); sq = fmaf(v, v, sq); }
-        for (int i = threadIdx.x; i < Hk * D; i += blockDim.x) { const float v = to_float(row[Hq * D + i]); sk = fmaf(v, v, sk); }
-        sq = block_sum(sq, scratch);
-        sk = block_sum(sk, scratch);
-        q_scale = 1.f / sqrtf(sq / (float)(Hq * D) + eps);
-        kn_scale = 1.f / sqrtf(sk / (float)(Hk * D) + eps);
+        float sums[2] = {0.f, 0.f};
+#pragma unroll 8
+        for (int i = threadIdx.x; i < Hq * D; i += blockDim.x) { const float v = to_float(row[i]); sums[0] = fmaf(v, v, sums[0]); }
+#pragma unroll 2
+        for (int i = threadIdx.x; i < Hk * D; i += blockDim.x) { const float v = to_float(row[Hq * D + i]); sums[1] = fmaf(v, v, sums[1]); }
+        block_sums<2>(sums, scratch);
+        q_scale = 1.f / sqrtf(sums[0] / (float)(Hq * D) + eps);
+        kn_scale = 1.f / sqrtf(sums[1] / (float)(Hk * D) + eps);
     }
     __syncthreads();
     const int per_head = D - half;  // work items a head: `half` pairs, then the lanes that pass
     const int page = slot / page_size, off = slot % page_size;
-    for (int it = threadIdx.x; it < (Hq + Hk) * per_head; it += blockDim.x) {
+    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    for (int it = first; it < (Hq + Hk) * per_head; it += step) {
         const int head = it / per_head, i = it % per_head;
         const bool is_q = head < Hq;
         const int base = head * D;  // keys follow the queries in the row
@@ -219,7 +222,7 @@ qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, 
     }
     if (pool) {
         const TI* vals = row + (size_t)(Hq + Hk) * D;
-        for (int i = threadIdx.x; i < Hk * V; i += blockDim.x) {
+        for (int i = first; i < Hk * V; i += step) {
             const int kh = i / V, d = i % V;
             pool[((((size_t)page * 2 + 1) * Hk + kh) * page_size + off) * Dp + d] = from_float<TK>(to_float(vals[i]));
         }
@@ -293,7 +296,8 @@ LLM_EXPORT int llm_qk_prepare(const void* proj, int in_dtype, int ldp, void* q_o
     const size_t smem = (size_t)(rot / 2 + 1) * sizeof(float2);
     auto go = [&](auto kernel, auto* in, auto* qo, auto* ko) {
         using TK = std::remove_pointer_t<decltype(ko)>;
-        return launch_pdl(kernel, dim3(N), dim3(256), smem, stream, in, ldp, qo, ldq, ko, ldk, (TK*)pool, slot_map, page_size, Dp, qw, kw,
+        const int rounds = ((Hq + Hk) * (D - rot / 2) + 255) / 256, room = 2 * 148 / N;
+        return launch_pdl(kernel, dim3(N, rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room)), dim3(256), smem, stream, in, ldp, qo, ldq, ko, ldk, (TK*)pool, slot_map, page_size, Dp, qw, kw,
                           eps, freq, rot, positions, k_scale, Hq, Hk, D, V);
     };
     if (in_dtype == LLM_F32 && q_dtype == LLM_F32 && k_dtype == LLM_F32)

@@ -1705,6 +1705,9 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
 # matrix of state per head, that route tokens to a few of many small feed-forward layers, or that run mixers side by
 # side (csrc/sigmoid_attention.cu, retention.cu, routing.cu).
 _SIGMOID_SPLIT_KEYS = 128  # a stretch of keys that one CTA sums up when a context is shared out
+# The same for the tensor-core kernel, whose tile is 32 keys: stretches of one tile put 600 keys on all sixteen shares, of 128 on five
+# (31.0 -> 20.8 us a layer of a decode step of four requests).
+_SIGMOID_MMA_SPLIT_KEYS = 32
 _SIGMOID_SPLIT_MAX_TOKENS = 64  # steps of more tokens have CTAs enough without cutting the keys
 _SIGMOID_SHARES = 16  # the tensor-core kernel's CTAs per tile of tokens: stretch s of the keys goes to share s % 16
 
@@ -1765,11 +1768,15 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
     longest = getattr(ctx, "max_context_len", None) or int(ctx.context_lens.max())
     if window:
         longest = min(longest, window + ctx.max_query_len)
-    split_keys = max(_SIGMOID_SPLIT_KEYS, -(-longest // (1024 * 32)) * 32)  # at most 1,024 stretches, of whole chunks of 32 keys
-    splits = 1 if n > _SIGMOID_SPLIT_MAX_TOKENS else max(1, -(-longest // split_keys))
-    parts = torch.empty((splits, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if splits > 1 else None
+    def stretches(keys):  # at most 1,024 of them, of whole chunks of 32 keys
+        keys = max(keys, -(-longest // (1024 * 32)) * 32)
+        return keys, 1 if n > _SIGMOID_SPLIT_MAX_TOKENS else max(1, -(-longest // keys))
+
     if q.dtype == torch.bfloat16 and not _FORCE_GENERIC_ATTENTION:
         # the tensor cores: tiles of 16 tokens of one request
+        split_keys, splits = stretches(_SIGMOID_MMA_SPLIT_KEYS)
+        shares = min(splits, _SIGMOID_SHARES)
+        parts = torch.empty((shares, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if splits > 1 else None
         cu = getattr(ctx, "host_cu_tokens", None) or ctx.cu_tokens.tolist()
         tiles = sum(-(-(b - a) // 16) for a, b in zip(cu[:-1], cu[1:]))
         code = _launch(
@@ -1782,10 +1789,12 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
             _check(code, "sigmoid_attention (tensor cores)")
             if splits > 1:
                 _check(_launch("llm_sigmoid_sum_parts", _ptr(parts), _ptr(out), _code(out.dtype), _ptr(ctx.positions), n,
-                               num_heads * value_dim, split_keys, int(window or 0), min(splits, _SIGMOID_SHARES), _stream()),
+                               num_heads * value_dim, split_keys, int(window or 0), shares, _stream()),
                        "sigmoid_attention (sum of the stretches)")
             return out
         add_launches(-1)  # sizes the kernel does not take: the general one below
+    split_keys, splits = stretches(_SIGMOID_SPLIT_KEYS)
+    parts = torch.empty((splits, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if splits > 1 else None
     code = _launch(
         "llm_sigmoid_attention", _ptr(q), _code(q.dtype), q.stride(0), _ptr(pool), _code(pool.dtype), _ptr(page_table),
         page_table.shape[1], _ptr(ctx.positions), _ptr(ctx.token_request), _ptr(head_bias), _ptr(head_mix), _ptr(out),
