@@ -1,11 +1,16 @@
 // Paged attention for any mix of query lengths, any key size up to 640 lanes, any value size up to 512 and any
-// group size: one warp per (token, query head).
+// group size: a (token, query head) is eight warps', which share the keys, or in steps of many tokens one warp's.
 //
 // This is the attention of the true 32-bit path and the fallback of the bfloat16 path for
 // shapes its faster kernels refuse.  Scores, the running maximum, the exponentials and the
 // weighted sum are 32-bit.  Keys are visited in chunks of 32 that start at multiples of 32 of
-// the absolute key position, so the order of every addition depends only on the query's
-// position (and the window), never on how the tokens were cut into steps or batched.
+// the absolute key position; chunk number c belongs to class c % 8, a class is summed up chunk by chunk, and the classes are joined
+// in their order, whoever had them: the order of every addition depends only on the query's position (and the window), never on
+// how the tokens were cut into steps or batched.
+//
+// Bound by latency where items are few (table -> key -> weights -> values, a chunk after the other): a decode step of two requests with 32
+// heads and 150 keys took 67 us a layer with a warp an item and takes 12 with a warp a class; 242 prompt tokens, whose warps fill the
+// SMs, take 64 and 139.
 //
 // A query at position p of request r sees keys max(0, p - window + 1) .. p (window <= 0: from 0), with a window also the
 // keys below keep_first; with chunk > 0 only those from the start of its own block of chunk positions on.
@@ -15,18 +20,28 @@
 
 namespace {
 
-constexpr int WARPS = 4;
+constexpr int CLASSES = 8;  // of chunks
+constexpr int MANY_WARPS = 4;  // items of a CTA where a warp has all classes of its item
 constexpr int MAX_DK = 640;  // most lanes of a query and a key
 constexpr int MAX_DV = 512;  // most lanes of a value
 
 // ACC: 32 value lanes each.  WIDE: the runs of a query and a key are read four lanes at a time (their lengths, strides and bases
 // allow it).  The order of every addition is that of the plain form.
-template <typename T, int ACC, bool WIDE>
-__global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsArgs<T> a) {
-    __shared__ __align__(16) float q_s[WARPS][MAX_DK];
+// SHARED: a CTA is one item and its warps the classes; else each of its warps is an item.
+template <typename T, int ACC, bool WIDE, bool SHARED>
+__global__ void __launch_bounds__((SHARED ? CLASSES : MANY_WARPS) * 32) attention_rows_kernel(const RowsArgs<T> a) {
+    constexpr int AHEAD = !SHARED || ACC > 4 ? 8 : ACC <= 2 ? 32 : 16;  // keys whose values are on their way at a time
+    __shared__ __align__(16) float q_all[SHARED ? 1 : MANY_WARPS][MAX_DK];
+    __shared__ float acc_s[SHARED ? CLASSES : 1][ACC * 32], ml_s[CLASSES][2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (item >= (long long)a.n_tokens * a.H) return;
+    const long long item = SHARED ? (long long)blockIdx.x : (long long)blockIdx.x * MANY_WARPS + warp;
+    if (item >= (long long)a.n_tokens * a.H) return;  // (whole CTAs where the CTA meets)
+    float* q_s = q_all[SHARED ? 0 : warp];
+    const int q_first = SHARED ? threadIdx.x : lane, q_step = SHARED ? CLASSES * 32 : 32;
+    auto meet = [&]() {
+        if (SHARED) __syncthreads();
+        else __syncwarp();
+    };
     const int t = (int)(item / a.H), h = (int)(item - (long long)t * a.H);
     const int r = a.token_request[t];
     const int q_begin = a.cu_tokens[r], q_len = a.cu_tokens[r + 1] - q_begin;
@@ -44,23 +59,39 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
     for (int i = 0; i < ACC; ++i) first[i] = 0.f;
     for (int map = 0; map < a.maps; ++map) {
         const T* qp = a.q0 + (long long)t * a.q0_token + (long long)h * a.q0_head + map * a.q_map;
-        __syncwarp();
-        for (int d = lane; d < a.d0; d += 32) q_s[warp][d] = to_float(qp[d]);
+        meet();
+        for (int d = q_first; d < a.d0; d += q_step) q_s[d] = to_float(qp[d]);
         if (a.d1 > 0) {
             const T* qr = a.q1 + (long long)t * a.q1_token + (long long)h * a.q1_head;
-            for (int d = lane; d < a.d1; d += 32) q_s[warp][a.d0 + d] = to_float(qr[d]);
+            for (int d = q_first; d < a.d1; d += q_step) q_s[a.d0 + d] = to_float(qr[d]);
         }
-        __syncwarp();
+        meet();
 
+        const int c_lo = (lo / 32) * 32, c_kept = ((kept + 31) / 32) * 32;  // the chunks of the kept keys end before c_kept
+        float all_m = -INFINITY, all_l = 0.f, all[ACC];  // the classes so far
+#pragma unroll
+        for (int i = 0; i < ACC; ++i) all[i] = 0.f;
+        auto join = [&](float m, float l, const float* acc, int pitch) {
+            if (m == -INFINITY) return;  // a class without a chunk
+            const float m_new = fmaxf(all_m, m), before = expf(all_m - m_new), share = expf(m - m_new);
+            all_m = m_new;
+            all_l = fmaf(l, share, all_l * before);
+#pragma unroll
+            for (int i = 0; i < ACC; ++i) all[i] = fmaf(acc[i * pitch], share, all[i] * before);
+        };
+#pragma unroll 1
+        for (int cls = SHARED ? warp : 0; cls < CLASSES; cls += SHARED ? CLASSES : 1) {
         float acc[ACC];
 #pragma unroll
         for (int i = 0; i < ACC; ++i) acc[i] = 0.f;
-        // a sink stands for a key of score sinks[h] and no value: the running maximum and sum start from it
-        float m = a.sinks ? a.sinks[h] : -INFINITY, l = a.sinks ? 1.f : 0.f;
+        // a sink stands for a key of score sinks[h] and no value: the first class's running maximum and sum start from it
+        const bool sink = a.sinks && cls == 0;
+        float m = sink ? a.sinks[h] : -INFINITY, l = sink ? 1.f : 0.f;
 
-        const int c_lo = (lo / 32) * 32, c_kept = ((kept + 31) / 32) * 32;  // the chunks of the kept keys end before c_kept
-        for (int c = kept > 0 ? 0 : c_lo; c <= pos; c += 32) {
-            if (c >= c_kept && c < c_lo) c = c_lo;  // nothing is seen between the kept keys and the window
+        auto mine_from = [&](int c) { return c + ((cls - c / 32) & (CLASSES - 1)) * 32; };  // the class's first chunk from c on
+        for (int c = mine_from(kept > 0 ? 0 : c_lo); c <= pos; c += CLASSES * 32) {
+            if (c >= c_kept && c < c_lo) c = mine_from(c_lo);  // nothing is seen between the kept keys and the window
+            if (c > pos) break;
             const int j = c + lane;
             const bool visible = (j >= lo && j <= pos) || j < kept;
             float s = -INFINITY;
@@ -76,12 +107,12 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
                     for (int d = 0; d < dk; d += 4) {
                         float kv[4], qv[4];
                         load4(kp + d, kv);
-                        load4(q_s[warp] + d, qv);
+                        load4(q_s + d, qv);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) dot = fmaf(qv[e], kv[e], dot);
                     }
                 } else {
-                    for (int d = 0; d < dk; ++d) dot = fmaf(q_s[warp][d], to_float(kp[d]), dot);
+                    for (int d = 0; d < dk; ++d) dot = fmaf(q_s[d], to_float(kp[d]), dot);
                 }
                 s = dot * a.scale;
                 if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
@@ -94,26 +125,46 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
 #pragma unroll
             for (int i = 0; i < ACC; ++i) acc[i] *= rescale;
             m = m_new;
-            // eight keys' values on their way at a time; a key of weight 0 is passed by
+            // a key of weight 0 is passed by
 #pragma unroll 1
-            for (int j0 = 0; j0 < min(32, pos - c + 1); j0 += 8) {
-                float v[8][ACC], pj[8];
+            for (int j0 = 0; j0 < min(32, pos - c + 1); j0 += AHEAD) {
+                float v[AHEAD][ACC], pj[AHEAD];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
+                for (int u = 0; u < AHEAD; ++u) {
                     pj[u] = __shfl_sync(0xffffffffu, p, j0 + u);
                     const T* vp = a.values + __shfl_sync(0xffffffffu, value_at, j0 + u);
 #pragma unroll
                     for (int i = 0; i < ACC; ++i) v[u][i] = pj[u] != 0.f && lane + 32 * i < dv ? to_float(vp[lane + 32 * i]) : 0.f;
                 }
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
+                for (int u = 0; u < AHEAD; ++u)
 #pragma unroll
                     for (int i = 0; i < ACC; ++i) acc[i] = pj[u] != 0.f ? fmaf(pj[u], v[u][i], acc[i]) : acc[i];
             }
         }
-        const float inv = 1.f / l;
+        if constexpr (SHARED) {
 #pragma unroll
-        for (int i = 0; i < ACC; ++i) first[i] = map == 0 ? acc[i] * inv : first[i] - a.diff_weight * (acc[i] * inv);
+            for (int i = 0; i < ACC; ++i) acc_s[cls][lane + 32 * i] = acc[i];
+            if (lane == 0) {
+                ml_s[cls][0] = m;
+                ml_s[cls][1] = l;
+            }
+        } else {
+            join(m, l, acc, 1);
+        }
+        }
+        if constexpr (SHARED) {
+            __syncthreads();
+#pragma unroll
+            for (int cls = 0; cls < CLASSES; ++cls) join(ml_s[cls][0], ml_s[cls][1], &acc_s[cls][lane], 32);
+        }
+        const float inv = 1.f / all_l;
+#pragma unroll
+        for (int i = 0; i < ACC; ++i) first[i] = map == 0 ? all[i] * inv : first[i] - a.diff_weight * (all[i] * inv);
+    }
+    if (SHARED) {
+        __syncthreads();  // the queries have been read by all
+        if (warp != 0) return;  // all warps hold the same
     }
     if (a.maps == 2) {
         float ss = 0.f;
@@ -123,7 +174,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
 #pragma unroll
         for (int i = 0; i < ACC; ++i) first[i] *= norm;
     }
-    float* y = q_s[warp];  // the queries have been read
+    float* y = q_s;  // the queries have been read
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < ACC; ++i)
@@ -137,14 +188,22 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_kernel(const RowsAr
 template <typename T, int ACC>
 int launch_rows_of(const RowsArgs<T>& a, cudaStream_t stream) {
     const long long items = (long long)a.n_tokens * a.H;
-    // few rows (decode steps): a warp a CTA, so that each has an SM of its own
-    const int warps = items <= 512 ? 1 : WARPS;
-    const long long blocks = (items + warps - 1) / warps;
+    // a warp a class until the items' own warps fill the SMs (2,048: 14 warps an SM); values of more than 256 lanes always (registers)
+    const bool shared = items <= 2048 || ACC > 8;
+    const long long blocks = shared ? items : (items + MANY_WARPS - 1) / MANY_WARPS;
     if (blocks > 0x7fffffffLL) return LLM_ERR_UNSUPPORTED;
     const bool wide = !(a.d0 & 3) && !(a.d1 & 3) && !((a.k_page | a.k_head | a.k_token | (a.maps == 2 ? a.k_map : 0)) & 3) &&
                       !((uintptr_t)a.keys & (4 * sizeof(T) - 1));
-    if (wide) attention_rows_kernel<T, ACC, true><<<(unsigned)blocks, warps * 32, 0, stream>>>(a);
-    else attention_rows_kernel<T, ACC, false><<<(unsigned)blocks, warps * 32, 0, stream>>>(a);
+    const unsigned grid = (unsigned)blocks, block = (shared ? CLASSES : MANY_WARPS) * 32;
+    if constexpr (ACC <= 8) {
+        if (!shared) {
+            if (wide) attention_rows_kernel<T, ACC, true, false><<<grid, block, 0, stream>>>(a);
+            else attention_rows_kernel<T, ACC, false, false><<<grid, block, 0, stream>>>(a);
+            return launch_status();
+        }
+    }
+    if (wide) attention_rows_kernel<T, ACC, true, true><<<grid, block, 0, stream>>>(a);
+    else attention_rows_kernel<T, ACC, false, true><<<grid, block, 0, stream>>>(a);
     return launch_status();
 }
 

@@ -1,0 +1,51 @@
+"""The general attention kernel: a row's bits are the same whether its item has eight warps (few items) or one (many), over the forms whose
+keys start and end in the middle of chunks."""
+
+import pytest
+import torch
+
+import test_attention_rows_few_gpu as rows
+from test_attention_rows_few_gpu import DEV, ops, rnd  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+FORMS = {
+    "plain": dict(d0=64, dv=64),
+    "odd": dict(d0=7, d1=6, dv=33),
+    "window": dict(d0=16, dv=130, window=70, slopes=True),
+    "kept": dict(d0=64, dv=64, window=40, keep_first=37, sinks=True),
+    "blocks": dict(d0=64, dv=64, chunk=96, softcap=5.0),
+    "two maps": dict(d0=32, dv=64, maps=2),
+    "wide": dict(d0=64, dv=300),
+}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("form", FORMS)
+def test_bits_do_not_depend_on_the_number_of_items(ops, form, dtype, monkeypatch):  # noqa: F811
+    monkeypatch.setattr(ops, "_FORCE_GENERIC_ATTENTION", True)
+    f = FORMS[form]
+    d0, d1, dv, maps, H, KV, page, n, context = f["d0"], f.get("d1", 0), f["dv"], f.get("maps", 1), 32, 8, 4, 65, 601
+    dk, pages = maps * d0 + d1, 160
+    keys, values = rnd(pages, KV, page, dk, seed=1, dtype=dtype), rnd(pages, KV, page, dv, seed=2, dtype=dtype)
+    q0, q1 = rnd(n, H, maps * d0, seed=3, dtype=dtype), rnd(n, H, d1, seed=4, dtype=dtype) if d1 else None
+    kw = dict(num_heads=H, num_kv_heads=KV, scale=dk**-0.5, window=f.get("window"), keep_first=f.get("keep_first"), chunk=f.get("chunk"), softcap=f.get("softcap"))
+    if f.get("slopes"):
+        kw["slopes"] = rnd(H, dtype=torch.float32, seed=5).abs() * 0.1
+    if f.get("sinks"):
+        kw["sinks"] = rnd(H, dtype=torch.float32, seed=6)
+    if maps == 2:
+        kw["differential"] = ops.DifferentialMaps(0.4, 1e-6, 0.5)
+
+    def run(first, count):  # the tokens [first, first + count) as a step of their own
+        table, ctx = rows.step((n,), (context,), page, pages, False)
+        ctx.context_lens = torch.tensor([context - n + first + count], dtype=torch.int32, device=DEV)
+        ctx.num_tokens = ctx.max_query_len = count
+        ctx.cu_tokens, ctx.token_request = torch.tensor([0, count], dtype=torch.int32, device=DEV), torch.zeros(count, dtype=torch.int32, device=DEV)
+        part = lambda x: None if x is None else x[first : first + count].contiguous()  # noqa: E731
+        return ops.attention_rows(part(q0), part(q1), keys.data_ptr(), (KV * page * dk, page * dk, dk), values.data_ptr(), (KV * page * dv, page * dv, dv), dv,
+                                  table, page, ctx, **kw)
+
+    whole = run(0, n)  # 2,080 items
+    for first, count in ((0, 1), (33, 1), (n - 2, 2), (0, 64)):
+        assert torch.equal(run(first, count), whole[first : first + count])
