@@ -94,6 +94,57 @@ __device__ __forceinline__ void route_row(const float* zr, const float* __restri
     if (shared_gate && lane == 0) wr[E] = shared_gate == 2 ? 1.f : 1.f / (1.f + expf(-zr[E]));
 }
 
+// The same for at most 32 experts, a lane each and everything in registers: a choice is a reduction of the scores as ordered integers and a
+// ballot (lowest index among equals) instead of ten shuffles through shared memory.  The same bits.
+__device__ __forceinline__ void route_row_32(const float* zr, const float* __restrict__ correction, float* wr, int E, int top, float scale, int renorm,
+                                             int shared_gate, int lane, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
+    const unsigned all = 0xffffffffu;
+    const bool mine = lane < E;
+    const float z = mine ? zr[lane] + (bias ? bias[lane] : 0.f) : -FLT_MAX;
+    float s;
+    if (sigmoid) {
+        s = mine ? 1.f / (1.f + expf(-z)) : 0.f;
+    } else {
+        const float m = warp_max(fmaxf(-FLT_MAX, z)), x = mine ? expf(z - m) : 0.f;
+        s = x * (1.f / warp_sum(x));
+    }
+    float c = mine ? s + (correction ? correction[lane] : 0.f) : -FLT_MAX;
+    if (groups > 0) {
+        const int size = E / groups, g = min(lane, E - 1) / size;
+        float first = -FLT_MAX, second = -FLT_MAX;
+        for (int i = 0; i < size; ++i) {
+            const float v = __shfl_sync(all, c, g * size + i);
+            if (v > first) { second = first; first = v; }
+            else if (v > second) second = v;
+        }
+        const float score = size > 1 ? first + second : first;
+        int ahead = 0;
+        for (int o = 0; o < groups; ++o) {
+            const float other = __shfl_sync(all, score, o * size);
+            ahead += other > score || (other == score && o < g);
+        }
+        if (ahead >= keep) c = -FLT_MAX;
+    }
+    // larger scores are larger integers (both zeros alike); 0: cannot be chosen
+    const unsigned bits = __float_as_uint(c + 0.f);
+    unsigned key = c > -FLT_MAX ? (bits & 0x80000000u ? ~bits : bits | 0x80000000u) : 0u;
+    bool chosen = false;
+    float chosen_sum = 0.f;
+    for (int k = 0; k < top; ++k) {
+        const unsigned best = __reduce_max_sync(all, key);
+        if (best == 0u) break;
+        const int arg = __ffs(__ballot_sync(all, key == best)) - 1;
+        chosen_sum += __shfl_sync(all, s, arg);
+        if (lane == arg) {
+            chosen = true;
+            key = 0u;
+        }
+    }
+    const float f = renorm ? scale / (chosen_sum + (sigmoid ? 1e-20f : 0.f)) : scale;
+    if (mine) wr[lane] = chosen ? s * f : 0.f;
+    if (shared_gate && lane == 0) wr[E] = shared_gate == 2 ? 1.f : 1.f / (1.f + expf(-zr[E]));
+}
+
 __global__ void __launch_bounds__(128)
 route_topk_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ correction, float* __restrict__ w, int N, int E,
                   int top, float scale, int renorm, int shared_gate) {
@@ -185,57 +236,81 @@ router_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, c
     }
 }
 
-// The same for steps of few tokens: one CTA a token, a warp a row of the router matrix at a time.  A warp's first row is on its way
-// before the kernel in front has ended (the weights depend on nothing).  The sums have the order of the kernel above.
+// The same for steps of few tokens: one CTA a token, a warp a row of the router matrix at a time.  The matrix is on its way before the
+// kernel in front has ended (the weights depend on nothing): a warp's first 1,024 lanes in registers, the rest of its rows in shared
+// memory, a lane's own elements.  Behind the wait stands one load of the token, a row's sums and the choice: 32 rows of 2,048 took 7.5 us
+// of a decode step with the second half of a row behind the wait and the choice in shared memory, and take 4.7.  The sums
+// have the order of the kernel above.
+constexpr int ROUTER_AHEAD = 8, ROUTER_STEP = ROUTER_AHEAD * 128;  // 16-byte pieces of a row that a lane has in registers; elements
+
+__host__ __device__ inline int router_steps_before(int warp, int rows, int warps, int per_row) {  // steps of the warps in front, less their first
+    const int each = rows / warps, more = rows % warps;
+    return warp * (each * per_row - 1) + (warp < more ? warp : more) * per_row;
+}
+
 template <typename TX>
 __global__ void __launch_bounds__(1024)
 router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
                   int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
-    constexpr int AHEAD = 8;  // 16-byte pieces of a row that a lane has in flight
-    extern __shared__ float sm[];  // z[rows], s[E], c[E], and the scores of runs of experts
+    extern __shared__ __align__(16) float sm[];  // the steps behind a warp's first [ROUTER_STEP each], x[K], z[rows], s[E], c[E], scores of runs
     pdl_trigger();
     const int rows = E + (shared_gate == 1), out_w = E + (shared_gate != 0), t = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const TX* xr = x + (size_t)t * ldx;
-    float4 w[AHEAD];
-    auto ask = [&](int e, int k0) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
+    float* ahead = sm + (size_t)router_steps_before(warp, rows, warps, per_row) * ROUTER_STEP;
+    float* x_s = sm + (size_t)(rows * per_row - warps) * ROUTER_STEP;
+    float* z_s = x_s + K;
+    float4 w[ROUTER_AHEAD];
 #pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            const int k = k0 + (i * 32 + lane) * 4;
-            w[i] = e < rows && k < K ? *reinterpret_cast<const float4*>(wr + (size_t)e * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    ask(warp, 0);
-    bool waited = false;
-    for (int e = warp; e < rows; e += warps) {
+    for (int i = 0; i < ROUTER_AHEAD; ++i) {
+        const int k = (i * 32 + lane) * 4;
+        w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)warp * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int e = warp, n = 0; e < rows; e += warps)
+        for (int step = e == warp ? 1 : 0; step < per_row; ++step, ++n)
+            for (int i = 0; i < ROUTER_AHEAD; ++i) {
+                const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
+                if (k < K)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(ahead + n * ROUTER_STEP + (i * 32 + lane) * 4)),
+                                 "l"(wr + (size_t)e * K + k));
+            }
+    asm volatile("cp.async.commit_group;\n" ::);
+    pdl_wait();
+    for (int k = threadIdx.x * 4; k < K; k += blockDim.x * 4) {
+        float v[4];
+        load4(x + (size_t)t * ldx + k, v);
+        store4(x_s + k, v);
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    for (int e = warp, n = 0; e < rows; e += warps) {
         float acc = 0.f;
-        for (int k0 = 0; k0 < K; k0 += AHEAD * 128) {
-            if (!waited) pdl_wait();
-            else ask(e, k0);
-            waited = true;
-            float xv[AHEAD][4];
+        for (int step = 0; step < per_row; ++step) {
+            const bool first = e == warp && step == 0;
 #pragma unroll
-            for (int i = 0; i < AHEAD; ++i) {
-                const int k = k0 + (i * 32 + lane) * 4;
-                xv[i][0] = xv[i][1] = xv[i][2] = xv[i][3] = 0.f;
-                if (k < K) load4(xr + k, xv[i]);
+            for (int i = 0; i < ROUTER_AHEAD; ++i) {
+                const int at = (i * 32 + lane) * 4, k = step * ROUTER_STEP + at;
+                if (k >= K) continue;
+                const float4 wv = first ? w[i] : *reinterpret_cast<const float4*>(ahead + n * ROUTER_STEP + at);
+                float xv[4];
+                load4(x_s + k, xv);
+                acc = fmaf(wv.x, xv[0], acc);
+                acc = fmaf(wv.y, xv[1], acc);
+                acc = fmaf(wv.z, xv[2], acc);
+                acc = fmaf(wv.w, xv[3], acc);
             }
-#pragma unroll
-            for (int i = 0; i < AHEAD; ++i) {
-                acc = fmaf(w[i].x, xv[i][0], acc);
-                acc = fmaf(w[i].y, xv[i][1], acc);
-                acc = fmaf(w[i].z, xv[i][2], acc);
-                acc = fmaf(w[i].w, xv[i][3], acc);
-            }
+            n += first ? 0 : 1;
         }
         acc = warp_sum(acc);
-        if (lane == 0) sm[e] = acc;
+        if (lane == 0) z_s[e] = acc;
     }
-    if (!waited) pdl_wait();
     __syncthreads();
     if (warp == 0) {
-        float* s = sm + rows;
-        route_row(sm, correction, out + (size_t)t * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep, s + 2 * E);
+        if (E <= 32) {
+            route_row_32(z_s, correction, out + (size_t)t * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
+        } else {
+            float* s = z_s + rows;
+            route_row(z_s, correction, out + (size_t)t * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep, s + 2 * E);
+        }
     }
 }
 
@@ -541,13 +616,18 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
     const int rows_all = E + (shared_gate == 1 ? 1 : 0);  // rows of the router's matrix (2: the last column of out is the constant 1)
     const size_t align = x_dtype == LLM_F32 ? 16 : 8;
     if (N <= 32 && K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)wr % 16 == 0 && (uintptr_t)x % align == 0) {
-        const size_t few = ((size_t)rows_all + 2 * E + groups) * sizeof(float);
-        const dim3 block(32 * (rows_all < 32 ? rows_all : 32));
-        if (x_dtype == LLM_F32)
-            return launch_pdl(router_few_kernel<float>, dim3(N), block, few, stream, (const float*)x, ldx, wr, correction, out, K, E, top, scale, renorm,
-                              shared_gate, bias, sigmoid, groups, keep);
-        return launch_pdl(router_few_kernel<bf>, dim3(N), block, few, stream, (const bf*)x, ldx, wr, correction, out, K, E, top, scale, renorm, shared_gate,
-                          bias, sigmoid, groups, keep);
+        const int warps = rows_all < 32 ? rows_all : 32, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
+        const size_t few = ((size_t)(rows_all * per_row - warps) * ROUTER_STEP + K + rows_all + 2 * E + groups) * sizeof(float);
+        auto go = [&](auto kernel, auto* xp) -> int {
+            if (few > 48 * 1024) {
+                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
+                if (e != cudaSuccess) return (int)e;
+            }
+            return launch_pdl(kernel, dim3(N), dim3(32 * warps), few, stream, xp, ldx, wr, correction, out, K, E, top, scale, renorm, shared_gate, bias, sigmoid,
+                              groups, keep);
+        };
+        // a matrix that the registers and the shared memory of a CTA hold (33 rows of 2,048: 148 KB); larger ones take the kernel below
+        if (few <= 200 * 1024) return x_dtype == LLM_F32 ? go(router_few_kernel<float>, (const float*)x) : go(router_few_kernel<bf>, (const bf*)x);
     }
     // tokens a CTA: one for steps of few tokens (more CTAs, more loads in flight a warp), two otherwise (three CTAs an SM), eight where
     // that leaves CTAs enough (the matrix passes through a CTA once for all of its tokens)
