@@ -230,6 +230,10 @@ router_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, c
     }
     __syncthreads();
     if (warp < TT && t0 + warp < N) {
+        if (E <= 32) {
+            route_row_32(z + warp * rows, correction, out + (size_t)(t0 + warp) * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
+            return;
+        }
         float* s = sm + (size_t)TT * rows + (size_t)warp * (2 * E + groups);
         route_row(z + warp * rows, correction, out + (size_t)(t0 + warp) * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups,
                   keep, s + 2 * E);
@@ -332,6 +336,7 @@ expert_act_scale_wide_kernel(const T* __restrict__ x, int ldx, const float* __re
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.y;
+#pragma unroll 4
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) * RUN; j < C; j += gridDim.x * blockDim.x * RUN) {
         const int b = j < E * ff ? j / ff : E;
         const float wt = w[(size_t)t * ldw + b];
@@ -383,6 +388,7 @@ expert_gated_act_kernel(const T* __restrict__ x, int ldx, T* __restrict__ y, int
         mine = table + (size_t)id * top;
     }
     pdl_wait();
+#pragma unroll 4
     for (int j = (blockIdx.x * blockDim.x + threadIdx.x) * RUN; j < C; j += gridDim.x * blockDim.x * RUN) {
         const bool shared = j >= E * ff;
         const int e = shared ? E : j / ff, i = shared ? j - E * ff : j - e * ff;
@@ -649,14 +655,20 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
     return x_dtype == LLM_F32 ? pick((const float*)x) : pick((const bf*)x);
 }
 
+// CTAs a token of the experts' activation, which has work for `blocks` of 256 threads with 16 bytes each: with many tokens a quarter of
+// them, four times 16 bytes a thread in flight (a CTA a run of 16 bytes a thread ended as soon as it had started: 1,801 tokens of a gated mixture 48.8 -> 41.0 us, 1,686 of a plain one 25.4 -> 18.7)
+static int activation_blocks(int blocks, int tokens) {
+    if (blocks > 64) blocks = 64;
+    return (long long)blocks * tokens > 8 * 4 * 148 ? (blocks + 3) / 4 : blocks;
+}
+
 LLM_EXPORT int llm_expert_act_scale(const void* x, int ldx, const float* w, int ldw, void* y, int ldy, int dtype, int N, int C, int E,
                                     int ff, int kind, cudaStream_t stream) {
     if (N <= 0 || C <= 0) return 0;
     if (E < 0 || ff <= 0 || (size_t)E * ff > (size_t)C || N > 65535) return LLM_ERR_BAD_ARGUMENT;
     const int run = dtype == LLM_F32 ? 4 : 8;
     if (ff % run == 0 && C % run == 0 && ldx % run == 0 && ldy % run == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0) {
-        const int per = 256 * run, blocks = (C + per - 1) / per;
-        const dim3 grid(blocks < 64 ? blocks : 64, N), block(256);
+        const dim3 grid(activation_blocks((C + 256 * run - 1) / (256 * run), N), N), block(256);
         if (dtype == LLM_F32)
             return launch_pdl(expert_act_scale_wide_kernel<float>, grid, block, 0, stream, (const float*)x, ldx, w, ldw, (float*)y, ldy, N, C, E, ff, kind);
         return launch_pdl(expert_act_scale_wide_kernel<__nv_bfloat16>, grid, block, 0, stream, (const __nv_bfloat16*)x, ldx, w, ldw,
@@ -677,8 +689,8 @@ LLM_EXPORT int llm_expert_gated_act(const void* x, int ldx, void* y, int ldy, in
     if (E < 0 || ff < 0 || fs < 0 || N > 65535 || (!w && (!ids || !table || top < 0 || vocab <= 0))) return LLM_ERR_BAD_ARGUMENT;
     const int run = dtype == LLM_F32 ? 4 : 8;
     const bool wide = ff % run == 0 && fs % run == 0 && ldx % run == 0 && ldy % run == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0;
-    const int per = 256 * (wide ? run : 1), blocks = (C + per - 1) / per;
-    const dim3 grid(blocks < 64 ? blocks : 64, N), block(256);
+    const int per = 256 * (wide ? run : 1);
+    const dim3 grid(activation_blocks((C + per - 1) / per, N), N), block(256);
     using bf = __nv_bfloat16;
     auto go = [&](auto kernel, auto* xp, auto* yp) {
         return launch_pdl(kernel, grid, block, 0, stream, xp, ldx, yp, ldy, w, ldw, ids, table, top, vocab, E, ff, fs, limit, limit_s, slope, up_shift);
