@@ -354,9 +354,10 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     static const int sms = [] {
         int dev = 0, n = 0;
         cudaGetDevice(&dev);
-        cudaFuncSetAttribute(experts_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UP_RING);
         return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
     }();
+    const cudaError_t set = cudaFuncSetAttribute(experts_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UP_RING);
+    if (set != cudaSuccess) return (int)set;
     const int most = (E * ff + fs) / (kind < 0 ? 8 : 16);
     const int code = launch_pdl(experts_up_kernel, dim3(most < sms ? most : sms), dim3(UP_THREADS), (size_t)p.up_slots * up_slot, stream, p);
     return code != 0 ? code : launch_pdl(experts_down_kernel, dim3(N / 16), dim3(DOWN_THREADS), 0, stream, p);

@@ -252,7 +252,8 @@ __host__ __device__ inline int router_steps_before(int warp, int rows, int warps
     return warp * (each * per_row - 1) + (warp < more ? warp : more) * per_row;
 }
 
-template <typename TX>
+// STAGED: registers and shared memory hold the matrix; else what is behind a warp's first step is read where it is used.
+template <typename TX, bool STAGED>
 __global__ void __launch_bounds__(1024)
 router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
                   int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
@@ -261,7 +262,7 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
     const int rows = E + (shared_gate == 1), out_w = E + (shared_gate != 0), t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
     float* ahead = sm + (size_t)router_steps_before(warp, rows, warps, per_row) * ROUTER_STEP;
-    float* x_s = sm + (size_t)(rows * per_row - warps) * ROUTER_STEP;
+    float* x_s = sm + (STAGED ? (size_t)(rows * per_row - warps) * ROUTER_STEP : 0);
     float* z_s = x_s + K;
     float4 w[ROUTER_AHEAD];
 #pragma unroll
@@ -269,7 +270,7 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
         const int k = (i * 32 + lane) * 4;
         w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)warp * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int e = warp, n = 0; e < rows; e += warps)
+    for (int e = warp, n = 0; STAGED && e < rows; e += warps)
         for (int step = e == warp ? 1 : 0; step < per_row; ++step, ++n)
             for (int i = 0; i < ROUTER_AHEAD; ++i) {
                 const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
@@ -290,11 +291,17 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
         float acc = 0.f;
         for (int step = 0; step < per_row; ++step) {
             const bool first = e == warp && step == 0;
+            if (!STAGED && !first)
+#pragma unroll
+                for (int i = 0; i < ROUTER_AHEAD; ++i) {
+                    const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
+                    w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)e * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
 #pragma unroll
             for (int i = 0; i < ROUTER_AHEAD; ++i) {
                 const int at = (i * 32 + lane) * 4, k = step * ROUTER_STEP + at;
                 if (k >= K) continue;
-                const float4 wv = first ? w[i] : *reinterpret_cast<const float4*>(ahead + n * ROUTER_STEP + at);
+                const float4 wv = !STAGED || first ? w[i] : *reinterpret_cast<const float4*>(ahead + n * ROUTER_STEP + at);
                 float xv[4];
                 load4(x_s + k, xv);
                 acc = fmaf(wv.x, xv[0], acc);
@@ -623,7 +630,9 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
     const size_t align = x_dtype == LLM_F32 ? 16 : 8;
     if (N <= 32 && K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)wr % 16 == 0 && (uintptr_t)x % align == 0) {
         const int warps = rows_all < 32 ? rows_all : 32, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
-        const size_t few = ((size_t)(rows_all * per_row - warps) * ROUTER_STEP + K + rows_all + 2 * E + groups) * sizeof(float);
+        const size_t rest = ((size_t)K + rows_all + 2 * E + groups) * sizeof(float), matrix = (size_t)(rows_all * per_row - warps) * ROUTER_STEP * sizeof(float);
+        const bool staged = matrix + rest <= 200 * 1024;  // 33 rows of 2,048: 148 KB
+        const size_t few = staged ? matrix + rest : rest;
         auto go = [&](auto kernel, auto* xp) -> int {
             if (few > 48 * 1024) {
                 const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
@@ -632,8 +641,10 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
             return launch_pdl(kernel, dim3(N), dim3(32 * warps), few, stream, xp, ldx, wr, correction, out, K, E, top, scale, renorm, shared_gate, bias, sigmoid,
                               groups, keep);
         };
-        // a matrix that the registers and the shared memory of a CTA hold (33 rows of 2,048: 148 KB); larger ones take the kernel below
-        if (few <= 200 * 1024) return x_dtype == LLM_F32 ? go(router_few_kernel<float>, (const float*)x) : go(router_few_kernel<bf>, (const bf*)x);
+        if (few <= 200 * 1024) {
+            if (x_dtype == LLM_F32) return staged ? go(router_few_kernel<float, true>, (const float*)x) : go(router_few_kernel<float, false>, (const float*)x);
+            return staged ? go(router_few_kernel<bf, true>, (const bf*)x) : go(router_few_kernel<bf, false>, (const bf*)x);
+        }
     }
     // tokens a CTA: one for steps of few tokens (more CTAs, more loads in flight a warp), two otherwise (three CTAs an SM), eight where
     // that leaves CTAs enough (the matrix passes through a CTA once for all of its tokens)

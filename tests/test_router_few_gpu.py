@@ -9,7 +9,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("K", [4, 1020, 1024, 1028, 2048, 4096])
-@pytest.mark.parametrize("experts, top, groups", [(1, 1, None), (5, 2, None), (32, 4, (4, 2)), (32, 32, None), (33, 3, None), (64, 5, (8, 3)), (30, 6, (30, 8))])
+@pytest.mark.parametrize("experts, top, groups", [(1, 1, None), (5, 2, None), (32, 4, (4, 2)), (32, 32, None), (33, 3, None), (64, 5, (8, 3)), (30, 6, (30, 8)), (200, 7, None)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_few_tokens_have_the_bits_of_many(K, experts, top, groups, dtype):
     from llmserve_triton_kernels_b200 import ops
