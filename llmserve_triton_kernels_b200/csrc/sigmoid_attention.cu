@@ -7,7 +7,8 @@
 //   out_h(i)   = sum_j w_h(i, j) v_c(h)(j)
 //
 // Nothing is normalised over keys, so the sum over keys may be cut anywhere and the pieces added: a long context is
-// shared out over `splits` CTAs in stretches of a fixed number of keys, counted from position 0, and the partial sums
+// shared out over `splits` CTAs in stretches of a fixed number of keys, counted from position 0 (stretch s is CTA s % splits's,
+// so that those of a window far behind position 0 are shared out like the first ones), and the partial sums
 // are added in the order of the stretches.  Scores, weights and sums are 32-bit.
 //
 // Also here: what a token's projections go through before they are keys and queries (an RMS norm over the whole
@@ -46,8 +47,9 @@ sigmoid_attention_kernel(const TQ* __restrict__ q, int ldq, const TC* __restrict
     pdl_trigger();
     const int pos = positions[t], req = token_request[t];
     const int first = window > 0 ? max(0, pos - window + 1) : 0;
-    // a stretch none of whose keys the token sees leaves its partial sums unwritten: the sum reads only stretches that have some
-    if (splits > 1 && (split * split_keys > pos || (split + 1) * split_keys <= first)) return;
+    // this CTA's stretches of those that the token sees; without one its partial sums stay unwritten, and the sum does not read them
+    const int stretch0 = first / split_keys, mine = stretch0 + (split + splits - stretch0 % splits) % splits;
+    if (mine * split_keys > pos) return;
     const int* table = page_table + (size_t)req * table_width;
     if (mix)
         for (int i = threadIdx.x; i < 32 * H; i += blockDim.x) {
@@ -57,12 +59,13 @@ sigmoid_attention_kernel(const TQ* __restrict__ q, int ldq, const TC* __restrict
     pdl_wait();
     for (int i = threadIdx.x; i < H * D; i += blockDim.x) sq[i] = to_float(q[(size_t)t * ldq + i]);
     __syncthreads();
-    int j_lo = max(first, split * split_keys), j_hi = min(pos, (split + 1) * split_keys - 1);  // inclusive
     float acc[VPL];
 #pragma unroll
     for (int m = 0; m < VPL; ++m) acc[m] = 0.f;
     const size_t plane = (size_t)KV * page_size * Dp;
     const int c_out = has_out ? h_out / group : 0;
+    for (int stretch = mine; stretch * split_keys <= pos; stretch += splits) {
+    const int j_lo = max(first, stretch * split_keys), j_hi = min(pos, (stretch + 1) * split_keys - 1);  // inclusive
     for (int j0 = (j_lo / CHUNK) * CHUNK; j0 <= j_hi; j0 += CHUNK) {
         const int j = j0 + lane;
         const bool seen = j >= j_lo && j <= j_hi;
@@ -111,6 +114,7 @@ sigmoid_attention_kernel(const TQ* __restrict__ q, int ldq, const TC* __restrict
             }
         }
         __syncthreads();
+    }
     }
     if (!has_out) return;
     if (splits > 1) {

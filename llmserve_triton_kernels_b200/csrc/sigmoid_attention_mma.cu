@@ -19,8 +19,8 @@ using namespace attn;
 constexpr int BM = 16;   // query tokens a CTA
 constexpr int HB = 16;   // output heads a CTA
 constexpr int THREADS = 512;
-constexpr int MAX_SHARES = 16;  // CTAs that share a tile's keys: stretch s goes to CTA s % 16, so that a step whose grid is made for the
-                                // longest context a pool allows does not launch hundreds of CTAs without keys
+constexpr int MAX_SHARES = 16;  // most CTAs that share a tile's keys: stretch s goes to CTA s % shares, so that a step whose grid is made for
+                                // the longest context a pool allows does not launch hundreds of CTAs without keys
 
 struct SigMmaParams {
     const __nv_bfloat16* q;
@@ -31,7 +31,7 @@ struct SigMmaParams {
     const float *bias, *mix;
     __nv_bfloat16* out;
     float* parts;  // [grid.z][N][H * V] partial sums when the keys are shared out over several CTAs (else null)
-    int N, R, H, KV, D, V, Dp, page_size, window, split_keys, splits;
+    int N, R, H, KV, D, V, Dp, page_size, window, split_keys;
     float scale, cap;
 };
 
@@ -79,15 +79,16 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
     const int pos0 = p.positions[t0];  // the tile's tokens stand at pos0, pos0 + 1, ...
     const int* table = p.page_table + (size_t)r * p.table_width;
     const size_t plane = (size_t)KV * p.page_size * p.Dp;
-    // the keys that any row of the tile sees; this CTA takes the stretches split, split + gridDim.z, ... of them
-    const int tile_first = p.window > 0 ? max(0, pos0 - p.window + 1) : 0, tile_last = pos0 + rows - 1;
-    {
-        bool any = false;
-        for (int s = split; s < p.splits && !any; s += gridDim.z)
-            any = max(tile_first, s * p.split_keys) <= min(tile_last, (s + 1) * p.split_keys - 1);
-        if (!any) return;  // the sum reads only the partial sums of CTAs that had keys
-    }
-    int first = 0, last = -1;  // of the stretch at hand
+    // the keys that any row of the tile sees, and of them this CTA's: the stretches s with s % shares == split, from the first one that
+    // the tile sees on, tile after tile (a stretch is whole tiles), the next one always on its way
+    const int tile_first = p.window > 0 ? max(0, pos0 - p.window + 1) : 0, last = pos0 + rows - 1, shares = gridDim.z;
+    const int stretch0 = tile_first / p.split_keys, mine = stretch0 + (split + shares - stretch0 % shares) % shares;
+    const int j_begin = max(mine * p.split_keys, tile_first / BN * BN);
+    auto next = [&](int j) {
+        j += BN;
+        return j % p.split_keys ? j : j + (shares - 1) * p.split_keys;
+    };
+    if (j_begin > last) return;  // the sum reads only the partial sums of CTAs that had keys
     pdl_wait();
     // the tile's queries, every head: 16 bytes a thread and turn; rows beyond the request's tokens are zeros
     {
@@ -133,15 +134,11 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
     const bool mixes = oct < 2;
     const bool mix_row = mixes && mi < rows;  // rows beyond the request's tokens keep weights of zero
 
-    for (int stretch = split; stretch < p.splits; stretch += gridDim.z) {
-    first = max(tile_first, stretch * p.split_keys);
-    last = min(tile_last, (stretch + 1) * p.split_keys - 1);
-    if (first > last) continue;
-    const int j_begin = (first / BN) * BN;
     load_keys(j_begin);
     load_values(j_begin);
     cp_async_commit();
-    for (int j0 = j_begin; j0 <= last; j0 += BN) {
+    for (int j0 = j_begin; j0 <= last;) {
+        const int j_next = next(j0);
         cp_async_wait<0>();
         __syncthreads();  // (A) this tile's keys and values have landed; everybody is done with the tile before
         // ---- 1. scores and weights of every head
@@ -174,7 +171,7 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
                 const int i = (lane >> 2) + half * 8;
                 const int pos = pos0 + i;
                 const int hi = i < rows ? min(pos, last) : -1;
-                const int lo = max(p.window > 0 ? max(0, pos - p.window + 1) : 0, first);
+                const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
                 if (hi < max(lo, j0)) {  // a row without a key in this tile (one beyond the request's tokens, as most rows of a decode step's tile)
 #pragma unroll
                     for (int n = 0; n < BN / 8; ++n)
@@ -203,7 +200,7 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
             }
         }
         __syncthreads();  // (B) every head's weights are in shared memory; nobody reads the keys any more
-        if (j0 + BN <= last) load_keys(j0 + BN);
+        if (j_next <= last) load_keys(j_next);
         cp_async_commit();
         // ---- 2. the heads' weights mixed, in 32-bit
         float m[8][2];
@@ -248,11 +245,11 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
             }
         }
         __syncthreads();  // (E) nobody reads this tile's values any more
-        if (j0 + BN <= last) load_values(j0 + BN);
+        if (j_next <= last) load_values(j_next);
         cp_async_commit();
+        j0 = j_next;
     }
     cp_async_wait<0>();
-    }  // stretches
     if (!has_out) return;
 #pragma unroll
     for (int n = 0; n < NV8; ++n)
@@ -261,7 +258,7 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
             const int i = (lane >> 2) + half * 8;
             if (i >= rows) continue;
             const size_t at = (size_t)(t0 + i) * H * V + (size_t)h_out * V + n * 8 + (lane & 3) * 2;
-            if (p.splits > 1)
+            if (shares > 1)
                 *reinterpret_cast<float2*>(p.parts + (size_t)split * p.N * H * V + at) = make_float2(O[n][half * 2], O[n][half * 2 + 1]);
             else
                 *reinterpret_cast<unsigned*>(p.out + at) = pack_bf16(O[n][half * 2], O[n][half * 2 + 1]);
@@ -269,13 +266,13 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
 }
 
 template <int NV8, int BN>
-int launch(const SigMmaParams& p, int tiles, size_t smem, cudaStream_t stream) {
+int launch(const SigMmaParams& p, int tiles, int shares, size_t smem, cudaStream_t stream) {
     auto kernel = sigmoid_attention_mma_kernel<NV8, BN>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    return launch_pdl(kernel, dim3(tiles, (p.H + HB - 1) / HB, p.splits < MAX_SHARES ? p.splits : MAX_SHARES), dim3(THREADS), smem, stream, p);
+    return launch_pdl(kernel, dim3(tiles, (p.H + HB - 1) / HB, shares), dim3(THREADS), smem, stream, p);
 }
 
 size_t smem_bytes(int H, int KV, int D, int V, int BN) {
@@ -288,16 +285,16 @@ size_t smem_bytes(int H, int KV, int D, int V, int BN) {
 
 // `tiles`: the sum over the requests of ceil(tokens / 16).  Returns LLM_ERR_UNSUPPORTED for sizes it does not take
 // (lanes that are no multiples of 16, values wider than 128 lanes, heads that do not fit the shared memory).
-// `splits` > 1: the keys are shared out in stretches of `split_keys` (a multiple of 32), stretch s to share s % shares with
-// shares = min(splits, 16), and the partial sums left in `parts [shares][N][H * V]` for llm_sigmoid_sum_parts.
+// `shares` > 1 (at most 16): the keys are shared out in stretches of `split_keys` (a multiple of 32) counted from position 0, stretch s
+// to share s % shares, and the partial sums left in `parts [shares][N][H * V]` for llm_sigmoid_sum_parts.
 LLM_EXPORT int llm_sigmoid_attention_mma(const void* q, int ldq, const void* pool, const int* page_table, int table_width,
                                          const int* positions, const int* cu_tokens, const float* bias, const float* mix, void* out,
                                          float* parts, int tiles, int N, int R, int H, int KV, int D, int V, int Dp, int page_size,
-                                         float scale, float cap, int window, int split_keys, int splits, cudaStream_t stream) {
+                                         float scale, float cap, int window, int split_keys, int shares, cudaStream_t stream) {
     if (tiles <= 0) return 0;
-    if (H <= 0 || KV <= 0 || H % KV || Dp < D || Dp < V || splits < 1 || splits > 65535 || (splits > 1 && (!parts || split_keys % 32 || split_keys < 32)))
+    if (H <= 0 || KV <= 0 || H % KV || Dp < D || Dp < V || shares < 1 || shares > MAX_SHARES || (shares > 1 && (!parts || split_keys % 32 || split_keys < 32)))
         return LLM_ERR_BAD_ARGUMENT;
-    if (splits == 1) split_keys = 1 << 30;
+    if (shares == 1) split_keys = 1 << 30;
     if (D % 16 || V % 16 || V > 128 || D > 256 || Dp % 8 || ldq % 8 || tiles > 1 << 30) return LLM_ERR_UNSUPPORTED;
     const size_t limit = 227 * 1024 - 64;
     int bn = 32;
@@ -305,8 +302,8 @@ LLM_EXPORT int llm_sigmoid_attention_mma(const void* q, int ldq, const void* poo
     const size_t smem = smem_bytes(H, KV, D, V, bn);
     if (smem > limit) return LLM_ERR_UNSUPPORTED;
     SigMmaParams p{(const __nv_bfloat16*)q, ldq, (const __nv_bfloat16*)pool, page_table, positions, cu_tokens, table_width, bias, mix,
-                   (__nv_bfloat16*)out, parts, N, R, H, KV, D, V, Dp, page_size, window, split_keys, splits, scale, cap};
-#define LLM_SIGMMA(NV8) (bn == 32 ? launch<NV8, 32>(p, tiles, smem, stream) : launch<NV8, 16>(p, tiles, smem, stream))
+                   (__nv_bfloat16*)out, parts, N, R, H, KV, D, V, Dp, page_size, window, split_keys, scale, cap};
+#define LLM_SIGMMA(NV8) (bn == 32 ? launch<NV8, 32>(p, tiles, shares, smem, stream) : launch<NV8, 16>(p, tiles, shares, smem, stream))
     switch (V / 16) {
         case 1: return LLM_SIGMMA(2);
         case 2: return LLM_SIGMMA(4);

@@ -1766,28 +1766,30 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
     n = q.shape[0]
     out = torch.empty((n, num_heads * value_dim), dtype=q.dtype, device=q.device)
     longest = getattr(ctx, "max_context_len", None) or int(ctx.context_lens.max())
-    if window:
-        longest = min(longest, window + ctx.max_query_len)
-    def stretches(keys):  # at most 1,024 of them, of whole chunks of 32 keys
-        keys = max(keys, -(-longest // (1024 * 32)) * 32)
-        return keys, 1 if n > _SIGMOID_SPLIT_MAX_TOKENS else max(1, -(-longest // keys))
+
+    def stretches(keys):
+        """Keys of a stretch (whole chunks of 32) and how many stretches a token may see (at most 1,025): a window, which may begin
+        anywhere in a stretch, one more than it fills."""
+        keys = max(keys, -(-(min(longest, window) if window else longest) // (1024 * 32)) * 32)
+        count = min(-(-longest // keys), -(-(window - 1) // keys) + 1) if window else -(-longest // keys)
+        return keys, 1 if n > _SIGMOID_SPLIT_MAX_TOKENS else max(1, count)
 
     if q.dtype == torch.bfloat16 and not _FORCE_GENERIC_ATTENTION:
         # the tensor cores: tiles of 16 tokens of one request
         split_keys, splits = stretches(_SIGMOID_MMA_SPLIT_KEYS)
         shares = min(splits, _SIGMOID_SHARES)
-        parts = torch.empty((shares, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if splits > 1 else None
+        parts = torch.empty((shares, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if shares > 1 else None
         cu = getattr(ctx, "host_cu_tokens", None) or ctx.cu_tokens.tolist()
         tiles = sum(-(-(b - a) // 16) for a, b in zip(cu[:-1], cu[1:]))
         code = _launch(
             "llm_sigmoid_attention_mma", _ptr(q), q.stride(0), _ptr(pool), _ptr(page_table), page_table.shape[1], _ptr(ctx.positions),
             _ptr(ctx.cu_tokens), _ptr(head_bias), _ptr(head_mix), _ptr(out), _ptr(parts), tiles, n, len(cu) - 1, num_heads, num_kv_heads,
-            key_dim, value_dim, pool.shape[4], pool.shape[3], float(scale), float(softcap or 0.0), int(window or 0), split_keys, splits,
+            key_dim, value_dim, pool.shape[4], pool.shape[3], float(scale), float(softcap or 0.0), int(window or 0), split_keys, shares,
             _stream(),
         )
         if code != 10002:
             _check(code, "sigmoid_attention (tensor cores)")
-            if splits > 1:
+            if shares > 1:
                 _check(_launch("llm_sigmoid_sum_parts", _ptr(parts), _ptr(out), _code(out.dtype), _ptr(ctx.positions), n,
                                num_heads * value_dim, split_keys, int(window or 0), shares, _stream()),
                        "sigmoid_attention (sum of the stretches)")

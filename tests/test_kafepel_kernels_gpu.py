@@ -90,6 +90,32 @@ def test_prepare_and_attention_against_plain(H, KV, D, V, rot, page_size, dtype,
     close(a, plain_ops.sigmoid_attention(q2, p2, table, ctx, **common, **more)[rows], tol, "keys shared out")
 
 
+@pytest.mark.parametrize("window", [1, 32, 33, 64, 127, 128, 300, 5000])
+@pytest.mark.parametrize("dtype,general,tol", [(torch.float32, False, 2e-5), (torch.bfloat16, False, 2e-2), (torch.bfloat16, True, 2e-2)])
+@pytest.mark.parametrize("lens, news", [([1000, 37, 530, 128], [1, 1, 1, 1]), ([1000, 700, 33], [5, 16, 2]), ([1500, 64], [48, 16]), ([97, 2900], [33, 31])])
+def test_windows_far_behind_which_the_context_starts(lens, news, window, dtype, general, tol, monkeypatch):
+    """Steps of up to 64 tokens share their keys out: a window ends long after position 0, wherever stretches of 32 or 128 keys
+    begin, and no partial sum is read that nobody wrote (whatever is allocated holds NaN)."""
+    ops = _ops()
+    monkeypatch.setattr(ops, "_FORCE_GENERIC_ATTENTION", general)
+    H, KV, D, V, page_size = 6, 2, 32, 48, 16
+    torch.manual_seed(window)
+    ctx, table, _, pages = paged_batch(lens, news, page_size)
+    pool = (torch.randn(pages, 2, KV, page_size, max(D, V), device=DEV) * 0.5).to(dtype)
+    q = torch.randn(ctx.num_tokens, H * D, device=DEV).to(dtype)
+    common = dict(num_heads=H, num_kv_heads=KV, key_dim=D, value_dim=V, scale=0.2, softcap=5.0, window=window,
+                  head_bias=torch.randn(H, device=DEV), head_mix=torch.randn(H, H, device=DEV))
+    want = plain_ops.sigmoid_attention(q, pool, table, ctx, **common)
+    empty = torch.empty
+
+    def unwritten(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        return t.fill_(torch.nan) if t.is_floating_point() else t
+
+    monkeypatch.setattr(torch, "empty", unwritten)
+    close(ops.sigmoid_attention(q, pool, table, ctx, **common), want, tol, f"window {window}")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("general", [False, True])
 @pytest.mark.parametrize("news", [[600, 1, 1], [1, 1, 1], [64, 2, 1]])
