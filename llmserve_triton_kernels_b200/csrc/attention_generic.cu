@@ -72,7 +72,7 @@ __global__ void __launch_bounds__((SHARED ? CLASSES : MANY_WARPS) * 32) attentio
 #pragma unroll
         for (int i = 0; i < ACC; ++i) all[i] = 0.f;
         auto join = [&](float m, float l, const float* acc, int pitch) {
-            if (m == -INFINITY) return;  // a class without a chunk
+            if (m == -INFINITY && l == l) return;  // a class without a key that weighs anything (one of NaN scores has a sum of NaN)
             const float m_new = fmaxf(all_m, m), before = expf(all_m - m_new), share = expf(m - m_new);
             all_m = m_new;
             all_l = fmaf(l, share, all_l * before);
@@ -118,9 +118,10 @@ __global__ void __launch_bounds__((SHARED ? CLASSES : MANY_WARPS) * 32) attentio
                 if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
                 s -= slope * (float)(pos - j);
             }
-            const float m_new = fmaxf(m, warp_max(s));  // finite: the chunk holds at least one visible key
-            const float p = visible ? expf(s - m_new) : 0.f;
-            const float rescale = expf(m - m_new);  // 0 on the first chunk (m = -inf)
+            const float m_new = fmaxf(m, warp_max(s));
+            const float m_use = m_new == -INFINITY ? 0.f : m_new;  // every score so far -inf (or NaN): weights of 0 (or NaN)
+            const float p = visible ? expf(s - m_use) : 0.f;
+            const float rescale = expf(m - m_use);  // 0 on the first chunk (m = -inf)
             l = l * rescale + warp_sum(p);
 #pragma unroll
             for (int i = 0; i < ACC; ++i) acc[i] *= rescale;

@@ -263,7 +263,7 @@ attention_rows_few_kernel(const RowsArgs<bf16> a, int splits, float* __restrict_
             ml_s[(warp * ROWS + row) * 2] = m[e];
             ml_s[(warp * ROWS + row) * 2 + 1] = l[e];
         }
-        if (m[e] != -INFINITY) {
+        if (l[e] != 0.f) {  // (NaN is not 0: a row whose scores are NaN is a part like any other)
             float* to = o_s + (warp * ROWS + row) * PITCH<DVW>;
 #pragma unroll
             for (int vg = 0; vg < VG; ++vg)
@@ -281,18 +281,19 @@ attention_rows_few_kernel(const RowsArgs<bf16> a, int splits, float* __restrict_
         const int row = i / quads, d = (i - row * quads) * 4, pair = MAPS == 2 ? row & 7 : row;
         if (pair >= rows_here) continue;
         const int first = DSPLIT == 1 ? 0 : d / DVW;  // the first of the warps that hold this lane
-        float M = -INFINITY, L = 0.f, ws[KG];
+        float M = -INFINITY, L = 0.f, ws[KG], ls[KG];
 #pragma unroll
         for (int k = 0; k < KG; ++k) {
             ws[k] = ml_s[((k * DSPLIT + first) * ROWS + row) * 2];
+            ls[k] = ml_s[((k * DSPLIT + first) * ROWS + row) * 2 + 1];
             M = fmaxf(M, ws[k]);
         }
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < KG; ++k) {
-            if (ws[k] == -INFINITY) continue;  // no key for this row: nothing was written
-            const float w = exp2f(ws[k] - M);
-            L = fmaf(w, ml_s[((k * DSPLIT + first) * ROWS + row) * 2 + 1], L);
+            if (ls[k] == 0.f) continue;  // no key for this row: nothing was written
+            const float w = ws[k] == -INFINITY ? 0.f : exp2f(ws[k] - M);  // (0: a sink of -inf, or NaN, which stays NaN)
+            L = fmaf(w, ls[k], L);
             const float4 v = *reinterpret_cast<const float4*>(o_s + ((k * DSPLIT + first) * ROWS + row) * PITCH<DVW> + (d - first * DVW));
             sum.x = fmaf(w, v.x, sum.x);
             sum.y = fmaf(w, v.y, sum.y);
@@ -302,7 +303,7 @@ attention_rows_few_kernel(const RowsArgs<bf16> a, int splits, float* __restrict_
         if constexpr (LEAVE) {
             const int R = row0 + row;
             const size_t at = ((size_t)(q_begin + R / group) * a.H + kvh * group + R % group) * splits + split;
-            if (M != -INFINITY) *reinterpret_cast<float4*>(part_o + at * dv + d) = sum;  // no key in this share: the merge does not use it
+            if (L != 0.f) *reinterpret_cast<float4*>(part_o + at * dv + d) = sum;  // no key in this share: the merge does not use it
             if (d == 0) {
                 part_ml[at * 2] = M;
                 part_ml[at * 2 + 1] = L;
@@ -326,7 +327,7 @@ attention_rows_few_kernel(const RowsArgs<bf16> a, int splits, float* __restrict_
                 const float ms = lane < splits ? load_of(cta_ml + row * 2, lane) : -INFINITY;
                 const float ls = lane < splits ? load_of(cta_ml + row * 2 + 1, lane) : 0.f;
                 const float M = warp_max(ms), w = ms == -INFINITY ? 0.f : exp2f(ms - M), total = warp_sum(w * ls);
-                const float inv = total > 0.f ? 1.f / total : 0.f;
+                const float inv = total == 0.f ? 0.f : 1.f / total;
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
                 for (int s = 0; s < splits; ++s) {
@@ -395,7 +396,8 @@ int launch_few(const RowsArgs<bf16>& a, int requests, int max_query_len, int spl
 // The shapes that the kernel takes: dk and dv <= 128, or (one map) dk <= 320 with dv <= 256; whole pieces of 32 key lanes and 64 value
 // lanes (shorter ones would leave threads without work: they stay with the kernel for many rows).  `splits` CTAs share a tile's keys: a
 // cluster (1, 2, 4 or 8) that writes the result, or, with out null, up to 32 that leave part_o [n_tokens * H * splits * dv] and part_ml
-// [n_tokens * H * splits * 2]; of a share without keys for a row only part_ml (-inf, 0) is written.
+// [n_tokens * H * splits * 2]; of a share without keys for a row only part_ml (-inf, 0) is written.  A NaN score makes its row NaN: a share
+// is left out by its sum, which is then NaN, and not by its maximum, which passes NaN by.
 int launch_rows_few(const RowsArgs<__nv_bfloat16>& a, int requests, int max_query_len, int splits, float* part_o, float* part_ml, cudaStream_t stream) {
     const int dk = a.maps * a.d0 + a.d1;
     const bool small = dk <= 64 && a.dv <= 64, medium = dk <= 128 && a.dv <= 128;

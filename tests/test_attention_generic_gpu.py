@@ -49,3 +49,45 @@ def test_bits_do_not_depend_on_the_number_of_items(ops, form, dtype, monkeypatch
     whole = run(0, n)  # 2,080 items
     for first, count in ((0, 1), (33, 1), (n - 2, 2), (0, 64)):
         assert torch.equal(run(first, count), whole[first : first + count])
+
+
+@pytest.mark.parametrize("n", [1, 300])  # eight warps an item, one
+@pytest.mark.parametrize("bad", ["query", "first key", "a chunk", "the newest key"])
+def test_nan_comes_out_where_it_is_seen(ops, bad, n):  # noqa: F811
+    """NaN in the only keys of a class of chunks does not leave with the class."""
+    H, page, d, context = 8, 4, 16, 301
+    pages = 80
+    q, keys, values = rnd(n, H, d, seed=1, dtype=torch.float32), rnd(pages, 1, page, d, seed=2, dtype=torch.float32), rnd(pages, 1, page, d, seed=3, dtype=torch.float32)
+    table, ctx = rows.step((n,), (context,), page, pages, False)
+    run = lambda: ops.attention_rows(q, None, keys.data_ptr(), (page * d, page * d, d), values.data_ptr(), (page * d, page * d, d), d, table, page, ctx,  # noqa: E731
+                                     num_heads=H, num_kv_heads=1, scale=0.25)
+    clean = run()
+    seen = torch.zeros(n, H, dtype=torch.bool, device=DEV)
+    if bad == "query":
+        q[-1, 2] = torch.nan
+        seen[-1, 2] = True
+    else:
+        first, last = {"first key": (0, 1), "a chunk": (64, 96), "the newest key": (context - 1, context)}[bad]
+        for j in range(first, last):
+            keys[int(table[0, j // page]), 0, j % page] = torch.nan
+        seen[torch.arange(context - n, context, device=DEV) >= first] = True
+    got = run()
+    assert bool(got[seen].isnan().all()) and torch.equal(got[~seen], clean[~seen])
+
+
+def test_keys_that_score_minus_infinity_weigh_nothing(ops):  # noqa: F811
+    """A whole chunk of them, in the first class and in others, and more of the class behind it: as in 64 bits."""
+    H, page, d, context = 4, 4, 16, 600
+    pages = 160
+    q, keys, values = rnd(1, H, d, seed=1, dtype=torch.float32), rnd(pages, 1, page, d, seed=2, dtype=torch.float32), rnd(pages, 1, page, d, seed=3, dtype=torch.float32)
+    q[..., 0] = 1.0
+    table, ctx = rows.step((1,), (context,), page, pages, False)
+    for first in (0, 64, 320):
+        for j in range(first, first + 32):
+            keys[int(table[0, j // page]), 0, j % page, 0] = -torch.inf
+    got = ops.attention_rows(q, None, keys.data_ptr(), (page * d, page * d, d), values.data_ptr(), (page * d, page * d, d), d, table, page, ctx,
+                             num_heads=H, num_kv_heads=1, scale=0.25)
+    order = table[0].long()
+    k, v = keys[order, 0].reshape(-1, d)[:context].double(), values[order, 0].reshape(-1, d)[:context].double()
+    want = torch.softmax(q[0].double() @ k.T * 0.25, -1) @ v
+    torch.testing.assert_close(got[0].double(), want, rtol=1e-5, atol=1e-6)

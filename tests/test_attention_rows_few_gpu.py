@@ -145,3 +145,62 @@ def test_merge_and_product_of_shares_some_without_keys(ops, splits, dv, n_out, s
     merged = (share[..., None] * o.double().nan_to_num()).sum(2) / (share * ml[..., 1].double()).sum(2)[..., None]
     want = torch.einsum("nhd,hmd->nhm", merged, w.double()).flatten(1) * torch.sigmoid(gate.double())
     torch.testing.assert_close(got.double(), want, rtol=2.0**-8, atol=1e-5 * dv)
+
+
+@pytest.mark.parametrize("leave", [False, True])
+@pytest.mark.parametrize("contexts", [(40, 9), (700, 2000), (130, 1)])
+@pytest.mark.parametrize("where", ["query", "first key", "newest key", "a key in the middle", "a tile of keys"])
+def test_nan_comes_out_where_it_is_seen(ops, where, contexts, leave, monkeypatch):
+    """A row that sees a NaN score is NaN, also where a warp's keys, or a whole share's, score nothing else; every other row is as it was."""
+    H, KV, page, dk, dv = 8, 1, 16, 288 if leave else 64, 256 if leave else 64
+    pages, n = sum(-(-c // page) for c in contexts) + 1, len(contexts)
+    q, keys = rnd(n, H, dk, seed=1), rnd(pages, KV, page, dk, seed=2)
+    values, w = rnd(pages, KV, page, dv, seed=3), rnd(H, 24, dv, seed=4)
+    table, ctx = step((1,) * n, contexts, page, pages, False)
+
+    def run():
+        out = ops.attention_rows(q, None, keys.data_ptr(), (KV * page * dk, page * dk, dk), values.data_ptr(), (KV * page * dv, page * dv, dv), dv, table, page, ctx,
+                                 num_heads=H, num_kv_heads=KV, scale=dk**-0.5, leave_parts=leave)
+        if isinstance(out, ops.AttentionParts):
+            return ops.merge_project_gate(out, w, None).view(n, H, -1)
+        return ops.head_linear(out, w) if leave else out
+
+    clean = run()
+    context = contexts[0]
+    at = {"first key": (0,), "newest key": (context - 1,), "a key in the middle": (context // 2,), "a tile of keys": range(16, 32)}.get(where)
+    if at is None:
+        q[0, 3] = torch.nan
+    else:
+        for j in at:
+            keys[int(table[0, j // page]), :, j % page] = torch.nan
+    bad = torch.zeros(n, H, dtype=torch.bool, device=DEV)
+    bad[0, 3 if at is None else slice(None)] = True
+    for rows_few in (ops._ROWS_FEW, 0):  # the kernel for many rows is no other way
+        monkeypatch.setattr(ops, "_ROWS_FEW", rows_few)
+        got = run()
+        assert bool(got[bad].isnan().all()), f"{where}: NaN was lost ({'many' if rows_few == 0 else 'few'} rows)"
+        if rows_few:
+            assert torch.equal(got[~bad], clean[~bad])
+        else:
+            assert bool(got[~bad].isfinite().all())
+
+
+@pytest.mark.parametrize("maps, sinks", [(1, True), (2, False)])
+def test_nan_beside_sinks_and_in_one_of_two_maps(ops, maps, sinks):
+    H, KV, page, d, dv, contexts = 8, 2, 16, 64, 64, (300, 20)
+    dk, pages = maps * d, 25
+    q, keys, values = rnd(2, H, dk, seed=1), rnd(pages, KV, page, dk, seed=2), rnd(pages, KV, page, dv, seed=3)
+    table, ctx = step((1, 1), contexts, page, pages, False)
+    kw = dict(num_heads=H, num_kv_heads=KV, scale=0.1)
+    if sinks:
+        kw["sinks"] = torch.where(torch.arange(H, device=DEV) % 2 == 0, -torch.inf, 0.5)  # (-inf: as if there were none)
+    if maps == 2:
+        kw["differential"] = ops.DifferentialMaps(0.4, 1e-6, 0.5)
+    run = lambda: ops.attention_rows(q, None, keys.data_ptr(), (KV * page * dk, page * dk, dk), values.data_ptr(), (KV * page * dv, page * dv, dv), dv, table, page, ctx, **kw)  # noqa: E731
+    clean = run()
+    assert bool(clean.isfinite().all())
+    keys[int(table[0, 0]), 1, 2, d * (maps - 1) :] = torch.nan  # key 2 of the first request, its last map's lanes alone
+    got = run()
+    seen = torch.zeros(2, H, dtype=torch.bool, device=DEV)
+    seen[0, H // KV :] = True
+    assert bool(got[seen].isnan().all()) and torch.equal(got[~seen], clean[~seen])
