@@ -96,6 +96,13 @@ __device__ __forceinline__ void block_sums(float (&v)[K], float* scratch) {
 
 static inline int launch_status() { return (int)cudaGetLastError(); }
 
+// SMs of the current device (asked for each time: a process may have several devices)
+static inline int device_sms() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+}
+
 // Programmatic dependent launch: a kernel launched through launch_pdl may start while the kernel
 // before it on the stream is still running.  It may set itself up (indices, barriers, loads of
 // weights and of the step's descriptor arrays, which no kernel writes) but must call pdl_wait()

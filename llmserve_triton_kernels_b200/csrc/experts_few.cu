@@ -351,11 +351,7 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     p.out = out; p.resid = resid; p.norm_w = norm_w; p.xw_out = (bf16*)xw_out; p.ss_out = ss_out; p.alpha = alpha; p.error_flag = error_flag;
     const int up_slot = 16 * (K * 2 + 64);
     p.up_slots = UP_RING / up_slot < MAX_SLOTS ? UP_RING / up_slot : MAX_SLOTS;
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
-    }();
+    const int sms = device_sms();
     const cudaError_t set = cudaFuncSetAttribute(experts_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UP_RING);
     if (set != cudaSuccess) return (int)set;
     const int most = (E * ff + fs) / (kind < 0 ? 8 : 16);

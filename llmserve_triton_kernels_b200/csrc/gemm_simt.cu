@@ -257,25 +257,13 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
     if (am < M && n0 + an < N) out[(size_t)am * ldo + n0 + an] = acc;
 }
 
-int f32_sm_count() {
-    static int count = 0;
-    if (count == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || count <= 0) count = 148;
-    }
-    return count;
-}
-
 template <int RM, int RN, int TR, int TC, int STAGES>
 int launch_tile(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     constexpr size_t smem = (size_t)STAGES * (RM + RN) * (BK + 4) * sizeof(float);
     auto kernel = gemm_f32_tile_kernel<RM, RN, TR, TC, STAGES>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {  // at every launch: the limit holds for the current device, and a process may have several
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
     }
     kernel<<<dim3((N + RN - 1) / RN, (M + RM - 1) / RM), (RM / TR) * (RN / TC), smem, stream>>>(x, w, out, M, N, K, ldx, ldw, ldo);
     return launch_status();
@@ -285,11 +273,9 @@ template <int MR, int STAGES>
 int launch_few(const float* x, const float* w, float* out, int M, int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
     constexpr size_t smem = few_bytes<MR, STAGES>();
     auto kernel = gemm_f32_few_kernel<MR, STAGES>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {  // at every launch: the limit holds for the current device, and a process may have several
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
     }
     return launch_pdl(kernel, dim3((N + FEW_N - 1) / FEW_N), dim3(FEW_THREADS), smem, stream, x, w, out, M, N, K, ldx, ldw, ldo);
 }
@@ -311,9 +297,9 @@ int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, 
     struct { int rm, rn, per_sm; double rate; } const kinds[4] = {{128, 128, 1, 1.0}, {64, 128, 2, 0.92}, {64, 64, 3, 0.85}, {32, 64, 4, 0.7}};
     int best = 0;
     double best_cost = 1e30;
+    const int sms = device_sms();
     for (int i = 0; i < 4; ++i) {
         const double tiles = (double)((M + kinds[i].rm - 1) / kinds[i].rm) * ((N + kinds[i].rn - 1) / kinds[i].rn);
-        const int sms = f32_sm_count();
         // tiles of the busiest SM, which runs them up to per_sm at a time at the full rate and one alone at less
         const double most = (double)(((long long)tiles + sms - 1) / sms);
         const double alone = most < kinds[i].per_sm ? 1.0 + 0.35 * (kinds[i].per_sm - most) / kinds[i].per_sm : 1.0;

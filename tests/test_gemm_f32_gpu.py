@@ -28,3 +28,45 @@ def test_rows_have_the_same_bits_in_every_kernel(n, k):
     pitched = torch.zeros(40, k + 8, device=DEV)
     pitched[:, :k] = x[:40]
     assert torch.equal(ops.linear(pitched[:7, :k], w), want[:7]) and torch.equal(ops.linear(pitched[:, :k], w), want[:40])
+
+
+SECOND_CONTEXT = """
+import ctypes, sys
+
+lib, cu = ctypes.CDLL(sys.argv[1]), ctypes.CDLL("libcuda.so.1")
+ok = lambda code: code and sys.exit(f"driver error {code}")
+ok(cu.cuInit(0))
+for turn in range(2):  # a context stands for a device: the library's kernels are set up in each
+    context, pointers = ctypes.c_void_p(), []
+    ok(cu.cuCtxCreate_v2(ctypes.byref(context), 0, 0))
+    M, N, K = 300, 96, 256
+    for elements in (M * K, N * K, M * N):
+        p = ctypes.c_uint64()
+        ok(cu.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(4 * elements)))
+        ok(cu.cuMemsetD32_v2(p, 0x3f800000, ctypes.c_size_t(elements)))  # ones
+        pointers.append(p)
+    x, w, out = (ctypes.c_void_p(p.value) for p in pointers)
+    for m in (1, 2, 4, 8, 16, 33, M):
+        code = lib.llm_gemm_simt(x, 0, w, 0, out, 0, m, N, K, K, K, N, None)
+        if code:
+            sys.exit(f"context {turn}, {m} rows: the launch was refused with {code}")
+        ok(cu.cuCtxSynchronize())
+        row = (ctypes.c_float * N)()
+        ok(cu.cuMemcpyDtoH_v2(row, ctypes.c_uint64(out.value + 4 * (m - 1) * N), ctypes.c_size_t(4 * N)))
+        assert list(row) == [float(K)] * N, (turn, m)
+print("same in both")
+"""
+
+
+def test_a_second_device_of_the_process():
+    """What a kernel needs before its launch is set up wherever it runs, not once a process: a second CUDA context has, as a second GPU has,
+    none of what was set in the first."""
+    import subprocess
+    import sys
+
+    from llmserve_triton_kernels_b200 import ops
+
+    ops.linear(torch.ones(1, 4, device=DEV), torch.ones(1, 4, device=DEV))
+    assert ops._F32 == 0
+    done = subprocess.run([sys.executable, "-c", SECOND_CONTEXT, str(ops.loaded_library_path())], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0 and "same in both" in done.stdout, done.stdout + done.stderr
