@@ -201,16 +201,19 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
             copy16_async(st + row * FEW_ROW + (piece % (FEW_K / 4)) * 4, k < K ? src : w, k < K);
         }
     };
-    // the weights do not depend on the kernel before: the first stages of them are on their way before its end
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-        if (s < stages) fetch_rows(s, true);
+    // w may be the work of the kernel in front: its first stages are brought into L2, where what that kernel still writes is seen, before that
+    // kernel's end, and copied from there behind it
+    if (tid < FEW_N)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(w + (size_t)min(n0 + tid, N - 1) * ldw), "r"(min(K, (STAGES - 1) * FEW_K) * 4) : "memory");
     pdl_trigger();
     pdl_wait();
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < stages) fetch_rows(s, false);
-        copies_commit();  // the first group carries the weights of all the first stages: they are waited for together
+        if (s < stages) {
+            fetch_rows(s, true);
+            fetch_rows(s, false);
+        }
+        copies_commit();
     }
     float acc = 0.f;
     const int an = tid % FEW_N, am = tid / FEW_N;  // the output that this thread adds up (am < MR)

@@ -550,7 +550,8 @@ def linear(x, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Te
     """``x [M, K] @ w [N, K]^T -> [M, N]``.  float32 operands run on the CUDA cores in true 32-bit
     (fixed summation order); bfloat16 operands accumulate in 32-bit on the tensor cores: up to 16 rows
     through the weight-streaming kernel, more through the vendor's library (or, where ``_GEMM_POLICY`` says so,
-    the own tcgen05 kernel from 128 rows on).  ``x`` may be a :class:`NormedInput`."""
+    the own tcgen05 kernel from 128 rows on).  ``x`` may be a :class:`NormedInput`.  In 32 bits ``w`` may be what the kernel in
+    front writes; in bfloat16 it is a weight, which the kernels ask for before the one in front has ended."""
     if isinstance(x, NormedInput):
         if x.shape[0] >= _TCGEN05_MIN_ROWS:
             out = _tcgen05_linear(x, w, out_dtype or x.dtype, 0, w.shape[0])

@@ -70,3 +70,34 @@ def test_a_second_device_of_the_process():
     assert ops._F32 == 0
     done = subprocess.run([sys.executable, "-c", SECOND_CONTEXT, str(ops.loaded_library_path())], capture_output=True, text=True, timeout=120)
     assert done.returncode == 0 and "same in both" in done.stdout, done.stdout + done.stderr
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 7, 16, 40])
+def test_operands_that_the_kernel_in_front_writes(m):
+    """Both operands are the work of a kernel that lets the product start before it has ended, and the buffers hold others until then."""
+    from llmserve_triton_kernels_b200 import ops
+
+    n, k, turns = 4000, 1028, 20
+    g = torch.Generator(device=DEV).manual_seed(m)
+    rows = torch.randn(turns, n + 16, k, generator=g, device=DEV)
+    ones = torch.ones(k, device=DEV)
+    left = torch.randn(m, k, generator=g, device=DEV)
+    ops.linear(left, ops.rmsnorm(rows[0].clone(), ones, 1e-5)[:n])  # what a capture may not do has been done
+    wants = []
+    for t in range(turns):
+        normed = ops.rmsnorm(rows[t].clone(), ones, 1e-5)
+        torch.cuda.synchronize()
+        wants.append((ops.linear(left, normed[:n]), ops.linear(normed[:m].clone(), normed[:n])))
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    stream, normed_rows = rows[0].clone(), torch.empty(n + 16, dtype=torch.int32, device=DEV)
+    torch.arange(n + 16, out=normed_rows)
+    with torch.cuda.graph(graph):
+        normed = ops.rmsnorm(stream, ones, 1e-5, rows=normed_rows)
+        a = ops.linear(left, normed[:n])
+        normed = ops.rmsnorm(stream, ones, 1e-5, rows=normed_rows)
+        b = ops.linear(normed[:m], normed[:n])
+    for t in range(turns):
+        stream.copy_(rows[t])
+        graph.replay()
+        assert torch.equal(a, wants[t][0]) and torch.equal(b, wants[t][1]), f"turn {t}"
