@@ -13,8 +13,9 @@
 // eight columns; a thread's 16 bytes of a row hold its operands of two k-steps if the tokens' lanes are permuted alike.
 //   up    a CTA an SM, a tile of 16 rows at a time, whole rows by bulk copies into a ring of three tiles (192 KB in flight), asked for by a
 //         warp of its own; each of sixteen warps takes every sixteenth piece of 32 k, its part of x in registers.
-//   down  a CTA 16 features, its sixteen warps the pieces of 32 k of the listed blocks in turn, straight into registers, two rounds of
-//         weights and activations on their way.
+//   down  a CTA 16 features, each of its sixteen warps pieces of 32 k of the listed blocks, straight into registers, two rounds of weights
+//         and activations on their way.  Which warp has a piece depends on the piece's place in w_down alone: a token's bits are the
+//         same whatever experts the other tokens use.
 // Behind its own tiles the up kernel has the down kernel's weights brought into L2, so that memory does not stand still between the two.
 // The shared expert's tiles (and, with a table, everybody's) are on their way before the kernel in front has ended.  The up kernel
 // lets its dependent start only behind its own wait, so the down kernel may make its list, and ask for its first weights, while
@@ -252,15 +253,36 @@ __global__ void __launch_bounds__(DOWN_THREADS, 1) experts_down_kernel(const Exp
     pdl_trigger();
     list_experts(p, list, &count, nullptr);  // the router ended before the up kernel let this one start
     __syncthreads();
-    const int total = pieces_s + count * pieces_e;
+    // The warp's pieces: the neighbouring pairs (whole lines of 128 bytes) whose number among all of w_down's columns is the warp's own modulo
+    // WARPS, of the shared expert, then of the listed ones.  So the order of a token's sums does not depend on the experts of others,
+    // whose pieces in between add zeros.
+    int block = pieces_s > 0 ? -1 : 0, at = -1, end = -1;  // `at`: the next piece, one of the block that ends at `end`
+    auto enter = [&]() {  // the block's first piece of this warp, or a later block's; at = -1: none is left
+        for (; block < count; ++block) {
+            const int a0 = (block < 0 ? p.E : list[block]) * pieces_e, pair = a0 >> 1, skip = (warp - pair) & (WARPS - 1);
+            at = skip == 0 ? a0 : (pair + skip) * 2;
+            end = a0 + (block < 0 ? pieces_s : pieces_e);
+            if (at < end) return;
+        }
+        at = -1;
+    };
+    enter();
+    auto take = [&]() {
+        if (at < 0) return -1;
+        const int k = at * 32;
+        at += (at & 1) ? 2 * WARPS - 1 : 1;
+        if (at >= end) {
+            ++block;
+            enter();
+        }
+        return k;
+    };
     const bf16 *row0 = p.w_down + (size_t)(n0 + g) * ldk + q * 8, *row1 = row0 + (size_t)8 * ldk, *tokens = p.act + (size_t)g * ldk + q * 8;
-    // a warp's round: two runs of two neighbouring pieces (whole lines of 128 bytes); first k of each, or -1
-    struct Round { uint4 a[DOWN_AHEAD][2], b[DOWN_AHEAD]; int k[DOWN_AHEAD]; };
-    auto ask = [&](Round& r, int n) {
+    struct Round { uint4 a[DOWN_AHEAD][2], b[DOWN_AHEAD]; int k[DOWN_AHEAD]; };  // first k of each piece, or -1
+    auto ask = [&](Round& r) {
 #pragma unroll
         for (int u = 0; u < DOWN_AHEAD; ++u) {
-            const int i = ((n * DOWN_AHEAD / 2 + u / 2) * WARPS + warp) * 2 + (u & 1), j = i - pieces_s;
-            r.k[u] = i >= total ? -1 : i < pieces_s ? p.E * p.ff + i * 32 : list[j / pieces_e] * p.ff + (j % pieces_e) * 32;
+            r.k[u] = take();
             r.a[u][0] = r.k[u] >= 0 ? load_weight(row0 + r.k[u]) : make_uint4(0, 0, 0, 0);
             r.a[u][1] = r.k[u] >= 0 ? load_weight(row1 + r.k[u]) : make_uint4(0, 0, 0, 0);
         }
@@ -275,19 +297,18 @@ __global__ void __launch_bounds__(DOWN_THREADS, 1) experts_down_kernel(const Exp
 #pragma unroll
         for (int u = 0; u < DOWN_AHEAD; ++u) mma_piece(c4, d4, r.a[u][0], r.a[u][1], r.b[u]);
     };
-    const int rounds = (total + DOWN_AHEAD * WARPS - 1) / (DOWN_AHEAD * WARPS);
     Round r0, r1;
-    ask(r0, 0);
-    ask(r1, 1);
+    ask(r0);
+    ask(r1);
     pdl_wait();
     ask_tokens(r0);
     ask_tokens(r1);
-    for (int n = 0; n < rounds; n += 2) {  // (pieces behind the last are zeros)
+    while (r0.k[0] >= 0) {  // (pieces behind the last are zeros)
         multiply(r0);
-        ask(r0, n + 2);
+        ask(r0);
         ask_tokens(r0);
         multiply(r1);
-        ask(r1, n + 3);
+        ask(r1);
         ask_tokens(r1);
     }
     *reinterpret_cast<float4*>(red[warp][lane]) = make_float4(c4[0] + d4[0], c4[1] + d4[1], c4[2] + d4[2], c4[3] + d4[3]);

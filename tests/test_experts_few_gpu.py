@@ -86,3 +86,28 @@ def test_what_it_does_not_take_goes_the_other_way():
     assert call(2, 64, 32, 32) is not None
     for args in ((9, 64, 32, 32), (2, 48, 32, 32), (2, 2080, 32, 32), (2, 64, 24, 32), (2, 64, 32, 48), (2, 64, 32, 32, torch.float32)):
         assert call(*args) is None, args
+
+
+@pytest.mark.parametrize("K, N, E, ff, fs", [(2048, 256, 32, 704, 1408), (256, 64, 37, 96, 0), (512, 32, 8, 1568, 800)])
+@pytest.mark.parametrize("form", ["gated", "silu"])
+def test_a_row_has_its_bits_whatever_the_other_tokens_use(K, N, E, ff, fs, form):
+    """The order of a token's sums depends on its own experts: beside others that use all experts, or its own, or none of them."""
+    from llmserve_triton_kernels_b200 import ops
+
+    per = 2 if form == "gated" else 1
+    x = rnd(8, K, seed=1)
+    w_up, w_down = rnd(per * (E * ff + fs), K, seed=2, scale=K**-0.5), rnd(N, E * ff + fs, seed=3, scale=ff**-0.5)
+    kw = dict(activation="silu") if form == "silu" else dict(limit=1.5, shared_limit=1.0, slope=1.702, up_shift=1.0)
+    g = torch.Generator().manual_seed(E)
+    wts = torch.zeros(8, E + 1, device=DEV)
+    for t in range(8):
+        wts[t, torch.randperm(E, generator=g)[: min(4, E)].to(DEV)] = 0.1 + 0.2 * t
+    wts[:, E] = 1.0
+    wts = wts[:, : E + (fs > 0)].contiguous()
+    run = lambda rows, w: ops.experts_few(x[rows].contiguous(), w_up, w_down, E, ff, fs, weights=w[rows].contiguous(), **kw)  # noqa: E731
+    alone = torch.cat([run([t], wts) for t in range(8)])
+    for count in (2, 3, 5, 8):
+        assert torch.equal(run(list(range(count)), wts), alone[:count]), f"{count} tokens"
+    crowded = wts.clone()
+    crowded[1:, :E] = 0.3  # the others use every expert
+    assert torch.equal(run(list(range(8)), crowded)[0], alone[0])
