@@ -362,8 +362,9 @@ attention_rows_few_kernel(const RowsArgs<bf16> a, int splits, float* __restrict_
     }
 }
 
+// a == null: nothing is launched, and `resident` becomes the number of CTAs that the device runs at once in clusters of `splits`
 template <int KB, int DVW, int DSPLIT, int MAPS, bool LEAVE>
-int launch_few(const RowsArgs<bf16>& a, int requests, int max_query_len, int splits, float* part_o, float* part_ml, cudaStream_t stream) {
+int launch_few(const RowsArgs<bf16>* a, int requests, int max_query_len, int splits, float* part_o, float* part_ml, cudaStream_t stream, int* resident) {
     constexpr bool QSMEM = KB > 4;
     constexpr size_t smem = ((size_t)WARPS * ROWS * (PITCH<DVW> + 2) + ROWS * 2 + (LEAVE ? 0 : ROWS * DVW * DSPLIT)) * sizeof(float) +
                             (QSMEM ? (size_t)ROWS * (KB * 32 + 32) * 2 : 0);
@@ -372,10 +373,10 @@ int launch_few(const RowsArgs<bf16>& a, int requests, int max_query_len, int spl
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    const long long tiles = ((long long)max_query_len * (a.H / a.KV) + ROWS / MAPS - 1) / (ROWS / MAPS);
-    if (tiles * splits > 0x7fffffffLL || a.KV > 65535 || requests > 65535) return LLM_ERR_UNSUPPORTED;
+    const long long tiles = a ? ((long long)max_query_len * (a->H / a->KV) + ROWS / MAPS - 1) / (ROWS / MAPS) : 1;
+    if (tiles * splits > 0x7fffffffLL || requests > 65535 || (a && a->KV > 65535)) return LLM_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * splits), a.KV, requests);
+    cfg.gridDim = dim3((unsigned)(tiles * splits), a ? a->KV : 1, requests);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -388,7 +389,33 @@ int launch_few(const RowsArgs<bf16>& a, int requests, int max_query_len, int spl
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = LEAVE ? 1 : 2;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, a, splits, part_o, part_ml);
+    if (a) return (int)cudaLaunchKernelEx(&cfg, kernel, *a, splits, part_o, part_ml);
+    if (LEAVE) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(resident, kernel, THREADS, smem);
+        *resident *= device_sms();
+        return (int)e;
+    }
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(resident, kernel, &cfg);
+    *resident *= splits;
+    return (int)e;
+}
+
+int pick_few(int dk, int dv, int maps, bool leave, const RowsArgs<bf16>* a, int requests, int max_query_len, int splits, float* part_o, float* part_ml,
+             cudaStream_t stream, int* resident) {
+    const bool small = dk <= 64 && dv <= 64, medium = dk <= 128 && dv <= 128;
+    if ((dk & 31) || (dv & 63) || !(medium || (maps == 1 && dk <= 320 && dv <= 256))) return LLM_ERR_UNSUPPORTED;
+    auto go = [&](auto of) { return of(a, requests, max_query_len, splits, part_o, part_ml, stream, resident); };
+    if (leave) {
+        if (maps != 1 || splits < 1 || splits > 32) return LLM_ERR_BAD_ARGUMENT;
+        if (small) return go(launch_few<2, 64, 1, 1, true>);
+        if (medium) return go(launch_few<4, 128, 1, 1, true>);
+        return dv <= 128 ? go(launch_few<10, 64, 2, 1, true>) : go(launch_few<10, 128, 2, 1, true>);
+    }
+    if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return LLM_ERR_BAD_ARGUMENT;  // clusters of any device
+    if (maps == 2) return small ? go(launch_few<2, 64, 1, 2, false>) : go(launch_few<4, 128, 1, 2, false>);
+    if (small) return go(launch_few<2, 64, 1, 1, false>);
+    if (medium) return go(launch_few<4, 128, 1, 1, false>);
+    return dv <= 128 ? go(launch_few<10, 64, 2, 1, false>) : go(launch_few<10, 128, 2, 1, false>);
 }
 
 }  // namespace
@@ -399,23 +426,15 @@ int launch_few(const RowsArgs<bf16>& a, int requests, int max_query_len, int spl
 // [n_tokens * H * splits * 2]; of a share without keys for a row only part_ml (-inf, 0) is written.  A NaN score makes its row NaN: a share
 // is left out by its sum, which is then NaN, and not by its maximum, which passes NaN by.
 int launch_rows_few(const RowsArgs<__nv_bfloat16>& a, int requests, int max_query_len, int splits, float* part_o, float* part_ml, cudaStream_t stream) {
-    const int dk = a.maps * a.d0 + a.d1;
-    const bool small = dk <= 64 && a.dv <= 64, medium = dk <= 128 && a.dv <= 128;
-    if (a.key_part != 0 || a.stats || (dk & 31) || (a.dv & 63) || !(medium || (a.maps == 1 && dk <= 320 && a.dv <= 256))) return LLM_ERR_UNSUPPORTED;
-    if (a.out == nullptr) {
-        if (a.maps != 1 || !part_o || !part_ml || splits > 32) return LLM_ERR_BAD_ARGUMENT;
-        if (small) return launch_few<2, 64, 1, 1, true>(a, requests, max_query_len, splits, part_o, part_ml, stream);
-        if (medium) return launch_few<4, 128, 1, 1, true>(a, requests, max_query_len, splits, part_o, part_ml, stream);
-        if (a.dv <= 128) return launch_few<10, 64, 2, 1, true>(a, requests, max_query_len, splits, part_o, part_ml, stream);
-        return launch_few<10, 128, 2, 1, true>(a, requests, max_query_len, splits, part_o, part_ml, stream);
-    }
-    if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return LLM_ERR_BAD_ARGUMENT;  // clusters of any device
-    if (a.maps == 2) {
-        if (small) return launch_few<2, 64, 1, 2, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
-        return launch_few<4, 128, 1, 2, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
-    }
-    if (small) return launch_few<2, 64, 1, 1, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
-    if (medium) return launch_few<4, 128, 1, 1, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
-    if (a.dv <= 128) return launch_few<10, 64, 2, 1, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
-    return launch_few<10, 128, 2, 1, false>(a, requests, max_query_len, splits, nullptr, nullptr, stream);
+    if (a.key_part != 0 || a.stats) return LLM_ERR_UNSUPPORTED;
+    if (a.out == nullptr && (!part_o || !part_ml)) return LLM_ERR_BAD_ARGUMENT;
+    return pick_few(a.maps * a.d0 + a.d1, a.dv, a.maps, a.out == nullptr, &a, requests, max_query_len, splits, part_o, part_ml, stream, nullptr);
+}
+
+// The CTAs of that kernel that the current device runs at once, `splits` of them a cluster (leave: none; partial results are left).  Clusters
+// do not fill the device: eight large CTAs need one group of SMs with eight free ones.  Negative: an error.
+LLM_EXPORT int llm_rows_few_resident(int dk, int dv, int maps, int leave, int splits) {
+    int resident = 0;
+    const int code = pick_few(dk, dv, maps, leave != 0, nullptr, 1, 1, splits, nullptr, nullptr, nullptr, &resident);
+    return code == 0 ? resident : -code;
 }

@@ -9,6 +9,8 @@ a CUDA device, or if the library cannot be built and loaded, the first call rais
 from __future__ import annotations
 
 import ctypes
+import functools
+import math
 import os
 import threading
 
@@ -55,6 +57,7 @@ _SIGNATURES = {
     "llm_attention_rows": [_vp, _ll, _ll, _i, _vp, _ll, _ll, _i, _vp, _ll, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _i, _i,
                            _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp, _vp, _ll, _i, _i, _f,
                            _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _vp],
+    "llm_rows_few_resident": [_i, _i, _i, _i, _i],
     "llm_attention_rows_mma": [_vp, _ll, _ll, _i, _vp, _ll, _ll, _i, _vp, _ll, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _i,
                                _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp, _ll, _i, _vp, _vp, _vp, _ll, _i, _i, _f,
                                _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _i, _i, _vp],
@@ -1165,26 +1168,47 @@ def head_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 # 512: 18.4 -> 12.4 us for one request, 22.1 -> 14.1 us for 8; all of 2,048 keys, 8 requests: 73.0 -> 38.9 us.
 _ROWS_SPLIT_KEYS = 128
 
-# Requests that bring at most so many rows (tokens times the query heads that share a key head), and at most 16 tokens, take the kernel
-# that cuts the keys over warps and merges in the cluster.  Measured against the kernel for many rows and its merge, back to back in a
-# graph: 32 heads on 8 of 64 lanes, window 512 of 2,000 keys: 13.4 -> 5.6 us for one token, 18.2 -> 7.5 for 8 requests, 14.4 -> 8.0
-# for 16 tokens of one (64 rows); all of 2,000 keys, 8 requests: 38.3 -> 14.4; two maps of 64 on values of 128, 128 rows: 20.3 ->
-# 11.3.  Latents of 256 + 32 with 32 heads (with the product behind them): 20.8 -> 12.1 at 32 rows, 25.1 -> 16.0 at 128, but 31.6 ->
-# 34.9 at 512, where sixteen rows a CTA read the keys too often.
+# Requests that bring at most so many rows (tokens times the query heads that share a key head), and at most 16 tokens, may take the kernel
+# that cuts the keys over warps and merges in the cluster (:func:`_few_plan` says when they do).
 _ROWS_FEW = 128
 
 
-def _few_splits(longest: int, base: int, dk: int, dv: int, leave: bool, bytes_a_split: int) -> int:
-    """How many CTAs share the keys of a tile of 16 rows, of which there are ``base``: a pass of a CTA takes 128 keys (64 where two warps
-    share the value lanes); an SM holds two such CTAs of short keys, else one.  CTAs of one cluster: a power of two up to 8."""
-    small = dk <= 64 and dv <= 64
-    want = -(-longest // (128 if dk <= 128 and dv <= 128 else 64))
-    room = max(1, (2 if small else 1) * _sm_count() // base)
-    if leave:
-        return max(1, min(want, room, 32, _SPLIT_SCRATCH_BYTES // bytes_a_split))
-    most = min(want, room, 8)
-    return 8 if most >= 8 else 4 if most >= 4 else 2 if most >= 2 else 1
+@functools.lru_cache(maxsize=512)
+def _few_resident(device: int, dk: int, dv: int, maps: int, leave: bool, splits: int) -> int:
+    """CTAs of that kernel that run at once, ``splits`` a cluster."""
+    resident = library().llm_rows_few_resident(dk, dv, maps, int(leave), splits)
+    _check(max(0, -resident), "attention_rows (CTAs at once)")
+    return max(1, resident)
 
+
+@functools.lru_cache(maxsize=1024)
+def _few_plan(device: int, longest: int, tiles: int, dk: int, dv: int, maps: int, leave: bool, most_splits: int, many_ctas: int, many_splits: int) -> int:
+    """How many CTAs share the keys of each of ``tiles`` tiles of 16 rows (0: the kernel for many rows is faster, with ``many_splits`` for
+    each of ``many_ctas`` tiles of 64).  Both kernels' times on a B200, in microseconds, by what they were measured at:
+
+    few rows: every wave of CTAs (an SM holds one, two of short runs; clusters of eight leave 28 of 148 SMs without work) starts and
+    merges in 3.8 to 7 and takes 2.4 to 2.85 a pass of 128 keys (64 where two warps share the value lanes).
+    many rows: a wave (two CTAs an SM) 8 (12 of long runs, with the merge of shares) and 0.068 (0.08) a key, and 4 for the merge of short ones.
+
+    Several tiles a request read its keys once each, where one of 64 rows reads them once.  Measured, many -> few (kernels back to back, one
+    CTA's context throughout): 32 heads on 8 of 64 lanes, 2,000 keys: 17.3 -> 8.1 for one request, 38.4 -> 14.8 for 8, 305 -> 169 for 128;
+    128 heads on a latent of 256 + 32 (8 tiles a request): 100 keys 25.5 -> 8.6 for one request, 29.1 -> 90.5 for 128; 2,000 keys
+    36.7 -> 50.7 for 8, 197 -> 642 for 128; 64 heads on 8 of 128, 4 tokens (2 tiles): 14.3 -> 9.0 for one request of 100 keys, 152 -> 181
+    for 32 of 2,000."""
+    small, long = dk <= 64 and dv <= 64, dk > 128 or dv > 128
+    start, a_pass, keys = (3.8, 2.4, 128) if small else (7.0, 2.85, 64) if long else (5.5, 2.35, 128)
+    best, best_us = 1, math.inf
+    want = -(-longest // keys)
+    shares = [max(1, min(want, _few_resident(device, dk, dv, maps, True, 1) // tiles, 32, most_splits))] if leave else (1, 2, 4, 8)
+    for splits in shares:
+        if splits > 1 and splits > want:
+            break
+        us = -(-tiles * splits // _few_resident(device, dk, dv, maps, leave, splits)) * (start + a_pass * -(-longest // (splits * keys)))
+        if us < best_us:
+            best, best_us = splits, us
+    alone, a_key = (12.0, 0.08) if long else (8.0, 0.068)
+    many_us = -(-many_ctas * many_splits // (2 * _sm_count())) * (alone + a_key * -(-longest // many_splits)) + (4.0 if many_splits > 1 and not (leave or long) else 0.0)
+    return best if best_us <= many_us else 0
 
 
 def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, page_table, page_size: int, ctx, *, num_heads: int,
@@ -1258,10 +1282,11 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
                and ((dk <= 128 and value_dim <= 128) or (maps == 1 and dk <= 320)))
         leave = leave_parts and splits > 1
         if few:
-            splits = _few_splits(longest, -(-most * group * maps // 16) * num_kv_heads * ctx.num_requests, dk, value_dim,
-                                 leave_parts, n * num_heads * value_dim * 4)
+            shares = _few_plan(q0.device.index or 0, longest, -(-most * group * maps // 16) * num_kv_heads * ctx.num_requests, dk, value_dim, maps, leave_parts,
+                               _SPLIT_SCRATCH_BYTES // (n * num_heads * value_dim * 4), ctas, splits)
+            few = 0 if shares == 0 else 2 if getattr(ctx, "steps_apart", False) else 1
+            splits = shares or splits
             leave = leave_parts and splits > 1
-            few = 2 if getattr(ctx, "steps_apart", False) else 1
         stats = torch.empty((n, num_heads, 2), dtype=torch.float32, device=q0.device) if want_stats else None
         part_o = part_ml = None
         if splits > 1 and (leave or not few):

@@ -204,3 +204,34 @@ def test_nan_beside_sinks_and_in_one_of_two_maps(ops, maps, sinks):
     seen = torch.zeros(2, H, dtype=torch.bool, device=DEV)
     seen[0, H // KV :] = True
     assert bool(got[seen].isnan().all()) and torch.equal(got[~seen], clean[~seen])
+
+
+@pytest.mark.parametrize("form", ["plain", "a short key in two runs", "whole group", "sink and gate", "two maps", "latent", "short latent"])
+def test_every_number_of_shares(ops, form, monkeypatch):
+    """However many CTAs share a tile's keys, more than there are keys for among them: the same result up to the order of its sums."""
+    f = dict(FORMS[form])
+    d0, d1, dv, H, KV, maps, page, contexts = f["d0"], f.get("d1", 0), f["dv"], f["H"], f["KV"], f.get("maps", 1), 16, (3, 200, 1100)
+    pages, n, dk = sum(-(-c // page) for c in contexts) + 1, len(contexts), maps * d0 + d1
+    keys, values = rnd(pages, KV, page, dk, seed=1), rnd(pages, KV, page, dv, seed=2)
+    q0, q1 = rnd(n, H, maps * d0, seed=3), rnd(n, H, d1, seed=4) if d1 else None
+    kw = dict(num_heads=H, num_kv_heads=KV, scale=dk**-0.5)
+    if f.get("sinks"):
+        kw.update(sinks=rnd(H, dtype=torch.float32, seed=6), gate=rnd(n, H * dv, dtype=torch.float32, seed=7))
+    if maps == 2:
+        kw["differential"] = ops.DifferentialMaps(0.4, 1e-6, 0.5)
+    table, ctx = step((1,) * n, contexts, page, pages, False)
+    run = lambda **more: ops.attention_rows(q0, q1, keys.data_ptr(), (KV * page * dk, page * dk, dk), values.data_ptr(), (KV * page * dv, page * dv, dv), dv, table, page, ctx, **kw, **more)  # noqa: E731
+    monkeypatch.setattr(ops, "_few_plan", lambda *a: 0)
+    want = run().float()
+    for shares in (1, 2, 4, 8):
+        monkeypatch.setattr(ops, "_few_plan", lambda *a: shares)
+        got = run().float()
+        # weights rounded to bfloat16 on either side (2^-9 of the largest), results too
+        assert float((got - want).abs().max()) <= 0.02 * float(want.abs().max()), f"{shares} shares"
+    if form in ("latent", "short latent"):
+        w = rnd(H, 16, dv, seed=5)
+        want = ops.head_linear(want.bfloat16(), w).flatten(1).float()
+        for shares in (2, 3, 9, 32):
+            monkeypatch.setattr(ops, "_few_plan", lambda *a: shares)
+            got = ops.merge_project_gate(run(leave_parts=True), w, None).float()
+            assert float((got - want).abs().max()) <= 0.03 * float(want.abs().max()), f"{shares} shares left"

@@ -1,0 +1,48 @@
+"""Which of two kernels a step takes, at sizes where both were timed on a B200: the faster one."""
+
+import pytest
+
+from llmserve_triton_kernels_b200 import ops
+
+
+@pytest.fixture
+def b200(monkeypatch):
+    monkeypatch.setattr(ops, "_sm_count", lambda: 148)
+    # what the device answers: clusters of eight large CTAs leave 28 SMs without work
+    at_once = {True: {1: 296, 2: 296, 4: 284, 8: 264}, False: {1: 148, 2: 148, 4: 132, 8: 120}}
+    monkeypatch.setattr(ops, "_few_resident", lambda device, dk, dv, maps, leave, splits: at_once[dk <= 64 and dv <= 64][1 if leave else splits])
+
+
+# (query heads, key heads, key lanes, value lanes, maps, partial results left), requests, keys, tokens a request
+MANY = [((128, 1, 288, 256, 1, False), 128, 2000, 1), ((128, 1, 288, 256, 1, False), 128, 100, 1), ((128, 1, 288, 256, 1, True), 8, 2000, 1),
+        ((32, 1, 288, 256, 1, False), 8, 2000, 4), ((32, 1, 288, 256, 1, False), 32, 2000, 4), ((16, 1, 128, 128, 1, False), 32, 2000, 4),
+        ((32, 8, 128, 128, 2, False), 32, 100, 4), ((32, 8, 128, 128, 2, False), 32, 2000, 4), ((64, 8, 128, 128, 1, False), 32, 100, 4),
+        ((64, 8, 128, 128, 1, False), 32, 2000, 4), ((32, 1, 288, 256, 1, False), 8, 2000, 1),
+        ((32, 1, 288, 256, 1, False), 32, 2000, 1)]
+FEW = [((32, 8, 64, 64, 1, False), 1, 100, 1), ((32, 8, 64, 64, 1, False), 128, 2000, 1), ((32, 8, 64, 64, 1, False), 32, 100, 4), ((32, 1, 288, 256, 1, True), 8, 2000, 1),
+       ((32, 1, 288, 256, 1, False), 32, 100, 1), ((128, 1, 288, 256, 1, True), 1, 2000, 1), ((128, 1, 288, 256, 1, False), 8, 100, 1), ((16, 1, 128, 128, 1, False), 128, 2000, 1),
+       ((32, 8, 128, 128, 2, False), 128, 2000, 1), ((32, 8, 128, 128, 2, False), 8, 100, 4), ((64, 8, 128, 128, 1, False), 8, 100, 4)]
+
+
+def few_plan(shape, requests, keys, tokens):
+    heads, kv, dk, dv, maps, leave = shape
+    rows, n = tokens * heads // kv * maps, requests * tokens
+    ctas = -(-rows // 64) * kv * requests
+    many_splits = max(1, min(-(-keys // 128), (2 if dv <= 128 else 1) * 148 // ctas, 16, ops._SPLIT_SCRATCH_BYTES // (n * heads * maps * dv * 4)))
+    return ops._few_plan.__wrapped__(0, keys, -(-rows // 16) * kv * requests, dk, dv, maps, leave, ops._SPLIT_SCRATCH_BYTES // (n * heads * dv * 4), ctas, many_splits)
+
+
+@pytest.mark.parametrize("call", MANY)
+def test_attention_of_many_tiles_stays_with_the_kernel_for_many_rows(b200, call):
+    assert few_plan(*call) == 0
+
+
+@pytest.mark.parametrize("call", FEW)
+def test_attention_of_few_rows_takes_the_kernel_for_them(b200, call):
+    assert few_plan(*call) > 0
+
+
+def test_clusters_that_do_not_fit_at_once_are_not_asked_for(b200):
+    # sixteen tiles: sixteen clusters of eight take two waves, sixteen of four one
+    assert few_plan((64, 8, 128, 128, 1, False), 1, 2000, 4) == 4
+    assert few_plan((64, 8, 128, 128, 1, False), 1, 2000, 1) == 8
