@@ -1112,7 +1112,7 @@ def latent_prepare(proj: torch.Tensor, positions: torch.Tensor, slot_map: torch.
     rows = torch.empty((proj.shape[0], rank + rot), dtype=proj.dtype, device=proj.device) if fresh else None
     q_up = None
     if w_up is not None:
-        _need(not fresh and latent_prepare_takes_up(proj, dim), "latent_prepare: the up product is for few bfloat16 tokens")
+        _need(not fresh and proj.dtype == torch.bfloat16 and proj.shape[0] <= 16 and dim % 16 == 0 and 16 <= dim <= 128, "latent_prepare: the up product is for few bfloat16 tokens")
         _need(w_up.dtype == proj.dtype and w_up.is_contiguous() and tuple(w_up.shape) == (heads, rank, dim), "latent_prepare: w_up [heads, rank, dim]")
         q_up = torch.empty((proj.shape[0], heads, rank), dtype=proj.dtype, device=proj.device)
     code = _launch("llm_latent_prepare", _ptr(proj), _code(proj.dtype), proj.stride(0), _ptr(q_rot), _ptr(rows), _ptr(positions),
@@ -1126,8 +1126,11 @@ def latent_prepare(proj: torch.Tensor, positions: torch.Tensor, slot_map: torch.
 
 def latent_prepare_takes_up(proj: torch.Tensor, dim: int) -> bool:
     """Whether :func:`latent_prepare` does the key up-projection of the queries too: steps of few tokens, whose product is bound by its
-    launch (the library's batched product took 2.5 us a layer and let nothing start before its end)."""
-    return proj.is_cuda and proj.dtype == torch.bfloat16 and proj.shape[0] <= 16 and dim % 16 == 0 and 16 <= dim <= 128
+    launch (the library's batched product took 2.5 us a layer and let nothing start before its end).  A thread multiplies a row of the
+    matrix with every token's lanes on the CUDA cores, so the line lies at tokens x lanes, where both ways take the same; one
+    launch against two, in microseconds: 256 lanes in all: 4.1 / 5.8 (16 heads of 64 on a latent of 256), 6.4 / 7.0 (32 of 128 on 512);
+    512: 6.9 / 5.8, 9.2 / 7.0; 1,024: 12.4 / 5.9, 15.1 / 7.1."""
+    return proj.is_cuda and proj.dtype == torch.bfloat16 and dim % 16 == 0 and 16 <= dim <= 128 and proj.shape[0] * dim < 512 and proj.shape[0] <= 16
 
 
 def unit_norm_kv_write(qkv: torch.Tensor, slot_map: torch.Tensor, pool: torch.Tensor, eps: float | None, heads: int, kv_heads: int,

@@ -46,3 +46,12 @@ def test_clusters_that_do_not_fit_at_once_are_not_asked_for(b200):
     # sixteen tiles: sixteen clusters of eight take two waves, sixteen of four one
     assert few_plan((64, 8, 128, 128, 1, False), 1, 2000, 4) == 4
     assert few_plan((64, 8, 128, 128, 1, False), 1, 2000, 1) == 8
+
+
+@pytest.mark.parametrize("tokens, dim, one_launch", [(1, 64, True), (1, 128, True), (4, 64, True), (2, 128, True), (8, 32, True), (7, 64, True), (15, 32, True),
+                                                     (8, 64, False), (4, 128, False), (8, 128, False), (16, 32, False), (16, 64, False), (16, 128, False), (1, 8, False), (1, 256, False)])
+def test_latent_queries_are_multiplied_beside_the_preparation_while_that_is_shorter(tokens, dim, one_launch):
+    class Rows:
+        is_cuda, dtype, shape = True, ops.torch.bfloat16, (tokens, 7)
+
+    assert ops.latent_prepare_takes_up(Rows, dim) == one_launch
