@@ -1679,32 +1679,46 @@ def expert_gated_act(x: torch.Tensor, experts: int, ff: int, shared_ff: int, lim
 
 
 _EXPERTS_FEW = 8  # tokens, see experts_few
+_EXPERTS_FEW_SHARE, _EXPERTS_FEW_EACH = 0.8, 2.5e6  # see experts_few_pay
+
+
+def experts_few_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int, row_bytes: int) -> bool:
+    """Whether reading only the used experts (:func:`experts_few`) is faster than the products over all of them, for tokens that choose
+    ``top`` of ``experts`` each; ``row_bytes``: bytes of all matrices an inner feature.  Fitted to 256 steps on a B200 (16 mixtures of 8 to
+    256 experts, inner sizes 64 to 5,632, 512 to 2,048 wide, 1 to 8 tokens, cold): the products over all take 8 us and 1.28 times their
+    bytes' time at the copy rate, the used ones 8 us, 1.6 times theirs and 0.6 us an expert (2.5 MB's time).  The choice is 0.8 % off the
+    faster way on average and takes no step more than 18 % slower.  All -> used, in microseconds: 32 experts of 704, 4 used, and a shared
+    one of 1,408: one token 64.0 -> 20.6, 4 65.1 -> 45.8, 7 65.0 -> 60.3, 8 65.3 -> 67.3; 16 of 512, 8 used: 2 tokens 19.9 -> 21.4, 8
+    20.0 -> 26.4; 64 of 64, 4 used: one 14.7 -> 10.7, 4 14.6 -> 17.1."""
+    used = experts * (1.0 - (1.0 - top / experts) ** tokens)
+    return (used * ff + shared_ff) * row_bytes + used * _EXPERTS_FEW_EACH <= _EXPERTS_FEW_SHARE * (experts * ff + shared_ff) * row_bytes
 
 
 def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, ff: int, shared_ff: int, *, activation: str | None = None,
                 limit: float = 0.0, shared_limit: float = 0.0, slope: float = 1.0, up_shift: float = 0.0, weights: torch.Tensor | None = None,
-                ids: torch.Tensor | None = None, table: torch.Tensor | None = None, sink: "ResidualSink | None" = None):
+                ids: torch.Tensor | None = None, table: torch.Tensor | None = None, sink: "ResidualSink | None" = None, top: int | None = None):
     """A mixture of experts for few bfloat16 tokens, of which only the experts that one of them uses are read: the product with ``w_up``,
     the activation (``activation``: one of :func:`expert_act_scale`'s; None: the bounded gated one of :func:`expert_gated_act`) times the
     tokens' weights, and the product with ``w_down``.  Returns ``[N, hidden]`` float32, or what ``sink.linear`` returns; None for
-    a step that it does not take.  Up to 8 tokens: with 4 of 32 experts each (2,048 wide, 704 inside, a shared one of 1,408), cold and
-    with the start of a graph, the two kernels took 27 us for one token, 49 for 4 and 70 for 8, whose experts are then two thirds of all,
-    against 70 for the products over all experts and the activation between them."""
+    a step that it does not take: of more than 8 tokens or other sizes than the kernels', or, with ``top`` (how many experts a token
+    uses), one that the products over all experts are faster for (:func:`experts_few_pay`)."""
     m, k = x.shape
     n, c = w_down.shape
     if not (x.is_cuda and x.dtype == torch.bfloat16 and m <= _EXPERTS_FEW and x.stride(1) == 1 and w_up.is_contiguous() and w_down.is_contiguous()):
         return None
     gated = activation is None
+    if top is not None and not experts_few_pay(m, experts, top, ff, shared_ff, 2 * ((2 if gated else 1) * k + n)):
+        return None
     _need(w_up.dtype == w_down.dtype == x.dtype and tuple(w_up.shape) == ((2 if gated else 1) * (experts * ff + shared_ff), k) and c == experts * ff + shared_ff,
           "experts_few: the stacked matrices do not match the experts")
-    ldw = top = vocab = 0
+    ldw = listed = vocab = 0
     if weights is not None:
         _need(weights.dtype == torch.float32 and weights.stride(1) == 1 and weights.shape[0] == m and weights.shape[1] >= experts + int(shared_ff > 0), "experts_few: weights are float32 [N, experts (+ 1)]")
         ldw = weights.stride(0)
     else:
         _i32(ids, "ids")
         _need(table is not None and table.dtype == torch.int32 and table.is_contiguous() and table.dim() == 2 and ids.numel() == m, "experts_few: table is int32 [vocab, top]")
-        vocab, top = table.shape
+        vocab, listed = table.shape
     resid = norm_w = out = xw = ss = None
     alpha = 1.0
     if sink is not None and sink.resid.is_contiguous() and tuple(sink.resid.shape) == (m, n):
@@ -1718,7 +1732,7 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
     act = torch.empty((m, c), dtype=x.dtype, device=x.device)
     code = _launch("llm_experts_few", _ptr(x), x.stride(0), _ptr(w_up), _ptr(w_down), _ptr(act), m, k, n, experts, ff, shared_ff,
                    -1 if gated else _UNARY_KINDS[activation], float(limit), float(shared_limit), float(slope), float(up_shift), _ptr(weights), ldw,
-                   _ptr(ids), _ptr(table), top, vocab, _ptr(out), _ptr(resid), _ptr(norm_w), _ptr(xw), _ptr(ss), float(alpha), _error_flag_ptr(), _stream())
+                   _ptr(ids), _ptr(table), listed, vocab, _ptr(out), _ptr(resid), _ptr(norm_w), _ptr(xw), _ptr(ss), float(alpha), _error_flag_ptr(), _stream())
     if code == 10002:
         add_launches(-1)
         return None

@@ -194,7 +194,7 @@ class RoutedMLP(FeedForward):
         if self.shared_size and not self.shared_gate:
             weights = torch.cat((weights, torch.ones_like(weights[:, :1])), dim=1)
         few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, activation=self.activation,
-                              weights=weights, sink=sink)
+                              weights=weights, sink=sink, top=self.top)
         if few is not None:
             return few
         act = ops.expert_act_scale(ops.linear(xt, self.w_up), weights, self.experts, self.expert_size, self.activation)
@@ -261,7 +261,8 @@ class TableRoutedMLP(FeedForward):
     def forward(self, x, ctx, sink=None):
         xt = x.materialize() if isinstance(x, ops.NormedInput) else x
         few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, limit=self.limit,
-                              shared_limit=self.shared_limit, slope=self.slope, up_shift=1.0, ids=ctx.token_ids, table=self.table, sink=sink)
+                              shared_limit=self.shared_limit, slope=self.slope, up_shift=1.0, ids=ctx.token_ids, table=self.table, sink=sink,
+                              top=self.top)
         if few is not None:
             return few
         act = ops.expert_gated_act(ops.linear(xt, self.w_up), self.experts, self.expert_size, self.shared_size, self.limit,
@@ -353,7 +354,8 @@ class RoutedGatedMLP(FeedForward):
         weights = ops.route(xt, self.w_router, self.correction, self.experts, self.top, self.router_scale, True, False, bias=self.b_router,
                             shared_one=self.shared_size > 0, scores=self.scores, groups=self.groups)
         few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, limit=self.limit,
-                              shared_limit=self.shared_limit, slope=self.slope, up_shift=self.up_shift, weights=weights, sink=sink)
+                              shared_limit=self.shared_limit, slope=self.slope, up_shift=self.up_shift, weights=weights, sink=sink,
+                              top=self.top)
         if few is not None:
             return few
         act = ops.expert_gated_act(ops.linear(xt, self.w_up), self.experts, self.expert_size, self.shared_size, self.limit, self.shared_limit,

@@ -55,3 +55,15 @@ def test_latent_queries_are_multiplied_beside_the_preparation_while_that_is_shor
         is_cuda, dtype, shape = True, ops.torch.bfloat16, (tokens, 7)
 
     assert ops.latent_prepare_takes_up(Rows, dim) == one_launch
+
+
+# hidden, experts, top, inner size, shared inner size, matrices an expert, tokens
+@pytest.mark.parametrize("used_alone, sizes", [
+    (True, (2048, 32, 4, 704, 1408, 3, 1)), (True, (2048, 32, 4, 704, 1408, 3, 4)), (True, (1024, 16, 2, 512, 1024, 2, 1)), (True, (1024, 16, 2, 512, 1024, 3, 3)),
+    (True, (2048, 256, 8, 256, 512, 3, 8)), (True, (2048, 8, 2, 5632, 0, 3, 2)), (True, (2048, 64, 8, 352, 704, 3, 5)),
+    (False, (1024, 16, 8, 512, 0, 3, 2)), (False, (1024, 16, 8, 512, 0, 3, 8)), (False, (512, 8, 2, 128, 0, 3, 1)), (False, (1024, 64, 4, 64, 256, 3, 4)),
+    (False, (2048, 16, 4, 704, 0, 3, 6)), (False, (2048, 8, 2, 1408, 0, 3, 8)), (False, (2048, 8, 2, 5632, 0, 3, 5)), (False, (64, 4, 2, 32, 0, 2, 1)),
+])
+def test_the_used_experts_are_read_alone_where_that_is_faster(used_alone, sizes):
+    hidden, experts, top, ff, shared, matrices, tokens = sizes
+    assert ops.experts_few_pay(tokens, experts, top, ff, shared, 2 * matrices * hidden) == used_alone

@@ -111,3 +111,41 @@ def test_a_row_has_its_bits_whatever_the_other_tokens_use(K, N, E, ff, fs, form)
     crowded = wts.clone()
     crowded[1:, :E] = 0.3  # the others use every expert
     assert torch.equal(run(list(range(8)), crowded)[0], alone[0])
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 5, 8])
+@pytest.mark.parametrize("kind", ["routed", "gated", "table"])
+@pytest.mark.parametrize("sunk", [False, True])
+def test_parts_give_the_same_either_way(kind, tokens, sunk, monkeypatch):
+    """A part whose used experts are read alone beside itself with the products over all experts."""
+    from types import SimpleNamespace
+
+    from llmserve_triton_kernels_b200 import ops
+    from llmserve_triton_kernels_b200.parts.feed_forward import RoutedGatedMLP, RoutedMLP, TableRoutedMLP
+
+    K, E, top, ff, fs = 1024, 32, 2, 512, 256
+    part = {"routed": lambda: RoutedMLP(K, E, top, ff, shared_size=fs, correction=False), "gated": lambda: RoutedGatedMLP(K, E, top, ff, fs),
+            "table": lambda: TableRoutedMLP(K, 64, E, top, ff, 7.0, fs)}[kind]()
+    tensors = {name: rnd(*spec.shape, seed=i, scale=0.05) for i, (name, spec) in enumerate(part.tensors().items())}
+    if kind == "table":
+        tensors["table"] = torch.rand(64, E, generator=torch.Generator().manual_seed(1)).argsort(1)[:, :top].to(DEV)
+    part.bind(tensors, torch.bfloat16, DEV)
+    x, ctx = rnd(tokens, K, seed=99), SimpleNamespace(token_ids=torch.arange(tokens, dtype=torch.int32, device=DEV) * 5)
+    launches, launch = [], ops._launch
+    monkeypatch.setattr(ops, "_launch", lambda name, *args: launches.append(name) or launch(name, *args))
+
+    def run():
+        launches.clear()
+        stream = rnd(tokens, K, dtype=torch.float32, seed=5)
+        out = part.forward(x, ctx, ops.ResidualSink(stream, None, 1e-5) if sunk else None)
+        return stream if sunk else out
+
+    monkeypatch.setattr(ops, "_EXPERTS_FEW_SHARE", 10.0)
+    got = run()
+    assert "llm_experts_few" in launches
+    monkeypatch.setattr(ops, "_EXPERTS_FEW_SHARE", 0.0)
+    want = run()
+    assert "llm_experts_few" not in launches
+    # inner activations rounded to bfloat16 on the one side before, on the other behind the product's rounding: 2^-8 of each
+    scale = float((want - (rnd(tokens, K, dtype=torch.float32, seed=5) if sunk else 0)).norm())
+    assert float((got - want).norm()) <= 8e-3 * scale
