@@ -1679,15 +1679,15 @@ def expert_gated_act(x: torch.Tensor, experts: int, ff: int, shared_ff: int, lim
 
 
 _EXPERTS_FEW = 8  # tokens, see experts_few
-_EXPERTS_FEW_SHARE, _EXPERTS_FEW_EACH = 0.8, 2.5e6  # see experts_few_pay
+_EXPERTS_FEW_SHARE, _EXPERTS_FEW_EACH = 0.78, 2.5e6  # see experts_few_pay
 
 
 def experts_few_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int, row_bytes: int) -> bool:
     """Whether reading only the used experts (:func:`experts_few`) is faster than the products over all of them, for tokens that choose
     ``top`` of ``experts`` each; ``row_bytes``: bytes of all matrices an inner feature.  Fitted to 256 steps on a B200 (16 mixtures of 8 to
-    256 experts, inner sizes 64 to 5,632, 512 to 2,048 wide, 1 to 8 tokens, cold): the products over all take 8 us and 1.28 times their
+    256 experts, inner sizes 64 to 5,632, 512 to 2,048 wide, 1 to 8 tokens, cold): the products over all take 8 us and 1.25 times their
     bytes' time at the copy rate, the used ones 8 us, 1.6 times theirs and 0.6 us an expert (2.5 MB's time).  The choice is 0.8 % off the
-    faster way on average and takes no step more than 18 % slower.  All -> used, in microseconds: 32 experts of 704, 4 used, and a shared
+    faster way on average and takes no step more than 16 % slower.  All -> used, in microseconds: 32 experts of 704, 4 used, and a shared
     one of 1,408: one token 64.0 -> 20.6, 4 65.1 -> 45.8, 7 65.0 -> 60.3, 8 65.3 -> 67.3; 16 of 512, 8 used: 2 tokens 19.9 -> 21.4, 8
     20.0 -> 26.4; 64 of 64, 4 used: one 14.7 -> 10.7, 4 14.6 -> 17.1."""
     used = experts * (1.0 - (1.0 - top / experts) ** tokens)
