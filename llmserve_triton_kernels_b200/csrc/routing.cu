@@ -95,7 +95,10 @@ __device__ __forceinline__ void route_row(const float* zr, const float* __restri
 }
 
 // The same for at most 32 experts, a lane each and everything in registers: a choice is a reduction of the scores as ordered integers and a
-// ballot (lowest index among equals) instead of ten shuffles through shared memory.  The same bits.
+// ballot (lowest index among equals) instead of ten shuffles through shared memory.  The same bits.  It starts up to 0.5 us later and each
+// choice is 0.2 us shorter, more with many experts: 4 of 32 experts 5.9 -> 4.3 us a launch, 2 of 32 5.0 -> 4.1, 2 of 8 4.0 -> 4.2.
+__host__ __device__ inline bool choice_in_registers(int E, int top, int groups) { return E <= 32 && (E > 16 || top >= 4 || groups > 0); }
+
 __device__ __forceinline__ void route_row_32(const float* zr, const float* __restrict__ correction, float* wr, int E, int top, float scale, int renorm,
                                              int shared_gate, int lane, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
     const unsigned all = 0xffffffffu;
@@ -161,8 +164,9 @@ route_topk_kernel(const float* __restrict__ z, int ldz, const float* __restrict_
 // The router's product and the choice in one kernel.  x: [N, K] (any type, read as 32-bit); wr: [E (+ 1), K] float32 (the last
 // row, if there is a shared gate, is the gate's); a CTA takes TT tokens (1, 2 or 8): a warp sums up the logits of four rows at a time for all of
 // them (a lane its share of the elements, then the lanes' sums: the same order whatever else is in the step), then a warp per token
-// chooses.
-template <typename TX, int TT>
+// chooses.  SMALL: the choice in registers (-1: asked at run time; one or two tokens a CTA have kernels of their own, because the
+// choice in registers beside the other costs the latter 0.4 us, eight have not, whose sums it costs 2 of 11 us to be compiled alone).
+template <typename TX, int TT, int SMALL>
 __global__ void __launch_bounds__(512)
 router_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
               int N, int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
@@ -230,21 +234,23 @@ router_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, c
     }
     __syncthreads();
     if (warp < TT && t0 + warp < N) {
-        if (E <= 32) {
+        if (SMALL == 1 || (SMALL < 0 && choice_in_registers(E, top, groups))) {
             route_row_32(z + warp * rows, correction, out + (size_t)(t0 + warp) * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
-            return;
+        } else {
+            float* s = sm + (size_t)TT * rows + (size_t)warp * (2 * E + groups);
+            route_row(z + warp * rows, correction, out + (size_t)(t0 + warp) * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups,
+                      keep, s + 2 * E);
         }
-        float* s = sm + (size_t)TT * rows + (size_t)warp * (2 * E + groups);
-        route_row(z + warp * rows, correction, out + (size_t)(t0 + warp) * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups,
-                  keep, s + 2 * E);
     }
 }
 
-// The same for steps of few tokens: one CTA a token, a warp a row of the router matrix at a time.  The matrix is on its way before the
-// kernel in front has ended (the weights depend on nothing): a warp's first 1,024 lanes in registers, the rest of its rows in shared
-// memory, a lane's own elements.  Behind the wait stands one load of the token, a row's sums and the choice: 32 rows of 2,048 took 7.5 us
-// of a decode step with the second half of a row behind the wait and the choice in shared memory, and take 4.7.  The sums
-// have the order of the kernel above.
+// The same for steps of few tokens, one CTA a token, in two forms whose sums have the order of the kernel above.
+//
+// Where registers and shared memory hold the matrix, all of it is on its way before the kernel in front has ended (the weights depend on
+// nothing): `warps` warps take a row at a time, a warp's first 1,024 lanes in registers, the rest of its rows in shared memory, a
+// lane's own elements.  Behind the wait stands one load of the token (by warps enough that each thread loads once), a row's sums and
+// the choice: 32 rows of 2,048 took 7.5 us of a decode step with the second half of a row behind the wait and the choice in shared
+// memory, and take 4.7.
 constexpr int ROUTER_AHEAD = 8, ROUTER_STEP = ROUTER_AHEAD * 128;  // 16-byte pieces of a row that a lane has in registers; elements
 
 __host__ __device__ inline int router_steps_before(int warp, int rows, int warps, int per_row) {  // steps of the warps in front, less their first
@@ -252,32 +258,35 @@ __host__ __device__ inline int router_steps_before(int warp, int rows, int warps
     return warp * (each * per_row - 1) + (warp < more ? warp : more) * per_row;
 }
 
-// STAGED: registers and shared memory hold the matrix; else what is behind a warp's first step is read where it is used.
-template <typename TX, bool STAGED>
+template <typename TX, bool SMALL>
 __global__ void __launch_bounds__(1024)
-router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
-                  int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
+router_staged_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
+                     int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep,
+                     int warps) {
     extern __shared__ __align__(16) float sm[];  // the steps behind a warp's first [ROUTER_STEP each], x[K], z[rows], s[E], c[E], scores of runs
     pdl_trigger();
     const int rows = E + (shared_gate == 1), out_w = E + (shared_gate != 0), t = blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
-    float* ahead = sm + (size_t)router_steps_before(warp, rows, warps, per_row) * ROUTER_STEP;
-    float* x_s = sm + (STAGED ? (size_t)(rows * per_row - warps) * ROUTER_STEP : 0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
+    const bool works = warp < warps;  // (the others only load the token)
+    float* ahead = sm + (works ? (size_t)router_steps_before(warp, rows, warps, per_row) * ROUTER_STEP : 0);
+    float* x_s = sm + (size_t)(rows * per_row - warps) * ROUTER_STEP;
     float* z_s = x_s + K;
     float4 w[ROUTER_AHEAD];
+    if (works) {
 #pragma unroll
-    for (int i = 0; i < ROUTER_AHEAD; ++i) {
-        const int k = (i * 32 + lane) * 4;
-        w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)warp * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < ROUTER_AHEAD; ++i) {
+            const int k = (i * 32 + lane) * 4;
+            w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)warp * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int e = warp, n = 0; e < rows; e += warps)
+            for (int step = e == warp ? 1 : 0; step < per_row; ++step, ++n)
+                for (int i = 0; i < ROUTER_AHEAD; ++i) {
+                    const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
+                    if (k < K)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(ahead + n * ROUTER_STEP + (i * 32 + lane) * 4)),
+                                     "l"(wr + (size_t)e * K + k));
+                }
     }
-    for (int e = warp, n = 0; STAGED && e < rows; e += warps)
-        for (int step = e == warp ? 1 : 0; step < per_row; ++step, ++n)
-            for (int i = 0; i < ROUTER_AHEAD; ++i) {
-                const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
-                if (k < K)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(ahead + n * ROUTER_STEP + (i * 32 + lane) * 4)),
-                                 "l"(wr + (size_t)e * K + k));
-            }
     asm volatile("cp.async.commit_group;\n" ::);
     pdl_wait();
     for (int k = threadIdx.x * 4; k < K; k += blockDim.x * 4) {
@@ -287,21 +296,15 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    for (int e = warp, n = 0; e < rows; e += warps) {
+    for (int e = works ? warp : rows, n = 0; e < rows; e += warps) {
         float acc = 0.f;
         for (int step = 0; step < per_row; ++step) {
             const bool first = e == warp && step == 0;
-            if (!STAGED && !first)
-#pragma unroll
-                for (int i = 0; i < ROUTER_AHEAD; ++i) {
-                    const int k = step * ROUTER_STEP + (i * 32 + lane) * 4;
-                    w[i] = k < K ? *reinterpret_cast<const float4*>(wr + (size_t)e * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
 #pragma unroll
             for (int i = 0; i < ROUTER_AHEAD; ++i) {
                 const int at = (i * 32 + lane) * 4, k = step * ROUTER_STEP + at;
                 if (k >= K) continue;
-                const float4 wv = !STAGED || first ? w[i] : *reinterpret_cast<const float4*>(ahead + n * ROUTER_STEP + at);
+                const float4 wv = first ? w[i] : *reinterpret_cast<const float4*>(ahead + n * ROUTER_STEP + at);
                 float xv[4];
                 load4(x_s + k, xv);
                 acc = fmaf(wv.x, xv[0], acc);
@@ -316,12 +319,62 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
     }
     __syncthreads();
     if (warp == 0) {
-        if (E <= 32) {
-            route_row_32(z_s, correction, out + (size_t)t * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
-        } else {
-            float* s = z_s + rows;
-            route_row(z_s, correction, out + (size_t)t * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep, s + 2 * E);
+        float* s = z_s + rows;
+        if constexpr (SMALL) route_row_32(z_s, correction, out + (size_t)t * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
+        else route_row(z_s, correction, out + (size_t)t * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep, s + 2 * E);
+    }
+}
+
+// Elsewhere only a warp's first row's first step is; what is behind it is read where it is used, and the token by each warp for itself.
+template <typename TX, bool SMALL>
+__global__ void __launch_bounds__(1024)
+router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ correction, float* __restrict__ out,
+                  int K, int E, int top, float scale, int renorm, int shared_gate, const float* __restrict__ bias, int sigmoid, int groups, int keep) {
+    constexpr int AHEAD = ROUTER_AHEAD;
+    extern __shared__ float sm[];  // z[rows], s[E], c[E], and the scores of runs
+    pdl_trigger();
+    const int rows = E + (shared_gate == 1), out_w = E + (shared_gate != 0), t = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const TX* xr = x + (size_t)t * ldx;
+    float4 w[AHEAD];
+    auto ask = [&](int e, int k0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int k = k0 + (i * 32 + lane) * 4;
+            w[i] = e < rows && k < K ? *reinterpret_cast<const float4*>(wr + (size_t)e * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+    };
+    ask(warp, 0);
+    bool waited = false;
+    for (int e = warp; e < rows; e += warps) {
+        float acc = 0.f;
+        for (int k0 = 0; k0 < K; k0 += AHEAD * 128) {
+            if (!waited) pdl_wait();
+            else ask(e, k0);
+            waited = true;
+            float xv[AHEAD][4];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                const int k = k0 + (i * 32 + lane) * 4;
+                xv[i][0] = xv[i][1] = xv[i][2] = xv[i][3] = 0.f;
+                if (k < K) load4(xr + k, xv[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                acc = fmaf(w[i].x, xv[i][0], acc);
+                acc = fmaf(w[i].y, xv[i][1], acc);
+                acc = fmaf(w[i].z, xv[i][2], acc);
+                acc = fmaf(w[i].w, xv[i][3], acc);
+            }
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) sm[e] = acc;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float* s = sm + rows;
+        if constexpr (SMALL) route_row_32(sm, correction, out + (size_t)t * out_w, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep);
+        else route_row(sm, correction, out + (size_t)t * out_w, s, s + E, E, top, scale, renorm, shared_gate, lane, bias, sigmoid, groups, keep, s + 2 * E);
     }
 }
 
@@ -630,21 +683,25 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
     const size_t align = x_dtype == LLM_F32 ? 16 : 8;
     if (N <= 32 && K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)wr % 16 == 0 && (uintptr_t)x % align == 0) {
         const int warps = rows_all < 32 ? rows_all : 32, per_row = (K + ROUTER_STEP - 1) / ROUTER_STEP;
-        const size_t rest = ((size_t)K + rows_all + 2 * E + groups) * sizeof(float), matrix = (size_t)(rows_all * per_row - warps) * ROUTER_STEP * sizeof(float);
-        const bool staged = matrix + rest <= 200 * 1024;  // 33 rows of 2,048: 148 KB
-        const size_t few = staged ? matrix + rest : rest;
-        auto go = [&](auto kernel, auto* xp) -> int {
-            if (few > 48 * 1024) {
-                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
+        const size_t rest = ((size_t)rows_all + 2 * E + groups) * sizeof(float);
+        const size_t staged = (size_t)(rows_all * per_row - warps) * ROUTER_STEP * sizeof(float) + (size_t)K * sizeof(float) + rest;
+        const int loads = (K / 4 + 31) / 32;  // warps of which a thread loads four elements of the token
+        const dim3 threads(32 * (loads > 32 ? 32 : loads > warps ? loads : warps));
+        auto go = [&](auto* xp, auto small) -> int {
+            constexpr bool SMALL = decltype(small)::value;
+            using TX = std::remove_const_t<std::remove_pointer_t<decltype(xp)>>;
+            if (staged > 200 * 1024 || rows_all < 4)  // (33 rows of 2,048 need 148 KB; of two or three rows the registers hold enough)
+                return launch_pdl(router_few_kernel<TX, SMALL>, dim3(N), dim3(32 * warps), rest, stream, xp, ldx, wr, correction, out, K, E, top, scale, renorm,
+                                  shared_gate, bias, sigmoid, groups, keep);
+            if (staged > 48 * 1024) {
+                const cudaError_t e = cudaFuncSetAttribute(router_staged_kernel<TX, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged);
                 if (e != cudaSuccess) return (int)e;
             }
-            return launch_pdl(kernel, dim3(N), dim3(32 * warps), few, stream, xp, ldx, wr, correction, out, K, E, top, scale, renorm, shared_gate, bias, sigmoid,
-                              groups, keep);
+            return launch_pdl(router_staged_kernel<TX, SMALL>, dim3(N), threads, staged, stream, xp, ldx, wr, correction, out, K, E, top, scale, renorm, shared_gate,
+                              bias, sigmoid, groups, keep, warps);
         };
-        if (few <= 200 * 1024) {
-            if (x_dtype == LLM_F32) return staged ? go(router_few_kernel<float, true>, (const float*)x) : go(router_few_kernel<float, false>, (const float*)x);
-            return staged ? go(router_few_kernel<bf, true>, (const bf*)x) : go(router_few_kernel<bf, false>, (const bf*)x);
-        }
+        auto pick = [&](auto* xp) { return choice_in_registers(E, top, groups) ? go(xp, std::true_type{}) : go(xp, std::false_type{}); };
+        return x_dtype == LLM_F32 ? pick((const float*)x) : pick((const bf*)x);
     }
     // tokens a CTA: one for steps of few tokens (more CTAs, more loads in flight a warp), two otherwise (three CTAs an SM), eight where
     // that leaves CTAs enough (the matrix passes through a CTA once for all of its tokens)
@@ -661,7 +718,9 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
     };
     auto pick = [&](auto* xp) -> int {
         using T = std::remove_const_t<std::remove_pointer_t<decltype(xp)>>;
-        return TT == 1 ? go(router_kernel<T, 1>, xp) : TT == 2 ? go(router_kernel<T, 2>, xp) : go(router_kernel<T, 8>, xp);
+        if (TT == 8) return go(router_kernel<T, 8, -1>, xp);
+        if (choice_in_registers(E, top, groups)) return TT == 1 ? go(router_kernel<T, 1, 1>, xp) : go(router_kernel<T, 2, 1>, xp);
+        return TT == 1 ? go(router_kernel<T, 1, 0>, xp) : go(router_kernel<T, 2, 0>, xp);
     };
     return x_dtype == LLM_F32 ? pick((const float*)x) : pick((const bf*)x);
 }
