@@ -84,10 +84,7 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
     const int tile_first = p.window > 0 ? max(0, pos0 - p.window + 1) : 0, last = pos0 + rows - 1, shares = gridDim.z;
     const int stretch0 = tile_first / p.split_keys, mine = stretch0 + (split + shares - stretch0 % shares) % shares;
     const int j_begin = max(mine * p.split_keys, tile_first / BN * BN);
-    auto next = [&](int j) {
-        j += BN;
-        return j % p.split_keys ? j : j + (shares - 1) * p.split_keys;
-    };
+    int left = (mine + 1) * p.split_keys - j_begin;  // keys of the stretch from the tile at hand on
     if (j_begin > last) return;  // the sum reads only the partial sums of CTAs that had keys
     pdl_wait();
     // the tile's queries, every head: 16 bytes a thread and turn; rows beyond the request's tokens are zeros
@@ -138,7 +135,12 @@ sigmoid_attention_mma_kernel(const SigMmaParams p) {
     load_values(j_begin);
     cp_async_commit();
     for (int j0 = j_begin; j0 <= last;) {
-        const int j_next = next(j0);
+        int j_next = j0 + BN;
+        left -= BN;
+        if (left == 0) {
+            j_next += (shares - 1) * p.split_keys;
+            left = p.split_keys;
+        }
         cp_async_wait<0>();
         __syncthreads();  // (A) this tile's keys and values have landed; everybody is done with the tile before
         // ---- 1. scores and weights of every head

@@ -1749,10 +1749,12 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
 # side (csrc/sigmoid_attention.cu, retention.cu, routing.cu).
 _SIGMOID_SPLIT_KEYS = 128  # a stretch of keys that one CTA sums up when a context is shared out
 # The same for the tensor-core kernel, whose tile is 32 keys: stretches of one tile put 600 keys on all sixteen shares, of 128 on five
-# (31.0 -> 20.8 us a layer of a decode step of four requests).
+# (31.0 -> 20.8 us a layer of a decode step of four requests).  As many shares as the SMs have room for, one CTA each: with sixteen
+# whatever the step, 64 requests (32 heads) took 50 us at 100 keys and 195 at 600, and take 30 and 122; at 6,000 keys, where two shares of
+# 64 tiles leave 20 of 148 SMs without work, sixteen were 4 % faster (12 % with 24 heads on 24), which the short contexts outweigh.
 _SIGMOID_MMA_SPLIT_KEYS = 32
 _SIGMOID_SPLIT_MAX_TOKENS = 64  # steps of more tokens have CTAs enough without cutting the keys
-_SIGMOID_SHARES = 16  # the tensor-core kernel's CTAs per tile of tokens: stretch s of the keys goes to share s % 16
+_SIGMOID_SHARES = 16  # the tensor-core kernel's most CTAs per tile of tokens: stretch s of the keys goes to share s % shares
 
 
 def qk_prepare(proj: torch.Tensor, positions: torch.Tensor | None, *, heads: int, kv_heads: int, dim: int, value_dim: int = 0,
@@ -1820,10 +1822,11 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
     if q.dtype == torch.bfloat16 and not _FORCE_GENERIC_ATTENTION:
         # the tensor cores: tiles of 16 tokens of one request
         split_keys, splits = stretches(_SIGMOID_MMA_SPLIT_KEYS)
-        shares = min(splits, _SIGMOID_SHARES)
-        parts = torch.empty((shares, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if shares > 1 else None
         cu = getattr(ctx, "host_cu_tokens", None) or ctx.cu_tokens.tolist()
         tiles = sum(-(-(b - a) // 16) for a, b in zip(cu[:-1], cu[1:]))
+        # (by the step's tiles alone, so that a token's order of sums does not follow from how long the others' contexts are)
+        shares = min(splits, _SIGMOID_SHARES, max(1, _sm_count() // max(1, tiles * -(-num_heads // 16))))
+        parts = torch.empty((shares, n, num_heads * value_dim), dtype=torch.float32, device=q.device) if shares > 1 else None
         code = _launch(
             "llm_sigmoid_attention_mma", _ptr(q), q.stride(0), _ptr(pool), _ptr(page_table), page_table.shape[1], _ptr(ctx.positions),
             _ptr(ctx.cu_tokens), _ptr(head_bias), _ptr(head_mix), _ptr(out), _ptr(parts), tiles, n, len(cu) - 1, num_heads, num_kv_heads,
