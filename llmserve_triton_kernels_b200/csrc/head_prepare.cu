@@ -271,7 +271,7 @@ LLM_EXPORT int llm_head_prepare(const void* proj, int in_dtype, int ldp, const f
         ((D | (rot / 2) | (Hk > 0 ? v_lanes | Dp : 0) | ldp | ldq) & 3) == 0 && aligned(proj) && aligned(bias) && aligned(q_out) && aligned(pool) &&
         aligned(qw) && aligned(kw)) {
         const int items = (Hq + Hk) * (D / 4 - rot / 8) + (Hk / maps) * (v_lanes / 4);
-        int shares = (2 * 148 + N - 1) / N, most = (items + 255) / 256;
+        int shares = (2 * device_sms() + N - 1) / N, most = (items + 255) / 256;
         if (shares > most) shares = most;
         const size_t wide_smem = (size_t)(rot / 2 + (v_freq ? V / 2 : 0) + 1) * sizeof(float2);
         auto wide = [&](auto kernel, auto* qo) {
@@ -285,7 +285,7 @@ LLM_EXPORT int llm_head_prepare(const void* proj, int in_dtype, int ldp, const f
     const size_t smem = ((size_t)WARPS * D + 1) * sizeof(float) + (size_t)(rot / 2 + 1 + (v_freq ? V / 2 : 0)) * sizeof(float2);
     auto go = [&](auto kernel, auto* in, auto* qo) {
         using TK = std::remove_pointer_t<decltype(qo)>;
-        const int rounds = (Hq + Hk + WARPS - 1) / WARPS, room = 2 * 148 / N;
+        const int rounds = (Hq + Hk + WARPS - 1) / WARPS, room = 2 * device_sms() / N;
         return launch_pdl(kernel, dim3(N, rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room)), dim3(WARPS * 32), smem, stream, in, ldp, bias, qo, ldq, (TK*)pool, slot_map, page_size, Dp, qw, kw,
                           eps, normed, freq, rot, positions, warm_coef, warm_every, Hq, Hk, D, V, values_are_keys, interleaved, v_keep, v_first, v_lambda, maps, v_freq,
                           (float2*)turn_out);

@@ -93,7 +93,9 @@ hyper_mix_norm_kernel(float* __restrict__ X, const Results res, const float* __r
 // The same where rows are 16-byte aligned multiples of four lanes, at most 4,096 of them: a thread has four neighbouring lanes of every copy
 // and result in flight at once, the read-in stays in registers up to the norm.  A CTA of W / 4 threads a row: bound by memory for
 // prompts (1,801 rows of 2,048 in four copies: 70 -> 27.4 us), by one load's latency for decoded tokens (12.5 -> 3.7 us a launch;
-// a loop of single lanes showed eight, one after the other).
+// a loop of single lanes showed eight, one after the other).  Five to eight copies spill a few registers (64 a thread at 1,024 threads)
+// and are faster all the same: eight of 4,096 lanes 106 -> 75 us for 1,024 rows, 16.6 -> 9.1 for one; of 1,024 lanes 22.9 -> 17.6 and
+// 5.4 -> 5.3.
 template <int S, typename TO>
 __global__ void __launch_bounds__(1024)
 hyper_mix_norm_wide_kernel(float* __restrict__ X, const Results res, const float* __restrict__ mix, const float* __restrict__ take,

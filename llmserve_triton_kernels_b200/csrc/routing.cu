@@ -729,7 +729,7 @@ LLM_EXPORT int llm_router(const void* x, int x_dtype, int ldx, const float* wr, 
 // them, four times 16 bytes a thread in flight (a CTA a run of 16 bytes a thread ended as soon as it had started: 1,801 tokens of a gated mixture 48.8 -> 41.0 us, 1,686 of a plain one 25.4 -> 18.7)
 static int activation_blocks(int blocks, int tokens) {
     if (blocks > 64) blocks = 64;
-    return (long long)blocks * tokens > 8 * 4 * 148 ? (blocks + 3) / 4 : blocks;
+    return (long long)blocks * tokens > 8 * 4 * device_sms() ? (blocks + 3) / 4 : blocks;
 }
 
 LLM_EXPORT int llm_expert_act_scale(const void* x, int ldx, const float* w, int ldw, void* y, int ldy, int dtype, int N, int C, int E,

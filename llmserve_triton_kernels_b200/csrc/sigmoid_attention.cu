@@ -300,7 +300,7 @@ LLM_EXPORT int llm_qk_prepare(const void* proj, int in_dtype, int ldp, void* q_o
     const size_t smem = (size_t)(rot / 2 + 1) * sizeof(float2);
     auto go = [&](auto kernel, auto* in, auto* qo, auto* ko) {
         using TK = std::remove_pointer_t<decltype(ko)>;
-        const int rounds = ((Hq + Hk) * (D - rot / 2) + 255) / 256, room = 2 * 148 / N;
+        const int rounds = ((Hq + Hk) * (D - rot / 2) + 255) / 256, room = 2 * device_sms() / N;
         return launch_pdl(kernel, dim3(N, rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room)), dim3(256), smem, stream, in, ldp, qo, ldq, ko, ldk, (TK*)pool, slot_map, page_size, Dp, qw, kw,
                           eps, freq, rot, positions, k_scale, Hq, Hk, D, V);
     };
