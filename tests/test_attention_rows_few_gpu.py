@@ -235,3 +235,54 @@ def test_every_number_of_shares(ops, form, monkeypatch):
             monkeypatch.setattr(ops, "_few_plan", lambda *a: shares)
             got = ops.merge_project_gate(run(leave_parts=True), w, None).float()
             assert float((got - want).abs().max()) <= 0.03 * float(want.abs().max()), f"{shares} shares left"
+
+
+@pytest.mark.parametrize("latent", [False, True])
+@pytest.mark.parametrize("news", [1, 3])
+@pytest.mark.parametrize("contexts", [(15, 16, 17), (31, 32, 33), (160, 144, 47), (2000, 1999, 1)])
+def test_the_newest_rows_are_the_work_of_the_kernel_in_front(ops, contexts, news, latent):
+    """Keys cached before the step are read while the kernel that writes the step's own rows still runs (``steps_apart``), and those are not:
+    the two kernels directly behind one another in a graph, other rows in their slots before every replay."""
+    contexts = tuple(max(c, news) for c in contexts)
+    H, KV, D, V, page, rank, rot, dim = 16, 4, 64, 64, 16, 128, 32, 64
+    pages = sum(-(-c // page) for c in contexts) + 2
+    n = news * len(contexts)
+    table, ctx = step((news,) * len(contexts), contexts, page, pages, True)
+    positions = [c - news + i for c in contexts for i in range(news)]
+    owner = ctx.token_request.tolist()
+    slots = torch.tensor([int(table[r, p // page]) * page + p % page for r, p in zip(owner, positions)], dtype=torch.int32, device=DEV)
+    pos = torch.tensor(positions, dtype=torch.int32, device=DEV)
+    if latent:
+        pool = rnd(pages, page, rank + rot, seed=1)
+        proj = rnd(n, H * (dim + rot) + rank + rot, seed=2)
+        weight, freq = torch.ones(rank, device=DEV), torch.rand(rot // 2, device=DEV)
+        q_lat = rnd(n, H, rank, seed=3)
+
+        def run():
+            q_rot = ops.latent_prepare(proj, pos, slots, pool, weight, freq, 1e-6, H, dim, rot, rank)
+            return ops.latent_paged_attention(q_lat, q_rot, pool, table, ctx, rank=rank, scale=0.08)
+    else:
+        pool = rnd(pages, 2, KV, page, D, seed=1)
+        proj = rnd(n, (H + KV) * D + KV * V, dtype=torch.float32, seed=2)
+
+        def run():
+            q = ops.head_prepare(proj, pos, heads=H, kv_heads=KV, dim=D, value_dim=V, q_weight=torch.ones(D, device=DEV), k_weight=torch.ones(D, device=DEV), eps=1e-6,
+                                 pool=pool, slot_map=slots)
+            return ops.paged_softmax_attention(q, pool, table, ctx, num_heads=H, num_kv_heads=KV, key_dim=D, value_dim=V, scale=0.125)
+
+    run()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    fresh, stale = proj.clone(), pool.clone()
+    for turn in range(12):
+        proj.copy_(fresh * (1.0 + turn) + turn)
+        pool.copy_(stale.roll(turn, 0) * 3.0)  # what the slots held before
+        graph.replay()
+        torch.cuda.synchronize()
+        early = got.clone()
+        ctx.steps_apart = False
+        pool.copy_(stale.roll(turn, 0) * 3.0)
+        want = run()
+        ctx.steps_apart = True
+        assert torch.equal(early, want), f"turn {turn}"
