@@ -196,7 +196,8 @@ LLM_EXPORT int llm_unit_norm_kv_write(void* qkv, int dtype, int ld, const int* s
     if (n <= 0) return 0;
     if (H <= 0 || KV <= 0 || dk <= 0 || dv <= 0 || D < dk || D < dv || page_size <= 0 || ld < (H + KV) * dk + KV * dv)
         return LLM_ERR_BAD_ARGUMENT;
-    const dim3 grid(n, n <= 64 ? (H + 2 * KV + 3) / 4 : 1);
+    // an item a warp up to 1,024 tokens (32 + 2 x 8 heads of 64, one CTA a token / several: 200 tokens 12.4 / 4.3 us, 600 12.8 / 8.2, 2,000 22.3 / 25.6)
+    const dim3 grid(n, n <= 1024 ? (H + 2 * KV + 3) / 4 : 1);
     if (dtype == LLM_F32)
         return launch_pdl(unit_norm_kv_write_kernel<float>, grid, dim3(128), 0, stream, (float*)qkv, ld, slot_map,
                           (float*)pool, eps, normed, H, KV, dk, dv, D, page_size);

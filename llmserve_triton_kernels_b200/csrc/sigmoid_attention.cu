@@ -154,9 +154,9 @@ sum_parts_kernel(const float* __restrict__ part, TO* __restrict__ out, const int
 //   rotate:  in every head, lanes i and i + rot/2 (i < rot/2) turn by position * freq[i]; lanes >= rot pass
 //   keys:    times k_scale
 //   queries go to q_out [N, Hq * D]; keys to k_out [N, Hk * D], or with the values into the token's slot of
-//   pool [pages, 2, Hk, page_size, Dp].  One CTA per token, or in steps of few tokens several that share its lanes, each of
+//   pool [pages, 2, Hk, page_size, Dp].  One CTA per token, or in steps of few tokens several that share its lanes (SHARED), each of
 //   which works out the token's angles and sums for itself.
-template <typename TI, typename TQ, typename TK>
+template <typename TI, typename TQ, typename TK, bool SHARED>
 __global__ void __launch_bounds__(256)
 qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, int ldq, TK* __restrict__ k_out, int ldk,
                   TK* __restrict__ pool, const int* __restrict__ slot_map, int page_size, int Dp, const float* __restrict__ qw,
@@ -179,9 +179,9 @@ qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, 
     float q_scale = 1.f, kn_scale = 1.f;
     if (qw) {
         float sums[2] = {0.f, 0.f};
-#pragma unroll 8
+#pragma unroll(SHARED ? 8 : 4)
         for (int i = threadIdx.x; i < Hq * D; i += blockDim.x) { const float v = to_float(row[i]); sums[0] = fmaf(v, v, sums[0]); }
-#pragma unroll 2
+#pragma unroll(SHARED ? 2 : 4)
         for (int i = threadIdx.x; i < Hk * D; i += blockDim.x) { const float v = to_float(row[Hq * D + i]); sums[1] = fmaf(v, v, sums[1]); }
         block_sums<2>(sums, scratch);
         q_scale = 1.f / sqrtf(sums[0] / (float)(Hq * D) + eps);
@@ -190,7 +190,7 @@ qk_prepare_kernel(const TI* __restrict__ proj, int ldp, TQ* __restrict__ q_out, 
     __syncthreads();
     const int per_head = D - half;  // work items a head: `half` pairs, then the lanes that pass
     const int page = slot / page_size, off = slot % page_size;
-    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    const int first = SHARED ? blockIdx.y * blockDim.x + threadIdx.x : threadIdx.x, step = SHARED ? gridDim.y * blockDim.x : blockDim.x;
     for (int it = first; it < (Hq + Hk) * per_head; it += step) {
         const int head = it / per_head, i = it % per_head;
         const bool is_q = head < Hq;
@@ -298,17 +298,20 @@ LLM_EXPORT int llm_qk_prepare(const void* proj, int in_dtype, int ldp, void* q_o
         return LLM_ERR_BAD_ARGUMENT;
     using bf = __nv_bfloat16;
     const size_t smem = (size_t)(rot / 2 + 1) * sizeof(float2);
-    auto go = [&](auto kernel, auto* in, auto* qo, auto* ko) {
+    const int rounds = ((Hq + Hk) * (D - rot / 2) + 255) / 256, room = 2 * device_sms() / N;
+    const int ctas = rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room);  // a token
+    auto go = [&](auto* in, auto* qo, auto* ko) {
+        using TI = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+        using TQ = std::remove_pointer_t<decltype(qo)>;
         using TK = std::remove_pointer_t<decltype(ko)>;
-        const int rounds = ((Hq + Hk) * (D - rot / 2) + 255) / 256, room = 2 * device_sms() / N;
-        return launch_pdl(kernel, dim3(N, rounds < room ? (rounds < 1 ? 1 : rounds) : (room < 1 ? 1 : room)), dim3(256), smem, stream, in, ldp, qo, ldq, ko, ldk, (TK*)pool, slot_map, page_size, Dp, qw, kw,
-                          eps, freq, rot, positions, k_scale, Hq, Hk, D, V);
+        return launch_pdl(ctas > 1 ? qk_prepare_kernel<TI, TQ, TK, true> : qk_prepare_kernel<TI, TQ, TK, false>, dim3(N, ctas), dim3(256), smem, stream, in, ldp, qo,
+                          ldq, ko, ldk, (TK*)pool, slot_map, page_size, Dp, qw, kw, eps, freq, rot, positions, k_scale, Hq, Hk, D, V);
     };
     if (in_dtype == LLM_F32 && q_dtype == LLM_F32 && k_dtype == LLM_F32)
-        return go(qk_prepare_kernel<float, float, float>, (const float*)proj, (float*)q_out, (float*)k_out);
+        return go((const float*)proj, (float*)q_out, (float*)k_out);
     if (in_dtype == LLM_F32 && q_dtype == LLM_BF16 && k_dtype == LLM_BF16)
-        return go(qk_prepare_kernel<float, bf, bf>, (const float*)proj, (bf*)q_out, (bf*)k_out);
+        return go((const float*)proj, (bf*)q_out, (bf*)k_out);
     if (in_dtype == LLM_BF16 && q_dtype == LLM_BF16 && k_dtype == LLM_BF16)
-        return go(qk_prepare_kernel<bf, bf, bf>, (const bf*)proj, (bf*)q_out, (bf*)k_out);
+        return go((const bf*)proj, (bf*)q_out, (bf*)k_out);
     return LLM_ERR_UNSUPPORTED;
 }
