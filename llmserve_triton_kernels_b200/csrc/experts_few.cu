@@ -18,8 +18,9 @@
 //         same whatever experts the other tokens use.
 // Behind its own tiles the up kernel has the down kernel's weights brought into L2, so that memory does not stand still between the two.
 // The shared expert's tiles (and, with a table, everybody's) are on their way before the kernel in front has ended.  The up kernel
-// lets its dependent start only behind its own wait, so the down kernel may make its list, and ask for its first weights, while
-// the up kernel runs: the router has ended by then.
+// lets its dependent start only behind its own wait, by when the router has ended: the down kernel makes its list without waiting.  Its CTAs
+// (128 registers x 512 threads, an SM's whole register file) start where an up CTA has ended, and ask for their first weights while
+// others still run.
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -205,7 +206,10 @@ __global__ void __launch_bounds__(UP_THREADS, 1) experts_up_kernel(const Experts
             const bf16* at = p.w_down + (size_t)n * ldk + (size_t)(shared ? p.E : list[b - (p.fs > 0 ? 1 : 0)]) * p.ff;
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(at), "r"((shared ? p.fs : p.ff) * 2) : "memory");
         }
-        return;  // the other warps wait for every tile that was asked for
+        // the other warps wait for every tile that was asked for, but not once a wait has given up: no copy is left on its way to a CTA that
+        // has ended
+        for (int n = max(0, asked - p.up_slots); n < asked; ++n) tma::mbar_wait(&full[n % p.up_slots], (n / p.up_slots) & 1);
+        return;
     }
     for (int n = 0; n < tiles; ++n) {
         const int s = n % p.up_slots;

@@ -1700,7 +1700,8 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
     """A mixture of experts for few bfloat16 tokens, of which only the experts that one of them uses are read: the product with ``w_up``,
     the activation (``activation``: one of :func:`expert_act_scale`'s; None: the bounded gated one of :func:`expert_gated_act`) times the
     tokens' weights, and the product with ``w_down``.  Returns ``[N, hidden]`` float32, or what ``sink.linear`` returns; None for
-    a step that it does not take: of more than 8 tokens or other sizes than the kernels', or, with ``top`` (how many experts a token
+    a step that it does not take: of more than 8 tokens, rows of more than 2,048 (a token's lanes wait in the warps' registers) or other
+    sizes than the kernels', or, with ``top`` (how many experts a token
     uses), one that the products over all experts are faster for (:func:`experts_few_pay`)."""
     m, k = x.shape
     n, c = w_down.shape
