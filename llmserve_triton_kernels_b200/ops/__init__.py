@@ -1202,9 +1202,10 @@ def _few_plan(device: int, longest: int, tiles: int, dk: int, dv: int, maps: int
     start, a_pass, keys = (3.8, 2.4, 128) if small else (7.0, 2.85, 64) if long else (5.5, 2.35, 128)
     best, best_us = 1, math.inf
     want = -(-longest // keys)
-    shares = [max(1, min(want, _few_resident(device, dk, dv, maps, True, 1) // tiles, 32, most_splits))] if leave else (1, 2, 4, 8)
+    # (partial results are left in two shares at least: the kernel that merges them on its way is shorter than a product of its own)
+    shares = [max(2, min(want, _few_resident(device, dk, dv, maps, True, 1) // tiles, 32, most_splits))] if leave else (1, 2, 4, 8)
     for splits in shares:
-        if splits > 1 and splits > want:
+        if splits > want and not leave and splits > 1:
             break
         us = -(-tiles * splits // _few_resident(device, dk, dv, maps, leave, splits)) * (start + a_pass * -(-longest // (splits * keys)))
         if us < best_us:
@@ -1285,7 +1286,8 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
                and ((dk <= 128 and value_dim <= 128) or (maps == 1 and dk <= 320)))
         leave = leave_parts and splits > 1
         if few:
-            shares = _few_plan(q0.device.index or 0, longest, -(-most * group * maps // 16) * num_kv_heads * ctx.num_requests, dk, value_dim, maps, leave_parts,
+            # (a captured step's context says the most keys that any step of its shape may have; whole prompts have their own tokens)
+            shares = _few_plan(q0.device.index or 0, min(longest, most) if getattr(ctx, "fresh_requests", False) else longest, -(-most * group * maps // 16) * num_kv_heads * ctx.num_requests, dk, value_dim, maps, leave_parts,
                                _SPLIT_SCRATCH_BYTES // (n * num_heads * value_dim * 4), ctas, splits)
             few = 0 if shares == 0 else 2 if getattr(ctx, "steps_apart", False) else 1
             splits = shares or splits

@@ -91,3 +91,22 @@ def test_keys_that_score_minus_infinity_weigh_nothing(ops):  # noqa: F811
     k, v = keys[order, 0].reshape(-1, d)[:context].double(), values[order, 0].reshape(-1, d)[:context].double()
     want = torch.softmax(q[0].double() @ k.T * 0.25, -1) @ v
     torch.testing.assert_close(got[0].double(), want, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("n", [1, 70])  # 32 heads: eight warps an item, one
+@pytest.mark.parametrize("context", [70, 96, 255, 256, 257, 288, 700])
+@pytest.mark.parametrize("window", [None, 33, 256])
+def test_beside_the_same_in_64_bits(ops, context, window, n):  # noqa: F811
+    H, KV, page, d, dv = 32, 8, 8, 24, 40
+    pages = -(-context // page) + 2
+    q, keys, values = rnd(n, H, d, seed=1, dtype=torch.float32), rnd(pages, KV, page, d, seed=2, dtype=torch.float32), rnd(pages, KV, page, dv, seed=3, dtype=torch.float32)
+    table, ctx = rows.step((n,), (context,), page, pages, False)
+    got = ops.attention_rows(q, None, keys.data_ptr(), (KV * page * d, page * d, d), values.data_ptr(), (KV * page * dv, page * dv, dv), dv, table, page, ctx,
+                             num_heads=H, num_kv_heads=KV, scale=0.3, window=window)
+    pick = lambda x: x[table[0].long()].transpose(1, 2).reshape(-1, KV, x.shape[-1])[:context].double().repeat_interleave(H // KV, 1)  # noqa: E731
+    scores = torch.einsum("nhd,jhd->hnj", q.double(), pick(keys)) * 0.3
+    pos, j = torch.arange(context - n, context, device=DEV)[:, None], torch.arange(context, device=DEV)[None]
+    scores = scores.masked_fill(~((j <= pos) & (j > pos - (window or context + 1))), -torch.inf)
+    want = torch.einsum("hnj,jhd->nhd", scores.softmax(-1), pick(values))
+    # 32-bit sums of up to 700 weights near 1e-2 and of 24 products a score: some ten roundings of 6e-8 behind one another
+    assert float((got.double() - want).norm()) <= 2e-6 * float(want.norm())
