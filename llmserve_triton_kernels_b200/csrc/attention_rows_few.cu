@@ -13,7 +13,8 @@
 //     in front is still writing its newest row to.
 //   * the CTAs that share a row tile are a thread-block cluster and merge through distributed shared memory: no partial results in
 //     memory and no second kernel.  (Latent attention leaves its partial results instead: the product behind it merges them.)
-// Measured on a B200 against the kernel for many rows and its merge, back to back in a graph (microseconds): 32 heads on 8 of 64 lanes,
+// Measured on a B200 against the kernel for many rows and its merge, back to back in a graph, the keys in L2 (microseconds; inside a decode
+// step, behind its weights, 7 to 9.5 where this says 5.6 to 8): 32 heads on 8 of 64 lanes,
 // window 512 of 2,000 keys: 13.4 -> 5.6 for one request, 18.2 -> 7.5 for 8; all of 2,000 keys, 8 requests: 38.3 -> 14.4; two maps of 64 on
 // values of 128: 17.9 -> 7.9; latents of 256 + 32 with 32 heads and the product behind them, 2,000 keys: 20.8 -> 12.1.
 #include <type_traits>

@@ -141,8 +141,8 @@ class RoutedMLP(FeedForward):
     them, one kernel that applies the activation and the token's
     weight of each expert's block of columns (0 for an expert the token did not choose, the gate for the shared one).
     The second product then sums over the experts by itself.  Every weight matrix is read once a step whatever the
-    tokens chose, which is what a decode step of several requests costs anyway; a prompt pays the products of the
-    experts its tokens did not choose."""
+    tokens chose; a prompt pays the products of the experts its tokens did not choose.  Steps of up to 8 tokens read the
+    used experts alone where that is faster (:func:`ops.experts_few`)."""
 
     graph_safe = True
     accepts_sink = True
@@ -220,7 +220,8 @@ class TableRoutedMLP(FeedForward):
     ``shared.down``.  As in :class:`RoutedMLP` all experts' gate and up matrices are stacked (the shared expert's last)
     and so are the down matrices side by side: a step is one product over every expert, one kernel that applies the
     bounds, the activation and the token's weight of each expert's block of columns (0 for an expert the table does not
-    give the token, whose columns are then not even read), and one product that sums over the experts by itself."""
+    give the token, whose columns are then not even read), and one product that sums over the experts by itself; up to 8
+    tokens may read the used experts alone."""
 
     graph_safe = True
     accepts_sink = True
@@ -294,7 +295,8 @@ class RoutedGatedMLP(FeedForward):
     As in :class:`TableRoutedMLP` all experts' gate and up matrices are stacked (the shared expert's last) and the down
     matrices stand side by side: a step is one kernel for the router (its 32-bit product, the choice and the weights), one
     product over every expert, one kernel for the activation times the token's weight of each expert's block of columns
-    (0, and nothing read, for an expert the token did not choose), and one product that sums over the experts by itself."""
+    (0, and nothing read, for an expert the token did not choose), and one product that sums over the experts by itself; up to
+    8 tokens may read the used experts alone."""
 
     graph_safe = True
     accepts_sink = True
