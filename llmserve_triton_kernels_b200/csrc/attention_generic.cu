@@ -9,7 +9,7 @@
 // how the tokens were cut into steps or batched.
 //
 // Bound by latency where items are few (table -> key -> weights -> values, a chunk after the other): a decode step of two requests with 32
-// heads and 150 keys took 67 us a layer with a warp an item and takes 12 with a warp a class; 242 prompt tokens, whose warps fill the
+// heads and 150 keys took 67 us a layer with a warp an item and takes 15 with a warp a class; 242 prompt tokens, whose warps fill the
 // SMs, take 64 and 139.
 //
 // A query at position p of request r sees keys max(0, p - window + 1) .. p (window <= 0: from 0), with a window also the

@@ -1,7 +1,7 @@
 // A mixture of small feed-forward layers for steps of few tokens (bfloat16, at most 8): only the experts that a token of the step
 // uses are read.
 //
-// In a decode step (1,408 + 704 x 4 of 32 experts, 2,048 wide) they took 10.7 + 8.4 us a layer for one token and 16.7 + 13.0 for three,
+// In a decode step (1,408 + 704 x 4 of 32 experts, 2,048 wide) they take 11.0 + 8.3 us a layer for one token and 17.1 + 12.5 for three,
 // where the products over all experts and the activation between them took 30.4 + 2.6 + 15.7.
 //
 // What bounds it: the bytes of the weights.  One token that uses 4 of 32 experts needs 52 of the 294 MB that the products over all

@@ -1752,7 +1752,7 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
 # side (csrc/sigmoid_attention.cu, retention.cu, routing.cu).
 _SIGMOID_SPLIT_KEYS = 128  # a stretch of keys that one CTA sums up when a context is shared out
 # The same for the tensor-core kernel, whose tile is 32 keys: stretches of one tile put 600 keys on all sixteen shares, of 128 on five
-# (31.0 -> 20.8 us a layer of a decode step of four requests).  As many shares as the SMs have room for, one CTA each: with sixteen
+# (31.0 -> 16.3 us a layer of a decode step of four requests, and 2.8 for the sum).  As many shares as the SMs have room for, one CTA each: with sixteen
 # whatever the step, 64 requests (32 heads) took 50 us at 100 keys and 195 at 600, and take 30 and 122; at 6,000 keys, where two shares of
 # 64 tiles leave 20 of 148 SMs without work, sixteen were 4 % faster (12 % with 24 heads on 24), which the short contexts outweigh.
 _SIGMOID_MMA_SPLIT_KEYS = 32
