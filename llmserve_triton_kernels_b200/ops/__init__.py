@@ -64,6 +64,8 @@ _SIGNATURES = {
     "llm_attention_tcgen05_general": [_vp, _i, _vp, _i, _vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,
                                       _vp, _ll, _vp, _f, _f, _f, _vp, _vp],
     "llm_experts_few": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp],
+    "llm_experts_many": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _f,
+                         _vp, _vp],
     "llm_gemm_simt_batched": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _vp],
     "llm_sample": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "llm_sigmoid_attention": [_vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i,
@@ -1744,6 +1746,58 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
     if resid is None:
         return out
     return NormedInput(xw, ss, sink.eps, sink.norm) if norm_w is not None else ADDED
+
+
+def experts_many_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int) -> bool:
+    """Whether the used experts' own products (:func:`experts_many`) are faster than the products over all experts."""
+    return tokens > _EXPERTS_FEW and top < experts
+
+
+def experts_many(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, ff: int, shared_ff: int, *, top: int, activation: str | None = None,
+                 limit: float = 0.0, shared_limit: float = 0.0, slope: float = 1.0, up_shift: float = 0.0, weights: torch.Tensor | None = None,
+                 ids: torch.Tensor | None = None, table: torch.Tensor | None = None, sink: "ResidualSink | None" = None):
+    """A mixture of experts for many bfloat16 tokens: the arguments of :func:`experts_few`, with ``top``, the most experts that a token uses.
+    Every token's row goes through the products of the experts that it uses and no others (csrc/experts_many.cu).  Returns ``[N, hidden]``
+    float32, or :data:`ADDED` where ``sink`` is given and takes it; None for sizes that the kernels do not take."""
+    m, k = x.shape
+    n, c = w_down.shape
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.stride(1) == 1 and w_up.is_contiguous() and w_down.is_contiguous()):
+        return None
+    gated = activation is None
+    _need(w_up.dtype == w_down.dtype == x.dtype and tuple(w_up.shape) == ((2 if gated else 1) * (experts * ff + shared_ff), k) and c == experts * ff + shared_ff,
+          "experts_many: the stacked matrices do not match the experts")
+    ldw = listed = vocab = 0
+    if weights is not None:
+        _need(weights.dtype == torch.float32 and weights.stride(1) == 1 and weights.shape[0] == m and weights.shape[1] >= experts + int(shared_ff > 0), "experts_many: weights are float32 [N, experts (+ 1)]")
+        ldw = weights.stride(0)
+    else:
+        _i32(ids, "ids")
+        _need(table is not None and table.dtype == torch.int32 and table.is_contiguous() and table.dim() == 2 and ids.numel() == m, "experts_many: table is int32 [vocab, top]")
+        vocab, listed = table.shape
+    resid = out = None
+    alpha = 1.0
+    if sink is not None and sink.resid.is_contiguous() and tuple(sink.resid.shape) == (m, n):
+        resid, alpha = sink.resid, sink.alpha
+    else:
+        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    cap = m * min(int(top), experts)
+    ints = torch.empty((experts * (2 * m + 1),), dtype=torch.int32, device=x.device)
+    act = torch.empty((cap, ff), dtype=x.dtype, device=x.device)
+    y = torch.empty((cap, n), dtype=torch.float32, device=x.device)
+    act_s = y_s = None
+    if shared_ff:
+        act_s = torch.empty((m, shared_ff), dtype=x.dtype, device=x.device)
+        y_s = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    code = _launch("llm_experts_many", _ptr(x), x.stride(0), _ptr(w_up), _ptr(w_down), m, k, n, experts, ff, shared_ff,
+                   -1 if gated else _UNARY_KINDS[activation], float(limit), float(shared_limit), float(slope), float(up_shift), _ptr(weights), ldw,
+                   _ptr(ids), _ptr(table), listed, vocab, _ptr(ints), cap, _ptr(act), _ptr(act_s), _ptr(y), _ptr(y_s), _ptr(out), _ptr(resid),
+                   float(alpha), _error_flag_ptr(), _stream())
+    if code == 10002:
+        add_launches(-1)
+        return None
+    _check(code, "experts_many")
+    add_launches(4)
+    return out if resid is None else ADDED
 
 
 # ------------------------------------------------------------------------------------------------

@@ -124,6 +124,15 @@ class DenseMLP(FeedForward):
 register_part("feed_forward", "dense_mlp", DenseMLP)
 
 
+def _used_experts(part, x, sink, **kw):
+    """What the kernels that read only the used experts return for a mixture, or None where the products over all experts are the way."""
+    sizes = (part.experts, part.expert_size, part.shared_size)
+    few = ops.experts_few(x, part.w_up, part.w_down, *sizes, sink=sink, top=part.top, **kw)
+    if few is not None or not ops.experts_many_pay(x.shape[0], part.experts, part.top, part.expert_size, part.shared_size):
+        return few
+    return ops.experts_many(x, part.w_up, part.w_down, *sizes, sink=sink, top=part.top, **kw)
+
+
 class RoutedMLP(FeedForward):
     """A mixture of small feed-forward layers ``down_e(act(up_e(x)))`` without biases, of which each token uses ``top``:
 
@@ -141,8 +150,8 @@ class RoutedMLP(FeedForward):
     them, one kernel that applies the activation and the token's
     weight of each expert's block of columns (0 for an expert the token did not choose, the gate for the shared one).
     The second product then sums over the experts by itself.  Every weight matrix is read once a step whatever the
-    tokens chose; a prompt pays the products of the experts its tokens did not choose.  Steps of up to 8 tokens read the
-    used experts alone where that is faster (:func:`ops.experts_few`)."""
+    tokens chose; a prompt pays the products of the experts its tokens did not choose.  Where that is faster the used experts run
+    alone: up to 8 tokens through :func:`ops.experts_few`, more through :func:`ops.experts_many`."""
 
     graph_safe = True
     accepts_sink = True
@@ -193,10 +202,9 @@ class RoutedMLP(FeedForward):
         weights = ops.route(xt, self.w_router, self.correction, self.experts, self.top, self.router_scale, self.renormalize, self.shared_gate)
         if self.shared_size and not self.shared_gate:
             weights = torch.cat((weights, torch.ones_like(weights[:, :1])), dim=1)
-        few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, activation=self.activation,
-                              weights=weights, sink=sink, top=self.top)
-        if few is not None:
-            return few
+        own = _used_experts(self, xt, sink, activation=self.activation, weights=weights)
+        if own is not None:
+            return own
         act = ops.expert_act_scale(ops.linear(xt, self.w_up), weights, self.experts, self.expert_size, self.activation)
         if sink is not None:
             handed_on = sink.linear(act, self.w_down)
@@ -220,8 +228,8 @@ class TableRoutedMLP(FeedForward):
     ``shared.down``.  As in :class:`RoutedMLP` all experts' gate and up matrices are stacked (the shared expert's last)
     and so are the down matrices side by side: a step is one product over every expert, one kernel that applies the
     bounds, the activation and the token's weight of each expert's block of columns (0 for an expert the table does not
-    give the token, whose columns are then not even read), and one product that sums over the experts by itself; up to 8
-    tokens may read the used experts alone."""
+    give the token, whose columns are then not even read), and one product that sums over the experts by itself; the used
+    experts may run alone, as there."""
 
     graph_safe = True
     accepts_sink = True
@@ -261,11 +269,10 @@ class TableRoutedMLP(FeedForward):
 
     def forward(self, x, ctx, sink=None):
         xt = x.materialize() if isinstance(x, ops.NormedInput) else x
-        few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, limit=self.limit,
-                              shared_limit=self.shared_limit, slope=self.slope, up_shift=1.0, ids=ctx.token_ids, table=self.table, sink=sink,
-                              top=self.top)
-        if few is not None:
-            return few
+        own = _used_experts(self, xt, sink, limit=self.limit, shared_limit=self.shared_limit, slope=self.slope, up_shift=1.0, ids=ctx.token_ids,
+                            table=self.table)
+        if own is not None:
+            return own
         act = ops.expert_gated_act(ops.linear(xt, self.w_up), self.experts, self.expert_size, self.shared_size, self.limit,
                                    self.shared_limit, self.slope, ids=ctx.token_ids, table=self.table)
         if sink is not None:
@@ -295,8 +302,8 @@ class RoutedGatedMLP(FeedForward):
     As in :class:`TableRoutedMLP` all experts' gate and up matrices are stacked (the shared expert's last) and the down
     matrices stand side by side: a step is one kernel for the router (its 32-bit product, the choice and the weights), one
     product over every expert, one kernel for the activation times the token's weight of each expert's block of columns
-    (0, and nothing read, for an expert the token did not choose), and one product that sums over the experts by itself; up to
-    8 tokens may read the used experts alone."""
+    (0, and nothing read, for an expert the token did not choose), and one product that sums over the experts by itself; the
+    used experts may run alone, as there."""
 
     graph_safe = True
     accepts_sink = True
@@ -355,11 +362,9 @@ class RoutedGatedMLP(FeedForward):
         xt = x.materialize() if isinstance(x, ops.NormedInput) else x
         weights = ops.route(xt, self.w_router, self.correction, self.experts, self.top, self.router_scale, True, False, bias=self.b_router,
                             shared_one=self.shared_size > 0, scores=self.scores, groups=self.groups)
-        few = ops.experts_few(xt, self.w_up, self.w_down, self.experts, self.expert_size, self.shared_size, limit=self.limit,
-                              shared_limit=self.shared_limit, slope=self.slope, up_shift=self.up_shift, weights=weights, sink=sink,
-                              top=self.top)
-        if few is not None:
-            return few
+        own = _used_experts(self, xt, sink, limit=self.limit, shared_limit=self.shared_limit, slope=self.slope, up_shift=self.up_shift, weights=weights)
+        if own is not None:
+            return own
         act = ops.expert_gated_act(ops.linear(xt, self.w_up), self.experts, self.expert_size, self.shared_size, self.limit, self.shared_limit,
                                    self.slope, weights=weights, up_shift=self.up_shift)
         if sink is not None:
