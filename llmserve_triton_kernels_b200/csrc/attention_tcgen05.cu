@@ -22,8 +22,12 @@
 // Keys past a request's length inside its last page, and pages outside the range a CTA needs, are
 // never looked at: a score outside [window start, position] is -inf before the exponential, and the
 // producer loads a page of the needed range in place of one outside it, so that no stale or released
-// page is touched.  Values of masked keys meet a probability of exactly zero; the cache pool holds only
-// finite numbers (it starts as zeros and is written by the projection kernels).
+// page is touched.  Values of masked keys meet a probability of exactly zero; what lies behind the request's last
+// token (stale rows of a page, in OWN the next request's) is made zeros in shared memory before the product.
+//
+// EXTRA: scores are capped and lose a distance bias before the softmax, or a window keeps the first keys (some operations more
+// a score, so a kernel of its own).  OWN: the keys and values are the step's own tokens, row by row and head by head, with lanes
+// behind the keys' first 64 that all heads share (latent attention's fresh part): no pages.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets *error_flag, the roles leave their loops,
 // tensor memory is freed and the kernel returns.
@@ -36,6 +40,8 @@
 namespace {
 
 using attn::AttnParams;
+
+constexpr float LOG2E = 1.4426950408889634f;
 
 constexpr int BM = 128, BN = 64, THREADS = 256, TMEM_COLS = 256;
 constexpr float LAZY = 8.f;  // log2 of how far a row's maximum may rise before its shift follows
@@ -50,13 +56,15 @@ constexpr float LAZY = 8.f;  // log2 of how far a row's maximum may rise before 
 //                  the softmax has read tile j; the other CTA of the SM fills the gap.
 //   64 and 128   : one tile of scores [0, 64); the output [64, 192); the queries [192, 224); probabilities [224, 256).  Three stages
 //                  (24 KB): 73 KB.
+//   96 and 64    : one tile of scores [0, 64); the output [64, 128); the queries [128, 176); probabilities [176, 208).  Three stages
+//                  (24 KB; a row's last 32 lanes lie in a piece of 64 of which the product reads the first half): 73 KB.
 template <int KD, int VD>
 struct Shape {
-    static constexpr bool Q_IN_TMEM = KD == 64;
-    static constexpr int S_BUFFERS = VD == 64 ? 2 : 1, STAGES = KD == 64 ? 3 : 2;
+    static constexpr bool Q_IN_TMEM = KD <= 96;
+    static constexpr int S_BUFFERS = KD == 64 && VD == 64 ? 2 : 1, STAGES = KD <= 96 ? 3 : 2;
     static constexpr int O_COL = S_BUFFERS * BN, Q_COL = O_COL + VD, P_COL = Q_IN_TMEM ? Q_COL + KD / 2 : O_COL + VD;
-    static constexpr int K_HALVES = KD / 64, V_HALVES = VD / 64;  // 64-wide pieces of a row of keys (queries), values: one TMA box each
-    static constexpr int K_BYTES = BN * KD * 2, V_BYTES = BN * VD * 2, STAGE_BYTES = K_BYTES + V_BYTES, Q_BYTES = Q_IN_TMEM ? 0 : BM * KD * 2;
+    static constexpr int K_HALVES = (KD + 63) / 64, V_HALVES = VD / 64;  // 64-wide pieces of a row of keys (queries), values: one TMA box each
+    static constexpr int K_BYTES = BN * K_HALVES * 128, V_BYTES = BN * VD * 2, STAGE_BYTES = K_BYTES + V_BYTES, Q_BYTES = Q_IN_TMEM ? 0 : BM * KD * 2;
     static constexpr size_t SMEM = 1024 + (size_t)Q_BYTES + (size_t)STAGES * STAGE_BYTES;
     static_assert(P_COL + BN / 2 <= TMEM_COLS, "tensor memory");
 };
@@ -77,13 +85,25 @@ struct TcParams {
     // One gate a head: the result times sigmoid(gate[token * gate_token + head]); null: none
     const float* gate;
     long long gate_token;
+    int gate_lanes;       // a gate a lane instead: gate[token * gate_token + head * VD + lane]
+    const float* sinks;   // [H], or null: a key of that score (not scaled) without a value
+    const float* slopes;  // [H], or null (EXTRA): scores lose slope * distance
+    float softcap;        // > 0 (EXTRA): softcap * tanh(score / softcap)
+    int keep_first, chunk;
+    // OWN: the lanes of the queries behind the first 64, and the (maximum, in units of log 2, and sum) of every row [tokens, H, 2] or null
+    const __nv_bfloat16* q1;
+    long long q_head, q1_token, q1_head;
+    int own_values, own_rot;  // the column of the values of head 0 in a row of keys and values, of the shared lanes in a row of theirs
+    float2* stats;
 };
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) { tma::mbar_arrive(bar); }
 
-template <int KD, int VD>
+// qmap: the queries (head size 128), in OWN the lanes that the heads share.
+template <int KD, int VD, bool EXTRA, bool OWN>
 __global__ void __launch_bounds__(THREADS, 2)
 attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kvmap) {
+    static_assert(OWN == (KD == 96), "the shared lanes are the last 32 of 96");
     using Sh = Shape<KD, VD>;
     constexpr int STAGES = Sh::STAGES, NBUF = Sh::S_BUFFERS, K_BYTES = Sh::K_BYTES, STAGE_BYTES = Sh::STAGE_BYTES;
     constexpr int K_HALVES = Sh::K_HALVES, V_HALVES = Sh::V_HALVES;
@@ -97,13 +117,23 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
     const int row0 = tile * BM;
     if (row0 >= q_len) return;
     const int rows_here = min(BM, q_len - row0);
-    const int pos0 = p.ctx_lens[r] - q_len;
+    const int ctx_len = OWN ? q_len : p.ctx_lens[r];  // the step's own tokens are counted from the first of them
+    const int pos0 = ctx_len - q_len;
     const int key_hi = pos0 + row0 + rows_here - 1;
-    const int key_lo = p.window > 0 ? max(0, pos0 + row0 - p.window + 1) : 0;
-    const int t_begin = key_lo / BN, n_tiles = key_hi / BN + 1 - t_begin;
+    auto first_seen = [&](int pos) {
+        const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+        return tp.chunk > 0 ? max(lo, pos - pos % tp.chunk) : lo;
+    };
+    const int key_lo = first_seen(pos0 + row0);
+    // with a window the keys below keep_first stay visible: their tiles come first, then the window's (one run where they meet)
+    const int kept = EXTRA && p.window > 0 ? min(tp.keep_first, key_lo) : 0;
+    const int kept_tiles = min((kept + BN - 1) / BN, key_lo / BN);
+    const int t_skip = key_lo / BN - kept_tiles;  // tiles between the two
+    const int n_tiles = key_hi / BN + 1 - t_skip;
+    auto tile_start = [&](int j) { return (j < kept_tiles ? j : j + t_skip) * BN; };
     // a key tile needs no mask if every row of the CTA sees all of it
     const int tile_pos_min = pos0 + row0;
-    const int tile_lo_max = p.window > 0 ? max(0, pos0 + row0 + rows_here - 1 - p.window + 1) : 0;
+    const int tile_lo_max = first_seen(pos0 + row0 + rows_here - 1);
 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -133,7 +163,7 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         gave_up = 0;
         tma::mbar_fence_init();
         tma::prefetch_map(&kvmap);
-        if (!Sh::Q_IN_TMEM) tma::prefetch_map(&qmap);
+        if (!Sh::Q_IN_TMEM || OWN) tma::prefetch_map(&qmap);
     }
     if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tma::smem_addr(&tmem_base)), "n"(TMEM_COLS) : "memory");
@@ -158,7 +188,7 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         const bool is_v = warp == 6;
         unsigned long long* full = is_v ? v_full : k_full;
         unsigned long long* empty = is_v ? v_empty : k_empty;
-        const int ps = p.page_size, pages_per_tile = BN / ps;
+        const int ps = OWN ? BN : p.page_size, pages_per_tile = BN / ps;
         const int lp_lo = key_lo / ps, lp_hi = key_hi / ps;
         const int* table = p.page_table + (size_t)r * p.table_width;
         if (!Sh::Q_IN_TMEM && !is_v && lane == 0) {
@@ -169,15 +199,17 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         // One box per page and 64-wide piece, each issued by a lane of its own (a thread's TMA instructions follow one another slowly;
         // several threads' overlap).  The page table is read 32 entries at a time; a page outside the needed range is
         // replaced by one inside it.
-        const int first_page = t_begin * pages_per_tile, halves = is_v ? V_HALVES : K_HALVES;
+        const int halves = is_v ? V_HALVES : K_HALVES;
         const int lane0 = is_v ? 0 : (q_head - head * tp.maps) * KD;  // where a row's lanes of this map begin
+        const int kept_hi = kept > 0 ? (kept - 1) / ps : -1;
         int my_page = 0, loaded_from = -32;
         bool alive = true;
         for (int j = 0; j < n_tiles && alive; ++j) {
-            const int s = j % STAGES, idx0 = j * pages_per_tile;
-            if (idx0 >= loaded_from + 32) {  // pages_per_tile divides 32: a tile's pages lie in one batch
-                loaded_from = idx0;
-                my_page = table[min(max(first_page + idx0 + lane, lp_lo), lp_hi)];
+            const int s = j % STAGES, key0 = tile_start(j), idx0 = key0 / ps;
+            if (!OWN && idx0 >= loaded_from + 32) {  // pages_per_tile divides 32: a tile's pages lie in one batch
+                loaded_from = idx0 - idx0 % 32;
+                const int idx = min(loaded_from + lane, lp_hi);
+                my_page = table[idx < lp_lo && idx > kept_hi ? lp_lo : idx];
             }
             if (lane == 0) {
                 if (gave_up || (j >= STAGES && !tma::mbar_wait(&empty[s], ((j / STAGES) - 1) & 1))) {
@@ -188,11 +220,17 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
                 }
             }
             alive = __shfl_sync(0xffffffffu, (int)alive, 0) != 0;
-            const int in_tile = lane / halves, half = lane % halves;
-            const int page = __shfl_sync(0xffffffffu, my_page, (idx0 - loaded_from + in_tile) & 31);
-            if (alive && in_tile < pages_per_tile) {
-                unsigned char* dst = kv_s + (size_t)s * STAGE_BYTES + (size_t)is_v * K_BYTES + (size_t)half * (BN * 128) + (size_t)in_tile * ps * 128;
-                tma::load_2d(dst, &kvmap, lane0 + half * 64, ((page * 2 + (int)is_v) * p.KV + kvh) * ps, &full[s]);
+            unsigned char* stage = kv_s + (size_t)s * STAGE_BYTES + (size_t)is_v * K_BYTES;
+            if constexpr (OWN) {
+                if (alive && lane == 0) {
+                    tma::load_2d(stage, &kvmap, is_v ? tp.own_values + head * VD : head * 64, q_begin + key0, &full[s]);
+                    if (!is_v) tma::load_2d(stage + BN * 128, &qmap, tp.own_rot, q_begin + key0, &full[s]);  // 32 lanes, zeros behind them
+                }
+            } else {
+                const int in_tile = lane / halves, half = lane % halves;
+                const int page = __shfl_sync(0xffffffffu, my_page, (idx0 - loaded_from + in_tile) & 31);
+                if (alive && in_tile < pages_per_tile)
+                    tma::load_2d(stage + (size_t)half * (BN * 128) + (size_t)in_tile * ps * 128, &kvmap, lane0 + half * 64, ((page * 2 + (int)is_v) * p.KV + kvh) * ps, &full[s]);
             }
         }
     } else if (warp == 5) {
@@ -228,41 +266,69 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         }
     } else if (warp == 7) {
         // ---- issuer of the second product: O += P_j V_j, as soon as the probabilities and the values are there ----
-        if (lane == 0) {
-            constexpr unsigned IDESC_PV = umma::idesc_bf16(BM, VD, true);
-            const unsigned o_tmem = tmem_base + O_COL, p_tmem = tmem_base + P_COL;
-            bool ok = true;
-            for (int j = 0; j < n_tiles && ok && !gave_up; ++j) {
-                const int s = j % STAGES;
-                ok = tma::mbar_wait(&v_full[s], (j / STAGES) & 1) && tma::mbar_wait(&p_full, j & 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                // the values lie [key][d]: B with N contiguous; 16 keys are two atoms of 8 rows, 2048 bytes further per step
-                // (a head of 128 lanes is two such pieces side by side, BN * 128 bytes apart: the leading offset)
-                const unsigned long long v_desc = umma::desc_sw128(kv_s + (size_t)s * STAGE_BYTES + K_BYTES, (V_HALVES > 1 ? BN * 128 : 1024) >> 4);
+        constexpr unsigned IDESC_PV = umma::idesc_bf16(BM, VD, true);
+        const unsigned o_tmem = tmem_base + O_COL, p_tmem = tmem_base + P_COL;
+        bool ok = true;  // the loop's head: as lane 0 has it
+        for (int j = 0; j < n_tiles && __shfl_sync(0xffffffffu, (int)(ok && !gave_up), 0); ++j) {
+            const int s = j % STAGES;
+            unsigned char* values = kv_s + (size_t)s * STAGE_BYTES + K_BYTES;
+            const int real = ctx_len - tile_start(j);  // keys of this tile that the request has
+            if (lane == 0) ok = tma::mbar_wait(&v_full[s], (j / STAGES) & 1);
+            if (real < BN) {
+                // rows that are not the request's: a probability of zero times what is no number would be none either
+                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0 && tma::mbar_wait(&v_full[s], (j / STAGES) & 1);
+                if (ok)
+                    for (int i = max(real, 0) * 8 + lane; i < BN * 8; i += 32)
 #pragma unroll
-                for (int k = 0; k < BN / 16; ++k)  // the output accumulates over the tiles
-                    umma::mma_bf16_ts(o_tmem, p_tmem + 8 * k, v_desc + (2048 >> 4) * k, IDESC_PV, k != 0 || j != 0);
-                umma::commit(&o_full);
-                umma::commit(&v_empty[s]);
+                        for (int h = 0; h < V_HALVES; ++h) reinterpret_cast<uint4*>(values + (size_t)h * (BN * 128))[i] = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                ok = __all_sync(0xffffffffu, ok);
             }
-            if (!ok) fail();
+            if (lane == 0) {
+                ok = ok && tma::mbar_wait(&p_full, j & 1);
+                if (ok) {
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    // the values lie [key][d]: B with N contiguous; 16 keys are two atoms of 8 rows, 2048 bytes further per step
+                    // (a head of 128 lanes is two such pieces side by side, BN * 128 bytes apart: the leading offset)
+                    const unsigned long long v_desc = umma::desc_sw128(values, (V_HALVES > 1 ? BN * 128 : 1024) >> 4);
+#pragma unroll
+                    for (int k = 0; k < BN / 16; ++k)  // the output accumulates over the tiles
+                        umma::mma_bf16_ts(o_tmem, p_tmem + 8 * k, v_desc + (2048 >> 4) * k, IDESC_PV, k != 0 || j != 0);
+                    umma::commit(&o_full);
+                    umma::commit(&v_empty[s]);
+                }
+            }
+            __syncwarp();
         }
+        if (!ok && lane == 0) fail();
     } else {
         // ---- softmax: thread = query row = lane of tensor memory ----
         const int row = warp * 32 + lane, tok = row0 + row;
         const bool row_ok = tok < q_len;
         const int pos = pos0 + tok;
-        const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+        const int lo = first_seen(pos), kept_of_row = EXTRA && p.window > 0 ? tp.keep_first : 0;
         const unsigned lane_base = tmem_base + ((unsigned)(warp * 32) << 16);
-        float m_run = -INFINITY, l_run = 0.f;
+        // a sink has been seen before the first key
+        float m_run = tp.sinks ? tp.sinks[head] * LOG2E : -INFINITY, l_run = tp.sinks ? 1.f : 0.f;
+        const float slope = EXTRA && tp.slopes ? tp.slopes[head] * LOG2E : 0.f;
+        const float cap2 = tp.softcap * LOG2E, cap_in = EXTRA && tp.softcap > 0.f ? 2.f * p.scale_log2 / tp.softcap : 0.f;
+        const float scale_log2 = EXTRA ? 1.f : p.scale_log2;  // what is left to do to a score
         bool ok = true;
         const unsigned o_taddr = lane_base + O_COL;
         if constexpr (Sh::Q_IN_TMEM) {  // the row's queries, as they lie in memory (two to a word), into the row's lane of tensor memory
             unsigned qw[32];
-            const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)(q_begin + tok) * p.q_stride + (size_t)q_head * KD);
+            if constexpr (OWN) {  // the last lanes first: 16 words, and 16 whose place the probabilities take
+                const uint4* rot = reinterpret_cast<const uint4*>(tp.q1 + (size_t)(q_begin + tok) * tp.q1_token + (size_t)head * tp.q1_head);
 #pragma unroll
-            for (int c = 0; c < KD / 8; ++c) {
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 u = row_ok && c < 4 ? rot[c] : make_uint4(0, 0, 0, 0);
+                    qw[4 * c] = u.x; qw[4 * c + 1] = u.y; qw[4 * c + 2] = u.z; qw[4 * c + 3] = u.w;
+                }
+                umma::tmem_st32(lane_base + Q_COL + 32, qw);
+            }
+            const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)(q_begin + tok) * p.q_stride + (OWN ? (size_t)head * tp.q_head : (size_t)q_head * KD));
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
                 const uint4 u = row_ok ? src[c] : make_uint4(0, 0, 0, 0);
                 qw[4 * c] = u.x; qw[4 * c + 1] = u.y; qw[4 * c + 2] = u.z; qw[4 * c + 3] = u.w;
             }
@@ -278,14 +344,15 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
 #define PH(i)
 #endif
         for (int j = 0; j < n_tiles; ++j) {
-            const int key_base = (t_begin + j) * BN;
+            const int key_base = tile_start(j);
             ok = __all_sync(0xffffffffu, !gave_up && tma::mbar_wait(&s_full[j % NBUF], (j / NBUF) & 1));
             PH(0)
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const bool whole = key_base + BN - 1 <= tile_pos_min && key_base >= tile_lo_max && rows_here == BM;
+            const bool whole = key_base + BN - 1 <= tile_pos_min && (key_base >= tile_lo_max || (EXTRA && key_base + BN <= kept)) && rows_here == BM;
             // the keys of this tile that the row sees are those with index (within the tile) in [see_lo, see_hi]
-            const int see_lo = row_ok ? lo - key_base : BN, see_hi = row_ok ? pos - key_base : -1;
+            // (and, in EXTRA, below see_kept)
+            const int see_lo = row_ok ? lo - key_base : BN, see_hi = row_ok ? pos - key_base : -1, see_kept = EXTRA ? kept_of_row - key_base : 0;
             // the row's 64 scores in one load; once they are in registers the buffer may take the scores two tiles on
             static_assert(BN == 64, "the softmax reads a tile's scores with one 64-column load");
             float v[BN];
@@ -297,18 +364,34 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             // the row's maximum (four chains, so that the comparisons do not wait for one another; the scale is
             // positive and is applied to the maximum alone)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            if constexpr (EXTRA) {
+                // the cap: tanh(t) = 1 - 2 / (e^(2t) + 1), through exp2 and a reciprocal (absolute error near 1e-7, which the cap
+                // multiplies: far below what the bfloat16 operands leave; both ends saturate to +-1)
+                if (tp.softcap > 0.f) {
+#pragma unroll
+                    for (int i = 0; i < BN; ++i) v[i] = cap2 * (1.f - __fdividef(2.f, exp2f(v[i] * cap_in) + 1.f));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < BN; ++i) v[i] *= p.scale_log2;
+                }
+                if (tp.slopes) {
+                    const float away = (float)(key_base - pos);
+#pragma unroll
+                    for (int i = 0; i < BN; ++i) v[i] = fmaf(slope, away + (float)i, v[i]);
+                }
+            }
             if (whole) {
 #pragma unroll
                 for (int i = 0; i < BN; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], v[i]);
             } else {
 #pragma unroll
                 for (int i = 0; i < BN; ++i) {
-                    const bool visible = i >= see_lo && i <= see_hi;
+                    const bool visible = (i >= see_lo || (EXTRA && i < see_kept)) && i <= see_hi;
                     v[i] = visible ? v[i] : -INFINITY;
                     mx4[i & 3] = fmaxf(mx4[i & 3], v[i]);
                 }
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
             // The output accumulates in tensor memory, scaled by 2^-m_run.  The row keeps its old shift while the new
             // maximum is less than 2^LAZY above it (any shift gives the same quotient in the end; probabilities then
             // reach 2^LAZY at most, which bfloat16 holds with its usual relative error), so the accumulated output
@@ -318,14 +401,14 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             const float m_new = grow ? m_cand : m_run;
             const float m_use = m_new == -INFINITY ? 0.f : m_new;
             const float alpha = attn::fast_exp2(m_run - m_use);  // 1 where the shift stays
-            const bool rescale = grow && m_run != -INFINITY;  // (a row that has seen no key yet has an output of zeros)
+            const bool rescale = grow && m_run != -INFINITY && j > 0;  // (a row that has seen no key yet has an output of zeros)
             m_run = m_new;
             PH(2)
             // the probabilities (a masked score is -inf: its probability is exactly 0), two to a word: the second
             // product's A operand, stored into the row's lane of tensor memory once the product before has read its own
             unsigned pw[BN / 2];
             float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // four chains, two per packed add
-            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(-m_use, -m_use);
+            const float2 scale2 = make_float2(scale_log2, scale_log2), shift2 = make_float2(-m_use, -m_use);
 #pragma unroll
             for (int c = 0; c < BN / 8; ++c) {
 #pragma unroll
@@ -387,9 +470,11 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             if (lane == 0) fail();
         } else if (n_tiles > 0) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            float inv = 1.f / l_run;
+            float inv = l_run == 0.f ? 0.f : 1.f / l_run;  // every key scored -inf: zeros
             __nv_bfloat16* dst = p.out + (size_t)(q_begin + tok) * p.out_stride + (size_t)head * VD;
-            if (tp.gate && row_ok) inv /= 1.f + expf(-tp.gate[(size_t)(q_begin + tok) * tp.gate_token + head]);
+            const float* gate = tp.gate ? tp.gate + (size_t)(q_begin + tok) * tp.gate_token + (tp.gate_lanes ? head * VD : head) : nullptr;
+            if (gate && !tp.gate_lanes && row_ok) inv /= 1.f + expf(-*gate);
+            if (OWN && tp.stats && row_ok) tp.stats[(size_t)(q_begin + tok) * p.H + head] = make_float2(m_run, l_run);
             if (tp.turn) {
                 const float4* cs = reinterpret_cast<const float4*>(tp.turn + (size_t)(q_begin + tok) * (VD / 2));  // two pairs each
 #pragma unroll 1
@@ -429,6 +514,16 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
                     for (int c = 0; c < 64; c += 4)
                         *reinterpret_cast<float4*>(raw + c) = make_float4(o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv);
                 } else if (row_ok) {
+                    if (gate && tp.gate_lanes) {
+#pragma unroll
+                        for (int c = 0; c < 64; c += 4) {
+                            const float4 g = *reinterpret_cast<const float4*>(gate + 64 * h + c);
+                            o[c] *= 1.f / (1.f + __expf(-g.x));
+                            o[c + 1] *= 1.f / (1.f + __expf(-g.y));
+                            o[c + 2] *= 1.f / (1.f + __expf(-g.z));
+                            o[c + 3] *= 1.f / (1.f + __expf(-g.w));
+                        }
+                    }
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         uint4 u;
@@ -493,22 +588,15 @@ join_maps_kernel(const float* __restrict__ raw, const int* __restrict__ token_re
 LLM_EXPORT int llm_attention_tcgen05_min_tokens() { return 128; }
 
 namespace {
-template <int KD, int VD>
-int launch_tcgen05(const TcParams& tp, const void* q, int q_stride, int n_tokens, const void* pool, long long kv_rows, int row_lanes,
-                   int page_size, unsigned grid_y, cudaStream_t stream) {
+template <int KD, int VD, bool EXTRA, bool OWN>
+int launch_tcgen05(const TcParams& tp, const CUtensorMap* qmap, const CUtensorMap* kvmap, unsigned grid_y, cudaStream_t stream) {
     using Sh = Shape<KD, VD>;
-    // one box of keys or values: a page's rows, 64 of the head's lanes; one box of queries: 128 tokens, 64 lanes of a head
-    const CUtensorMap* kvmap = tma::cached_map_2d_bf16(pool, (uint64_t)kv_rows, (uint64_t)row_lanes, (uint64_t)row_lanes, (uint32_t)page_size, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap* qmap = Sh::Q_IN_TMEM ? kvmap
-                                            : tma::cached_map_2d_bf16(q, (uint64_t)n_tokens, (uint64_t)tp.a.H * tp.maps * KD, (uint64_t)q_stride, BM, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!kvmap || !qmap) return LLM_ERR_UNSUPPORTED;
-    static bool configured = false;  // per head size
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    return launch_pdl(attention_tcgen05_kernel<KD, VD>, dim3((unsigned)(tp.a.H * tp.maps), grid_y), dim3(THREADS), Sh::SMEM, stream, tp, *qmap, *kvmap);
+    auto kernel = attention_tcgen05_kernel<KD, VD, EXTRA, OWN>;
+    // at every launch: the limit holds for the current device, and a process may have several
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    return launch_pdl(kernel, dim3((unsigned)(tp.a.H * tp.maps), grid_y), dim3(THREADS), Sh::SMEM, stream, tp, *qmap, *kvmap);
 }
 
 struct Differential {  // how two maps meet (raw == null: one map a head)
@@ -517,19 +605,31 @@ struct Differential {  // how two maps meet (raw == null: one map a head)
     const int* token_request;
 };
 
+struct Options {  // as in TcParams
+    const float2* turn;
+    const float* gate;
+    long long gate_token;
+    int gate_lanes;
+    const float *sinks, *slopes;
+    float softcap;
+    int keep_first, chunk;
+};
+
 int attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, const void* pool, long long pool_pages, const int* page_table,
                       int table_width, const int* cu_tokens, const int* ctx_lens, int requests, int n_tokens, int H, int KV, int KD, int VD,
-                      int row_lanes, int page_size, int window, float scale, int min_tokens, int max_tokens, const float2* turn, const float* gate,
-                      long long gate_token, const Differential& diff, int* error_flag, cudaStream_t stream) {
+                      int row_lanes, int page_size, int window, float scale, int min_tokens, int max_tokens, const Options& opt,
+                      const Differential& diff, int* error_flag, cudaStream_t stream) {
     if (n_tokens <= 0 || requests <= 0 || max_tokens < min_tokens) return 0;
     const bool sizes = (KD == 64 && (VD == 64 || VD == 128)) || (KD == 128 && VD == 128);
     if (!sizes || (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64)) return LLM_ERR_UNSUPPORTED;
     const int maps = diff.raw ? 2 : 1;
     if (H <= 0 || KV <= 0 || H % KV || table_width <= 0 || min_tokens < 1 || !(scale > 0.f) || row_lanes < maps * KD || row_lanes < VD ||
-        (diff.raw && (turn || gate || !diff.token_request)))
+        (diff.raw && (opt.turn || opt.gate || opt.sinks || !diff.token_request)) || (opt.turn && opt.gate && opt.gate_lanes) || opt.keep_first < 0 ||
+        opt.chunk < 0)
         return LLM_ERR_BAD_ARGUMENT;
     if ((q_stride & 7) || (out_stride & 7) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)pool & 127) || q_stride < H * maps * KD ||
-        (row_lanes & 7) || ((uintptr_t)turn & 15) || ((uintptr_t)diff.raw & 15))
+        (row_lanes & 7) || ((uintptr_t)opt.turn & 15) || ((uintptr_t)diff.raw & 15) ||
+        (opt.gate && opt.gate_lanes && (((uintptr_t)opt.gate & 15) || (opt.gate_token & 3))))
         return LLM_ERR_UNSUPPORTED;
     const long long kv_rows = pool_pages * 2 * KV * page_size;
     if (kv_rows <= 0 || kv_rows > 0x7fffffffLL) return LLM_ERR_UNSUPPORTED;
@@ -553,15 +653,26 @@ int attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, co
     tp.error_flag = error_flag;
     tp.maps = maps;
     tp.raw = diff.raw;
-    tp.turn = turn;
-    tp.gate = gate;
-    tp.gate_token = gate_token;
+    tp.turn = opt.turn;
+    tp.gate = opt.gate;
+    tp.gate_token = opt.gate_token;
+    tp.gate_lanes = opt.gate_lanes;
+    tp.sinks = opt.sinks;
+    tp.slopes = opt.slopes;
+    tp.softcap = opt.softcap;
+    tp.keep_first = opt.keep_first;
+    tp.chunk = opt.chunk;
     const long long y = (long long)requests * tp.tiles_per_request;
     if (y > 65535) return LLM_ERR_UNSUPPORTED;
+    // one box of keys or values: a page's rows, 64 of the head's lanes; one box of queries: 128 tokens, 64 lanes of a head
+    const CUtensorMap* kvmap = tma::cached_map_2d_bf16(pool, (uint64_t)kv_rows, (uint64_t)row_lanes, (uint64_t)row_lanes, (uint32_t)page_size, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    const CUtensorMap* qmap = KD == 64 ? kvmap
+                                       : tma::cached_map_2d_bf16(q, (uint64_t)n_tokens, (uint64_t)H * maps * KD, (uint64_t)q_stride, BM, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    const bool extra = opt.slopes || opt.softcap > 0.f || (opt.keep_first > 0 && window > 0);
     int code;
-    if (KD == 64 && VD == 64) code = launch_tcgen05<64, 64>(tp, q, q_stride, n_tokens, pool, kv_rows, row_lanes, page_size, (unsigned)y, stream);
-    else if (KD == 64) code = launch_tcgen05<64, 128>(tp, q, q_stride, n_tokens, pool, kv_rows, row_lanes, page_size, (unsigned)y, stream);
-    else code = launch_tcgen05<128, 128>(tp, q, q_stride, n_tokens, pool, kv_rows, row_lanes, page_size, (unsigned)y, stream);
+    if (KD == 64 && VD == 64) code = extra ? launch_tcgen05<64, 64, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<64, 64, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
+    else if (KD == 64) code = extra ? launch_tcgen05<64, 128, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<64, 128, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
+    else code = extra ? launch_tcgen05<128, 128, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<128, 128, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
     if (code != 0 || maps == 1) return code;
     const long long items = (long long)n_tokens * H;
     auto join = [&](auto kernel) {
@@ -581,20 +692,68 @@ LLM_EXPORT int llm_attention_tcgen05(const void* q, int q_stride, void* out, int
                                      int requests, int n_tokens, int H, int KV, int D, int page_size, int window, float scale,
                                      int min_tokens, int max_tokens, int* error_flag, cudaStream_t stream) {
     return attention_tcgen05(q, q_stride, out, out_stride, pool, pool_pages, page_table, table_width, cu_tokens, ctx_lens, requests, n_tokens, H, KV, D, D,
-                             D, page_size, window, scale, min_tokens, max_tokens, nullptr, nullptr, 0, Differential{}, error_flag, stream);
+                             D, page_size, window, scale, min_tokens, max_tokens, Options{}, Differential{}, error_flag, stream);
 }
 
 // The same with keys of KD and values of VD lanes (64 and 64, 64 and 128, 128 and 128) in rows of row_lanes; `turn` [tokens, VD / 2] pairs
-// (cos, sin) or null: values that turn back; `gate` (row pitch gate_token) or null: one gate a head; `raw` [tokens, H, 2, VD] (32-bit
-// scratch) or null: two score maps a head, whose results meet as u / sqrt(mean(u^2) + diff_eps) * diff_scale, u = a1 - diff_weight * a2
-// (a second launch; without turn and gate).
+// (cos, sin) or null: values that turn back; `gate` (row pitch gate_token) or null: one gate a head, with gate_lanes one a lane (not with
+// turn); `sinks` and `slopes` [H] or null; softcap (0: none); keep_first (with a window) and chunk (0: none) as in llm_attention_rows;
+// `raw` [tokens, H, 2, VD] (32-bit scratch) or null: two score maps a head, whose results meet as u / sqrt(mean(u^2) + diff_eps) *
+// diff_scale, u = a1 - diff_weight * a2 (a second launch; without turn, gate and sinks).
 LLM_EXPORT int llm_attention_tcgen05_general(const void* q, int q_stride, void* out, int out_stride, const void* pool, long long pool_pages,
                                              const int* page_table, int table_width, const int* token_request, const int* cu_tokens,
                                              const int* ctx_lens, int requests, int n_tokens, int H, int KV, int KD, int VD, int row_lanes,
                                              int page_size, int window, float scale, int min_tokens, int max_tokens, const void* turn,
-                                             const float* gate, long long gate_token, float* raw, float diff_weight, float diff_eps,
+                                             const float* gate, long long gate_token, int gate_lanes, const float* sinks, const float* slopes,
+                                             float softcap, int keep_first, int chunk, float* raw, float diff_weight, float diff_eps,
                                              float diff_scale, int* error_flag, cudaStream_t stream) {
     const Differential diff = {raw, diff_weight, diff_eps, diff_scale, token_request};
+    const Options opt = {(const float2*)turn, gate, gate_token, gate_lanes, sinks, slopes, softcap, keep_first, chunk};
     return attention_tcgen05(q, q_stride, out, out_stride, pool, pool_pages, page_table, table_width, cu_tokens, ctx_lens, requests, n_tokens, H, KV, KD, VD,
-                             row_lanes, page_size, window, scale, min_tokens, max_tokens, (const float2*)turn, gate, gate_token, diff, error_flag, stream);
+                             row_lanes, page_size, window, scale, min_tokens, max_tokens, opt, diff, error_flag, stream);
+}
+
+// Attention over the step's own tokens of every request that brings at least min_tokens: keys of 64 + 32 lanes, values of 64.  q0
+// [tokens, H, 64] and q1 [tokens, H, 32] (strides in elements); kv [tokens, kv_stride]: head h's 64 key lanes from column h * 64, its
+// values from values_col + h * 64; rot [tokens, rot_stride]: the key lanes that all heads share are the row's last 32, from rot_col;
+// out [tokens, H * 64]; stats [tokens, H, 2] or null: every row's maximum (in units of log 2) and sum.
+LLM_EXPORT int llm_attention_tcgen05_own(const void* q0, long long q0_token, long long q0_head, const void* q1, long long q1_token, long long q1_head,
+                                         void* out, int out_stride, const void* kv, int kv_stride, int values_col, const void* rot, int rot_stride,
+                                         int rot_col, const int* cu_tokens, int requests, int n_tokens, int H, int window, float scale, int min_tokens,
+                                         int max_tokens, float* stats, int* error_flag, cudaStream_t stream) {
+    if (n_tokens <= 0 || requests <= 0 || max_tokens < min_tokens) return 0;
+    if (H <= 0 || min_tokens < 1 || !(scale > 0.f) || values_col < H * 64 || kv_stride < values_col + H * 64 || rot_col < 0 || rot_col + 32 != rot_stride)
+        return LLM_ERR_BAD_ARGUMENT;
+    if (((q0_token | q0_head | q1_token | q1_head | out_stride | kv_stride | values_col | rot_stride | rot_col) & 7) || q0_token > 0x7fffffffLL ||
+        (((uintptr_t)q0 | (uintptr_t)q1 | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)rot) & 15) || ((uintptr_t)stats & 7))
+        return LLM_ERR_UNSUPPORTED;
+    TcParams tp = {};
+    tp.a.q = (const __nv_bfloat16*)q0;
+    tp.q1 = (const __nv_bfloat16*)q1;
+    tp.q_head = q0_head;
+    tp.q1_token = q1_token;
+    tp.q1_head = q1_head;
+    tp.a.q_stride = (int)q0_token;
+    tp.a.out = (__nv_bfloat16*)out;
+    tp.a.out_stride = out_stride;
+    tp.a.cu_tokens = cu_tokens;
+    tp.a.H = H;
+    tp.a.KV = H;
+    tp.a.G = 1;
+    tp.a.page_size = BN;
+    tp.a.window = window;
+    tp.a.scale_log2 = scale * LOG2E;
+    tp.min_tokens = min_tokens;
+    tp.tiles_per_request = (max_tokens + BM - 1) / BM;
+    tp.error_flag = error_flag;
+    tp.maps = 1;
+    tp.own_values = values_col;
+    tp.own_rot = rot_col;
+    tp.stats = (float2*)stats;
+    const long long y = (long long)requests * tp.tiles_per_request;
+    if (y > 65535) return LLM_ERR_UNSUPPORTED;
+    // (the rows' last 32 lanes in boxes of 64: behind a row's end a box is filled with zeros)
+    const CUtensorMap* kvmap = tma::cached_map_2d_bf16(kv, (uint64_t)n_tokens, (uint64_t)values_col + H * 64, (uint64_t)kv_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    const CUtensorMap* rotmap = tma::cached_map_2d_bf16(rot, (uint64_t)n_tokens, (uint64_t)rot_stride, (uint64_t)rot_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    return launch_tcgen05<96, 64, false, true>(tp, rotmap, kvmap, (unsigned)y, stream);
 }

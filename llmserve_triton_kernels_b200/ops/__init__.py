@@ -62,7 +62,8 @@ _SIGNATURES = {
                                _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp, _ll, _i, _vp, _vp, _vp, _ll, _i, _i, _f,
                                _i, _i, _ll, _ll, _f, _f, _f, _vp, _i, _i, _i, _vp],
     "llm_attention_tcgen05_general": [_vp, _i, _vp, _i, _vp, _ll, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,
-                                      _vp, _ll, _vp, _f, _f, _f, _vp, _vp],
+                                      _vp, _ll, _i, _vp, _vp, _f, _i, _i, _vp, _f, _f, _f, _vp, _vp],
+    "llm_attention_tcgen05_own": [_vp, _ll, _ll, _vp, _ll, _ll, _vp, _i, _vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp, _vp, _vp],
     "llm_experts_few": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp],
     "llm_experts_many": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _f,
                          _vp, _vp],
@@ -133,6 +134,7 @@ _TC_ATTENTION_ENABLED = True
 _TC_ATTENTION_HEAD_DIMS = (64, 128)
 _TC_ATTENTION_PAGE_SIZES = (8, 16, 32, 64)
 _TC_ATTENTION_MIN_TOKENS = 128  # a request with at least this many tokens in the step: attention on tcgen05
+_TC_ATTENTION_JOIN_TOKENS = 32  # where that kernel runs, requests of at least so many go along (tiles of their own beside the others')
 _TCGEN05_MIN_ROWS = 128  # from this many rows a bfloat16 product runs on tcgen05 with TMA-fed tiles (own kernel)
 _DECODE_LINEAR_MAX_ROWS = 16  # up to this many rows a bfloat16 matrix product streams the weights once (own kernel)
 _FORCE_GENERIC_ATTENTION = False  # tests switch the tensor-core attention off to reach the general kernel in bfloat16
@@ -771,8 +773,9 @@ def paged_attention(
         # requests that bring at least 128 tokens: 128-token tiles of one head on tcgen05 (head sizes 64 and 128, pages
         # of 8 to 64 keys); the others: rows of (token, group member) on mma.sync, 64 rows a tile or the split-key shape
         tc_min = 0
-        if head_dim in _TC_ATTENTION_HEAD_DIMS and pool.shape[3] in _TC_ATTENTION_PAGE_SIZES and _TC_ATTENTION_ENABLED:
-            tc_min = _TC_ATTENTION_MIN_TOKENS
+        if (head_dim in _TC_ATTENTION_HEAD_DIMS and pool.shape[3] in _TC_ATTENTION_PAGE_SIZES and _TC_ATTENTION_ENABLED
+                and (getattr(ctx, "max_query_len", None) or max(_token_counts(ctx))) >= _TC_ATTENTION_MIN_TOKENS):
+            tc_min = _TC_ATTENTION_JOIN_TOKENS
         num_requests, tc_longest, small, max_rows_large, other_rows = _attention_route(ctx, group, tc_min)
         if tc_longest:
             code = _launch(
@@ -1223,7 +1226,7 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
                    leave_parts: bool = False, sinks: torch.Tensor | None = None, gate: torch.Tensor | None = None,
                    keep_first: int | None = None, chunk: int | None = None, softcap: float | None = None, gate_per_head: bool = False,
                    differential: "DifferentialMaps | None" = None, turn: torch.Tensor | None = None, turn_neighbours: bool = False,
-                   out: torch.Tensor | None = None, skip_from: int = 0):
+                   out: torch.Tensor | None = None, skip_from: int = 0, stats: torch.Tensor | None = None):
     """Attention in its general form: queries ``q0 [N, H, d0]`` and optionally ``q1 [N, H, d1]`` (lanes behind q0's),
     keys and values addressed by ``(page, head, token)`` strides in elements, an optional bias ``-slopes[h] * distance``.
     Returns ``[N, H, value_dim]``.
@@ -1231,7 +1234,8 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
     ``key_part`` (bfloat16 on the tensor cores only): 1 = only the keys cached before this step; 2 = only the step's own
     tokens, whose keys and values lie token by token (``keys`` lanes ``[0, fresh_d0)`` per head, ``keys1`` the lanes
     behind them, one row a token for all heads).  With ``want_stats`` the result is ``(out, stats [N, H, 2])``: each row's
-    maximum score and sum of exponentials (a row without keys: ``-inf, 0``, and an output that is not to be read), for :func:`merge_two_parts`.
+    maximum score and sum of exponentials (a row without keys: ``-inf, 0``, and an output that is not to be read), for :func:`merge_two_parts`
+    (in ``stats`` where the caller has a place for it).
     ``leave_parts``: where the keys are cut over several CTAs the partial results are not merged but returned as an
     :class:`AttentionParts`, for a kernel that merges them on its way (:func:`merge_project_gate`).
     ``sinks`` (float32 ``[H]``): every head's softmax has one more term ``exp(sinks[h])`` in its denominator, with no key and
@@ -1294,7 +1298,8 @@ def attention_rows(q0, q1, keys, k_strides, values, v_strides, value_dim: int, p
             few = 0 if shares == 0 else 2 if getattr(ctx, "steps_apart", False) else 1
             splits = shares or splits
             leave = leave_parts and splits > 1
-        stats = torch.empty((n, num_heads, 2), dtype=torch.float32, device=q0.device) if want_stats else None
+        if want_stats and stats is None:
+            stats = torch.empty((n, num_heads, 2), dtype=torch.float32, device=q0.device)
         part_o = part_ml = None
         if splits > 1 and (leave or not few):
             part_o = torch.empty((n * num_heads * maps * splits * value_dim,), dtype=torch.float32, device=q0.device)
@@ -1407,10 +1412,28 @@ def fresh_latent_attention(q_plain: torch.Tensor, q_rot: torch.Tensor, kv: torch
     rot = fresh.shape[1] - rank
     _need(kv.is_contiguous() and fresh.is_contiguous() and kv.shape[1] == heads * (dim + value_dim), "fresh_latent_attention: kv [N, H dim | H vdim]")
     element = kv.element_size()
+    out = torch.empty((n, heads, value_dim), dtype=kv.dtype, device=kv.device)
+    stats = torch.empty((n, heads, 2), dtype=torch.float32, device=kv.device) if want_stats else None
+    taken = 0
+    if (kv.dtype == torch.bfloat16 and (dim, rot, value_dim) == (64, 32, 64) and _TC_ATTENTION_ENABLED and not _FORCE_GENERIC_ATTENTION
+            and ctx.max_query_len >= _TC_ATTENTION_MIN_TOKENS and q_plain.stride(2) == 1 and q_rot.stride(2) == 1):
+        counts = _token_counts(ctx)
+        code = _launch(
+            "llm_attention_tcgen05_own", _ptr(q_plain), q_plain.stride(0), q_plain.stride(1), _ptr(q_rot), q_rot.stride(0), q_rot.stride(1),
+            _ptr(out), out.stride(0), _ptr(kv), kv.stride(0), heads * dim, _ptr(fresh), fresh.stride(0), rank, _ptr(ctx.cu_tokens), len(counts), n,
+            heads, int(window or 0), float(scale), _TC_ATTENTION_JOIN_TOKENS, max(counts), _ptr(stats), _error_flag_ptr(), _stream(),
+        )
+        if code == 10002:
+            add_launches(-1)
+        else:
+            _check(code, "fresh_latent_attention (tcgen05)")
+            taken = _TC_ATTENTION_JOIN_TOKENS
+            if min(counts) >= taken:
+                return (out, stats) if want_stats else out
     return attention_rows(q_plain, q_rot, kv.data_ptr(), (0, dim, kv.stride(0)), kv.data_ptr() + heads * dim * element,
                           (0, value_dim, kv.stride(0)), value_dim, page_table, 1, ctx, num_heads=heads, num_kv_heads=heads,
                           scale=scale, window=window, key_part=2, keys1=fresh.data_ptr() + rank * element, k1_token=rank + rot,
-                          fresh_d0=dim, want_stats=want_stats)
+                          fresh_d0=dim, want_stats=want_stats, out=out, skip_from=taken, stats=stats)
 
 
 def biased_paged_attention(qkv: torch.Tensor, pool: torch.Tensor, page_table: torch.Tensor, ctx, *, num_heads: int, num_kv_heads: int,
@@ -1426,9 +1449,14 @@ def biased_paged_attention(qkv: torch.Tensor, pool: torch.Tensor, page_table: to
     q = qkv.as_strided((qkv.shape[0], num_heads, key_dim), (qkv.stride(0), key_dim, 1), qkv.storage_offset())
     head, page = page_size * row, 2 * num_kv_heads * page_size * row
     values = pool.data_ptr() + num_kv_heads * head * pool.element_size()
-    out = attention_rows(q, None, _ptr(pool), (page, head, row), values, (page, head, row), value_dim, page_table, page_size, ctx,
-                         num_heads=num_heads, num_kv_heads=num_kv_heads, scale=scale, window=window, slopes=slopes)
-    return out.view(qkv.shape[0], num_heads * value_dim)
+    out = torch.empty((qkv.shape[0], num_heads * value_dim), dtype=qkv.dtype, device=qkv.device)
+    taken, rest = _tcgen05_softmax_attention(qkv[:, : num_heads * key_dim], pool, page_table, ctx, out, num_heads, num_kv_heads, key_dim, value_dim, scale,
+                                             window, None, None, None, slopes=slopes)
+    if not taken or rest:
+        attention_rows(q, None, _ptr(pool), (page, head, row), values, (page, head, row), value_dim, page_table, page_size, ctx,
+                       num_heads=num_heads, num_kv_heads=num_kv_heads, scale=scale, window=window, slopes=slopes,
+                       out=out.view(qkv.shape[0], num_heads, value_dim), skip_from=taken)
+    return out
 
 
 def paged_softmax_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Tensor, ctx, *, num_heads: int, num_kv_heads: int,
@@ -1457,9 +1485,10 @@ def paged_softmax_attention(q: torch.Tensor, pool: torch.Tensor, page_table: tor
     if out is None:
         out = torch.empty((q.shape[0], num_heads * value_dim), dtype=q.dtype, device=q.device)
     taken = 0  # requests of at least so many tokens that the tcgen05 kernel has taken
-    if sinks is None and not keep_first and not chunk and not softcap and slopes is None and not turn_neighbours and (gate is None or gate_per_head):
+    if not turn_neighbours:
         taken, rest = _tcgen05_softmax_attention(q, pool, page_table, ctx, out, num_heads, num_kv_heads, key_dim // (2 if differential is not None else 1),
-                                                 value_dim, scale, window, gate, differential, turn)
+                                                 value_dim, scale, window, gate, differential, turn, sinks=sinks, slopes=slopes, softcap=softcap,
+                                                 keep_first=keep_first, chunk=chunk, gate_per_head=gate_per_head)
         if taken and not rest:
             return out
     o3 = out.as_strided((q.shape[0], num_heads, value_dim), (out.stride(0), value_dim, 1), out.storage_offset())
@@ -1486,17 +1515,24 @@ _TC_SOFTMAX_SIZES = ((64, 64), (64, 128), (128, 128))  # lanes of a key (of one 
 
 
 def _tcgen05_softmax_attention(q, pool, page_table, ctx, out, heads: int, kv_heads: int, key_dim: int, value_dim: int, scale: float,
-                               window, gate, differential, turn) -> tuple[int, bool]:
-    """The part of :func:`paged_softmax_attention` that the tcgen05 kernel takes: bfloat16 requests that bring at least
-    ``_TC_ATTENTION_MIN_TOKENS`` tokens.  Returns ``(that number or 0 if it took none, whether other requests are left)``."""
+                               window, gate, differential, turn, sinks=None, slopes=None, softcap=None, keep_first=None, chunk=None,
+                               gate_per_head: bool = True) -> tuple[int, bool]:
+    """The part of :func:`paged_softmax_attention` that the tcgen05 kernel takes: bfloat16 requests of at least ``_TC_ATTENTION_JOIN_TOKENS``
+    tokens in a step in which one brings ``_TC_ATTENTION_MIN_TOKENS`` or more.  Returns ``(the fewest tokens of a request that it took or 0
+    if it took none, whether other requests are left)``."""
     if (q.dtype != torch.bfloat16 or _FORCE_GENERIC_ATTENTION or not _TC_ATTENTION_ENABLED or (key_dim, value_dim) not in _TC_SOFTMAX_SIZES
-            or pool.shape[3] not in _TC_ATTENTION_PAGE_SIZES or (differential is not None and (gate is not None or turn is not None))
-            or ctx.max_query_len < _TC_ATTENTION_MIN_TOKENS):
+            or pool.shape[3] not in _TC_ATTENTION_PAGE_SIZES or (differential is not None and (gate is not None or turn is not None or sinks is not None))
+            or (turn is not None and gate is not None and not gate_per_head) or ctx.max_query_len < _TC_ATTENTION_MIN_TOKENS):
         return 0, True
     if turn is not None:
         _need(turn.dtype == torch.float32 and turn.is_contiguous() and tuple(turn.shape) == (q.shape[0], value_dim // 2, 2), "turn: float32 [N, value_dim / 2, 2]")
     if gate is not None:
-        _need(gate.dtype == torch.float32 and gate.dim() == 2 and gate.stride(1) == 1 and gate.shape[0] == q.shape[0] and gate.shape[1] >= heads, "the gate must be float32 [N, heads]")
+        _need(gate.dtype == torch.float32 and gate.dim() == 2 and gate.stride(1) == 1 and gate.shape[0] == q.shape[0]
+              and gate.shape[1] >= heads * (1 if gate_per_head else value_dim), "the gate must be float32 [N, heads * value_dim] (or [N, heads])")
+    for t, what in ((sinks, "sinks"), (slopes, "slopes")):
+        _need(t is None or (t.dtype == torch.float32 and t.numel() == heads and t.is_contiguous()), f"{what} must be float32 [heads]")
+    keep_first, chunk, softcap = int(keep_first or 0) if window else 0, int(chunk or 0), float(softcap or 0.0)
+    _need(keep_first >= 0 and chunk >= 0 and softcap >= 0.0, "attention: keep_first, chunk and softcap are not negative")
     _i32(page_table, "page_table")
     counts = _token_counts(ctx)
     n = q.shape[0]
@@ -1507,15 +1543,16 @@ def _tcgen05_softmax_attention(q, pool, page_table, ctx, out, heads: int, kv_hea
     code = _launch(
         "llm_attention_tcgen05_general", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(pool), pool.shape[0], _ptr(page_table), page_table.shape[1],
         _ptr(ctx.token_request), _ptr(ctx.cu_tokens), _ptr(ctx.context_lens), len(counts), n, heads, kv_heads, key_dim, value_dim, pool.shape[4], pool.shape[3],
-        int(window or 0), float(scale), _TC_ATTENTION_MIN_TOKENS, max(counts), _ptr(turn), _ptr(gate), 0 if gate is None else gate.stride(0), _ptr(raw),
-        float(weight), float(eps), float(post), _error_flag_ptr(), _stream(),
+        int(window or 0), float(scale), _TC_ATTENTION_JOIN_TOKENS, max(counts), _ptr(turn), _ptr(gate), 0 if gate is None else gate.stride(0),
+        int(not gate_per_head), _ptr(sinks), _ptr(slopes), softcap, keep_first, chunk, _ptr(raw), float(weight), float(eps), float(post),
+        _error_flag_ptr(), _stream(),
     )
     if code == 10002:
         add_launches(-1)
         return 0, True
     _check(code, "paged_softmax_attention (tcgen05)")
     add_launches(int(raw is not None))
-    return _TC_ATTENTION_MIN_TOKENS, min(counts) < _TC_ATTENTION_MIN_TOKENS
+    return _TC_ATTENTION_JOIN_TOKENS, min(counts) < _TC_ATTENTION_JOIN_TOKENS
 
 
 def head_prepare(proj: torch.Tensor, positions: torch.Tensor | None, *, heads: int, kv_heads: int, dim: int, value_dim: int = 0,

@@ -1,0 +1,99 @@
+"""Attention of prompt portions on tcgen05 with everything that designs put around the softmax, and over a step's own tokens, beside the
+plain statement: edges of the 128-token and 64-key tiles, windows, kept keys and blocks that leave tiles out, small requests that go along,
+rows behind a request's end that hold NaN."""
+
+import pytest
+import torch
+
+import plain_ops
+from test_kafepel_kernels_gpu import DEV, _ops, close, paged_batch
+
+pytestmark = pytest.mark.gpu
+
+OPTIONS = {
+    "sinks": dict(sinks=True), "sinks far above and below": dict(sinks="far"), "gate": dict(gate=True), "sinks, gate, window": dict(sinks=True, gate=True, window=70),
+    "bias and window": dict(slopes=True, window=100), "cap": dict(softcap=5.0), "kept, window, cap, bias": dict(window=33, keep_first=16, softcap=20.0, slopes=True),
+    "many kept": dict(window=130, keep_first=200), "kept over a tile's edge": dict(window=40, keep_first=65), "blocks": dict(chunk=100),
+    "blocks and window": dict(chunk=64, window=33), "one gate a head": dict(gate="head", sinks=True),
+}
+
+
+@pytest.mark.parametrize("what", OPTIONS)
+@pytest.mark.parametrize("H,KV,D,V,page_size", [(4, 2, 64, 64, 16), (3, 1, 64, 128, 8), (2, 2, 128, 128, 64)])
+def test_options_against_plain(H, KV, D, V, page_size, what):
+    ops = _ops()
+    torch.manual_seed(H * 100 + D)
+    more = dict(OPTIONS[what])
+    ctx, table, _, pages = paged_batch([700, 129, 300, 65, 40, 9], [300, 129, 128, 32, 31, 1], page_size)
+    N, bf = ctx.num_tokens, torch.bfloat16
+    pool = (torch.randn(pages, 2, KV, page_size, max(D, V), device=DEV) * 0.7).to(bf)
+    for r, n in enumerate([700, 129, 300, 65]):  # what an earlier request left behind this one's last token
+        if n % page_size:
+            pool[int(table[r, n // page_size]), :, :, n % page_size :] = torch.nan
+    q = torch.randn(N, H * D + 8, device=DEV).to(bf)[:, : H * D]
+    if more.get("sinks"):
+        more["sinks"] = torch.randn(H, device=DEV) * 2.0 if more["sinks"] is True else torch.tensor([200.0, -200.0, float("-inf"), 3.0], device=DEV)[:H].contiguous()
+    if more.get("gate"):
+        more["gate_per_head"] = more["gate"] == "head"
+        more["gate"] = torch.randn(N, 4 + H * V + 8, device=DEV)[:, 4 : 4 + H * V]
+    if more.get("slopes"):
+        more["slopes"] = torch.rand(H, device=DEV) * 0.2
+    common = dict(num_heads=H, num_kv_heads=KV, key_dim=D, value_dim=V, scale=0.3)
+    want = plain_ops.paged_softmax_attention(q, pool, table, ctx, **common, **more)
+    launches = ops.launch_count()
+    got = ops.paged_softmax_attention(q, pool, table, ctx, **common, **more)
+    assert ops.launch_count() == launches + 2  # requests of 32 tokens and more here, the others there
+    close(got, want, 2e-2, what)
+    if "slopes" in more and not more.get("softcap"):
+        got = ops.biased_paged_attention(q, pool, table, ctx, **common, slopes=more["slopes"], window=more["window"])
+        close(got, want, 2e-2, what + " (a projection's rows)")
+
+
+def test_every_key_scores_minus_infinity():
+    """A row without a finite score is zeros; one NaN score leaves its row NaN; the rows beside them are as without them."""
+    ops = _ops()
+    ctx, table, _, pages = paged_batch([200], [200], 16)
+    pool = torch.randn(pages, 2, 1, 16, 64, device=DEV).bfloat16()
+    pool[:, 0, :, :, 0] = 1.0
+    q = torch.randn(200, 64, device=DEV).bfloat16()
+    common = dict(num_heads=1, num_kv_heads=1, key_dim=64, value_dim=64, scale=0.3)
+    same = ops.paged_softmax_attention(q, pool, table, ctx, **common)
+    q[3, 0], q[150, 0], q[160, 5] = -torch.inf, -torch.inf, torch.nan
+    got = ops.paged_softmax_attention(q, pool, table, ctx, **common)
+    assert bool((got[3] == 0).all()) and bool((got[150] == 0).all()) and bool(got[160].isnan().all())
+    rest = torch.ones(200, dtype=torch.bool)
+    rest[[3, 150, 160]] = False
+    assert same.isfinite().all() and torch.equal(got[rest], same[rest])
+
+
+@pytest.mark.parametrize("window", [None, 1, 64, 100])
+@pytest.mark.parametrize("news", [[300, 129, 40, 5], [128], [1025, 33]])
+def test_a_steps_own_tokens(news, window):
+    ops = _ops()
+    H, rank, bf = 3, 72, torch.bfloat16
+    ctx, table, _, _ = paged_batch([n + 17 * i for i, n in enumerate(news)], news, 16)
+    N = sum(news)
+    torch.manual_seed(N)
+    proj = torch.randn(N, H * 96 + 8, device=DEV).to(bf)
+    q = proj.as_strided((N, H, 64), (proj.stride(0), 96, 1))
+    q_rot, kv, fresh = torch.randn(N, H, 32, device=DEV).to(bf), torch.randn(N, H * 128, device=DEV).to(bf), torch.randn(N, rank + 32, device=DEV).to(bf)
+    args = dict(dim=64, value_dim=64, rank=rank, scale=0.2, window=window)
+    out, stats = ops.fresh_latent_attention(q, q_rot, kv, fresh, table, ctx, **args)
+    alone = ops.fresh_latent_attention(q, q_rot, kv, fresh, table, ctx, **args, want_stats=False)
+    assert torch.equal(out, alone)
+    cu = ctx.cu_tokens.tolist()
+    for a, b in zip(cu, cu[1:]):
+        qs = torch.cat((q[a:b], q_rot[a:b]), -1).double()
+        ks = torch.cat((kv[a:b, : H * 64].view(-1, H, 64), fresh[a:b, None, rank:].expand(-1, H, -1)), -1).double()
+        s = torch.einsum("ihd,jhd->hij", qs, ks) * 0.2
+        i, j = torch.arange(b - a, device=DEV)[:, None], torch.arange(b - a, device=DEV)[None]
+        s = s.masked_fill((j > i) | ((i - j >= window) if window else torch.zeros_like(i - j, dtype=torch.bool)), -torch.inf)
+        want = torch.einsum("hij,jhd->ihd", s.softmax(-1), kv[a:b, H * 64 :].view(-1, H, 64).double())
+        close(out[a:b], want, 1e-2, f"tokens {a} to {b}")
+        log_sum = stats[a:b, :, 0].double() * 0.6931471805599453 + stats[a:b, :, 1].double().log()
+        torch.testing.assert_close(log_sum, s.logsumexp(-1).T, rtol=1e-5, atol=1e-4)
+    # the next request's rows are nobody else's
+    if len(news) > 1:
+        kv[cu[1] : cu[2]] = torch.nan
+        fresh[cu[1] : cu[2]] = torch.nan
+        assert torch.equal(ops.fresh_latent_attention(q, q_rot, kv, fresh, table, ctx, **args, want_stats=False)[: cu[1]], out[: cu[1]])
