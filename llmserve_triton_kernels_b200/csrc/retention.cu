@@ -285,6 +285,69 @@ retention_scan_kernel(const float* __restrict__ q, int ldq, const float* __restr
     }
 }
 
+// The same walk for steps of few tokens a request, bound by the way to memory and back: a warp owns 16 columns of one (request, head) and
+// nothing is shared with another.  Lane (part, quarter) holds rows part * DPT .. of the quarter's four columns, from the state's rows
+// straight into registers and back (64 bytes a row), and reads the lanes of q, k and z that its rows meet.  A sum's parts and their order
+// are those of the kernel above, so a token has the same bits in both.  D = 8 * DPT, V a multiple of 16, rows on 16 bytes.
+template <typename TV, int DPT, bool GATED>
+__global__ void __launch_bounds__(64)
+scan_step_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk, const TV* __restrict__ v, int ldv,
+                 const float* __restrict__ decay, float* __restrict__ states, const int* __restrict__ state_slots, const int* __restrict__ cu_tokens,
+                 float* __restrict__ out, int H, int V, const float* __restrict__ z, int ldz, const float* __restrict__ zbias, float inv_tau, float q_scale) {
+    constexpr int D = DPT * TPC;
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, part = lane >> 2, h = blockIdx.y, r = blockIdx.z;
+    const int column = (blockIdx.x * 2 + (threadIdx.x >> 5)) * 16 + (lane & 3) * 4;
+    if (column >= V) return;  // (a warp's columns are there together)
+    const int begin = cu_tokens[r], end = cu_tokens[r + 1];
+    float* state = states + ((size_t)state_slots[r] * H + h) * D * V + (size_t)part * DPT * V + column;
+    const float gamma = GATED ? 1.f : decay[h];
+    float bias[GATED ? DPT : 1];
+#pragma unroll
+    for (int i = 0; i < (GATED ? DPT : 1); ++i) bias[i] = GATED && zbias ? zbias[h * D + part * DPT + i] : 0.f;
+    pdl_wait();
+    float S[DPT][4];
+#pragma unroll
+    for (int i = 0; i < DPT; ++i) load4(state + (size_t)i * V, S[i]);
+    // a token's lanes, the next one's on their way while one is walked
+    struct Token { float q[DPT], k[DPT], z[GATED ? DPT : 4], v[4]; };
+    auto fetch = [&](int t, Token& w) {
+        const size_t lanes = (size_t)h * D + part * DPT;
+        load4(v + (size_t)t * ldv + (size_t)h * V + column, w.v);
+#pragma unroll
+        for (int i = 0; i < DPT; i += 4) {
+            load4(q + (size_t)t * ldq + lanes + i, *reinterpret_cast<float(*)[4]>(w.q + i));
+            load4(k + (size_t)t * ldk + lanes + i, *reinterpret_cast<float(*)[4]>(w.k + i));
+            if constexpr (GATED) load4(z + (size_t)t * ldz + lanes + i, *reinterpret_cast<float(*)[4]>(w.z + i));
+        }
+    };
+    Token now, next;
+    if (begin < end) fetch(begin, now);
+    for (int t = begin; t < end; ++t, now = next) {
+        if (t + 1 < end) fetch(t + 1, next);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < DPT; ++i) {
+            const float a = GATED ? decay_of(now.z[GATED ? i : 0] + bias[GATED ? i : 0], inv_tau) : gamma;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                S[i][c] = fmaf(a, S[i][c], now.k[i] * now.v[c]);
+                acc[c] = fmaf(S[i][c], now.q[i], acc[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 16);
+            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 8);
+            acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 4);
+            if (GATED) acc[c] *= q_scale;
+        }
+        if (part == 0) store4(out + ((size_t)t * H + h) * V + column, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < DPT; ++i) store4(state + (size_t)i * V, S[i]);
+}
+
 // From the stretches' end states (the first from the true state, the others from zero) to the state at every stretch's
 // start and the slot's new state:  start_1 = end_0;  start_(s+1) = decay^(length_s) start_s + end_s.  One thread an element.
 // `spans` [requests * NS, H, D] (or null): row by row, what stands in place of decay^(length_s) where every token chose its decays.
@@ -353,13 +416,27 @@ int scan_launch(bool gated, const float* q, int ldq, const float* k, int ldk, co
         return LLM_ERR_BAD_ARGUMENT;
     if (v_dtype != LLM_F32 && v_dtype != LLM_BF16) return LLM_ERR_BAD_ARGUMENT;
     const int NS = stretches;
+    using bf = __nv_bfloat16;
+    // steps of few tokens: the kernel without shared memory where the sizes and rows allow
+    auto on16 = [](const void* a) { return ((uintptr_t)a & 15) == 0; };
+    if (few_tokens && NS == 1 && (D == 32 || D == 64 || D == 128) && V % 16 == 0 && !((ldq | ldk | ldv | ldz) & 3) && on16(q) && on16(k) && on16(z) &&
+        on16(states) && on16(out) && ((uintptr_t)v & (v_dtype == LLM_F32 ? 15 : 7)) == 0 && requests <= 65535) {
+        auto step = [&](auto kernel, auto* vp) {
+            return launch_pdl(kernel, dim3((V / 16 + 1) / 2, H, requests), dim3(64), 0, stream, q, ldq, k, ldk, vp, ldv, decay, states, state_slots, cu_tokens, out, H, V,
+                              z, ldz, zbias, inv_tau, q_scale);
+        };
+#define LLM_STEP2(DPT, G) (v_dtype == LLM_F32 ? step(scan_step_kernel<float, DPT, G>, (const float*)v) : step(scan_step_kernel<bf, DPT, G>, (const bf*)v))
+#define LLM_STEP(G) (D == 32 ? LLM_STEP2(4, G) : D == 64 ? LLM_STEP2(8, G) : LLM_STEP2(16, G))
+        return gated ? LLM_STEP(true) : LLM_STEP(false);
+#undef LLM_STEP
+#undef LLM_STEP2
+    }
     // steps of few tokens a request (decode steps) move the state more than they compute: 16 columns a CTA, more CTAs
     const int cpt = few_tokens ? 1 : D <= 64 ? 4 : D <= 128 ? 2 : 1, cols = GROUPS * cpt;
     const dim3 grid((V + cols - 1) / cols, H, requests * NS), block(GROUPS * TPC);
     float* ends = scratch;
     float* starts = scratch ? scratch + (size_t)requests * NS * H * D * V : nullptr;
     float* spans = scratch && gated ? starts + (size_t)requests * NS * H * D * V : nullptr;
-    using bf = __nv_bfloat16;
     auto go = [&](auto kernel, auto* vp, int dpt, int tb) -> int {
         const int ds = dpt * TPC;
         const size_t smem = ((size_t)ds * (cols + 1) + 4 + (size_t)(gated ? 6 : 4) * tb * (dpt + 4) * TPC + (size_t)2 * tb * cols) * sizeof(float);
