@@ -1,35 +1,37 @@
 // A mixture of small feed-forward layers for steps of few tokens (bfloat16, at most 8): only the experts that a token of the step
 // uses are read.
 //
-// In a decode step (1,408 + 704 x 4 of 32 experts, 2,048 wide) they take 11.0 + 8.3 us a layer for one token and 17.1 + 12.5 for three,
-// where the products over all experts and the activation between them took 30.4 + 2.6 + 15.7.
-//
 // What bounds it: the bytes of the weights.  One token that uses 4 of 32 experts needs 52 of the 294 MB that the products over all
 // experts read; eight tokens need about two thirds.  Two kernels, the activation in the first one's end:
 //   up    act[t, j] = act(x W_up^T) * weight[t, expert of j]           (gated: gate and up rows of the same feature in one tile)
 //   down  y[t, n] = sum over the used experts' j of act[t, j] W_down[n, j], plain or added to the residual stream
-// Which experts are used is known on the device alone (the router's weights, or the table's row of each token id): every CTA makes the
-// list and walks the tiles of the listed blocks.  The products are mma.sync m16n8k16, the weights its sixteen rows and the tokens its
+// Which experts are used is known on the device alone (the router's weights, or the table's row of each token id): every warp makes the
+// list and walks the listed blocks.  The products are mma.sync m16n8k16, the weights its sixteen rows and the tokens its
 // eight columns; a thread's 16 bytes of a row hold its operands of two k-steps if the tokens' lanes are permuted alike.
-//   up    a CTA an SM, a tile of 16 rows at a time, whole rows by bulk copies into a ring of three tiles (192 KB in flight), asked for by a
-//         warp of its own; each of sixteen warps takes every sixteenth piece of 32 k, its part of x in registers.
-//   down  a CTA 16 features, each of its sixteen warps pieces of 32 k of the listed blocks, straight into registers, two rounds of weights
-//         and activations on their way.  Which warp has a piece depends on the piece's place in w_down alone: a token's bits are the
-//         same whatever experts the other tokens use.
-// Behind its own tiles the up kernel has the down kernel's weights brought into L2, so that memory does not stand still between the two.
-// The shared expert's tiles (and, with a table, everybody's) are on their way before the kernel in front has ended.  The up kernel
-// lets its dependent start only behind its own wait, by when the router has ended: the down kernel makes its list without waiting.  Its CTAs
-// (128 registers x 512 threads, an SM's whole register file) start where an up CTA has ended, and ask for their first weights while
-// others still run.
+//
+// Both kernels are CTAs of eight warps, every warp with a ring of TMA boxes of its own (as in linear_stream.cuh), so that neither a meeting
+// of the CTA nor another warp's pace stands between a box's arrival and the next one's request:
+//   up    a CTA an SM, a tile of 16 rows at a time; a warp has one or two boxes of 128 k of every tile and its part of x in registers.
+//         The warps' sums wait in shared memory and meet once every four tiles.
+//   down  a CTA 16 features; boxes of 64 k, the tokens' lanes of the same k behind the weights in the slot.  Which warp has a box depends on
+//         the box's place in w_down alone: a token's bits are the same whatever experts the other tokens use.
+// An up CTA and a down CTA share an SM (at most 120 registers x 256 threads and 227 KB together): the up kernel lets its dependent start
+// behind its own wait, by when the router has ended, so that the down kernel makes its list and asks for its first boxes while the up
+// kernel runs, which also brings the rest of the down kernel's weights into L2 behind its own.  The shared expert's boxes (and, with a
+// table, everybody's) are on their way before the kernel in front has ended.
 #include "common.cuh"
+#include "linear_stream.cuh"
 #include "tma.cuh"
 
 namespace {
 
 using bf16 = __nv_bfloat16;
-constexpr int MAX_M = 8, MAX_E = 256, WARPS = 16, UP_THREADS = WARPS * 32 + 32, UP_KB = 4, DOWN_THREADS = WARPS * 32, DOWN_AHEAD = 4, MAX_SLOTS = 8;
+constexpr int MAX_M = 8, MAX_E = 256, WARPS = 8, THREADS = WARPS * 32, MEET = 4;  // MEET: tiles between two meetings of the up kernel
+constexpr int UP_BOXK = 128, UP_KB = 2, UP_SLOTS = 3, UP_SLOT = 16 * UP_BOXK;  // elements of a slot; UP_KB: most boxes a warp has of a tile
+constexpr int DOWN_BOXK = 64, DOWN_SLOTS = 3, DOWN_SLOT = (16 + MAX_M) * DOWN_BOXK;
 constexpr size_t AHEAD_BYTES = 32 << 20;  // the most of w_down that the up kernel brings into L2
-constexpr int UP_RING = 196 * 1024;  // three tiles of 2,048 k
+constexpr size_t UP_SMEM = 1024 + (size_t)WARPS * UP_SLOTS * UP_SLOT * 2 + 2 * (size_t)MEET * WARPS * 32 * 16;
+constexpr size_t DOWN_SMEM = 1024 + (size_t)WARPS * DOWN_SLOTS * DOWN_SLOT * 2 + (size_t)WARPS * 32 * 16;
 
 struct Experts {
     const bf16 *x, *w_up, *w_down;
@@ -45,30 +47,15 @@ struct Experts {
     bf16* xw_out;
     float* ss_out;
     float alpha;
-    int up_slots;
     int* error_flag;
 };
 
-__device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+using lin::feature_row;  // which row of eight in a box holds the weights of MMA row g
+
 // both k-steps of a piece of 32 k: a0, a1: rows g and g + 8 of the weights, b: column g of the tokens
 __device__ __forceinline__ void mma_piece(float (&c)[4], float (&d)[4], const uint4& a0, const uint4& a1, const uint4& b) {
-    mma_bf16(c, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
-    mma_bf16(d, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
-}
-// weights are read once: no place in L1
-__device__ __forceinline__ uint4 load_weight(const bf16* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-// `bytes` (a multiple of 16) into shared memory, counted on `bar`
-__device__ __forceinline__ void copy_bulk(void* to, const void* from, unsigned bytes, unsigned long long* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(tma::smem_addr(to)), "l"(from), "r"(bytes), "r"(tma::smem_addr(bar)) : "memory");
+    lin::mma_bf16(c, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
+    lin::mma_bf16(d, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
 }
 
 __device__ __forceinline__ float weight_of(const Experts& p, int m, int e) {
@@ -81,11 +68,10 @@ __device__ __forceinline__ float weight_of(const Experts& p, int m, int e) {
     return w;
 }
 
-// The used experts in ascending order, and (wt_s not null) every token's weight of every expert and of the shared one, by warp 0; the
-// caller meets before it reads them.
-__device__ __forceinline__ void list_experts(const Experts& p, short* list, int* count, float (*wt_s)[MAX_E + 1]) {
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
+// The used experts in ascending order, by the calling warp for itself (list: its own place), and where wt_s is given every token's weight of
+// every expert and of the shared one.  Returns their number.
+__device__ __forceinline__ int list_experts(const Experts& p, unsigned char* list, float (*wt_s)[MAX_E + 1]) {
+    const int lane = threadIdx.x & 31;
     int n = 0;
     if (wt_s && lane < p.M && p.fs > 0) wt_s[lane][p.E] = weight_of(p, lane, p.E);
     for (int e0 = 0; e0 < p.E; e0 += 32) {
@@ -100,10 +86,11 @@ __device__ __forceinline__ void list_experts(const Experts& p, short* list, int*
             if (wt_s && e < p.E) wt_s[m][e] = wt[m];
         }
         const unsigned mask = __ballot_sync(0xffffffffu, used);
-        if (used) list[n + __popc(mask & ((1u << lane) - 1))] = (short)e;
+        if (used) list[n + __popc(mask & ((1u << lane) - 1))] = (unsigned char)e;
         n += __popc(mask);
     }
-    if (lane == 0) *count = n;
+    __syncwarp();
+    return n;
 }
 
 __device__ __forceinline__ float activate(float v, int kind) {
@@ -113,226 +100,283 @@ __device__ __forceinline__ float activate(float v, int kind) {
     return v;
 }
 
-// The sixteen warps' sums of a lane's four values, in order.
-__device__ __forceinline__ void add_up(const float (*red)[32][4], int lane, float (&s)[4]) {
+// The warps' sums of a lane's four values, in order.
+__device__ __forceinline__ void add_up(const float4* red, int lane, float (&s)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) s[i] = 0.f;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
-        float part[4];
-        load4(red[w][lane], part);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[i] += part[i];
+        const float4 part = red[w * 32 + lane];
+        s[0] += part.x; s[1] += part.y; s[2] += part.z; s[3] += part.w;
     }
 }
 
-__global__ void __launch_bounds__(UP_THREADS, 1) experts_up_kernel(const Experts p) {
-    extern __shared__ __align__(128) unsigned char ring[];  // [slots][16][2 K + 64]
-    __shared__ short list[MAX_E];
-    __shared__ int count, gave_up;
-    __shared__ __align__(16) float red[2][WARPS][32][4];
+// map: w_up in boxes of 8 (gated) or 16 rows and two neighbouring pieces of 64 k where `whole` (rows are whole pieces), else one piece.
+__global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid_constant__ CUtensorMap map, const int whole) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ unsigned char lists[WARPS][MAX_E];
     __shared__ float wt_s[MAX_M][MAX_E + 1];
-    __shared__ __align__(8) unsigned long long full[MAX_SLOTS], empty[MAX_SLOTS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    __shared__ __align__(8) unsigned long long full[WARPS][UP_SLOTS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, fr = feature_row(g);
+    bf16* rings = reinterpret_cast<bf16*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    bf16* ring = rings + (size_t)warp * UP_SLOTS * UP_SLOT;
+    float4* red = reinterpret_cast<float4*>(rings + (size_t)WARPS * UP_SLOTS * UP_SLOT);  // [2][MEET][WARPS][32]
     const bool gated = p.kind < 0, known = p.weights == nullptr;  // the table's experts do not depend on the kernel in front
     const int step = gated ? 8 : 16, tiles_e = p.ff / step, tiles_s = p.fs / step, per = gated ? 2 : 1;
-    const int pitch = p.K * 2 + 64, slot_bytes = 16 * pitch;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < p.up_slots; ++s) {
-            tma::mbar_init(&full[s], 1);
-            tma::mbar_init(&empty[s], WARPS);
-        }
+    const int kblocks = (p.K + UP_BOXK - 1) / UP_BOXK, my_kb = kblocks > warp ? (kblocks - 1 - warp) / WARPS + 1 : 0;
+    unsigned long long* my_full = full[warp];
+    unsigned char* list = lists[warp];
+    if (lane == 0) {
+        for (int s = 0; s < UP_SLOTS; ++s) tma::mbar_init(&my_full[s], 1);
         tma::mbar_fence_init();
-        gave_up = 0;
+        if (warp == 0) tma::prefetch_map(&map);
     }
-    if (known) list_experts(p, list, &count, wt_s);
-    __syncthreads();
+    __syncwarp();
+    int count = known ? list_experts(p, list, warp == 0 ? wt_s : nullptr) : 0;
     // tile v: the shared expert's first, then the listed experts'
     auto place = [&](int v, int& e, int& f0) {
         e = v < tiles_s ? p.E : list[(v - tiles_s) / tiles_e];
         f0 = (v < tiles_s ? v : (v - tiles_s) % tiles_e) * step;
     };
-    auto fail = [&]() {
-        gave_up = 1;
-        if (p.error_flag) atomicExch(p.error_flag, 1);
-    };
-    // the asking warp asks for the CTA's n-th tile, sixteen lanes a row each
-    auto ask = [&](int n) {
+    auto tiles_of = [&](int total) { return (int)blockIdx.x < total ? (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0; };
+    int tiles = tiles_of(tiles_s + count * tiles_e), armed = 0, a_tile = 0, a_kb = warp;
+    // asks for the warp's next box (lane 0)
+    auto arm = [&]() {
         int e, f0;
-        place(blockIdx.x + n * gridDim.x, e, f0);
-        const int s = n % p.up_slots;
-        if (lane == 0) tma::mbar_expect_tx(&full[s], 16 * p.K * 2);
-        __syncwarp();
-        if (lane < 16) {
-            const size_t row = (size_t)e * per * p.ff + f0 + (gated && lane >= 8 ? (e == p.E ? p.fs : p.ff) + lane - 8 : lane);
-            copy_bulk(ring + (size_t)s * slot_bytes + lane * pitch, p.w_up + row * p.K, p.K * 2, &full[s]);
+        place(blockIdx.x + a_tile * gridDim.x, e, f0);
+        const int s = armed % UP_SLOTS, rows = gated ? 8 : 16;
+        const int row = e * per * p.ff + f0;  // (of the gate, whose up rows lie ff or fs further)
+        bf16* dst = ring + (size_t)s * UP_SLOT;
+        tma::mbar_expect_tx(&my_full[s], UP_SLOT * 2);
+        for (int half = 0; half < per; ++half, dst += 8 * UP_BOXK) {
+            const int r = row + half * (e == p.E ? p.fs : p.ff);
+            if (whole) tma::load_3d(dst, &map, 0, r, a_kb * 2, &my_full[s]);
+            else {
+                tma::load_2d(dst, &map, a_kb * UP_BOXK, r, &my_full[s]);
+                tma::load_2d(dst + rows * 64, &map, a_kb * UP_BOXK + 64, r, &my_full[s]);
+            }
+        }
+        ++armed;
+        a_kb += WARPS;
+        if (a_kb >= kblocks) {
+            a_kb = warp;
+            ++a_tile;
         }
     };
-    int asked = 0, total = known ? tiles_s + count * tiles_e : tiles_s;
-    auto mine = [&]() { return (int)blockIdx.x < total ? (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0; };
-    if (warp == WARPS)
-        for (const int n = min(mine(), p.up_slots); asked < n; ++asked) ask(asked);
+    auto fill = [&](int consumed) {
+        if (lane == 0)
+            while (armed < tiles * my_kb && armed < consumed + UP_SLOTS) arm();
+    };
+    fill(0);
     pdl_wait();
     pdl_trigger();  // behind the wait: see above
-    uint4 xb[UP_KB];
-    if (warp < WARPS) {
+    uint4 xb[UP_KB][4];
 #pragma unroll
-        for (int i = 0; i < UP_KB; ++i) {
-            const int k = (warp + i * WARPS) * 32;
-            xb[i] = k < p.K && g < p.M ? *reinterpret_cast<const uint4*>(p.x + (size_t)g * p.ldx + k + q * 8) : make_uint4(0, 0, 0, 0);
+    for (int j = 0; j < UP_KB; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = (warp + j * WARPS) * UP_BOXK + i * 32;
+            xb[j][i] = k < p.K && g < p.M ? __ldcg(reinterpret_cast<const uint4*>(p.x + (size_t)g * p.ldx + k + q * 8)) : make_uint4(0, 0, 0, 0);
         }
-    }
     if (!known) {
-        list_experts(p, list, &count, wt_s);
-        __syncthreads();
-        total = tiles_s + count * tiles_e;
+        count = list_experts(p, list, warp == 0 ? wt_s : nullptr);
+        tiles = tiles_of(tiles_s + count * tiles_e);
+        fill(0);
     }
-    const int tiles = mine(), lda = p.E * p.ff + p.fs;
-    if (warp == WARPS) {
-        for (; asked < tiles; ++asked) {
-            if (asked >= p.up_slots && !__all_sync(0xffffffffu, tma::mbar_wait(&empty[asked % p.up_slots], (asked / p.up_slots - 1) & 1))) {
-                fail();
-                break;
-            }
-            ask(asked);
-        }
-        // the down kernel's weights on their way into L2 behind this kernel's: memory does not stand still while this one ends and that one
-        // starts (row by row of a block, dealt over the CTAs)
-        const int blocks = (p.fs > 0 ? 1 : 0) + count, ldk = p.E * p.ff + p.fs;
+    const int lda = p.E * p.ff + p.fs;
+    int unit = 0;
+    bool gave_up = false, ahead = false;
+    // the down kernel's weights on their way into L2 behind this kernel's: memory does not stand still while this one ends (row by row of
+    // a block, dealt over the CTAs' warps)
+    auto bring_ahead = [&]() {
+        if (ahead) return;
+        ahead = true;
+        const int blocks = (p.fs > 0 ? 1 : 0) + count;
         const int items = (int)min((long long)blocks * p.N, (long long)(AHEAD_BYTES / (2 * (size_t)max(p.ff, p.fs))));
-        for (int i = blockIdx.x * 32 + lane; i < items; i += gridDim.x * 32) {
+        for (int i = (blockIdx.x * WARPS + warp) * 32 + lane; i < items; i += gridDim.x * THREADS) {
             const int b = i / p.N, n = i - b * p.N;
             const bool shared = p.fs > 0 && b == 0;
-            const bf16* at = p.w_down + (size_t)n * ldk + (size_t)(shared ? p.E : list[b - (p.fs > 0 ? 1 : 0)]) * p.ff;
+            const bf16* at = p.w_down + (size_t)n * lda + (size_t)(shared ? p.E : list[b - (p.fs > 0 ? 1 : 0)]) * p.ff;
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(at), "r"((shared ? p.fs : p.ff) * 2) : "memory");
         }
-        // the other warps wait for every tile that was asked for, but not once a wait has given up: no copy is left on its way to a CTA that
-        // has ended
-        for (int n = max(0, asked - p.up_slots); n < asked; ++n) tma::mbar_wait(&full[n % p.up_slots], (n / p.up_slots) & 1);
-        return;
-    }
-    for (int n = 0; n < tiles; ++n) {
-        const int s = n % p.up_slots;
-        if (!*(volatile int*)&gave_up && !tma::mbar_wait(&full[s], (n / p.up_slots) & 1)) fail();
-        const unsigned char* row = ring + (size_t)s * slot_bytes + g * pitch + q * 16;
-        float c[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
+    };
+    for (int t0 = 0, round = 0; t0 < tiles; t0 += MEET, ++round) {
+        const int t1 = min(tiles, t0 + MEET);
+        float4* mine = red + (size_t)(round & 1) * MEET * WARPS * 32;
+        for (int t = t0; t < t1; ++t) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < UP_KB; ++i) {
-            const int k = (warp + i * WARPS) * 32;
-            if (k < p.K) mma_piece(c, d, *reinterpret_cast<const uint4*>(row + k * 2), *reinterpret_cast<const uint4*>(row + 8 * pitch + k * 2), xb[i]);
+            for (int j = 0; j < UP_KB; ++j) {
+                if (j >= my_kb) break;
+                if (unit + UP_SLOTS >= tiles * my_kb) bring_ahead();  // the warp's last box has been asked for
+                const int s = unit % UP_SLOTS;
+                if (!gave_up && !tma::mbar_wait(&my_full[s], (unit / UP_SLOTS) & 1)) {
+                    gave_up = true;
+                    if (p.error_flag) atomicExch(p.error_flag, 1);
+                }
+                // [2 pieces of 64 k][rows][64], the 16 bytes c of row r at c ^ (r & 7); gated: eight rows of the gate, then of the up
+                const bf16* slot = ring + (size_t)s * UP_SLOT + fr * 64;
+                uint4 a[4][2];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bf16* at = slot + (i >> 1) * (gated ? 8 * 64 : 16 * 64) + ((((i & 1) << 2) | q) ^ fr) * 8;
+                    a[i][0] = *reinterpret_cast<const uint4*>(at);
+                    a[i][1] = *reinterpret_cast<const uint4*>(at + (gated ? 8 * UP_BOXK : 8 * 64));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_piece(c, d, a[i][0], a[i][1], xb[j][i]);
+                __syncwarp();  // the products have been issued: every lane's pieces are in registers, and the slot may take the next box
+                ++unit;
+                fill(unit);
+            }
+            mine[((t - t0) * WARPS + warp) * 32 + lane] = make_float4(c[0] + d[0], c[1] + d[1], c[2] + d[2], c[3] + d[3]);
         }
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&empty[s]);
-        *reinterpret_cast<float4*>(red[n & 1][warp][lane]) = make_float4(c[0] + d[0], c[1] + d[1], c[2] + d[2], c[3] + d[3]);
-        // the sixteen warps meet; the other buffer of sums is written next, and this one read until the meeting after that
-        asm volatile("bar.sync 1, %0;\n" ::"n"(WARPS * 32) : "memory");
-        if (warp != n % WARPS) continue;
-        int e, f0;
-        place(blockIdx.x + n * gridDim.x, e, f0);
-        float sum[4];
-        add_up(red[n & 1], lane, sum);
+        if (t1 == tiles) bring_ahead();  // (a warp without boxes)
+        __syncthreads();  // this buffer of sums is written again two meetings on
+        for (int t = t0 + warp; t < t1; t += WARPS) {
+            int e, f0;
+            place(blockIdx.x + t * gridDim.x, e, f0);
+            float sum[4];
+            add_up(mine + (size_t)(t - t0) * WARPS * 32, lane, sum);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {  // token 2 q + i; sum[i]: row g, sum[i + 2]: row g + 8
-            const int m = 2 * q + i;
-            if (m >= p.M) continue;
-            const float wt = wt_s[m][e];
-            bf16* y = p.act + (size_t)m * lda + (size_t)e * p.ff + f0 + g;
-            if (gated) {
-                const float lim = e == p.E ? p.limit_s : p.limit, gc = fminf(sum[i], lim), uc = fminf(fmaxf(sum[i + 2], -lim), lim);
-                y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : gc / (1.f + expf(-p.slope * gc)) * (uc + p.up_shift) * wt);
-            } else {
-                y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i], p.kind) * wt);
-                y[8] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i + 2], p.kind) * wt);
+            for (int i = 0; i < 2; ++i) {  // token 2 q + i; sum[i]: row g, sum[i + 2]: row g + 8
+                const int m = 2 * q + i;
+                if (m >= p.M) continue;
+                const float wt = wt_s[m][e];
+                bf16* y = p.act + (size_t)m * lda + (size_t)e * p.ff + f0 + fr;
+                if (gated) {
+                    const float lim = e == p.E ? p.limit_s : p.limit, gc = fminf(sum[i], lim), uc = fminf(fmaxf(sum[i + 2], -lim), lim);
+                    y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : gc / (1.f + expf(-p.slope * gc)) * (uc + p.up_shift) * wt);
+                } else {
+                    y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i], p.kind) * wt);
+                    y[8] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i + 2], p.kind) * wt);
+                }
             }
         }
     }
+    // every box that was asked for has been waited for; where a wait gave up, once more, so that no copy lands after the CTA has left
+    if (gave_up && lane == 0)
+        for (int n = max(0, armed - UP_SLOTS); n < armed; ++n) tma::mbar_wait(&my_full[n % UP_SLOTS], (n / UP_SLOTS) & 1);
 }
 
-__global__ void __launch_bounds__(DOWN_THREADS, 1) experts_down_kernel(const Experts p) {
-    __shared__ short list[MAX_E];
-    __shared__ int count;
-    __shared__ __align__(16) float red[WARPS][32][4];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const int n0 = blockIdx.x * 16, ldk = p.E * p.ff + p.fs, pieces_e = p.ff >> 5, pieces_s = p.fs >> 5;
-    pdl_trigger();
-    list_experts(p, list, &count, nullptr);  // the router ended before the up kernel let this one start
-    __syncthreads();
-    // The warp's pieces: the neighbouring pairs (whole lines of 128 bytes) whose number among all of w_down's columns is the warp's own modulo
-    // WARPS, of the shared expert, then of the listed ones.  So the order of a token's sums does not depend on the experts of others,
-    // whose pieces in between add zeros.
-    int block = pieces_s > 0 ? -1 : 0, at = -1, end = -1;  // `at`: the next piece, one of the block that ends at `end`
-    auto enter = [&]() {  // the block's first piece of this warp, or a later block's; at = -1: none is left
-        for (; block < count; ++block) {
-            const int a0 = (block < 0 ? p.E : list[block]) * pieces_e, pair = a0 >> 1, skip = (warp - pair) & (WARPS - 1);
-            at = skip == 0 ? a0 : (pair + skip) * 2;
-            end = a0 + (block < 0 ? pieces_s : pieces_e);
-            if (at < end) return;
+// map: w_down in boxes of 16 rows and 64 columns; act_map: act in boxes of 8 rows (what is not there reads as zeros) and 64 columns.
+__global__ void __maxnreg__(120) experts_down_kernel(const Experts p, const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap act_map) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ unsigned char lists[WARPS][MAX_E];
+    __shared__ __align__(8) unsigned long long full[WARPS][DOWN_SLOTS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, fr = feature_row(g);
+    bf16* rings = reinterpret_cast<bf16*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    bf16* ring = rings + (size_t)warp * DOWN_SLOTS * DOWN_SLOT;
+    float4* red = reinterpret_cast<float4*>(rings + (size_t)WARPS * DOWN_SLOTS * DOWN_SLOT);  // [WARPS][32]
+    const int n0 = blockIdx.x * 16, boxes_e = (p.ff + DOWN_BOXK - 1) / DOWN_BOXK, boxes_s = (p.fs + DOWN_BOXK - 1) / DOWN_BOXK;
+    unsigned long long* my_full = full[warp];
+    unsigned char* list = lists[warp];
+    if (lane == 0) {
+        for (int s = 0; s < DOWN_SLOTS; ++s) tma::mbar_init(&my_full[s], 1);
+        tma::mbar_fence_init();
+        if (warp == 0) {
+            tma::prefetch_map(&map);
+            tma::prefetch_map(&act_map);
         }
-        at = -1;
-    };
-    enter();
-    auto take = [&]() {
-        if (at < 0) return -1;
-        const int k = at * 32;
-        at += (at & 1) ? 2 * WARPS - 1 : 1;
-        if (at >= end) {
-            ++block;
-            enter();
-        }
-        return k;
-    };
-    const bf16 *row0 = p.w_down + (size_t)(n0 + g) * ldk + q * 8, *row1 = row0 + (size_t)8 * ldk, *tokens = p.act + (size_t)g * ldk + q * 8;
-    struct Round { uint4 a[DOWN_AHEAD][2], b[DOWN_AHEAD]; int k[DOWN_AHEAD]; };  // first k of each piece, or -1
-    auto ask = [&](Round& r) {
-#pragma unroll
-        for (int u = 0; u < DOWN_AHEAD; ++u) {
-            r.k[u] = take();
-            r.a[u][0] = r.k[u] >= 0 ? load_weight(row0 + r.k[u]) : make_uint4(0, 0, 0, 0);
-            r.a[u][1] = r.k[u] >= 0 ? load_weight(row1 + r.k[u]) : make_uint4(0, 0, 0, 0);
-        }
-    };
-    auto ask_tokens = [&](Round& r) {
-#pragma unroll
-        for (int u = 0; u < DOWN_AHEAD; ++u)
-            r.b[u] = r.k[u] >= 0 && g < p.M ? __ldcg(reinterpret_cast<const uint4*>(tokens + r.k[u])) : make_uint4(0, 0, 0, 0);
-    };
-    float c4[4] = {0.f, 0.f, 0.f, 0.f}, d4[4] = {0.f, 0.f, 0.f, 0.f};
-    auto multiply = [&](const Round& r) {
-#pragma unroll
-        for (int u = 0; u < DOWN_AHEAD; ++u) mma_piece(c4, d4, r.a[u][0], r.a[u][1], r.b[u]);
-    };
-    Round r0, r1;
-    ask(r0);
-    ask(r1);
-    pdl_wait();
-    ask_tokens(r0);
-    ask_tokens(r1);
-    while (r0.k[0] >= 0) {  // (pieces behind the last are zeros)
-        multiply(r0);
-        ask(r0);
-        ask_tokens(r0);
-        multiply(r1);
-        ask(r1);
-        ask_tokens(r1);
     }
-    *reinterpret_cast<float4*>(red[warp][lane]) = make_float4(c4[0] + d4[0], c4[1] + d4[1], c4[2] + d4[2], c4[3] + d4[3]);
+    __syncwarp();
+    pdl_trigger();
+    const int count = list_experts(p, list, nullptr);  // the router ended before the up kernel let this one start
+    // The warp's boxes: those whose number among all of w_down's (boxes_e an expert, the shared one's last) is the warp's own modulo WARPS,
+    // of the shared expert, then of the listed ones.  So the order of a token's sums does not depend on the experts of others, whose
+    // boxes in between add zeros.
+    struct Walk {
+        int block, box;  // block -1: the shared expert's
+    };
+    auto expert = [&](const Walk& w) { return w.block < 0 ? p.E : (int)list[w.block]; };
+    auto enter = [&](Walk& w) { w.box = w.block < count ? (warp - expert(w) * boxes_e) & (WARPS - 1) : 0; };
+    // moves on to a box that exists; false: none is left
+    auto settle = [&](Walk& w) {
+        while (w.block < count && w.box >= (w.block < 0 ? boxes_s : boxes_e)) {
+            ++w.block;
+            enter(w);
+        }
+        return w.block < count;
+    };
+    Walk ask = {-1, 0};
+    enter(ask);
+    Walk use = ask;
+    int armed = 0;
+    bool may_read = false;  // the tokens' lanes are there
+    auto column = [&](const Walk& w) { return expert(w) * p.ff + w.box * DOWN_BOXK; };
+    auto fill = [&](int consumed) {  // lane 0
+        while (armed < consumed + DOWN_SLOTS && settle(ask)) {
+            const int s = armed % DOWN_SLOTS, k = column(ask);
+            bf16* dst = ring + (size_t)s * DOWN_SLOT;
+            tma::mbar_expect_tx(&my_full[s], DOWN_SLOT * 2);
+            tma::load_2d(dst, &map, k, n0, &my_full[s]);
+            if (may_read) tma::load_2d(dst + 16 * DOWN_BOXK, &act_map, k, 0, &my_full[s]);
+            ++armed;
+            ask.box += WARPS;
+        }
+    };
+    if (lane == 0) fill(0);
+    pdl_wait();
+    if (lane == 0) {
+        may_read = true;
+        Walk w = use;
+        for (int n = 0; n < armed; ++n, w.box += WARPS)
+            if (settle(w)) tma::load_2d(ring + (size_t)n * DOWN_SLOT + 16 * DOWN_BOXK, &act_map, column(w), 0, &my_full[n]);
+    }
+    // what the end needs besides the sums
+    float before[4] = {0.f, 0.f, 0.f, 0.f}, norm_w[2] = {0.f, 0.f};
+    if (warp == 0 && p.resid) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int m = 2 * q + (i & 1), n = n0 + fr + (i >> 1) * 8;
+            if (m < p.M) before[i] = __ldcg(p.resid + (size_t)m * p.N + n);
+            if (p.norm_w) norm_w[i >> 1] = p.norm_w[n];
+        }
+    }
+    float c[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
+    int unit = 0;
+    bool gave_up = false;
+    for (; settle(use); use.box += WARPS) {
+        const int s = unit % DOWN_SLOTS;
+        if (!gave_up && !tma::mbar_wait(&my_full[s], (unit / DOWN_SLOTS) & 1)) {
+            gave_up = true;
+            if (p.error_flag) atomicExch(p.error_flag, 1);
+        }
+        const bf16 *w = ring + (size_t)s * DOWN_SLOT + fr * 64, *x = ring + (size_t)s * DOWN_SLOT + 16 * DOWN_BOXK + g * 64;
+        uint4 a[2][2], b[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            a[i][0] = *reinterpret_cast<const uint4*>(w + (((i << 2) | q) ^ fr) * 8);
+            a[i][1] = *reinterpret_cast<const uint4*>(w + 8 * 64 + (((i << 2) | q) ^ fr) * 8);
+            b[i] = *reinterpret_cast<const uint4*>(x + (((i << 2) | q) ^ g) * 8);
+        }
+        mma_piece(c, d, a[0][0], a[0][1], b[0]);
+        // an expert's last box may hold 32 columns of its neighbour
+        if (use.box * DOWN_BOXK + 32 < (use.block < 0 ? p.fs : p.ff)) mma_piece(c, d, a[1][0], a[1][1], b[1]);
+        __syncwarp();  // the products have been issued: every lane's pieces are in registers, and the slot may take the next box
+        ++unit;
+        if (lane == 0) fill(unit);
+    }
+    red[warp * 32 + lane] = make_float4(c[0] + d[0], c[1] + d[1], c[2] + d[2], c[3] + d[3]);
+    if (gave_up && lane == 0)
+        for (int n = max(0, armed - DOWN_SLOTS); n < armed; ++n) tma::mbar_wait(&my_full[n % DOWN_SLOTS], (n / DOWN_SLOTS) & 1);
     __syncthreads();
     if (warp != 0) return;
     float s[4], ss[2] = {0.f, 0.f};
     add_up(red, lane, s);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int m = 2 * q + (i & 1), n = n0 + g + (i >> 1) * 8;
+        const int m = 2 * q + (i & 1), n = n0 + fr + (i >> 1) * 8;
         if (m >= p.M) continue;
         const size_t at = (size_t)m * p.N + n;
         if (!p.resid) {
             p.out[at] = s[i];
             continue;
         }
-        const float r = fmaf(p.alpha, s[i], p.resid[at]);
+        const float r = fmaf(p.alpha, s[i], before[i]);
         p.resid[at] = r;
         if (p.norm_w) {
-            p.xw_out[at] = __float2bfloat16_rn(r * p.norm_w[n]);
+            p.xw_out[at] = __float2bfloat16_rn(r * norm_w[i >> 1]);
             ss[i & 1] = fmaf(r, r, ss[i & 1]);
         }
     }
@@ -365,7 +409,7 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
         kind == 2 || kind > 3 || fs < 0)
         return LLM_ERR_BAD_ARGUMENT;
     auto aligned = [](const void* a) { return ((uintptr_t)a & 15) == 0; };
-    if (M > MAX_M || K < 32 || K > WARPS * UP_KB * 32 || (K & 31) || ff < 32 || (ff & 31) || (fs & 31) || N < 16 || (N & 15) || E < 1 || E > MAX_E ||
+    if (M > MAX_M || K < 32 || K > WARPS * UP_KB * UP_BOXK || (K & 31) || ff < 32 || (ff & 31) || (fs & 31) || N < 16 || (N & 15) || E < 1 || E > MAX_E ||
         (ldx & 7) || !aligned(x) || !aligned(w_up) || !aligned(w_down) || !aligned(act))
         return LLM_ERR_UNSUPPORTED;
     Experts p = {};
@@ -374,12 +418,23 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     p.limit = limit; p.limit_s = limit_s; p.slope = slope; p.up_shift = up_shift;
     p.weights = weights; p.ldw = ldw; p.ids = ids; p.table = table; p.top = top; p.vocab = vocab;
     p.out = out; p.resid = resid; p.norm_w = norm_w; p.xw_out = (bf16*)xw_out; p.ss_out = ss_out; p.alpha = alpha; p.error_flag = error_flag;
-    const int up_slot = 16 * (K * 2 + 64);
-    p.up_slots = UP_RING / up_slot < MAX_SLOTS ? UP_RING / up_slot : MAX_SLOTS;
-    const int sms = device_sms();
-    const cudaError_t set = cudaFuncSetAttribute(experts_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UP_RING);
-    if (set != cudaSuccess) return (int)set;
+    const int sms = device_sms(), per = kind < 0 ? 2 : 1, C = E * ff + fs;
+    const bool whole = K % 64 == 0;  // rows are whole pieces of 64 k: two of them in one box
+    CUtensorMap up_map, act_map;
+    if (!(whole ? tma::make_map_row_pieces_bf16(&up_map, w_up, (uint64_t)per * C, K, kind < 0 ? 8 : 16)
+                : tma::make_map_2d_bf16(&up_map, w_up, (uint64_t)per * C, K, K, kind < 0 ? 8 : 16, 64, CU_TENSOR_MAP_SWIZZLE_128B)))
+        return LLM_ERR_UNSUPPORTED;
+    const CUtensorMap* down_map = tma::cached_map_2d_bf16(w_down, N, C, C, 16, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!down_map || !tma::make_map_2d_bf16(&act_map, act, M, C, C, MAX_M, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B)) return LLM_ERR_UNSUPPORTED;
+    // at every launch: the limits hold for the current device, and a process may have several; all of the SM's memory as shared memory, so
+    // that CTAs of both kernels share it
+    for (int k = 0; k < 2; ++k) {
+        const void* kernel = k == 0 ? (const void*)experts_up_kernel : (const void*)experts_down_kernel;
+        cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k == 0 ? UP_SMEM : DOWN_SMEM));
+        if (set == cudaSuccess) set = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (set != cudaSuccess) return (int)set;
+    }
     const int most = (E * ff + fs) / (kind < 0 ? 8 : 16);
-    const int code = launch_pdl(experts_up_kernel, dim3(most < sms ? most : sms), dim3(UP_THREADS), (size_t)p.up_slots * up_slot, stream, p);
-    return code != 0 ? code : launch_pdl(experts_down_kernel, dim3(N / 16), dim3(DOWN_THREADS), 0, stream, p);
+    const int code = launch_pdl(experts_up_kernel, dim3(most < sms ? most : sms), dim3(THREADS), UP_SMEM, stream, p, up_map, (int)whole);
+    return code != 0 ? code : launch_pdl(experts_down_kernel, dim3(N / 16), dim3(THREADS), DOWN_SMEM, stream, p, *down_map, act_map);
 }
