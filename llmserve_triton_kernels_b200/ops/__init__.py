@@ -72,7 +72,6 @@ _SIGNATURES = {
     "llm_sigmoid_attention": [_vp, _i, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i,
                               _i, _i, _vp],
     "llm_sigmoid_attention_mma": [_vp, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp],
-    "llm_sigmoid_attention_step": [_vp, _i, _vp, _ll, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _vp],
     "llm_sigmoid_sum_parts": [_vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
     "llm_qk_prepare": [_vp, _i, _i, _vp, _i, _i, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _f, _vp, _i, _vp, _f, _i, _i, _i, _i, _i, _vp],
     "llm_retention_scan": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i, _vp],
@@ -1914,19 +1913,6 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
         count = min(-(-longest // keys), -(-(window - 1) // keys) + 1) if window else -(-longest // keys)
         return keys, 1 if n > _SIGMOID_SPLIT_MAX_TOKENS else max(1, count)
 
-    if q.dtype == torch.bfloat16 and not _FORCE_GENERIC_ATTENTION and n == getattr(ctx, "num_requests", 0) and getattr(ctx, "max_query_len", 0) == 1:
-        # one token a request: as many CTAs a token as SMs have room for (by the number of tokens alone, so that a token's order of sums
-        # does not follow from the contexts)
-        shares = next(s for s in (8, 4, 2, 1) if s == 1 or s * n <= _sm_count())
-        code = _launch(
-            "llm_sigmoid_attention_step", _ptr(q), q.stride(0), _ptr(pool), pool.shape[0], _ptr(page_table), page_table.shape[1], _ptr(ctx.positions),
-            _ptr(ctx.token_request), _ptr(head_bias), _ptr(head_mix), _ptr(out), n, num_heads, num_kv_heads, key_dim, value_dim, pool.shape[4],
-            pool.shape[3], float(scale), float(softcap or 0.0), int(window or 0), shares, _stream(),
-        )
-        if code != 10002:
-            _check(code, "sigmoid_attention (one token a request)")
-            return out
-        add_launches(-1)
     if q.dtype == torch.bfloat16 and not _FORCE_GENERIC_ATTENTION:
         # the tensor cores: tiles of 16 tokens of one request
         split_keys, splits = stretches(_SIGMOID_MMA_SPLIT_KEYS)
