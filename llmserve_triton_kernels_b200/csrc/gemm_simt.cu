@@ -295,18 +295,16 @@ int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, 
     if (M <= 4) return launch_few<4, 4>(x, w, out, M, N, K, ldx, ldw, ldo, stream);
     if (M <= 8) return launch_few<8, 3>(x, w, out, M, N, K, ldx, ldw, ldo, stream);
     if (M <= 16) return launch_few<16, 3>(x, w, out, M, N, K, ldx, ldw, ldo, stream);
-    // the tile that takes the least time by its share of the CUDA cores' rate when the SMs are full of it, and how full they are:
-    // small outputs want small tiles, so that every SM has one
-    struct { int rm, rn, per_sm; double rate; } const kinds[4] = {{128, 128, 1, 1.0}, {64, 128, 2, 0.92}, {64, 64, 3, 0.85}, {32, 64, 4, 0.7}};
+    // the tile that takes the least time by how many of them the busiest SM has.  Measured (2,048 k, 17 to 300 rows of 1,024 to 11,264
+    // features, microseconds; n tiles of an SM): 232 n, 145 n, 27 + 59 n and 32 + 31 n.  242 rows: 2,560 features 145 with 64 x 64, 118 with 32 x 64;
+    // 2,048 features 88 and 104; 11,264 features 322 and 338.
+    struct { int rm, rn; double once, each; } const kinds[4] = {{128, 128, 0., 232.}, {64, 128, 0., 145.}, {64, 64, 27., 59.}, {32, 64, 32., 31.}};
     int best = 0;
     double best_cost = 1e30;
     const int sms = device_sms();
     for (int i = 0; i < 4; ++i) {
-        const double tiles = (double)((M + kinds[i].rm - 1) / kinds[i].rm) * ((N + kinds[i].rn - 1) / kinds[i].rn);
-        // tiles of the busiest SM, which runs them up to per_sm at a time at the full rate and one alone at less
-        const double most = (double)(((long long)tiles + sms - 1) / sms);
-        const double alone = most < kinds[i].per_sm ? 1.0 + 0.35 * (kinds[i].per_sm - most) / kinds[i].per_sm : 1.0;
-        const double cost = most * kinds[i].rm * kinds[i].rn / kinds[i].rate * alone;
+        const long long tiles = (long long)((M + kinds[i].rm - 1) / kinds[i].rm) * ((N + kinds[i].rn - 1) / kinds[i].rn);
+        const double cost = kinds[i].once + kinds[i].each * (double)((tiles + sms - 1) / sms);
         if (cost < best_cost) {
             best_cost = cost;
             best = i;
