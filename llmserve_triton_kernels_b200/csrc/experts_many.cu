@@ -10,9 +10,9 @@
 // products over all experts with the token's weight as a factor, which ran before, did eight times the operations for 4 of 32 experts.
 //
 // The products are tcgen05 with the WEIGHTS as the 128 rows of the tile and an expert's tokens as its columns: an expert has as many
-// tokens as it has, and N goes up to 256 in steps of 16 where M is 128 whatever there is to do.  One persistent CTA an SM walks (group,
+// tokens as it has, and N goes up to 64, 128 or 256 (the fewer, the deeper the ring) in steps of 16 where M is 128 whatever there is to do.  One persistent CTA an SM walks (group,
 // tile of features, tile of tokens), the shared expert's tiles first (the largest), token tiles innermost so that neighbours in time share
-// weights in L2.  Warp 0 brings operands by TMA through a ring of four slots (where the experts are gated a box of eight rows of gate, of up, of
+// weights in L2.  Warp 0 brings operands by TMA through a ring of slots (where the experts are gated a box of eight rows of gate, of up, of
 // gate ..., so that a feature's two sums lie eight lanes apart in tensor memory), warp 1 issues the products into one of two accumulators,
 // warps 2-5 end the tile before meanwhile.
 // Every wait is bounded; one that gives up sets the error flag, and the roles run to their end.
@@ -20,11 +20,13 @@
 #include "tma.cuh"
 #include "umma.cuh"
 
+#include <type_traits>
+
 namespace {
 
 using bf16 = __nv_bfloat16;
-constexpr int MAX_E = 256, BM = 128, BK = 64, MAX_N = 256, THREADS = 192, STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2, SLOT_BYTES = A_BYTES + MAX_N * BK * 2, X_BOX = 32;
+constexpr int MAX_E = 256, BM = 128, BK = 64, THREADS = 192;
+constexpr int A_BYTES = BM * BK * 2, X_BOX = 32;
 constexpr int CHUNK = 32;  // tokens that the epilogue turns round in shared memory at a time
 
 struct Many {
@@ -90,7 +92,8 @@ struct Groups {
     int row0[MAX_E + 1], rows[MAX_E + 1], tile0[MAX_E + 2];
 };
 
-__device__ __forceinline__ int token_tiles(int rows) { return (rows + MAX_N - 1) / MAX_N; }
+template <int NT>
+__device__ __forceinline__ int token_tiles(int rows) { return (rows + NT - 1) / NT; }
 
 __device__ __forceinline__ int sum_up_to(int v, int lane) {
 #pragma unroll
@@ -101,10 +104,11 @@ __device__ __forceinline__ int sum_up_to(int v, int lane) {
     return v;
 }
 
-// By one warp; the caller meets before it reads.
+// By one warp; the caller meets before it reads.  NT: most tokens of a tile.
+template <int NT>
 __device__ __forceinline__ void find_groups(const Many& p, Groups* g, int tiles_s, int tiles_e) {
     const int lane = threadIdx.x & 31;
-    int rows = 0, tiles = p.fs > 0 ? tiles_s * token_tiles(p.T) : 0;
+    int rows = 0, tiles = p.fs > 0 ? tiles_s * token_tiles<NT>(p.T) : 0;
     if (lane == 0) {
         g->row0[0] = 0;
         g->rows[0] = p.fs > 0 ? p.T : 0;
@@ -116,7 +120,7 @@ __device__ __forceinline__ void find_groups(const Many& p, Groups* g, int tiles_
         const int mine = e < p.E ? __ldcg(p.counts + e) : 0, sum = sum_up_to(mine, lane);
         // a token has no more experts than the caller made room for; whatever the counts say, nobody leaves the buffers
         const int from = min(rows + sum - mine, p.cap), n = min(mine, p.cap - from);
-        const int t_sum = sum_up_to(tiles_e * token_tiles(n), lane);
+        const int t_sum = sum_up_to(tiles_e * token_tiles<NT>(n), lane);
         if (e < p.E) {
             g->row0[e + 1] = from;
             g->rows[e + 1] = n;
@@ -133,9 +137,10 @@ struct Tile {
 };
 
 // `cursor`: the last group looked at (tiles are walked in order).
+template <int NT>
 __device__ __forceinline__ Tile tile_at(const Groups& g, int tile, int& cursor, int step) {
     while (tile >= g.tile0[cursor + 1]) ++cursor;
-    const int rows = g.rows[cursor], over = token_tiles(rows), each = ((rows + over - 1) / over + 15) & ~15;
+    const int rows = g.rows[cursor], over = token_tiles<NT>(rows), each = ((rows + over - 1) / over + 15) & ~15;
     const int local = tile - g.tile0[cursor];
     Tile t;
     t.group = cursor;
@@ -163,18 +168,19 @@ enum { UP, UP_GATED, DOWN };
 
 // rows: the experts' rows of x (up) or of act (down); rows_s: x, or the shared expert's act, all in boxes of X_BOX rows;
 // w, w_s: the experts' and the shared expert's matrix (the same map where they are not gated).
-template <int WHAT>
+template <int WHAT, int NT, int STAGES>
 __global__ void __launch_bounds__(THREADS)
 experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_map, const __grid_constant__ CUtensorMap rows_s_map,
                        const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap w_s_map) {
     constexpr int STEP = WHAT == UP_GATED ? 64 : 128;  // features a tile
+    constexpr int SLOT_BYTES = A_BYTES + NT * BK * 2;
     constexpr int PITCH = STEP * 2 + 32;               // bytes from token to token in the epilogue's pieces
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* turn = ring + (size_t)STAGES * SLOT_BYTES;  // [2][CHUNK][PITCH]
     __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drained;
     __shared__ Groups groups;
-    __shared__ float factor[MAX_N];
+    __shared__ float factor[NT];
     __shared__ unsigned tmem_base;
     __shared__ volatile int gave_up;
 
@@ -199,13 +205,13 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
         tma::prefetch_map(&w_s_map);
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tma::smem_addr(&tmem_base)), "n"(2 * MAX_N) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tma::smem_addr(&tmem_base)), "n"(2 * NT) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     pdl_trigger();
     pdl_wait();
     const int width_e = WHAT == DOWN ? p.N : p.ff, width_s = WHAT == DOWN ? p.N : p.fs;
-    if (warp == 0) find_groups(p, &groups, (width_s + STEP - 1) / STEP, (width_e + STEP - 1) / STEP);
+    if (warp == 0) find_groups<NT>(p, &groups, (width_s + STEP - 1) / STEP, (width_e + STEP - 1) / STEP);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -223,7 +229,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
         int it = 0;
         bool ok = true;  // the same in all lanes
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            const Tile t = tile_at(groups, tile, cursor, STEP);
+            const Tile t = tile_at<NT>(groups, tile, cursor, STEP);
             const bool shared = t.group == 0;
             const int e = t.group - 1, kblocks = (inner(t.group) + BK - 1) / BK;
             const int n_boxes = (t.n + X_BOX - 1) / X_BOX, row = groups.row0[t.group] + t.row + lane * X_BOX;
@@ -256,11 +262,11 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
         int it = 0, i = 0;
         bool ok = true;  // the same in all lanes
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++i) {
-            const Tile t = tile_at(groups, tile, cursor, STEP);
+            const Tile t = tile_at<NT>(groups, tile, cursor, STEP);
             const int kblocks = (inner(t.group) + BK - 1) / BK;
             const unsigned idesc = umma::idesc_bf16(BM, t.n, false);
             const int buf = i & 1;
-            const unsigned d_tmem = tmem_base + buf * MAX_N;
+            const unsigned d_tmem = tmem_base + buf * NT;
             ok = __all_sync(0xffffffffu, i < 2 || tma::mbar_wait(&acc_empty[buf], ((i >> 1) - 1) & 1));
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             for (int kb = 0; kb < kblocks && ok; ++kb, ++it) {
@@ -291,13 +297,13 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
         const int quarter = warp & 3, mine = threadIdx.x - 64;  // mine: 0 .. 127
         int i = 0, piece = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
-            const Tile t = tile_at(groups, tile, cursor, STEP);
+            const Tile t = tile_at<NT>(groups, tile, cursor, STEP);
             const bool shared = t.group == 0;
             const int e = t.group - 1, buf = i & 1;
             const size_t row0 = (size_t)groups.row0[t.group] + t.row;
             if constexpr (WHAT != DOWN) {  // the tokens' weights of this expert, once everybody has read those of the tile before
                 meet_128();
-                for (int c = mine; c < MAX_N; c += 128) {
+                for (int c = mine; c < NT; c += 128) {
                     const int token = c < t.valid ? (shared ? t.row + c : __ldcg(p.list + (size_t)e * p.T + t.row + c)) : -1;
                     factor[c] = token >= 0 ? weight_of(p, token, shared ? p.E : e) : 0.f;
                 }
@@ -306,7 +312,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
             if (!ok) fail();
             if (any_of_128(!ok)) break;  // the four warps meet in a tile's pieces: they leave together
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const unsigned lane_base = tmem_base + buf * MAX_N + ((unsigned)(quarter * 32) << 16);
+            const unsigned lane_base = tmem_base + buf * NT + ((unsigned)(quarter * 32) << 16);
             if constexpr (WHAT == DOWN) {
                 const int n = t.f0 + quarter * 32 + lane;
                 float* y = (shared ? p.y_s : p.y) + row0 * p.N + n;
@@ -334,7 +340,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
                         // other token and gets what it lacks
                         const bool has_up = lane & 8;
                         unsigned char* at = dst + (quarter * 16 + (lane >> 4) * 8 + (lane & 7)) * 2 + (has_up ? PITCH : 0);
-                        const float* f = factor + c + (has_up ? 1 : 0);  // (c is a multiple of 32 below MAX_N)
+                        const float* f = factor + c + (has_up ? 1 : 0);  // (c is a multiple of 32 below NT)
 #pragma unroll
                         for (int j = 0; j < 32; j += 2) {
                             const float other = __shfl_xor_sync(0xffffffffu, has_up ? v[j] : v[j + 1], 8);
@@ -363,7 +369,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "n"(2 * MAX_N) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "n"(2 * NT) : "memory");
     }
 }
 
@@ -452,11 +458,11 @@ bool make_gated_map(CUtensorMap* map, const bf16* w, int experts, int ff, int K)
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int WHAT>
+template <int WHAT, int NT, int STAGES>
 int launch_product(const Many& p, const CUtensorMap& rows, const CUtensorMap& rows_s, const CUtensorMap& w, const CUtensorMap& w_s, cudaStream_t stream) {
     constexpr int STEP = WHAT == UP_GATED ? 64 : 128;
-    constexpr size_t smem = (size_t)STAGES * SLOT_BYTES + 1024 + (WHAT == DOWN ? 0 : 2 * CHUNK * (STEP * 2 + 32));
-    auto kernel = experts_product_kernel<WHAT>;
+    constexpr size_t smem = (size_t)STAGES * (A_BYTES + NT * BK * 2) + 1024 + (WHAT == DOWN ? 0 : 2 * CHUNK * (STEP * 2 + 32));
+    auto kernel = experts_product_kernel<WHAT, NT, STAGES>;
     // at every launch: the limit holds for the current device, and a process may have several
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -466,12 +472,13 @@ int launch_product(const Many& p, const CUtensorMap& rows, const CUtensorMap& ro
 }  // namespace
 
 // x [T, K] (row stride ldx) through the used experts: arguments as llm_experts_few, any number of tokens.  cap: rows that act [cap, ff] and
-// y [cap, N] have room for (tokens x experts of a token); act_s [T, fs] and y_s [T, N] for the shared expert; ints: E + 2 E T words.
+// y [cap, N] have room for (tokens x experts of a token); act_s [T, fs] and y_s [T, N] for the shared expert; ints: E + 2 E T words.  width: most tokens of a tile,
+// 64, 128 or 256.
 // Needs K, ff and fs multiples of 8, N a multiple of 4, K <= 2 N, E <= 256; LLM_ERR_UNSUPPORTED otherwise, and then nothing has been launched.
 LLM_EXPORT int llm_experts_many(const void* x, int ldx, const void* w_up, const void* w_down, int T, int K, int N, int E, int ff, int fs, int kind,
                                 float limit, float limit_s, float slope, float up_shift, const float* weights, int ldw, const int* ids,
                                 const int* table, int listed, int vocab, int* ints, int cap, void* act, void* act_s, float* y, float* y_s, float* out,
-                                float* resid, float alpha, int* error_flag, cudaStream_t stream) {
+                                float* resid, float alpha, int width, int* error_flag, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (K < 8 || ff < 8 || ((K | ff | fs | ldx) & 7) || (N & 3) || N <= 0 || K > 2 * N || E < 1 || E > MAX_E || cap < 1 || fs < 0 || T > (1 << 20)) return LLM_ERR_UNSUPPORTED;
     if (((uintptr_t)x | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)act_s | (uintptr_t)y | (uintptr_t)y_s | (uintptr_t)out | (uintptr_t)resid) & 15)
@@ -505,9 +512,14 @@ LLM_EXPORT int llm_experts_many(const void* x, int ldx, const void* w_up, const 
     if (code) return code;
     code = launch_pdl(experts_gather_kernel, dim3(T), dim3(128), 0, stream, p, (const bf16*)x, ldx, xs);
     if (code) return code;
-    code = kind < 0 ? launch_product<UP_GATED>(p, x_rows, x_boxes, up, up_s, stream) : launch_product<UP>(p, x_rows, x_boxes, up, up_s, stream);
-    if (code) return code;
-    code = launch_product<DOWN>(p, act_rows, act_s_rows, down, down, stream);
+    auto products = [&](auto width, auto stages) {
+        constexpr int NT = decltype(width)::value, STAGES = decltype(stages)::value;
+        const int up_code = kind < 0 ? launch_product<UP_GATED, NT, STAGES>(p, x_rows, x_boxes, up, up_s, stream) : launch_product<UP, NT, STAGES>(p, x_rows, x_boxes, up, up_s, stream);
+        return up_code ? up_code : launch_product<DOWN, NT, STAGES>(p, act_rows, act_s_rows, down, down, stream);
+    };
+    code = width <= 64 ? products(std::integral_constant<int, 64>{}, std::integral_constant<int, 8>{})
+         : width <= 128 ? products(std::integral_constant<int, 128>{}, std::integral_constant<int, 6>{})
+                        : products(std::integral_constant<int, 256>{}, std::integral_constant<int, 4>{});
     if (code) return code;
     return launch_pdl(experts_combine_kernel, dim3(T), dim3(256), 0, stream, p);
 }

@@ -65,7 +65,7 @@ _SIGNATURES = {
                                       _vp, _ll, _i, _vp, _vp, _f, _i, _i, _vp, _f, _f, _f, _vp, _vp],
     "llm_attention_tcgen05_own": [_vp, _ll, _ll, _vp, _ll, _ll, _vp, _i, _vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp, _vp, _vp],
     "llm_experts_few": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp],
-    "llm_experts_many": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _f,
+    "llm_experts_many": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _f, _vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _f, _i,
                          _vp, _vp],
     "llm_gemm_simt_batched": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _vp],
     "llm_sample": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
@@ -1790,6 +1790,16 @@ def experts_many_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: in
     return tokens > _EXPERTS_FEW and top < experts
 
 
+_EXPERTS_MANY_WIDTH: int | None = None  # tests and measurements choose the most tokens of a tile; None: the rule below
+
+
+def _experts_many_width(tokens: int, experts: int, top: int) -> int:
+    """The most tokens of a tile of :func:`experts_many`."""
+    if _EXPERTS_MANY_WIDTH:
+        return _EXPERTS_MANY_WIDTH
+    return 64 if tokens <= 256 else 128 if tokens <= 1024 else 256
+
+
 def experts_many(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, ff: int, shared_ff: int, *, top: int, activation: str | None = None,
                  limit: float = 0.0, shared_limit: float = 0.0, slope: float = 1.0, up_shift: float = 0.0, weights: torch.Tensor | None = None,
                  ids: torch.Tensor | None = None, table: torch.Tensor | None = None, sink: "ResidualSink | None" = None):
@@ -1828,7 +1838,7 @@ def experts_many(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, expe
     code = _launch("llm_experts_many", _ptr(x), x.stride(0), _ptr(w_up), _ptr(w_down), m, k, n, experts, ff, shared_ff,
                    -1 if gated else _UNARY_KINDS[activation], float(limit), float(shared_limit), float(slope), float(up_shift), _ptr(weights), ldw,
                    _ptr(ids), _ptr(table), listed, vocab, _ptr(ints), cap, _ptr(act), _ptr(act_s), _ptr(y), _ptr(y_s), _ptr(out), _ptr(resid),
-                   float(alpha), _error_flag_ptr(), _stream())
+                   float(alpha), _experts_many_width(m, experts, cap // m), _error_flag_ptr(), _stream())
     if code == 10002:
         add_launches(-1)
         return None

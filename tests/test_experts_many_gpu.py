@@ -34,9 +34,11 @@ def stated(x, w_up, w_down, E, ff, fs, wts, act, limits, slope, shift):
 
 @pytest.mark.parametrize("m", [1, 9, 40, 257, 530])
 @pytest.mark.parametrize("K, N, E, ff, fs", [(2048, 2048, 32, 704, 1408), (72, 36, 5, 40, 0), (1024, 1000, 37, 64, 136), (128, 128, 2, 8, 264), (64, 256, 256, 128, 0)])
-@pytest.mark.parametrize("form", ["gated", "table", "relu2", "silu", "gelu_tanh"])
-def test_used_experts_alone(m, K, N, E, ff, fs, form):
+@pytest.mark.parametrize("form, width", [("gated", 64), ("gated", 128), ("gated", 256), ("table", 128), ("relu2", 256), ("silu", 64), ("gelu_tanh", 128)])
+def test_used_experts_alone(m, K, N, E, ff, fs, form, width, monkeypatch):
     from llmserve_triton_kernels_b200 import ops
+
+    monkeypatch.setattr(ops, "_EXPERTS_MANY_WIDTH", width)  # most tokens of a tile
 
     act = form if form in ("relu2", "silu", "gelu_tanh") else None
     per, top = 1 if act else 2, min(4, E - 1)
