@@ -16,9 +16,13 @@
 //   down  a CTA 16 features; boxes of 64 k, the tokens' lanes of the same k behind the weights in the slot.  Which warp has a box depends on
 //         the box's place in w_down alone: a token's bits are the same whatever experts the other tokens use.
 // An up CTA and a down CTA share an SM (at most 120 registers x 256 threads and 227 KB together): the up kernel lets its dependent start
-// behind its own wait, by when the router has ended, so that the down kernel makes its list and asks for its first boxes while the up
-// kernel runs, which also brings the rest of the down kernel's weights into L2 behind its own.  The shared expert's boxes (and, with a
-// table, everybody's) are on their way before the kernel in front has ended.
+// behind its own wait, by when the router has ended, so that the down kernel makes its list and asks for its first boxes (10 MB) while the up
+// kernel runs.  The shared expert's boxes (and, with a table, everybody's) are on their way before the kernel in front has ended.
+// Measured (us for both behind a router, weights in memory; before: sixteen warps that met at every tile, a down kernel whose registers kept it
+// off every SM until the up kernel had left, its weights brought into L2 by the up kernel): 32 experts of 704, 4 used, a shared one of
+// 1,408, 2,048 wide: one token 20.4 -> 17.6, 3 34.0 -> 31.9, 8 55.5 -> 51.6; 8 experts of 5,632, 2 used: 45.9 -> 40.5, 8 tokens 131 -> 109; 128 of
+// 192, 8 used: 20.0 -> 14.5, 8 tokens 66.4 -> 51.0.  The up kernel bringing the down kernel's weights into L2 costs 2 to 11 us of that;
+// rings of 4 to 6 boxes in the up kernel (and fewer in the other, or one CTA an SM) 1 to 7 us.
 #include "common.cuh"
 #include "linear_stream.cuh"
 #include "tma.cuh"
@@ -29,7 +33,6 @@ using bf16 = __nv_bfloat16;
 constexpr int MAX_M = 8, MAX_E = 256, WARPS = 8, THREADS = WARPS * 32, MEET = 4;  // MEET: tiles between two meetings of the up kernel
 constexpr int UP_BOXK = 128, UP_KB = 2, UP_SLOTS = 3, UP_SLOT = 16 * UP_BOXK;  // elements of a slot; UP_KB: most boxes a warp has of a tile
 constexpr int DOWN_BOXK = 64, DOWN_SLOTS = 3, DOWN_SLOT = (16 + MAX_M) * DOWN_BOXK;
-constexpr size_t AHEAD_BYTES = 32 << 20;  // the most of w_down that the up kernel brings into L2
 constexpr size_t UP_SMEM = 1024 + (size_t)WARPS * UP_SLOTS * UP_SLOT * 2 + 2 * (size_t)MEET * WARPS * 32 * 16;
 constexpr size_t DOWN_SMEM = 1024 + (size_t)WARPS * DOWN_SLOTS * DOWN_SLOT * 2 + (size_t)WARPS * 32 * 16;
 
@@ -185,21 +188,7 @@ __global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid
     }
     const int lda = p.E * p.ff + p.fs;
     int unit = 0;
-    bool gave_up = false, ahead = false;
-    // the down kernel's weights on their way into L2 behind this kernel's: memory does not stand still while this one ends (row by row of
-    // a block, dealt over the CTAs' warps)
-    auto bring_ahead = [&]() {
-        if (ahead) return;
-        ahead = true;
-        const int blocks = (p.fs > 0 ? 1 : 0) + count;
-        const int items = (int)min((long long)blocks * p.N, (long long)(AHEAD_BYTES / (2 * (size_t)max(p.ff, p.fs))));
-        for (int i = (blockIdx.x * WARPS + warp) * 32 + lane; i < items; i += gridDim.x * THREADS) {
-            const int b = i / p.N, n = i - b * p.N;
-            const bool shared = p.fs > 0 && b == 0;
-            const bf16* at = p.w_down + (size_t)n * lda + (size_t)(shared ? p.E : list[b - (p.fs > 0 ? 1 : 0)]) * p.ff;
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(at), "r"((shared ? p.fs : p.ff) * 2) : "memory");
-        }
-    };
+    bool gave_up = false;
     for (int t0 = 0, round = 0; t0 < tiles; t0 += MEET, ++round) {
         const int t1 = min(tiles, t0 + MEET);
         float4* mine = red + (size_t)(round & 1) * MEET * WARPS * 32;
@@ -208,7 +197,6 @@ __global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid
 #pragma unroll
             for (int j = 0; j < UP_KB; ++j) {
                 if (j >= my_kb) break;
-                if (unit + UP_SLOTS >= tiles * my_kb) bring_ahead();  // the warp's last box has been asked for
                 const int s = unit % UP_SLOTS;
                 if (!gave_up && !tma::mbar_wait(&my_full[s], (unit / UP_SLOTS) & 1)) {
                     gave_up = true;
@@ -231,7 +219,6 @@ __global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid
             }
             mine[((t - t0) * WARPS + warp) * 32 + lane] = make_float4(c[0] + d[0], c[1] + d[1], c[2] + d[2], c[3] + d[3]);
         }
-        if (t1 == tiles) bring_ahead();  // (a warp without boxes)
         __syncthreads();  // this buffer of sums is written again two meetings on
         for (int t = t0 + warp; t < t1; t += WARPS) {
             int e, f0;
