@@ -1785,19 +1785,50 @@ def experts_few(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, exper
     return NormedInput(xw, ss, sink.eps, sink.norm) if norm_w is not None else ADDED
 
 
-def experts_many_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int) -> bool:
-    """Whether the used experts' own products (:func:`experts_many`) are faster than the products over all experts."""
-    return tokens > _EXPERTS_FEW and top < experts
-
-
+_EXPERTS_MANY_MIN = 128  # tokens, see experts_many_pay
 _EXPERTS_MANY_WIDTH: int | None = None  # tests and measurements choose the most tokens of a tile; None: the rule below
 
 
-def _experts_many_width(tokens: int, experts: int, top: int) -> int:
-    """The most tokens of a tile of :func:`experts_many`."""
-    if _EXPERTS_MANY_WIDTH:
-        return _EXPERTS_MANY_WIDTH
-    return 64 if tokens <= 256 else 128 if tokens <= 1024 else 256
+def _experts_many_tiles(tokens: int, experts: int, top: int, ff: int, shared_ff: int, gated: bool) -> tuple[int, float, float, int]:
+    """``(the most tokens of a tile of experts_many, tiles of the busiest SM in the first product, tokens of an average tile, tiles of an
+    expert's rows)``, the experts evenly used: the width (64, 128 or 256) whose busiest SM has the least to do, a tile costing as much as 80
+    tokens whatever it holds.  Measured (used experts, us with 64 / 128 / 256): 32 experts of 704, 4 used, a shared one of 1,408: 256 tokens 96 / 98 /
+    110, 512 120 / 106 / 118, 1,024 191 / 149 / 141, 1,800 317 / 243 / 212; 8 of 7,168, 2 used: 256 tokens 385 / 327 / 341."""
+    used = experts * (1.0 - (1.0 - top / experts) ** tokens)
+    rows = tokens * top / used
+    step, best = (64 if gated else 128), None
+    for width in (_EXPERTS_MANY_WIDTH,) if _EXPERTS_MANY_WIDTH else (64, 128, 256):
+        of_expert, of_shared = math.ceil((rows + math.sqrt(rows)) / width), math.ceil(tokens / width)
+        n_e, n_s = -(-math.ceil(rows / of_expert) // 16) * 16, -(-math.ceil(tokens / of_shared) // 16) * 16
+        a, b = used * math.ceil(ff / step) * of_expert, float(math.ceil(shared_ff / step) * of_shared)
+        n, each = (a * n_e + b * n_s) / (a + b), math.ceil((a + b) / _sm_count())
+        if best is None or each * (80.0 + n) < best[1] * (80.0 + best[2]):
+            best = (width, each, n, of_expert)
+    return best
+
+
+def experts_many_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int, gated: bool, hidden: int) -> bool:
+    """Whether the used experts' own products (:func:`experts_many`) are faster than the products over all experts.  Both ways' times fitted
+    to 130 steps on a B200 (13 mixtures of 4 to 256 experts, inner sizes 64 to 7,168, 256 to 4,096 wide, 9 to 4,096 tokens): a fixed part and
+    the root of the squares of the weights' bytes at the copy rate and of the operations (all experts: at 1.31 PFLOP/s; the used ones: by the
+    busiest SM's tiles), for the used ones also the rows that travel between the kernels.  The choice takes no step of that sweep more than 1 %
+    slower than the faster way; under 128 tokens the two are within a few per cent wherever the used ones are faster at all.  All -> used (us): 32
+    experts of 704, 4 used, a shared one of 1,408: 256 tokens 104 -> 96, 512 137 -> 106, 1,800 404 -> 212; 8 of 1,408, 2 used: 512 90 -> 89, 1,800
+    194 -> 140; 16 of 704, 8 used: 1,800 232 -> 284."""
+    if tokens < _EXPERTS_MANY_MIN or top >= experts:
+        return False
+    width, each, n, of_expert = _experts_many_tiles(tokens, experts, top, ff, shared_ff, gated)
+    per = 3 if gated else 2
+    used = experts * (1.0 - (1.0 - top / experts) ** tokens)
+    row, flops = per * hidden * 2 / 6.55e6, 2.0 * tokens * (experts * ff + shared_ff) * per * hidden  # us an inner feature's weights
+    time_all = 18.0 + math.hypot(1.54 * (experts * ff + shared_ff) * row, flops / 1.31e9)
+    of_shared = math.ceil(tokens / width) if shared_ff else 0
+    tiles = used * of_expert + of_shared
+    inner = (used * of_expert * ff + of_shared * shared_ff) / tiles
+    up = each * (80.0 + n) * hidden / 64
+    down = math.ceil(math.ceil(hidden / 128) * tiles / _sm_count()) * (80.0 + n) * (inner / 64 + 4)
+    time_used = 26.0 + math.hypot(1.11 * (used * ff + shared_ff) * row, (1.47 * up + 3.4 * down) / 1e3) + 1.96 * tokens * (top + 1) * hidden * 12 / 6.55e6
+    return 1.03 * time_used < time_all
 
 
 def experts_many(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, experts: int, ff: int, shared_ff: int, *, top: int, activation: str | None = None,
@@ -1838,7 +1869,7 @@ def experts_many(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, expe
     code = _launch("llm_experts_many", _ptr(x), x.stride(0), _ptr(w_up), _ptr(w_down), m, k, n, experts, ff, shared_ff,
                    -1 if gated else _UNARY_KINDS[activation], float(limit), float(shared_limit), float(slope), float(up_shift), _ptr(weights), ldw,
                    _ptr(ids), _ptr(table), listed, vocab, _ptr(ints), cap, _ptr(act), _ptr(act_s), _ptr(y), _ptr(y_s), _ptr(out), _ptr(resid),
-                   float(alpha), _experts_many_width(m, experts, cap // m), _error_flag_ptr(), _stream())
+                   float(alpha), _experts_many_tiles(m, experts, cap // m, ff, shared_ff, gated)[0], _error_flag_ptr(), _stream())
     if code == 10002:
         add_launches(-1)
         return None

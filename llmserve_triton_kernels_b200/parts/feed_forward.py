@@ -128,7 +128,7 @@ def _used_experts(part, x, sink, **kw):
     """What the kernels that read only the used experts return for a mixture, or None where the products over all experts are the way."""
     sizes = (part.experts, part.expert_size, part.shared_size)
     few = ops.experts_few(x, part.w_up, part.w_down, *sizes, sink=sink, top=part.top, **kw)
-    if few is not None or not ops.experts_many_pay(x.shape[0], part.experts, part.top, part.expert_size, part.shared_size):
+    if few is not None or not ops.experts_many_pay(x.shape[0], part.experts, part.top, part.expert_size, part.shared_size, kw.get("activation") is None, x.shape[1]):
         return few
     return ops.experts_many(x, part.w_up, part.w_down, *sizes, sink=sink, top=part.top, **kw)
 

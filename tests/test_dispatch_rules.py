@@ -67,3 +67,18 @@ def test_latent_queries_are_multiplied_beside_the_preparation_while_that_is_shor
 def test_the_used_experts_are_read_alone_where_that_is_faster(used_alone, sizes):
     hidden, experts, top, ff, shared, matrices, tokens = sizes
     assert ops.experts_few_pay(tokens, experts, top, ff, shared, 2 * matrices * hidden) == used_alone
+
+
+def test_experts_of_many_tokens_run_alone_where_that_was_measured_faster(monkeypatch):
+    """Steps on both sides of the line, with both ways' times on a B200 (microseconds)."""
+    from llmserve_triton_kernels_b200 import ops
+
+    monkeypatch.setattr(ops, "_sm_count", lambda: 148)
+    for tokens, experts, top, ff, shared, gated, hidden, everybody, used in (
+        (512, 32, 4, 704, 1408, True, 2048, 137, 106), (1800, 32, 4, 704, 1408, True, 2048, 404, 212), (120, 32, 4, 704, 1408, True, 2048, 90, 90),
+        (1024, 32, 4, 704, 1408, False, 2048, 165, 137), (256, 32, 4, 704, 1408, False, 2048, 79, 84), (512, 16, 2, 512, 1024, True, 1024, 51, 57),
+        (1800, 16, 2, 512, 1024, True, 1024, 106, 93), (4096, 16, 2, 512, 1024, False, 1024, 143, 148), (1800, 16, 8, 704, 1408, True, 2048, 232, 284),
+        (4096, 8, 6, 512, 0, True, 512, 85, 171), (1800, 8, 2, 1408, 0, True, 2048, 194, 140), (4096, 4, 2, 2816, 0, True, 1024, 253, 277),
+    ):
+        assert ops.experts_many_pay(tokens, experts, top, ff, shared, gated, hidden) == (used < 0.98 * everybody), (tokens, experts, hidden)
+    assert not ops.experts_many_pay(4096, 8, 8, 704, 0, True, 2048)  # every token uses every expert
