@@ -268,37 +268,42 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         // ---- issuer of the second product: O += P_j V_j, as soon as the probabilities and the values are there ----
         constexpr unsigned IDESC_PV = umma::idesc_bf16(BM, VD, true);
         const unsigned o_tmem = tmem_base + O_COL, p_tmem = tmem_base + P_COL;
-        bool ok = true;  // the loop's head: as lane 0 has it
-        for (int j = 0; j < n_tiles && __shfl_sync(0xffffffffu, (int)(ok && !gave_up), 0); ++j) {
+        bool ok = true;
+        auto multiply = [&](int j) {  // lane 0
             const int s = j % STAGES;
-            unsigned char* values = kv_s + (size_t)s * STAGE_BYTES + K_BYTES;
-            const int real = ctx_len - tile_start(j);  // keys of this tile that the request has
-            if (lane == 0) ok = tma::mbar_wait(&v_full[s], (j / STAGES) & 1);
-            if (real < BN) {
-                // rows that are not the request's: a probability of zero times what is no number would be none either
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0 && tma::mbar_wait(&v_full[s], (j / STAGES) & 1);
-                if (ok)
-                    for (int i = max(real, 0) * 8 + lane; i < BN * 8; i += 32)
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            // the values lie [key][d]: B with N contiguous; 16 keys are two atoms of 8 rows, 2048 bytes further per step
+            // (a head of 128 lanes is two such pieces side by side, BN * 128 bytes apart: the leading offset)
+            const unsigned long long v_desc = umma::desc_sw128(kv_s + (size_t)s * STAGE_BYTES + K_BYTES, (V_HALVES > 1 ? BN * 128 : 1024) >> 4);
 #pragma unroll
-                        for (int h = 0; h < V_HALVES; ++h) reinterpret_cast<uint4*>(values + (size_t)h * (BN * 128))[i] = make_uint4(0, 0, 0, 0);
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                ok = __all_sync(0xffffffffu, ok);
+            for (int k = 0; k < BN / 16; ++k)  // the output accumulates over the tiles
+                umma::mma_bf16_ts(o_tmem, p_tmem + 8 * k, v_desc + (2048 >> 4) * k, IDESC_PV, k != 0 || j != 0);
+            umma::commit(&o_full);
+            umma::commit(&v_empty[s]);
+        };
+        // only the request's last tile may hold rows that are not the request's
+        const int real = ctx_len - tile_start(n_tiles - 1), whole_tiles = n_tiles - (real < BN ? 1 : 0);
+        if (lane == 0)
+            for (int j = 0; j < whole_tiles && ok && !gave_up; ++j) {
+                ok = tma::mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1) && tma::mbar_wait(&p_full, j & 1);
+                if (ok) multiply(j);
             }
+        __syncwarp();
+        if (whole_tiles < n_tiles && __shfl_sync(0xffffffffu, (int)(ok && !gave_up), 0)) {
+            // a probability of zero times what is no number would be none either: those rows become zeros
+            const int j = whole_tiles, s = j % STAGES;
+            uint4* values = reinterpret_cast<uint4*>(kv_s + (size_t)s * STAGE_BYTES + K_BYTES);
+            ok = __all_sync(0xffffffffu, tma::mbar_wait(&v_full[s], (j / STAGES) & 1));
+            if (ok)
+                for (int i = real * 8 + lane; i < BN * 8; i += 32)
+#pragma unroll
+                    for (int h = 0; h < V_HALVES; ++h) values[h * (BN * 8) + i] = make_uint4(0, 0, 0, 0);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
             if (lane == 0) {
                 ok = ok && tma::mbar_wait(&p_full, j & 1);
-                if (ok) {
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    // the values lie [key][d]: B with N contiguous; 16 keys are two atoms of 8 rows, 2048 bytes further per step
-                    // (a head of 128 lanes is two such pieces side by side, BN * 128 bytes apart: the leading offset)
-                    const unsigned long long v_desc = umma::desc_sw128(values, (V_HALVES > 1 ? BN * 128 : 1024) >> 4);
-#pragma unroll
-                    for (int k = 0; k < BN / 16; ++k)  // the output accumulates over the tiles
-                        umma::mma_bf16_ts(o_tmem, p_tmem + 8 * k, v_desc + (2048 >> 4) * k, IDESC_PV, k != 0 || j != 0);
-                    umma::commit(&o_full);
-                    umma::commit(&v_empty[s]);
-                }
+                if (ok) multiply(j);
             }
-            __syncwarp();
         }
         if (!ok && lane == 0) fail();
     } else {
