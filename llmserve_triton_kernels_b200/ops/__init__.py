@@ -1681,7 +1681,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
     _i32(cu_tokens, "cu_tokens")
     out = torch.empty((q.shape[0], heads, value_dim), dtype=torch.float32, device=q.device)
     few = 0 < int(max_query_len) <= 16
-    stretches = _scan_stretches(few, dim, value_dim, heads, int(num_requests), int(max_query_len))
+    stretches = _scan_stretches(few, dim, value_dim, heads, int(num_requests), int(max_query_len), q.shape[0], True)
     scratch = None
     if stretches > 1:  # the stretches' end states, start states and products of decays
         scratch = torch.empty((int(num_requests) * stretches * heads * (2 * dim * value_dim + dim),), dtype=torch.float32, device=q.device)
@@ -1992,11 +1992,30 @@ def sigmoid_attention(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Ten
 _RETENTION_MIN_STRETCH = 64  # tokens a stretch of a long request has at least
 
 
-def _scan_stretches(few: bool, dim: int, value_dim: int, heads: int, requests: int, max_query_len: int) -> int:
-    """Into how many stretches the scans (csrc/retention.cu) cut a long request, so that the GPU has CTAs enough."""
+def _scan_stretches(few: bool, dim: int, value_dim: int, heads: int, requests: int, max_query_len: int, tokens: int, gated: bool = False) -> int:
+    """Into how many stretches the scans (csrc/retention.cu) cut a long request.  So many that the GPU has CTAs enough, but at most 8; keys
+    of up to 64 lanes: the number that a fit to their times expects to be the fastest, where it expects 12 % less time than of that (it
+    mistakes the order of closer ones; wider keys it mistook by up to 40 %).  A walk takes 8 us and 0.142 us a token (gated 0.33), as often
+    as its CTAs fill the SMs (what fits into their shared memory; half of a started round counts in full); requests shorter than the longest
+    leave room.  In stretches there are two walks, the start states between them, and each CTA's states to bring (the last term).  Measured
+    (heads of 64 by 128, us for all launches): one request of 1,801 tokens, 16 heads, gated: 8 stretches 202, 13 140, 16 195; 8 heads: 8 169,
+    24 91; two of 4,096, 4 heads: 8 171, 18 102; not gated, four requests of up to 600 and 16 heads: 1 112, 3 90, 5 102; four of 300: 1 66,
+    4 88; eight of 128: 1 39, 2 70."""
     cols = 16 if few else 64 if dim <= 64 else 32 if dim <= 128 else 16  # columns of the state that one CTA owns
     ctas = -(-value_dim // cols) * heads * requests
-    return max(1, min(8, max_query_len // _RETENTION_MIN_STRETCH, -(-4 * _sm_count() // ctas), 65535 // max(1, requests)))
+    enough = max(1, min(8, max_query_len // _RETENTION_MIN_STRETCH, -(-4 * _sm_count() // ctas), 65535 // max(1, requests)))
+    if few or dim > 64:
+        return enough
+    each, start, bring, an_sm = (0.33, 14.0, 0.032, 3 if dim > 32 else 5) if gated else (0.142, 8.0, 0.01, 2 if dim > 32 else 3)
+    busy = ctas / requests * tokens / max(1, max_query_len)
+
+    def expected(n: int) -> float:
+        rounds = busy * n / (an_sm * _sm_count())
+        walk = (8.0 + max_query_len / n * each) * max(1.0, (rounds + math.ceil(rounds)) / 2)
+        return walk if n == 1 else start + 2 * walk + ctas * n * bring
+
+    best = min(range(1, max(1, min(24, max_query_len // _RETENTION_MIN_STRETCH, 65535 // max(1, requests))) + 1), key=expected)
+    return best if expected(best) < 0.88 * expected(enough) else enough
 
 
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, states: torch.Tensor,
@@ -2016,7 +2035,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     _i32(cu_tokens, "cu_tokens")
     out = torch.empty((q.shape[0], heads, value_dim), dtype=torch.float32, device=q.device)
     few = 0 < int(max_query_len) <= 16  # a decode step, or portions of a few tokens
-    stretches = _scan_stretches(few, dim, value_dim, heads, int(num_requests), int(max_query_len))
+    stretches = _scan_stretches(few, dim, value_dim, heads, int(num_requests), int(max_query_len), q.shape[0])
     scratch = None
     if stretches > 1:
         scratch = torch.empty((2, int(num_requests) * stretches, heads, dim, value_dim), dtype=torch.float32, device=q.device)

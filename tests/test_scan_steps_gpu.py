@@ -39,3 +39,31 @@ def test_a_token_has_the_same_bits_in_steps_of_any_length(H, D, V, v_dtype, gate
             got[torch.tensor(rows, device=DEV)] = scan(rows, news, mine)
             at = [a + n for a, n in zip(at, news)]
         assert torch.equal(got, want) and torch.equal(mine, whole), f"portions of {cut}"
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_long_requests_walk_in_the_expected_number_of_stretches(gated, monkeypatch):
+    """Every number of stretches that the rule may choose gives the same outputs and states to the sums' rounding: 24 (the most), one that fills
+    the SMs once, and 1, for requests of which one has fewer tokens than there are stretches."""
+    ops = _ops()
+    heads, dim, value_dim, lens = 4, 64, 48, [1600, 7, 300]
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    q, k, z = (0.3 * torch.randn(sum(lens), heads * dim, device=DEV, generator=gen) for _ in range(3))
+    v = torch.randn(sum(lens), heads * value_dim, device=DEV, generator=gen)
+    start = torch.randn(4, heads, dim, value_dim, device=DEV, generator=gen)
+    cu = torch.tensor([0, 1600, 1607, 1907], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
+
+    def run():
+        states = start.clone()
+        args = (states, slots, cu, 3, heads, dim, value_dim, max(lens))
+        out = ops.gated_scan(q, k, v, z, None, 0.1, 1.0, *args) if gated else ops.retention_scan(q, k, v, torch.linspace(0.9, 0.99, heads, device=DEV), *args)
+        return out, states
+
+    assert ops._scan_stretches(False, dim, value_dim, heads, 1, 1600, 1600, gated) > 8
+    monkeypatch.setattr(ops, "_scan_stretches", lambda *a: 1)
+    want = run()
+    for n in (13, 24):
+        monkeypatch.setattr(ops, "_scan_stretches", lambda *a, n=n: n)
+        for got, ref in zip(run(), want):  # 32-bit sums of some hundred decaying terms in another order: 2^-24 * sqrt(1600) * their size
+            assert (got - ref).abs().max() <= 4e-6 * ref.abs().max()
