@@ -1720,17 +1720,16 @@ def expert_gated_act(x: torch.Tensor, experts: int, ff: int, shared_ff: int, lim
 
 
 _EXPERTS_FEW = 8  # tokens, see experts_few
-_EXPERTS_FEW_SHARE, _EXPERTS_FEW_EACH = 0.78, 2.5e6  # see experts_few_pay
+_EXPERTS_FEW_SHARE, _EXPERTS_FEW_EACH = 0.76, 0.95e6  # see experts_few_pay
 
 
 def experts_few_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: int, row_bytes: int) -> bool:
     """Whether reading only the used experts (:func:`experts_few`) is faster than the products over all of them, for tokens that choose
-    ``top`` of ``experts`` each; ``row_bytes``: bytes of all matrices an inner feature.  Fitted to 256 steps on a B200 (16 mixtures of 8 to
-    256 experts, inner sizes 64 to 5,632, 512 to 2,048 wide, 1 to 8 tokens, cold): the products over all take 8 us and 1.25 times their
-    bytes' time at the copy rate, the used ones 8 us, 1.6 times theirs and 0.6 us an expert (2.5 MB's time).  The choice is 0.8 % off the
-    faster way on average and takes no step more than 16 % slower.  All -> used, in microseconds: 32 experts of 704, 4 used, and a shared
-    one of 1,408: one token 64.0 -> 20.6, 4 65.1 -> 45.8, 7 65.0 -> 60.3, 8 65.3 -> 67.3; 16 of 512, 8 used: 2 tokens 19.9 -> 21.4, 8
-    20.0 -> 26.4; 64 of 64, 4 used: one 14.7 -> 10.7, 4 14.6 -> 17.1."""
+    ``top`` of ``experts`` each; ``row_bytes``: bytes of all matrices an inner feature.  Fitted to 72 steps on a B200 (12 mixtures of 4 to
+    256 experts, inner sizes 64 to 5,632, 512 to 2,048 wide, 1 to 8 tokens, cold): the used experts' bytes take 1 / 0.76 of the time that the
+    products over all take for theirs, and an expert costs 0.95 MB's time beside.  The choice is 0.9 % off the faster way on average and takes no
+    step more than 28 % slower (one of 13 us).  All -> used, in microseconds: 32 experts of 704, 4 used, and a shared one of 1,408: one token 61.8 -> 17.5,
+    4 62.1 -> 40.0, 8 62.2 -> 51.0; 16 of 704, 8 used: one token 37.7 -> 26.7, 3 38.0 -> 42.8; 64 of 64, 4 used: one 12.9 -> 8.4, 6 13.0 -> 14.1."""
     used = experts * (1.0 - (1.0 - top / experts) ** tokens)
     return (used * ff + shared_ff) * row_bytes + used * _EXPERTS_FEW_EACH <= _EXPERTS_FEW_SHARE * (experts * ff + shared_ff) * row_bytes
 
