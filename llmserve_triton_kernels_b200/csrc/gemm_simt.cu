@@ -297,7 +297,8 @@ int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, 
     if (M <= 16) return launch_few<16, 3>(x, w, out, M, N, K, ldx, ldw, ldo, stream);
     // the tile that takes the least time by how many of them the busiest SM has.  Measured (2,048 k, 17 to 300 rows of 1,024 to 11,264
     // features, microseconds; n tiles of an SM): 232 n, 145 n, 27 + 59 n and 32 + 31 n.  242 rows: 2,560 features 145 with 64 x 64, 118 with 32 x 64;
-    // 2,048 features 88 and 104; 11,264 features 322 and 338.
+    // 2,048 features 88 and 104; 11,264 features 322 and 338.  Against the rule before (the areas of the busiest SM's tiles at assumed rates): 11,264
+    // features, 200 rows 365 -> 310, 300 479 -> 377, 512 709 -> 604; 2,048 features, 700 rows 197 -> 173; most sizes as they were.
     struct { int rm, rn; double once, each; } const kinds[4] = {{128, 128, 0., 232.}, {64, 128, 0., 145.}, {64, 64, 27., 59.}, {32, 64, 32., 31.}};
     int best = 0;
     double best_cost = 1e30;

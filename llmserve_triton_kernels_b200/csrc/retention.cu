@@ -288,7 +288,8 @@ retention_scan_kernel(const float* __restrict__ q, int ldq, const float* __restr
 // The same walk for steps of few tokens a request, bound by the way to memory and back: a warp owns 16 columns of one (request, head) and
 // nothing is shared with another.  Lane (part, quarter) holds rows part * DPT .. of the quarter's four columns, from the state's rows
 // straight into registers and back (64 bytes a row), and reads the lanes of q, k and z that its rows meet.  A sum's parts and their order
-// are those of the kernel above, so a token has the same bits in both.  D = 8 * DPT, V a multiple of 16, rows on 16 bytes.
+// are those of the kernel above, so a token has the same bits in both.  D = 8 * DPT, V a multiple of 16, rows on 16 bytes.  Measured (us a
+// layer, one token a request; the kernel above before): four requests, 16 heads of 64 by 128 12.4 -> 2.95, one request with gates 8.6 -> 2.96.
 template <typename TV, int DPT, bool GATED>
 __global__ void __launch_bounds__(64)
 scan_step_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk, const TV* __restrict__ v, int ldv,
