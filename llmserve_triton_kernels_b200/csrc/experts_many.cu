@@ -9,7 +9,7 @@
 // What bounds it: the weights' bytes up to about 1,500 tokens (32 experts of 704 in 2,048: 294 MB a layer), beyond that the tensor cores; the
 // products over all experts with the token's weight as a factor, which ran before, did eight times the operations for 4 of 32 experts.
 // Measured (us a layer, all products over all experts -> these launches): 32 experts of 704, 4 used, a shared one of 1,408, 2,048 wide, 1,801
-// tokens 387 -> 187 (up 89 at 0.45 of the tensor peak, down 65, combine 19, gather 8, sort 6); 256 tokens 104 -> 96, 512 137 -> 106.  Rows
+// tokens 387 -> 187 (up 89 at 0.42 of the tensor peak, down 65, combine 19, gather 8, sort 6); 256 tokens 104 -> 96, 512 137 -> 106.  Rows
 // gathered by the product itself (TMA, four rows a box) took 375 at 1,800 tokens.
 //
 // The products are tcgen05 with the WEIGHTS as the 128 rows of the tile and an expert's tokens as its columns: an expert has as many

@@ -134,7 +134,11 @@ _TC_ATTENTION_ENABLED = True
 _TC_ATTENTION_HEAD_DIMS = (64, 128)
 _TC_ATTENTION_PAGE_SIZES = (8, 16, 32, 64)
 _TC_ATTENTION_MIN_TOKENS = 128  # a request with at least this many tokens in the step: attention on tcgen05
-_TC_ATTENTION_JOIN_TOKENS = 32  # where that kernel runs, requests of at least so many go along (tiles of their own beside the others')
+# Where that kernel runs, requests of at least so many go along (tiles of their own beside the others').  A request of 512 tokens and, in a
+# launch of their own -> along (us, 32 heads of 64): 4 of 32 28.3 -> 12.9, 4 of 100 25.4 -> 13.3, 16 of 32 23.3 -> 21.9, 4 of 64 behind 1,000 cached
+# 79.6 -> 33.4.  Of fewer tokens it depends on what is cached: 7 of 24 behind 500 39.1 -> 28.7, but 31 of 24 behind 300 51.6 -> 62.5; 3 of 16 behind
+# 1,500 33.0 -> 42.0.
+_TC_ATTENTION_JOIN_TOKENS = 32
 _TCGEN05_MIN_ROWS = 128  # from this many rows a bfloat16 product runs on tcgen05 with TMA-fed tiles (own kernel)
 _DECODE_LINEAR_MAX_ROWS = 16  # up to this many rows a bfloat16 matrix product streams the weights once (own kernel)
 _FORCE_GENERIC_ATTENTION = False  # tests switch the tensor-core attention off to reach the general kernel in bfloat16
