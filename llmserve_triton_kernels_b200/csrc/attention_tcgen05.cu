@@ -596,14 +596,13 @@ LLM_EXPORT int llm_attention_tcgen05_min_tokens() { return 128; }
 
 namespace {
 template <int KD, int VD, bool EXTRA, bool OWN>
-int launch_tcgen05(const TcParams& tp, const CUtensorMap* qmap, const CUtensorMap* kvmap, unsigned grid_y, cudaStream_t stream) {
+int launch_tcgen05(const TcParams& tp, const CUtensorMap& qmap, const CUtensorMap& kvmap, unsigned grid_y, cudaStream_t stream) {
     using Sh = Shape<KD, VD>;
-    if (!kvmap || !qmap) return LLM_ERR_UNSUPPORTED;
     auto kernel = attention_tcgen05_kernel<KD, VD, EXTRA, OWN>;
     // at every launch: the limit holds for the current device, and a process may have several
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
     if (e != cudaSuccess) return (int)e;
-    return launch_pdl(kernel, dim3((unsigned)(tp.a.H * tp.maps), grid_y), dim3(THREADS), Sh::SMEM, stream, tp, *qmap, *kvmap);
+    return launch_pdl(kernel, dim3((unsigned)(tp.a.H * tp.maps), grid_y), dim3(THREADS), Sh::SMEM, stream, tp, qmap, kvmap);
 }
 
 struct Differential {  // how two maps meet (raw == null: one map a head)
@@ -672,9 +671,10 @@ int attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, co
     const long long y = (long long)requests * tp.tiles_per_request;
     if (y > 65535) return LLM_ERR_UNSUPPORTED;
     // one box of keys or values: a page's rows, 64 of the head's lanes; one box of queries: 128 tokens, 64 lanes of a head
-    const CUtensorMap* kvmap = tma::cached_map_2d_bf16(pool, (uint64_t)kv_rows, (uint64_t)row_lanes, (uint64_t)row_lanes, (uint32_t)page_size, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap* qmap = KD == 64 ? kvmap
-                                       : tma::cached_map_2d_bf16(q, (uint64_t)n_tokens, (uint64_t)H * maps * KD, (uint64_t)q_stride, BM, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    CUtensorMap kvmap, qmap;
+    if (!tma::cached_map_2d_bf16(&kvmap, pool, (uint64_t)kv_rows, (uint64_t)row_lanes, (uint64_t)row_lanes, (uint32_t)page_size, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return LLM_ERR_UNSUPPORTED;
+    if (KD == 64) qmap = kvmap;
+    else if (!tma::make_map_2d_bf16(&qmap, q, (uint64_t)n_tokens, (uint64_t)H * maps * KD, (uint64_t)q_stride, BM, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return LLM_ERR_UNSUPPORTED;
     const bool extra = opt.slopes || opt.softcap > 0.f || (opt.keep_first > 0 && window > 0);
     int code;
     if (KD == 64 && VD == 64) code = extra ? launch_tcgen05<64, 64, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<64, 64, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
@@ -760,7 +760,9 @@ LLM_EXPORT int llm_attention_tcgen05_own(const void* q0, long long q0_token, lon
     const long long y = (long long)requests * tp.tiles_per_request;
     if (y > 65535) return LLM_ERR_UNSUPPORTED;
     // (the rows' last 32 lanes in boxes of 64: behind a row's end a box is filled with zeros)
-    const CUtensorMap* kvmap = tma::cached_map_2d_bf16(kv, (uint64_t)n_tokens, (uint64_t)values_col + H * 64, (uint64_t)kv_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap* rotmap = tma::cached_map_2d_bf16(rot, (uint64_t)n_tokens, (uint64_t)rot_stride, (uint64_t)rot_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    CUtensorMap kvmap, rotmap;
+    if (!tma::make_map_2d_bf16(&kvmap, kv, (uint64_t)n_tokens, (uint64_t)values_col + H * 64, (uint64_t)kv_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !tma::make_map_2d_bf16(&rotmap, rot, (uint64_t)n_tokens, (uint64_t)rot_stride, (uint64_t)rot_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+        return LLM_ERR_UNSUPPORTED;
     return launch_tcgen05<96, 64, false, true>(tp, rotmap, kvmap, (unsigned)y, stream);
 }

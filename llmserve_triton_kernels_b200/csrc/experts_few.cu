@@ -407,12 +407,13 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     p.out = out; p.resid = resid; p.norm_w = norm_w; p.xw_out = (bf16*)xw_out; p.ss_out = ss_out; p.alpha = alpha; p.error_flag = error_flag;
     const int sms = device_sms(), per = kind < 0 ? 2 : 1, C = E * ff + fs;
     const bool whole = K % 64 == 0;  // rows are whole pieces of 64 k: two of them in one box
-    CUtensorMap up_map, act_map;
+    CUtensorMap up_map, down_map, act_map;
     if (!(whole ? tma::make_map_row_pieces_bf16(&up_map, w_up, (uint64_t)per * C, K, kind < 0 ? 8 : 16)
                 : tma::make_map_2d_bf16(&up_map, w_up, (uint64_t)per * C, K, K, kind < 0 ? 8 : 16, 64, CU_TENSOR_MAP_SWIZZLE_128B)))
         return LLM_ERR_UNSUPPORTED;
-    const CUtensorMap* down_map = tma::cached_map_2d_bf16(w_down, N, C, C, 16, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (!down_map || !tma::make_map_2d_bf16(&act_map, act, M, C, C, MAX_M, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B)) return LLM_ERR_UNSUPPORTED;
+    if (!tma::cached_map_2d_bf16(&down_map, w_down, N, C, C, 16, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !tma::make_map_2d_bf16(&act_map, act, M, C, C, MAX_M, DOWN_BOXK, CU_TENSOR_MAP_SWIZZLE_128B))
+        return LLM_ERR_UNSUPPORTED;
     // at every launch: the limits hold for the current device, and a process may have several; all of the SM's memory as shared memory, so
     // that CTAs of both kernels share it
     for (int k = 0; k < 2; ++k) {
@@ -423,5 +424,5 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     }
     const int most = (E * ff + fs) / (kind < 0 ? 8 : 16);
     const int code = launch_pdl(experts_up_kernel, dim3(most < sms ? most : sms), dim3(THREADS), UP_SMEM, stream, p, up_map, (int)whole);
-    return code != 0 ? code : launch_pdl(experts_down_kernel, dim3(N / 16), dim3(THREADS), DOWN_SMEM, stream, p, *down_map, act_map);
+    return code != 0 ? code : launch_pdl(experts_down_kernel, dim3(N / 16), dim3(THREADS), DOWN_SMEM, stream, p, down_map, act_map);
 }

@@ -303,13 +303,14 @@ int launch(const void* x, int ldx, const void* w, int w_rows, const GemmParams& 
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    const CUtensorMap* xmap = tma::cached_map_2d_bf16(x, p.M, p.K, ldx, BM, BK, CU_TENSOR_MAP_SWIZZLE_128B);
-    const CUtensorMap* wmap = tma::cached_map_2d_bf16(w, w_rows, p.K, p.K, BN, BK, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (!xmap || !wmap) return LLM_ERR_UNSUPPORTED;
+    CUtensorMap xmap, wmap;
+    if (!tma::make_map_2d_bf16(&xmap, x, p.M, p.K, ldx, BM, BK, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !tma::cached_map_2d_bf16(&wmap, w, w_rows, p.K, p.K, BN, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+        return LLM_ERR_UNSUPPORTED;
     const long long tiles = (long long)((p.N + BN - 1) / BN) * ((p.M + BM - 1) / BM);
     if (tiles > 0x7fffffffLL) return LLM_ERR_UNSUPPORTED;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());  // one CTA per SM walks its share of the tiles
-    return launch_pdl(kernel, dim3(grid), dim3(THREADS), smem, stream, p, *xmap, *wmap);
+    return launch_pdl(kernel, dim3(grid), dim3(THREADS), smem, stream, p, xmap, wmap);
 }
 
 }  // namespace

@@ -61,10 +61,11 @@ inline bool make_map_row_pieces_bf16(CUtensorMap* map, const void* base, uint64_
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Maps are cached by (address, shape, box): weights and cache pools live for the life of the model, and
-// activations of a shape come back to the same addresses from a caching allocator.  Null if the driver refuses.
-inline const CUtensorMap* cached_map_2d_bf16(const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
-                                             uint32_t box_cols, CUtensorMapSwizzle swizzle) {
+// The same from a cache by (address, shape, box), for what lives as long as the model: weights and cache pools.  (Activations have a map
+// made at each call, 41 ns where the cache takes 16: their shapes are as many as there are step sizes.)  The map is the caller's own copy, taken under the lock: the cache
+// empties itself when it is full, and neither that nor another thread's call reaches a map that was handed out.
+inline bool cached_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
+                               uint32_t box_cols, CUtensorMapSwizzle swizzle) {
     struct Key {
         const void* p;
         uint64_t rows, cols, ld;
@@ -85,12 +86,15 @@ inline const CUtensorMap* cached_map_2d_bf16(const void* base, uint64_t rows, ui
     static std::mutex lock;
     std::lock_guard<std::mutex> guard(lock);
     const Key key{base, rows, cols, ld, box_rows, box_cols, (int)swizzle};
-    auto it = maps.find(key);
-    if (it != maps.end()) return &it->second;
-    if (maps.size() > 4096) maps.clear();
-    CUtensorMap map;
-    if (!make_map_2d_bf16(&map, base, rows, cols, ld, box_rows, box_cols, swizzle)) return nullptr;
-    return &maps.emplace(key, map).first->second;
+    const auto it = maps.find(key);
+    if (it != maps.end()) {
+        *map = it->second;
+        return true;
+    }
+    if (!make_map_2d_bf16(map, base, rows, cols, ld, box_rows, box_cols, swizzle)) return false;
+    if (maps.size() >= 4096) maps.clear();
+    maps.emplace(key, *map);
+    return true;
 }
 
 // ---- device -----------------------------------------------------------------------------------
