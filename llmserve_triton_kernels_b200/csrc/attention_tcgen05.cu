@@ -20,9 +20,9 @@
 // the output are 32-bit; probabilities are rounded to bfloat16 for the second product, as in the mma.sync kernel.
 //
 // Keys past a request's length inside its last page, and pages outside the range a CTA needs, are
-// never looked at: a score outside [window start, position] is -inf before the exponential, and the
-// producer loads a page of the needed range in place of one outside it, so that no stale or released
-// page is touched.  Values of masked keys meet a probability of exactly zero; what lies behind the request's last
+// never looked at: a score outside [window start, position] is -inf before the exponential, and in place of a page outside
+// the needed range the producer asks for a box outside the pool, which the TMA unit fills with zeros, so that no stale or
+// released page is touched.  Values of masked keys meet a probability of exactly zero; what lies behind the request's last
 // token (stale rows of a page, in OWN the next request's) is made zeros in shared memory before the product.
 //
 // EXTRA: scores are capped and lose a distance bias before the softmax, or a window keeps the first keys (some operations more
@@ -199,8 +199,7 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             for (int h = 0; h < K_HALVES; ++h) tma::load_2d(q_s + (size_t)h * (BM * 128), &qmap, q_head * KD + h * 64, q_begin + row0, &q_full);
         }
         // One box per page and 64-wide piece, each issued by a lane of its own (a thread's TMA instructions follow one another slowly;
-        // several threads' overlap).  The page table is read 32 entries at a time; a page outside the needed range is
-        // replaced by one inside it.
+        // several threads' overlap).  The page table is read 32 entries at a time.
         const int halves = is_v ? V_HALVES : K_HALVES;
         const int lane0 = is_v ? 0 : (q_head - head * tp.maps) * KD;  // where a row's lanes of this map begin
         const int kept_hi = kept > 0 ? (kept - 1) / ps : -1;
@@ -210,8 +209,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             const int s = j % STAGES, key0 = tile_start(j), idx0 = key0 / ps;
             if (!OWN && idx0 >= loaded_from + 32) {  // pages_per_tile divides 32: a tile's pages lie in one batch
                 loaded_from = idx0 - idx0 % 32;
-                const int idx = min(loaded_from + lane, lp_hi);
-                my_page = table[idx < lp_lo && idx > kept_hi ? lp_lo : idx];
+                const int idx = loaded_from + lane;
+                my_page = idx <= lp_hi && (idx >= lp_lo || idx <= kept_hi) ? table[idx] : -1;
             }
             if (lane == 0) {
                 if (gave_up || (j >= STAGES && !tma::mbar_wait(&empty[s], ((j / STAGES) - 1) & 1))) {
@@ -231,8 +230,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             } else {
                 const int in_tile = lane / halves, half = lane % halves;
                 const int page = __shfl_sync(0xffffffffu, my_page, (idx0 - loaded_from + in_tile) & 31);
-                if (alive && in_tile < pages_per_tile)
-                    tma::load_2d(stage + (size_t)half * (BN * 128) + (size_t)in_tile * ps * 128, &kvmap, lane0 + half * 64, ((page * 2 + (int)is_v) * p.KV + kvh) * ps, &full[s]);
+                if (alive && in_tile < pages_per_tile)  // (no page: the rows in front of the pool)
+                    tma::load_2d(stage + (size_t)half * (BN * 128) + (size_t)in_tile * ps * 128, &kvmap, lane0 + half * 64, page < 0 ? -ps : ((page * 2 + (int)is_v) * p.KV + kvh) * ps, &full[s]);
             }
         }
     } else if (warp == 5) {

@@ -50,6 +50,32 @@ def test_options_against_plain(H, KV, D, V, page_size, what, monkeypatch):
         close(got, want, 2e-2, what + " (a projection's rows)")
 
 
+@pytest.mark.parametrize("more", [dict(window=1), dict(window=4), dict(window=7, keep_first=3), dict(window=3, keep_first=70), dict(chunk=50, window=5),
+                                  dict(chunk=50), dict(chunk=50, window=5, keep_first=20), dict(sinks=True, window=4)], ids=str)
+@pytest.mark.parametrize("D,V,page_size", [(64, 64, 8), (64, 128, 16), (128, 128, 32), (64, 64, 64)])
+def test_a_tail_whose_window_lies_in_the_last_page(D, V, page_size, more, monkeypatch):
+    """Tail tiles of 1 to 8 rows that need the request's last, partly filled page alone: what stands behind its end is nobody's, wherever in
+    a tile of keys the pages that are not needed would have been."""
+    ops = _ops()
+    torch.manual_seed(D + page_size)
+    news = [129, 130, 132, 136, 33]
+    ctx, table, _, pages = paged_batch([n + old for n, old in zip(news, (21, 0, 300, 1, 40))], news, page_size)
+    pool = torch.randn(pages, 2, 2, page_size, max(D, V), device=DEV).bfloat16()
+    for r, n in enumerate(ctx.context_lens.tolist()):
+        if n % page_size:
+            pool[int(table[r, n // page_size]), :, :, n % page_size :] = torch.nan
+    q = torch.randn(ctx.num_tokens, 2 * D, device=DEV).bfloat16()
+    more = dict(more, sinks=torch.randn(2, device=DEV)) if more.get("sinks") else more
+    common = dict(num_heads=2, num_kv_heads=2, key_dim=D, value_dim=V, scale=0.3)
+    got = ops.paged_softmax_attention(q, pool, table, ctx, **common, **more)
+    if "chunk" in more and "keep_first" in more:  # kept keys stay visible from every block: the kernels' reading, which the plain statement does not share
+        monkeypatch.setattr(ops, "_TC_ATTENTION_ENABLED", False)
+        want = ops.paged_softmax_attention(q, pool, table, ctx, **common, **more)
+    else:
+        want = plain_ops.paged_softmax_attention(q, pool, table, ctx, **common, **more)
+    close(got, want, 2e-2, str(more))
+
+
 def test_every_key_scores_minus_infinity():
     """A row without a finite score is zeros; one NaN score leaves its row NaN; the rows beside them are as without them."""
     ops = _ops()
