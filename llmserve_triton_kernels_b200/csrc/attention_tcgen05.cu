@@ -25,11 +25,14 @@
 // released page is touched.  Values of masked keys meet a probability of exactly zero; what lies behind the request's last
 // token (stale rows of a page, in OWN the next request's) is made zeros in shared memory before the product.
 //
-// EXTRA: scores are capped and lose a distance bias before the softmax, or a window keeps the first keys (some operations more
-// a score, so a kernel of its own).  OWN: the keys and values are the step's own tokens, row by row and head by head, with lanes
-// behind the keys' first 64 that all heads share (latent attention's fresh part): no pages.
-// Measured (us a layer, one request; before, on mma.sync): 1,801 tokens with sinks and gates a lane 161 -> 47; 1,500 tokens of latent
-// attention's own part 120 -> 34, with a window and a distance bias 120 -> 41.
+// PLAIN, SIDE, EXTRA: kernels of their own for the plain softmax with or without a window, for what stands beside a softmax (sinks, gates,
+// values that turn, two maps, blocks), and for what changes a score as well (a cap, a distance bias, a window that keeps the first keys: some
+// operations more a score).  In one kernel the plain softmax was slower for what it does not use (us, 32 heads of 64, all in one -> apart: 2,041
+// tokens 54.9 -> 52.5, 4,096 123.8 -> 119.2, 1,801 of the general entry 42.4 -> 38.6, its sinks 42.4 -> 41.4, values that turn 43.0 -> 44.4; 32 heads
+// of 128, 4,096 tokens 141.8 -> 138.3).  OWN: the keys and values are the step's own tokens, row by row and head by head, with
+// lanes behind the keys' first 64 that all heads share (latent attention's fresh part): no pages.
+// Measured (us a layer, one request; before, on mma.sync): 1,801 tokens, 32 heads of 64, sinks 140 -> 41, gates a lane 150 -> 52, a distance bias 147
+// -> 58, a cap 173 -> 83; latent attention's own part, 16 heads 117 -> 39.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets *error_flag, the roles leave their loops,
 // tensor memory is freed and the kernel returns.
@@ -38,6 +41,8 @@
 #include <cstdio>
 #endif
 #include "umma.cuh"
+
+#include <type_traits>
 
 namespace {
 
@@ -101,17 +106,21 @@ struct TcParams {
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) { tma::mbar_arrive(bar); }
 
+enum Form { PLAIN, SIDE, EXTRA_FORM, OWN_FORM };  // see above
+
 // qmap: the queries (head size 128), in OWN the lanes that the heads share.
-template <int KD, int VD, bool EXTRA, bool OWN>
+template <int KD, int VD, Form FORM>
 __global__ void __launch_bounds__(THREADS, 2)
 attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kvmap) {
+    constexpr bool EXTRA = FORM == EXTRA_FORM, OWN = FORM == OWN_FORM, WITH_SIDE = FORM == SIDE || EXTRA;
     static_assert(OWN == (KD == 96), "the shared lanes are the last 32 of 96");
     using Sh = Shape<KD, VD>;
     constexpr int STAGES = Sh::STAGES, NBUF = Sh::S_BUFFERS, K_BYTES = Sh::K_BYTES, STAGE_BYTES = Sh::STAGE_BYTES;
     constexpr int K_HALVES = Sh::K_HALVES, V_HALVES = Sh::V_HALVES;
     constexpr int O_COL = Sh::O_COL, Q_COL = Sh::Q_COL, P_COL = Sh::P_COL;
     const AttnParams& p = tp.a;
-    const int q_head = blockIdx.x, head = q_head / tp.maps, kvh = head / p.G;
+    const int maps = WITH_SIDE ? tp.maps : 1, chunk = WITH_SIDE ? tp.chunk : 0;
+    const int q_head = blockIdx.x, head = q_head / maps, kvh = head / p.G;
     const int r = blockIdx.y / tp.tiles_per_request;
     const int tile = tp.tiles_per_request - 1 - (int)(blockIdx.y % tp.tiles_per_request);  // long tiles first
     const int q_begin = p.cu_tokens[r], q_len = p.cu_tokens[r + 1] - q_begin;
@@ -124,7 +133,7 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
     const int key_hi = pos0 + row0 + rows_here - 1;
     auto first_seen = [&](int pos) {
         const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
-        return tp.chunk > 0 ? max(lo, pos - pos % tp.chunk) : lo;
+        return chunk > 0 ? max(lo, pos - pos % chunk) : lo;
     };
     const int key_lo = first_seen(pos0 + row0);
     // with a window the keys below keep_first stay visible: their tiles come first, then the window's (one run where they meet)
@@ -132,7 +141,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
     const int kept_tiles = min((kept + BN - 1) / BN, key_lo / BN);
     const int t_skip = key_lo / BN - kept_tiles;  // tiles between the two
     const int n_tiles = key_hi / BN + 1 - t_skip;
-    auto tile_start = [&](int j) { return (j < kept_tiles ? j : j + t_skip) * BN; };
+    auto tile_number = [&](int j) { return j < kept_tiles ? j : j + t_skip; };
+    auto tile_start = [&](int j) { return tile_number(j) * BN; };
     // a key tile needs no mask if every row of the CTA sees all of it
     const int tile_pos_min = pos0 + row0;
     const int tile_lo_max = first_seen(pos0 + row0 + rows_here - 1);
@@ -201,12 +211,12 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         // One box per page and 64-wide piece, each issued by a lane of its own (a thread's TMA instructions follow one another slowly;
         // several threads' overlap).  The page table is read 32 entries at a time.
         const int halves = is_v ? V_HALVES : K_HALVES;
-        const int lane0 = is_v ? 0 : (q_head - head * tp.maps) * KD;  // where a row's lanes of this map begin
+        const int lane0 = is_v ? 0 : (q_head - head * maps) * KD;  // where a row's lanes of this map begin
         const int kept_hi = kept > 0 ? (kept - 1) / ps : -1;
         int my_page = 0, loaded_from = -32;
         bool alive = true;
         for (int j = 0; j < n_tiles && alive; ++j) {
-            const int s = j % STAGES, key0 = tile_start(j), idx0 = key0 / ps;
+            const int s = j % STAGES, number = tile_number(j), idx0 = number * pages_per_tile;
             if (!OWN && idx0 >= loaded_from + 32) {  // pages_per_tile divides 32: a tile's pages lie in one batch
                 loaded_from = idx0 - idx0 % 32;
                 const int idx = loaded_from + lane;
@@ -224,8 +234,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             unsigned char* stage = kv_s + (size_t)s * STAGE_BYTES + (size_t)is_v * K_BYTES;
             if constexpr (OWN) {
                 if (alive && lane == 0) {
-                    tma::load_2d(stage, &kvmap, is_v ? tp.own_values + head * VD : head * 64, q_begin + key0, &full[s]);
-                    if (!is_v) tma::load_2d(stage + BN * 128, &qmap, tp.own_rot, q_begin + key0, &full[s]);  // 32 lanes, zeros behind them
+                    tma::load_2d(stage, &kvmap, is_v ? tp.own_values + head * VD : head * 64, q_begin + number * BN, &full[s]);
+                    if (!is_v) tma::load_2d(stage + BN * 128, &qmap, tp.own_rot, q_begin + number * BN, &full[s]);  // 32 lanes, zeros behind them
                 }
             } else {
                 const int in_tile = lane / halves, half = lane % halves;
@@ -315,7 +325,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
         const int lo = first_seen(pos), kept_of_row = EXTRA && p.window > 0 ? tp.keep_first : 0;
         const unsigned lane_base = tmem_base + ((unsigned)(warp * 32) << 16);
         // a sink has been seen before the first key
-        float m_run = tp.sinks ? tp.sinks[head] * LOG2E : -INFINITY, l_run = tp.sinks ? 1.f : 0.f;
+        const bool sink = WITH_SIDE && tp.sinks;
+        float m_run = sink ? tp.sinks[head] * LOG2E : -INFINITY, l_run = sink ? 1.f : 0.f;
         const float slope = EXTRA && tp.slopes ? tp.slopes[head] * LOG2E : 0.f;
         const float cap2 = tp.softcap * LOG2E, cap_in = EXTRA && tp.softcap > 0.f ? 2.f * p.scale_log2 / tp.softcap : 0.f;
         const float scale_log2 = EXTRA ? 1.f : p.scale_log2;  // what is left to do to a score
@@ -478,10 +489,10 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             float inv = l_run == 0.f ? 0.f : 1.f / l_run;  // every key scored -inf: zeros
             __nv_bfloat16* dst = p.out + (size_t)(q_begin + tok) * p.out_stride + (size_t)head * VD;
-            const float* gate = tp.gate ? tp.gate + (size_t)(q_begin + tok) * tp.gate_token + (tp.gate_lanes ? head * VD : head) : nullptr;
+            const float* gate = WITH_SIDE && tp.gate ? tp.gate + (size_t)(q_begin + tok) * tp.gate_token + (tp.gate_lanes ? head * VD : head) : nullptr;
             if (gate && !tp.gate_lanes && row_ok) inv /= 1.f + expf(-*gate);
             if (OWN && tp.stats && row_ok) tp.stats[(size_t)(q_begin + tok) * p.H + head] = make_float2(m_run, l_run);
-            if (tp.turn) {
+            if (WITH_SIDE && tp.turn) {
                 const float4* cs = reinterpret_cast<const float4*>(tp.turn + (size_t)(q_begin + tok) * (VD / 2));  // two pairs each
 #pragma unroll 1
                 for (int h = 0; h < VD / 2; h += 32) {
@@ -514,8 +525,8 @@ attention_tcgen05_kernel(const TcParams tp, const __grid_constant__ CUtensorMap 
             for (int h = 0; h < V_HALVES; ++h) {
                 float o[64];
                 umma::tmem_ld64(o_taddr + 64 * h, o);  // (by all lanes of the warp: the load is the warp's)
-                if (row_ok && tp.raw) {
-                    float* raw = tp.raw + ((size_t)(q_begin + tok) * (p.H * tp.maps) + q_head) * VD + 64 * h;
+                if (WITH_SIDE && row_ok && tp.raw) {
+                    float* raw = tp.raw + ((size_t)(q_begin + tok) * (p.H * maps) + q_head) * VD + 64 * h;
 #pragma unroll
                     for (int c = 0; c < 64; c += 4)
                         *reinterpret_cast<float4*>(raw + c) = make_float4(o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv);
@@ -594,10 +605,10 @@ join_maps_kernel(const float* __restrict__ raw, const int* __restrict__ token_re
 LLM_EXPORT int llm_attention_tcgen05_min_tokens() { return 128; }
 
 namespace {
-template <int KD, int VD, bool EXTRA, bool OWN>
+template <int KD, int VD, Form FORM>
 int launch_tcgen05(const TcParams& tp, const CUtensorMap& qmap, const CUtensorMap& kvmap, unsigned grid_y, cudaStream_t stream) {
     using Sh = Shape<KD, VD>;
-    auto kernel = attention_tcgen05_kernel<KD, VD, EXTRA, OWN>;
+    auto kernel = attention_tcgen05_kernel<KD, VD, FORM>;
     // at every launch: the limit holds for the current device, and a process may have several
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
     if (e != cudaSuccess) return (int)e;
@@ -675,10 +686,17 @@ int attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, co
     if (KD == 64) qmap = kvmap;
     else if (!tma::make_map_2d_bf16(&qmap, q, (uint64_t)n_tokens, (uint64_t)H * maps * KD, (uint64_t)q_stride, BM, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return LLM_ERR_UNSUPPORTED;
     const bool extra = opt.slopes || opt.softcap > 0.f || (opt.keep_first > 0 && window > 0);
-    int code;
-    if (KD == 64 && VD == 64) code = extra ? launch_tcgen05<64, 64, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<64, 64, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
-    else if (KD == 64) code = extra ? launch_tcgen05<64, 128, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<64, 128, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
-    else code = extra ? launch_tcgen05<128, 128, true, false>(tp, qmap, kvmap, (unsigned)y, stream) : launch_tcgen05<128, 128, false, false>(tp, qmap, kvmap, (unsigned)y, stream);
+    const bool side = maps > 1 || opt.turn || opt.gate || opt.sinks || opt.chunk > 0;
+    auto form = [&](auto kd, auto vd) {
+        constexpr int K = decltype(kd)::value, V = decltype(vd)::value;
+        return extra  ? launch_tcgen05<K, V, EXTRA_FORM>(tp, qmap, kvmap, (unsigned)y, stream)
+               : side ? launch_tcgen05<K, V, SIDE>(tp, qmap, kvmap, (unsigned)y, stream)
+                      : launch_tcgen05<K, V, PLAIN>(tp, qmap, kvmap, (unsigned)y, stream);
+    };
+    using std::integral_constant;
+    const int code = KD == 128  ? form(integral_constant<int, 128>{}, integral_constant<int, 128>{})
+                     : VD == 64 ? form(integral_constant<int, 64>{}, integral_constant<int, 64>{})
+                                : form(integral_constant<int, 64>{}, integral_constant<int, 128>{});
     if (code != 0 || maps == 1) return code;
     const long long items = (long long)n_tokens * H;
     auto join = [&](auto kernel) {
@@ -763,5 +781,5 @@ LLM_EXPORT int llm_attention_tcgen05_own(const void* q0, long long q0_token, lon
     if (!tma::make_map_2d_bf16(&kvmap, kv, (uint64_t)n_tokens, (uint64_t)values_col + H * 64, (uint64_t)kv_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !tma::make_map_2d_bf16(&rotmap, rot, (uint64_t)n_tokens, (uint64_t)rot_stride, (uint64_t)rot_stride, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B))
         return LLM_ERR_UNSUPPORTED;
-    return launch_tcgen05<96, 64, false, true>(tp, rotmap, kvmap, (unsigned)y, stream);
+    return launch_tcgen05<96, 64, OWN_FORM>(tp, rotmap, kvmap, (unsigned)y, stream);
 }
