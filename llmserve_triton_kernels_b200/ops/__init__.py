@@ -134,11 +134,7 @@ _TC_ATTENTION_ENABLED = True
 _TC_ATTENTION_HEAD_DIMS = (64, 128)
 _TC_ATTENTION_PAGE_SIZES = (8, 16, 32, 64)
 _TC_ATTENTION_MIN_TOKENS = 128  # a request with at least this many tokens in the step: attention on tcgen05
-# Where that kernel runs, requests of at least so many go along (tiles of their own beside the others').  A request of 512 tokens and, in a
-# launch of their own -> along (us, 32 heads of 64): 4 of 32 28.3 -> 12.9, 4 of 100 25.4 -> 13.3, 16 of 32 23.3 -> 21.9, 4 of 64 behind 1,000 cached
-# 79.6 -> 33.4.  Of fewer tokens it depends on what is cached: 7 of 24 behind 500 39.1 -> 28.7, but 31 of 24 behind 300 51.6 -> 62.5; 3 of 16 behind
-# 1,500 33.0 -> 42.0.
-_TC_ATTENTION_JOIN_TOKENS = 32
+_TC_ATTENTION_JOIN_TOKENS, _TC_ATTENTION_JOIN_CROWDED, _TC_ATTENTION_JOIN_CROWDED_GENERAL = 32, 64, 48  # where that kernel runs, smaller requests that go along, see _tc_join_tokens
 _TCGEN05_MIN_ROWS = 128  # from this many rows a bfloat16 product runs on tcgen05 with TMA-fed tiles (own kernel)
 _DECODE_LINEAR_MAX_ROWS = 16  # up to this many rows a bfloat16 matrix product streams the weights once (own kernel)
 _FORCE_GENERIC_ATTENTION = False  # tests switch the tensor-core attention off to reach the general kernel in bfloat16
@@ -779,7 +775,7 @@ def paged_attention(
         tc_min = 0
         if (head_dim in _TC_ATTENTION_HEAD_DIMS and pool.shape[3] in _TC_ATTENTION_PAGE_SIZES and _TC_ATTENTION_ENABLED
                 and (getattr(ctx, "max_query_len", None) or max(_token_counts(ctx))) >= _TC_ATTENTION_MIN_TOKENS):
-            tc_min = _TC_ATTENTION_JOIN_TOKENS
+            tc_min = _tc_join_tokens(ctx, num_heads, head_dim, head_dim, _TC_ATTENTION_JOIN_CROWDED)
         num_requests, tc_longest, small, max_rows_large, other_rows = _attention_route(ctx, group, tc_min)
         if tc_longest:
             code = _launch(
@@ -1510,6 +1506,22 @@ def _token_counts(ctx) -> list[int]:
     return [b - a for a, b in zip(cu, cu[1:])]
 
 
+def _tc_join_tokens(ctx, heads: int, key_dim: int, value_dim: int, crowded: int) -> int:
+    """From how many tokens on a request goes along with one of ``_TC_ATTENTION_MIN_TOKENS`` through the tcgen05 kernel, whose CTAs are 128 rows of
+    a head (of a score map).  Along, a request of 32 tokens fills a quarter of its tiles, which costs nothing while all tiles are on the SMs at
+    once (two a SM).  Measured (us, in a launch of their own -> along; a request of 512 tokens and): 32 heads of 64 over 4 of keys, 4 requests of 32
+    tokens behind 300 keys 23.8 -> 15.1, 16 of them 24.3 -> 37.1, 63 behind 2,000 209 -> 379; of 64 tokens 4 24.6 -> 15.4, 16 37.1 -> 37.6, 63 109 -> 118;
+    beside one of 2,000 tokens 16 of 32 behind 1,000 108 -> 132.  With sinks and gates the general kernels, which are slower, are what they leave: 16
+    of 32 tokens behind 300 keys 64 -> 59, 32 of them 72 -> 96, 32 of 48 103 -> 98.  Wider heads or values gain in nearly every case: 32 heads of 128 over 8, 16 of 32
+    tokens behind 1,000 keys 78 -> 79, 63 of them 263 -> 257, 4 of 64 behind 300 34 -> 17; the worst, 63 of 32 with nothing cached beside 128
+    tokens, 33 -> 41.  (Capped scores beside a request of 128 tokens: one of 32 tokens behind 1,500 keys takes 1.4 times as long, four 1.2.)  Requests of
+    fewer than 32 tokens stay apart: 31 of 24 behind 300 keys 51.6 -> 62.5."""
+    if (key_dim, value_dim) != (64, 64):
+        return _TC_ATTENTION_JOIN_TOKENS
+    tiles = sum(-(-c // 128) for c in _token_counts(ctx) if c >= _TC_ATTENTION_JOIN_TOKENS)
+    return _TC_ATTENTION_JOIN_TOKENS if tiles * heads <= 2 * _sm_count() else crowded
+
+
 def _most_tokens_below(ctx, limit: int) -> int:
     """The most tokens that a request with fewer than ``limit`` tokens brings."""
     return max((c for c in _token_counts(ctx) if c < limit), default=1)
@@ -1521,7 +1533,7 @@ _TC_SOFTMAX_SIZES = ((64, 64), (64, 128), (128, 128))  # lanes of a key (of one 
 def _tcgen05_softmax_attention(q, pool, page_table, ctx, out, heads: int, kv_heads: int, key_dim: int, value_dim: int, scale: float,
                                window, gate, differential, turn, sinks=None, slopes=None, softcap=None, keep_first=None, chunk=None,
                                gate_per_head: bool = True) -> tuple[int, bool]:
-    """The part of :func:`paged_softmax_attention` that the tcgen05 kernel takes: bfloat16 requests of at least ``_TC_ATTENTION_JOIN_TOKENS``
+    """The part of :func:`paged_softmax_attention` that the tcgen05 kernel takes: bfloat16 requests of at least :func:`_tc_join_tokens`
     tokens in a step in which one brings ``_TC_ATTENTION_MIN_TOKENS`` or more.  Returns ``(the fewest tokens of a request that it took or 0
     if it took none, whether other requests are left)``."""
     if (q.dtype != torch.bfloat16 or _FORCE_GENERIC_ATTENTION or not _TC_ATTENTION_ENABLED or (key_dim, value_dim) not in _TC_SOFTMAX_SIZES
@@ -1544,10 +1556,11 @@ def _tcgen05_softmax_attention(q, pool, page_table, ctx, out, heads: int, kv_hea
     if differential is not None:
         raw = torch.empty((n, heads, 2, value_dim), dtype=torch.float32, device=q.device)
     weight, eps, post = (differential.weight, differential.eps, differential.scale) if differential is not None else (0.0, 0.0, 0.0)
+    join = _tc_join_tokens(ctx, heads * (1 if differential is None else 2), key_dim, value_dim, _TC_ATTENTION_JOIN_CROWDED_GENERAL)
     code = _launch(
         "llm_attention_tcgen05_general", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(pool), pool.shape[0], _ptr(page_table), page_table.shape[1],
         _ptr(ctx.token_request), _ptr(ctx.cu_tokens), _ptr(ctx.context_lens), len(counts), n, heads, kv_heads, key_dim, value_dim, pool.shape[4], pool.shape[3],
-        int(window or 0), float(scale), _TC_ATTENTION_JOIN_TOKENS, max(counts), _ptr(turn), _ptr(gate), 0 if gate is None else gate.stride(0),
+        int(window or 0), float(scale), join, max(counts), _ptr(turn), _ptr(gate), 0 if gate is None else gate.stride(0),
         int(not gate_per_head), _ptr(sinks), _ptr(slopes), softcap, keep_first, chunk, _ptr(raw), float(weight), float(eps), float(post),
         _error_flag_ptr(), _stream(),
     )
@@ -1556,7 +1569,7 @@ def _tcgen05_softmax_attention(q, pool, page_table, ctx, out, heads: int, kv_hea
         return 0, True
     _check(code, "paged_softmax_attention (tcgen05)")
     add_launches(int(raw is not None))
-    return _TC_ATTENTION_JOIN_TOKENS, min(counts) < _TC_ATTENTION_JOIN_TOKENS
+    return join, min(counts) < join
 
 
 def head_prepare(proj: torch.Tensor, positions: torch.Tensor | None, *, heads: int, kv_heads: int, dim: int, value_dim: int = 0,

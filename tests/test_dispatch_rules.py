@@ -82,3 +82,22 @@ def test_experts_of_many_tokens_run_alone_where_that_was_measured_faster(monkeyp
     ):
         assert ops.experts_many_pay(tokens, experts, top, ff, shared, gated, hidden) == (used < 0.98 * everybody), (tokens, experts, hidden)
     assert not ops.experts_many_pay(4096, 8, 8, 704, 0, True, 2048)  # every token uses every expert
+
+
+# heads (times maps), key lanes, value lanes, long request, riders, their tokens, whether they were faster along with it
+@pytest.mark.parametrize("heads,dk,dv,long,riders,tokens,along", [
+    (32, 64, 64, 512, 4, 32, True), (32, 64, 64, 512, 16, 32, False), (32, 64, 64, 512, 63, 32, False), (32, 64, 64, 128, 8, 32, True), (32, 64, 64, 2000, 16, 32, False),
+    (32, 64, 64, 512, 16, 100, True), (32, 64, 64, 2000, 63, 64, True), (8, 64, 64, 512, 16, 32, True), (32, 128, 128, 512, 63, 48, True), (64, 128, 128, 512, 16, 32, True),
+    (32, 64, 128, 1800, 32, 32, True), (32, 96, 64, 512, 32, 32, True), (32, 64, 64, 512, 4, 24, False), (32, 128, 128, 512, 31, 24, False)])
+def test_small_requests_go_along_with_a_long_one_where_that_is_faster(b200, heads, dk, dv, long, riders, tokens, along):
+    class Step:
+        host_cu_tokens = [0, long, *(long + tokens * (i + 1) for i in range(riders))]
+
+    assert (tokens >= ops._tc_join_tokens(Step, heads, dk, dv, ops._TC_ATTENTION_JOIN_CROWDED)) == along
+
+
+def test_small_requests_beside_the_general_form_in_a_crowd(b200):
+    class Step:
+        host_cu_tokens = [0, 512, *(512 + 48 * (i + 1) for i in range(32))]
+
+    assert ops._tc_join_tokens(Step, 32, 64, 64, ops._TC_ATTENTION_JOIN_CROWDED_GENERAL) == 48
