@@ -639,10 +639,11 @@ int attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, co
     const bool sizes = (KD == 64 && (VD == 64 || VD == 128)) || (KD == 128 && VD == 128);
     if (!sizes || (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64)) return LLM_ERR_UNSUPPORTED;
     const int maps = diff.raw ? 2 : 1;
-    if (H <= 0 || KV <= 0 || H % KV || table_width <= 0 || min_tokens < 1 || !(scale > 0.f) || row_lanes < maps * KD || row_lanes < VD ||
+    if (H <= 0 || KV <= 0 || H % KV || table_width <= 0 || min_tokens < 1 || row_lanes < maps * KD || row_lanes < VD ||
         (diff.raw && (opt.turn || opt.gate || opt.sinks || !diff.token_request)) || (opt.turn && opt.gate && opt.gate_lanes) || opt.keep_first < 0 ||
         opt.chunk < 0)
         return LLM_ERR_BAD_ARGUMENT;
+    if (!(scale > 0.f)) return LLM_ERR_UNSUPPORTED;  // a row's maximum is taken before the scale
     if ((q_stride & 7) || (out_stride & 7) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)pool & 127) || q_stride < H * maps * KD ||
         (row_lanes & 7) || ((uintptr_t)opt.turn & 15) || ((uintptr_t)diff.raw & 15) ||
         (opt.gate && opt.gate_lanes && (((uintptr_t)opt.gate & 15) || (opt.gate_token & 3))))
@@ -715,6 +716,7 @@ LLM_EXPORT int llm_attention_tcgen05(const void* q, int q_stride, void* out, int
                                      const int* page_table, int table_width, const int* cu_tokens, const int* ctx_lens,
                                      int requests, int n_tokens, int H, int KV, int D, int page_size, int window, float scale,
                                      int min_tokens, int max_tokens, int* error_flag, cudaStream_t stream) {
+    if (!(scale > 0.f)) return LLM_ERR_BAD_ARGUMENT;
     return attention_tcgen05(q, q_stride, out, out_stride, pool, pool_pages, page_table, table_width, cu_tokens, ctx_lens, requests, n_tokens, H, KV, D, D,
                              D, page_size, window, scale, min_tokens, max_tokens, Options{}, Differential{}, error_flag, stream);
 }
@@ -746,8 +748,9 @@ LLM_EXPORT int llm_attention_tcgen05_own(const void* q0, long long q0_token, lon
                                          int rot_col, const int* cu_tokens, int requests, int n_tokens, int H, int window, float scale, int min_tokens,
                                          int max_tokens, float* stats, int* error_flag, cudaStream_t stream) {
     if (n_tokens <= 0 || requests <= 0 || max_tokens < min_tokens) return 0;
-    if (H <= 0 || min_tokens < 1 || !(scale > 0.f) || values_col < H * 64 || kv_stride < values_col + H * 64 || rot_col < 0 || rot_col + 32 != rot_stride)
+    if (H <= 0 || min_tokens < 1 || values_col < H * 64 || kv_stride < values_col + H * 64 || rot_col < 0 || rot_col + 32 != rot_stride)
         return LLM_ERR_BAD_ARGUMENT;
+    if (!(scale > 0.f)) return LLM_ERR_UNSUPPORTED;
     if (((q0_token | q0_head | q1_token | q1_head | out_stride | kv_stride | values_col | rot_stride | rot_col) & 7) || q0_token > 0x7fffffffLL ||
         (((uintptr_t)q0 | (uintptr_t)q1 | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)rot) & 15) || ((uintptr_t)stats & 7))
         return LLM_ERR_UNSUPPORTED;

@@ -124,3 +124,21 @@ def test_a_steps_own_tokens(news, window):
         kv[cu[1] : cu[2]] = torch.nan
         fresh[cu[1] : cu[2]] = torch.nan
         assert torch.equal(ops.fresh_latent_attention(q, q_rot, kv, fresh, table, ctx, **args, want_stats=False)[: cu[1]], out[: cu[1]])
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.3])
+def test_scales_that_are_not_positive_go_the_old_way(scale):
+    ops = _ops()
+    torch.manual_seed(7)
+    ctx, table, _, pages = paged_batch([300, 40], [200, 40], 16)
+    pool, q = torch.randn(pages, 2, 2, 16, 64, device=DEV).bfloat16(), torch.randn(240, 128, device=DEV).bfloat16()
+    for more in (dict(sinks=torch.randn(2, device=DEV)), dict(softcap=5.0), dict(slopes=torch.rand(2, device=DEV) * 0.2), dict(chunk=64)):
+        common = dict(num_heads=2, num_kv_heads=2, key_dim=64, value_dim=64, scale=scale, **more)
+        close(ops.paged_softmax_attention(q, pool, table, ctx, **common), plain_ops.paged_softmax_attention(q, pool, table, ctx, **common), 2e-2, str(more))
+    kv, q_rot, fresh = torch.randn(240, 256, device=DEV).bfloat16(), torch.randn(240, 2, 32, device=DEV).bfloat16(), torch.randn(240, 72 + 32, device=DEV).bfloat16()
+    got = ops.fresh_latent_attention(q.view(240, 2, 64), q_rot, kv, fresh, table, ctx, dim=64, value_dim=64, rank=72, scale=scale, window=None, want_stats=False)
+    for a, b in ((0, 200), (200, 240)):
+        k = torch.cat((kv[a:b, :128].view(-1, 2, 64), fresh[a:b, None, 72:].expand(-1, 2, -1)), -1).float()
+        s = torch.einsum("ihd,jhd->hij", torch.cat((q[a:b].view(-1, 2, 64), q_rot[a:b]), -1).float(), k) * scale
+        s = s.masked_fill(torch.ones_like(s[0], dtype=torch.bool).triu(1), -torch.inf)
+        close(got[a:b], torch.einsum("hij,jhd->ihd", s.softmax(-1), kv[a:b, 128:].view(-1, 2, 64).float()), 1e-2, f"tokens {a} to {b}")
