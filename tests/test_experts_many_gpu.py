@@ -64,6 +64,7 @@ def test_used_experts_alone(m, K, N, E, ff, fs, form, width, monkeypatch):
     for e in range(E):
         if not bool((wts[:, e] != 0).any()):
             w_up[e * per * ff : (e + 1) * per * ff] = torch.nan
+            w_down[:, e * ff : (e + 1) * ff] = torch.nan
     want = stated(x, w_up, w_down, E, ff, fs, wts, act, (1.5, 1.0), 1.702, 1.0)
     got = ops.experts_many(x, w_up, w_down, E, ff, fs, **kw, top=top)
     # the activations are rounded to bfloat16 (2^-9 each, signs at random), the sums are 32-bit
