@@ -85,3 +85,23 @@ def test_what_it_does_not_take_goes_the_other_way():
     assert ops.experts_many(x, w_up, w_down, 4, 12, 0, **kw) is None  # rows that do not start on 16 bytes
     assert ops.launch_count() == before
     assert ops.experts_many(x.float(), w_up.float(), w_down.float(), 4, 12, 0, **kw) is None
+
+
+def test_many_tokens_wide_rows_and_a_table_with_repeats():
+    """More tokens than the sort's CTA has threads, rows of more pieces than the gather asks for in advance, a table row that names an expert
+    twice and token ids outside the table (which read its first row, as in the products over all experts)."""
+    from llmserve_triton_kernels_b200 import ops
+
+    m, K, N, E, ff, fs = 1100, 2304, 1152, 4, 24, 8
+    x, w_up, w_down = rnd(m, K), rnd(2 * (E * ff + fs), K, seed=1, scale=K**-0.5), rnd(N, E * ff + fs, seed=2, scale=ff**-0.5)
+    table = torch.tensor([[1, 3], [2, 2], [0, 1], [3, 0]], dtype=torch.int32, device=DEV)
+    ids = torch.arange(m, dtype=torch.int32, device=DEV) % 6 - 1  # -1 and 4 are outside
+    rows = table[torch.where((ids < 0) | (ids > 3), 0, ids).long()].long()
+    wts = torch.zeros(m, E + 1, device=DEV).scatter(1, rows, 0.5)
+    wts[:, E] = 1.0
+    kw = dict(limit=1.5, shared_limit=1.0, slope=1.0, up_shift=1.0, ids=ids, table=table)
+    got = ops.experts_many(x, w_up, w_down, E, ff, fs, **kw, top=2)
+    want = stated(x, w_up, w_down, E, ff, fs, wts, None, (1.5, 1.0), 1.0, 1.0)
+    assert float((got.double() - want).norm()) <= 3e-3 * float(want.norm())
+    act = ops.expert_gated_act(ops.linear(x, w_up), E, ff, fs, 1.5, 1.0, 1.0, ids=ids, table=table)
+    assert float((got.double() - ops.linear(act, w_down).double()).norm()) <= 1e-2 * float(want.norm())
