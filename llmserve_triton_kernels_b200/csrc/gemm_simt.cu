@@ -299,6 +299,12 @@ int launch_f32(const float* x, const float* w, float* out, int M, int N, int K, 
     // features, microseconds; n tiles of an SM): 232 n, 145 n, 27 + 59 n and 32 + 31 n.  242 rows: 2,560 features 145 with 64 x 64, 118 with 32 x 64;
     // 2,048 features 88 and 104; 11,264 features 322 and 338.  Against the rule before (the areas of the busiest SM's tiles at assumed rates): 11,264
     // features, 200 rows 365 -> 310, 300 479 -> 377, 512 709 -> 604; 2,048 features, 700 rows 197 -> 173; most sizes as they were.
+    // From 64 to 8,192 k (571 products, 17 to 2,000 rows of 256 to 32,000 features) every tile's time is in proportion to k, so the choice does
+    // not depend on it: from 1,024 k on it is 0.2 % off the fastest tile on average and 16 at the most (at 5,632 k 0.1 and 3, the rule before 3.1 and
+    // 29).  Below, the mean is 3 % (before: 3 as well) and single products are up to 60 % off, all with a last tile that stands beyond the matrix: its
+    // threads read the last row over and over, all from one place of L2 (256 k, 200 rows of 2,048 features: 29.8 with 64 x 64, 18.5 with 32 x 64; 242 rows:
+    // 16.4 and 18.5).  Zeros there, other rows, or last tiles that end with the matrix cost full tiles of 64 x 64 1 to 9 %.  64 x 128 is chosen where it ties
+    // with two tiles of 64 x 64 an SM, and is 1 to 11 % faster than they are there (200 rows of 4,096 features: 153.6 and 163.9).
     struct { int rm, rn; double once, each; } const kinds[4] = {{128, 128, 0., 232.}, {64, 128, 0., 145.}, {64, 64, 27., 59.}, {32, 64, 32., 31.}};
     int best = 0;
     double best_cost = 1e30;
