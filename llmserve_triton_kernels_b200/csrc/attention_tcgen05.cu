@@ -599,12 +599,6 @@ join_maps_kernel(const float* __restrict__ raw, const int* __restrict__ token_re
     for (int e = 0; e < W; e += 2) *reinterpret_cast<__nv_bfloat162*>(o + e) = __floats2bfloat162_rn(u[e] * norm, u[e + 1] * norm);
 }
 
-}  // namespace
-
-// The fewest tokens a request must bring for this kernel to take it (its CTAs are 128 tokens of one head).
-LLM_EXPORT int llm_attention_tcgen05_min_tokens() { return 128; }
-
-namespace {
 template <int KD, int VD, Form FORM>
 int launch_tcgen05(const TcParams& tp, const CUtensorMap& qmap, const CUtensorMap& kvmap, unsigned grid_y, cudaStream_t stream) {
     using Sh = Shape<KD, VD>;

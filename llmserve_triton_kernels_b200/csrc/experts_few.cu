@@ -16,14 +16,16 @@
 //   down  a CTA 16 features; boxes of 64 k, the tokens' lanes of the same k behind the weights in the slot.  Which warp has a box depends on
 //         the box's place in w_down alone: a token's bits are the same whatever experts the other tokens use.
 // An up CTA and a down CTA share an SM (at most 120 registers x 256 threads and 227 KB together): the up kernel lets its dependent start
-// behind its own wait, by when the router has ended, so that the down kernel makes its list and asks for its first boxes (10 MB) while the up
-// kernel runs.  The shared expert's boxes (and, with a table, everybody's) are on their way before the kernel in front has ended.
+// behind its own wait, by when the router has ended, so that the down kernel makes its list and asks for its first boxes (the weights' 48 KB
+// a CTA: 6.3 MB at 2,048 wide) while the up kernel runs.  The shared expert's boxes (and, with a table, everybody's) are on their way before
+// the kernel in front has ended.
 // Measured (us for both behind a router, weights in memory; before: sixteen warps that met at every tile, a down kernel whose registers kept it
 // off every SM until the up kernel had left, its weights brought into L2 by the up kernel): 32 experts of 704, 4 used, a shared one of
 // 1,408, 2,048 wide: one token 20.4 -> 17.6, 3 34.0 -> 31.9, 8 55.5 -> 51.6; 8 experts of 5,632, 2 used: 45.9 -> 40.5, 8 tokens 131 -> 109; 128 of
 // 192, 8 used: 20.0 -> 14.5, 8 tokens 66.4 -> 51.0.  The up kernel bringing the down kernel's weights into L2 costs 2 to 11 us of that;
 // rings of 4 to 6 boxes in the up kernel (and fewer in the other, or one CTA an SM) 1 to 7 us.
 #include "common.cuh"
+#include "experts.cuh"
 #include "linear_stream.cuh"
 #include "tma.cuh"
 
@@ -41,10 +43,7 @@ struct Experts {
     bf16* act;  // [M, E * ff + fs]: only used blocks are written and read
     int ldx, M, K, N, E, ff, fs, kind;  // kind: -1 gated, else the activation
     float limit, limit_s, slope, up_shift;
-    const float* weights;  // [M, ldw], or null:
-    int ldw;
-    const int *ids, *table;
-    int top, vocab;
+    experts::Weights weights;
     float *out, *resid;  // out [M, N], or resid [M, N] += alpha * y
     const float* norm_w;  // with resid: xw_out = resid * norm_w, ss_out [N / 16, M] = sums of resid^2
     bf16* xw_out;
@@ -61,28 +60,18 @@ __device__ __forceinline__ void mma_piece(float (&c)[4], float (&d)[4], const ui
     lin::mma_bf16(d, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
 }
 
-__device__ __forceinline__ float weight_of(const Experts& p, int m, int e) {
-    if (p.weights) return __ldcg(p.weights + (size_t)m * p.ldw + e);
-    if (e == p.E) return 1.f;
-    int id = p.ids[m];
-    if (id < 0 || id >= p.vocab) id = 0;
-    float w = 0.f;
-    for (int c = 0; c < p.top; ++c) w = p.table[(size_t)id * p.top + c] == e ? 1.f / (float)p.top : w;
-    return w;
-}
-
 // The used experts in ascending order, by the calling warp for itself (list: its own place), and where wt_s is given every token's weight of
 // every expert and of the shared one.  Returns their number.
 __device__ __forceinline__ int list_experts(const Experts& p, unsigned char* list, float (*wt_s)[MAX_E + 1]) {
     const int lane = threadIdx.x & 31;
     int n = 0;
-    if (wt_s && lane < p.M && p.fs > 0) wt_s[lane][p.E] = weight_of(p, lane, p.E);
+    if (wt_s && lane < p.M && p.fs > 0) wt_s[lane][p.E] = p.weights.of(lane, p.E);
     for (int e0 = 0; e0 < p.E; e0 += 32) {
         const int e = e0 + lane;
         float wt[MAX_M];
         bool used = false;
 #pragma unroll
-        for (int m = 0; m < MAX_M; ++m) wt[m] = m < p.M && e < p.E ? weight_of(p, m, e) : 0.f;
+        for (int m = 0; m < MAX_M; ++m) wt[m] = m < p.M && e < p.E ? p.weights.of(m, e) : 0.f;
 #pragma unroll
         for (int m = 0; m < MAX_M; ++m) {
             used |= wt[m] != 0.f;
@@ -94,13 +83,6 @@ __device__ __forceinline__ int list_experts(const Experts& p, unsigned char* lis
     }
     __syncwarp();
     return n;
-}
-
-__device__ __forceinline__ float activate(float v, int kind) {
-    if (kind == 0) { const float r = fmaxf(v, 0.f); return r * r; }                                    // relu^2
-    if (kind == 1) return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));  // gelu (tanh)
-    if (kind == 3) return v / (1.f + expf(-v));                                                        // silu
-    return v;
 }
 
 // The warps' sums of a lane's four values, in order.
@@ -124,7 +106,7 @@ __global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid
     bf16* rings = reinterpret_cast<bf16*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     bf16* ring = rings + (size_t)warp * UP_SLOTS * UP_SLOT;
     float4* red = reinterpret_cast<float4*>(rings + (size_t)WARPS * UP_SLOTS * UP_SLOT);  // [2][MEET][WARPS][32]
-    const bool gated = p.kind < 0, known = p.weights == nullptr;  // the table's experts do not depend on the kernel in front
+    const bool gated = p.kind < 0, known = p.weights.w == nullptr;  // the table's experts do not depend on the kernel in front
     const int step = gated ? 8 : 16, tiles_e = p.ff / step, tiles_s = p.fs / step, per = gated ? 2 : 1;
     const int kblocks = (p.K + UP_BOXK - 1) / UP_BOXK, my_kb = kblocks > warp ? (kblocks - 1 - warp) / WARPS + 1 : 0;
     unsigned long long* my_full = full[warp];
@@ -235,8 +217,8 @@ __global__ void __maxnreg__(120) experts_up_kernel(const Experts p, const __grid
                     const float lim = e == p.E ? p.limit_s : p.limit, gc = fminf(sum[i], lim), uc = fminf(fmaxf(sum[i + 2], -lim), lim);
                     y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : gc / (1.f + expf(-p.slope * gc)) * (uc + p.up_shift) * wt);
                 } else {
-                    y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i], p.kind) * wt);
-                    y[8] = __float2bfloat16_rn(wt == 0.f ? 0.f : activate(sum[i + 2], p.kind) * wt);
+                    y[0] = __float2bfloat16_rn(wt == 0.f ? 0.f : experts::activate(sum[i], p.kind) * wt);
+                    y[8] = __float2bfloat16_rn(wt == 0.f ? 0.f : experts::activate(sum[i + 2], p.kind) * wt);
                 }
             }
         }
@@ -403,7 +385,7 @@ LLM_EXPORT int llm_experts_few(const void* x, int ldx, const void* w_up, const v
     p.x = (const bf16*)x; p.w_up = (const bf16*)w_up; p.w_down = (const bf16*)w_down; p.act = (bf16*)act;
     p.ldx = ldx; p.M = M; p.K = K; p.N = N; p.E = E; p.ff = ff; p.fs = fs; p.kind = kind;
     p.limit = limit; p.limit_s = limit_s; p.slope = slope; p.up_shift = up_shift;
-    p.weights = weights; p.ldw = ldw; p.ids = ids; p.table = table; p.top = top; p.vocab = vocab;
+    p.weights = {weights, ldw, ids, table, top, vocab, E};
     p.out = out; p.resid = resid; p.norm_w = norm_w; p.xw_out = (bf16*)xw_out; p.ss_out = ss_out; p.alpha = alpha; p.error_flag = error_flag;
     const int sms = device_sms(), per = kind < 0 ? 2 : 1, C = E * ff + fs;
     const bool whole = K % 64 == 0;  // rows are whole pieces of 64 k: two of them in one box

@@ -20,6 +20,7 @@
 // warps 2-5 end the tile before meanwhile.
 // Every wait is bounded; one that gives up sets the error flag, and the roles run to their end.
 #include "common.cuh"
+#include "experts.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
 
@@ -36,10 +37,7 @@ struct Many {
     int T, K, N, E, ff, fs, cap;  // cap: rows of act and y (tokens x experts of a token)
     int kind;                     // -1 gated, else the activation
     float limit, limit_s, slope, up_shift;
-    const float* weights;  // [T, ldw], or null:
-    int ldw;
-    const int *ids, *table;
-    int listed, vocab;
+    experts::Weights weights;
     int *counts, *list, *place;  // [E], [E, T] tokens of an expert, [T, E] a token's row among its expert's
     bf16 *act, *act_s;           // [cap, ff], [T, fs]
     float *y, *y_s;              // [cap, N], [T, N]
@@ -47,23 +45,6 @@ struct Many {
     float alpha;
     int* error_flag;
 };
-
-__device__ __forceinline__ float weight_of(const Many& p, int t, int e) {
-    if (p.weights) return __ldcg(p.weights + (size_t)t * p.ldw + e);
-    if (e == p.E) return 1.f;
-    int id = p.ids[t];
-    if (id < 0 || id >= p.vocab) id = 0;
-    float w = 0.f;
-    for (int c = 0; c < p.listed; ++c) w = p.table[(size_t)id * p.listed + c] == e ? 1.f / (float)p.listed : w;
-    return w;
-}
-
-__device__ __forceinline__ float activate(float v, int kind) {
-    if (kind == 0) { const float r = fmaxf(v, 0.f); return r * r; }                                    // relu^2
-    if (kind == 1) return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));  // gelu (tanh)
-    if (kind == 3) return v / (1.f + expf(-v));                                                        // silu
-    return v;
-}
 
 __global__ void __launch_bounds__(1024) experts_sort_kernel(const Many p) {
     __shared__ int of_warp[32];
@@ -73,7 +54,7 @@ __global__ void __launch_bounds__(1024) experts_sort_kernel(const Many p) {
     int base = 0;
     for (int t0 = 0; t0 < p.T; t0 += blockDim.x) {
         const int t = t0 + threadIdx.x;
-        const bool uses = t < p.T && weight_of(p, t, e) != 0.f;
+        const bool uses = t < p.T && p.weights.of(t, e) != 0.f;
         const unsigned mask = __ballot_sync(0xffffffffu, uses);
         if (lane == 0) of_warp[warp] = __popc(mask);
         __syncthreads();
@@ -310,7 +291,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
                 meet_128();
                 for (int c = mine; c < NT; c += 128) {
                     const int token = c < t.valid ? (shared ? t.row + c : __ldcg(p.list + (size_t)e * p.T + t.row + c)) : -1;
-                    factor[c] = token >= 0 ? weight_of(p, token, shared ? p.E : e) : 0.f;
+                    factor[c] = token >= 0 ? p.weights.of(token, shared ? p.E : e) : 0.f;
                 }
             }
             const bool ok = !gave_up && tma::mbar_wait(&acc_full[buf], (i >> 1) & 1);
@@ -355,7 +336,7 @@ experts_product_kernel(const Many p, const __grid_constant__ CUtensorMap rows_ma
                     } else {
                         unsigned char* at = dst + (quarter * 32 + lane) * 2;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) *reinterpret_cast<bf16*>(at + j * PITCH) = __float2bfloat16_rn(activate(v[j], p.kind) * factor[c + j]);
+                        for (int j = 0; j < 32; ++j) *reinterpret_cast<bf16*>(at + j * PITCH) = __float2bfloat16_rn(experts::activate(v[j], p.kind) * factor[c + j]);
                     }
                     meet_128();
                     for (int q = mine; q < CHUNK * (STEP / 8); q += 128) {
@@ -385,7 +366,7 @@ __device__ __forceinline__ int rows_of_token(const Many& p, int t, int* rows) {
     for (int e0 = 0; e0 < p.E; e0 += 32) {
         const int e = e0 + lane;
         const int mine = e < p.E ? __ldcg(p.counts + e) : 0, sum = sum_up_to(mine, lane);
-        const bool uses = e < p.E && weight_of(p, t, e) != 0.f;
+        const bool uses = e < p.E && p.weights.of(t, e) != 0.f;
         const int at = uses ? __ldcg(p.place + (size_t)t * p.E + e) : 0;
         const unsigned mask = __ballot_sync(0xffffffffu, uses);
         if (uses) rows[n + __popc(mask & ((1u << lane) - 1))] = min(before + sum - mine + at, p.cap - 1);
@@ -508,7 +489,7 @@ LLM_EXPORT int llm_experts_many(const void* x, int ldx, const void* w_up, const 
     Many p = {};
     p.T = T; p.K = K; p.N = N; p.E = E; p.ff = ff; p.fs = fs; p.cap = cap; p.kind = kind;
     p.limit = limit; p.limit_s = limit_s; p.slope = slope; p.up_shift = up_shift;
-    p.weights = weights; p.ldw = ldw; p.ids = ids; p.table = table; p.listed = listed; p.vocab = vocab;
+    p.weights = {weights, ldw, ids, table, listed, vocab, E};
     p.counts = ints; p.list = ints + E; p.place = ints + E + (size_t)E * T;
     p.act = (bf16*)act; p.act_s = (bf16*)act_s; p.y = y; p.y_s = y_s; p.out = out; p.resid = resid; p.alpha = alpha; p.error_flag = error_flag;
 

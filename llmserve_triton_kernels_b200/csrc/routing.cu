@@ -3,6 +3,7 @@
 //
 // The router's scores, the choice and the weights are 32-bit.
 #include "common.cuh"
+#include "experts.cuh"
 
 #include <float.h>
 
@@ -378,13 +379,6 @@ router_few_kernel(const TX* __restrict__ x, int ldx, const float* __restrict__ w
     }
 }
 
-__device__ __forceinline__ float activate(float v, int kind) {
-    if (kind == 0) { const float r = fmaxf(v, 0.f); return r * r; }                                                // relu^2
-    if (kind == 1) return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));              // gelu (tanh)
-    if (kind == 3) return v / (1.f + expf(-v));                                                                    // silu
-    return v;
-}
-
 // y[t, j] = act(x[t, j]) * w[t, block(j)]: block(j) = j / ff for j < E * ff, and E for the columns behind them (a
 // shared expert's).  x, y: [N, C].  In two forms: 16 bytes a thread, where every run of 16 bytes lies within one expert's
 // block (ff a multiple of the run) and rows start on 16-byte boundaries; element by element elsewhere.
@@ -405,7 +399,7 @@ expert_act_scale_wide_kernel(const T* __restrict__ x, int ldx, const float* __re
         if (wt != 0.f) {
             raw = *reinterpret_cast<const uint4*>(x + (size_t)t * ldx + j);
 #pragma unroll
-            for (int e = 0; e < RUN; ++e) v[e] = from_float<T>(activate(to_float(v[e]), kind) * wt);
+            for (int e = 0; e < RUN; ++e) v[e] = from_float<T>(experts::activate(to_float(v[e]), kind) * wt);
         }
         *reinterpret_cast<uint4*>(y + (size_t)t * ldy + j) = raw;
     }
@@ -421,7 +415,7 @@ expert_act_scale_kernel(const T* __restrict__ x, int ldx, const float* __restric
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < C; j += gridDim.x * blockDim.x) {
         const int b = j < E * ff ? j / ff : E;
         const float wt = w[(size_t)t * ldw + b];
-        y[(size_t)t * ldy + j] = from_float<T>(wt == 0.f ? 0.f : activate(to_float(x[(size_t)t * ldx + j]), kind) * wt);
+        y[(size_t)t * ldy + j] = from_float<T>(wt == 0.f ? 0.f : experts::activate(to_float(x[(size_t)t * ldx + j]), kind) * wt);
     }
 }
 
