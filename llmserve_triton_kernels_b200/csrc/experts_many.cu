@@ -8,9 +8,9 @@
 //
 // What bounds it: the weights' bytes up to about 1,500 tokens (32 experts of 704 in 2,048: 294 MB a layer), beyond that the tensor cores; the
 // products over all experts with the token's weight as a factor, which ran before, did eight times the operations for 4 of 32 experts.
-// Measured (us a layer, all products over all experts -> these launches): 32 experts of 704, 4 used, a shared one of 1,408, 2,048 wide, 1,801
-// tokens 387 -> 187 (up 89 at 0.42 of the tensor peak, down 65, combine 19, gather 8, sort 6); 256 tokens 104 -> 96, 512 137 -> 106.  Rows
-// gathered by the product itself (TMA, four rows a box) took 375 at 1,800 tokens.
+// Measured (us a layer, launches back to back, weights from memory; products over all experts -> these launches): 32 experts of 704, 4 used, a
+// shared one of 1,408, 2,048 wide: 256 tokens 88 -> 78, 512 127 -> 89, 1,024 222 -> 121, 1,801 383 -> 183 (up 89 at 0.42 of the tensor peak, down
+// 67, combine 19, gather 8, sort 6).  Rows gathered by the product itself (TMA, four rows a box) were no faster than all experts.
 //
 // The products are tcgen05 with the WEIGHTS as the 128 rows of the tile and an expert's tokens as its columns: an expert has as many
 // tokens as it has, and N goes up to 64, 128 or 256 (the fewer, the deeper the ring) in steps of 16 where M is 128 whatever there is to do.  One persistent CTA an SM walks (group,

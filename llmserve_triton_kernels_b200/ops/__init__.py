@@ -1808,8 +1808,8 @@ _EXPERTS_MANY_WIDTH: int | None = None  # tests and measurements choose the most
 def _experts_many_tiles(tokens: int, experts: int, top: int, ff: int, shared_ff: int, gated: bool) -> tuple[int, float, float, int]:
     """``(the most tokens of a tile of experts_many, tiles of the busiest SM in the first product, tokens of an average tile, tiles of an
     expert's rows)``, the experts evenly used: the width (64, 128 or 256) whose busiest SM has the least to do, a tile costing as much as 80
-    tokens whatever it holds.  Measured (used experts, us with 64 / 128 / 256): 32 experts of 704, 4 used, a shared one of 1,408: 256 tokens 96 / 98 /
-    110, 512 120 / 106 / 118, 1,024 191 / 149 / 141, 1,800 317 / 243 / 212; 8 of 7,168, 2 used: 256 tokens 385 / 327 / 341."""
+    tokens whatever it holds.  Measured (used experts, us with 64 / 128 / 256, each layer behind a write of 256 MB): 32 experts of 704, 4 used, a shared one
+    of 1,408: 256 tokens 92 / 93 / 108, 512 125 / 109 / 121, 1,024 176 / 149 / 136, 1,801 281 / 199 / 190; 8 of 7,168, 2 used: 256 tokens 208 / 165 / 173."""
     used = experts * (1.0 - (1.0 - top / experts) ** tokens)
     rows = tokens * top / used
     step, best = (64 if gated else 128), None
@@ -1828,9 +1828,9 @@ def experts_many_pay(tokens: int, experts: int, top: int, ff: int, shared_ff: in
     to 130 steps on a B200 (13 mixtures of 4 to 256 experts, inner sizes 64 to 7,168, 256 to 4,096 wide, 9 to 4,096 tokens): a fixed part and
     the root of the squares of the weights' bytes at the copy rate and of the operations (all experts: at 1.31 PFLOP/s; the used ones: by the
     busiest SM's tiles), for the used ones also the rows that travel between the kernels.  The choice takes no step of that sweep more than 1 %
-    slower than the faster way; under 128 tokens the two are within a few per cent wherever the used ones are faster at all.  All -> used (us): 32
-    experts of 704, 4 used, a shared one of 1,408: 256 tokens 104 -> 96, 512 137 -> 106, 1,800 404 -> 212; 8 of 1,408, 2 used: 512 90 -> 89, 1,800
-    194 -> 140; 16 of 704, 8 used: 1,800 232 -> 284."""
+    slower than the faster way; under 128 tokens the two are within a few per cent wherever the used ones are faster at all.  All -> used (us, each
+    layer behind a write of 256 MB): 32 experts of 704, 4 used, a shared one of 1,408: 256 tokens 102 -> 94, 512 136 -> 111, 1,801 372 -> 190; 8 of 1,408,
+    2 used: 512 80 -> 81, 1,801 179 -> 127; 16 of 704, 8 used: 1,801 187 -> 231."""
     if tokens < _EXPERTS_MANY_MIN or top >= experts:
         return False
     width, each, n, of_expert = _experts_many_tiles(tokens, experts, top, ff, shared_ff, gated)
