@@ -142,3 +142,24 @@ def test_scales_that_are_not_positive_go_the_old_way(scale):
         s = torch.einsum("ihd,jhd->hij", torch.cat((q[a:b].view(-1, 2, 64), q_rot[a:b]), -1).float(), k) * scale
         s = s.masked_fill(torch.ones_like(s[0], dtype=torch.bool).triu(1), -torch.inf)
         close(got[a:b], torch.einsum("hij,jhd->ihd", s.softmax(-1), kv[a:b, 128:].view(-1, 2, 64).float()), 1e-2, f"tokens {a} to {b}")
+
+
+@pytest.mark.parametrize("H,KV,D,general,plain", [(4, 2, 64, 32, 32), (16, 4, 64, 48, 64), (16, 4, 128, 32, 32)])
+def test_a_crowd_of_small_requests_beside_a_long_one(H, KV, D, general, plain, monkeypatch):
+    """Forty requests on both sides of every threshold: which of them go along, and everybody's rows."""
+    ops = _ops()
+    torch.manual_seed(H + D)
+    news = [200, *(31 + i % 40 for i in range(39))]
+    ctx, table, _, pages = paged_batch([n + 13 * (i % 7) for i, n in enumerate(news)], news, 16)
+    pool = torch.randn(pages, 2, KV, 16, D, device=DEV).bfloat16()
+    qkv = torch.randn(ctx.num_tokens, (H + 2 * KV) * D, device=DEV).bfloat16()
+    q = qkv[:, : H * D]
+    common = dict(num_heads=H, num_kv_heads=KV, key_dim=D, value_dim=D, scale=0.2)
+    taken, kernel = [], ops._tcgen05_softmax_attention
+    monkeypatch.setattr(ops, "_tcgen05_softmax_attention", lambda *a, **k: taken.append(kernel(*a, **k)) or taken[-1])
+    for more in ({}, dict(sinks=torch.randn(H, device=DEV)), dict(slopes=torch.rand(H, device=DEV) * 0.1)):
+        close(ops.paged_softmax_attention(q, pool, table, ctx, **common, **more), plain_ops.paged_softmax_attention(q, pool, table, ctx, **common, **more), 2e-2, str(more))
+    assert taken == [(general, True)] * 3
+    assert ops._tc_join_tokens(ctx, H, D, D, ops._TC_ATTENTION_JOIN_CROWDED) == plain
+    got = ops.paged_attention(qkv, pool, table, ctx, num_heads=H, num_kv_heads=KV, head_dim=D, scale=0.2)
+    close(got, plain_ops.paged_softmax_attention(q, pool, table, ctx, **common), 2e-2, "the plain form")
